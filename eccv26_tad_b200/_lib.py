@@ -1,10 +1,13 @@
-"""ctypes binding of ``libsvtad.so`` (declared in ``include/svtad.h``).
+"""ctypes binding of ``libsvtad.so`` (declared in ``include/svtad.h``), and the extension ``_native`` over it.
 
 The library is the only implementation behind this package: if it is missing, importing this
 module raises - there is no eager / CPU fallback.
 """
 import ctypes
+import importlib.util
 import os
+
+import torch  # noqa: F401  (its libraries must be loaded before the extension that links to them)
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libsvtad.so")
@@ -31,6 +34,7 @@ SIGNATURES = {
     "svtad_conv_dgrad": (c_int, [c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_p, c_p, c_sz, c_p]),
     "svtad_conv_wgrad": (c_int, [c_p, c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_p, c_sz, c_p]),
     "svtad_conv_bwd": (c_int, [c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_p, c_p, c_sz, c_p]),
+    "svtad_conv_bwd_typed": (c_int, [c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_int, c_p, c_p, c_sz, c_p]),
     "svtad_static_workspace_bytes": (c_sz, []),
     "svtad_conv_wgrad_static": (c_int, [c_p, c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_p]),
     "svtad_allreduce_stage_bytes": (c_sz, [c_i64]),
@@ -62,6 +66,25 @@ def load():
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+class _Native:
+    """The extension behind the module and the table functions (csrc/native.cpp), linked to libsvtad.so beside it;
+    loaded at the first use, as the library is.  Its functions become plain attributes of this object."""
+
+    def __getattr__(self, name):
+        path = os.path.join(_PKG, "_native.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is missing: build it with `python -m eccv26_tad_b200.build`")
+        load()
+        spec = importlib.util.spec_from_file_location(__package__ + "._native", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        self.__dict__.update({k: v for k, v in vars(mod).items() if not k.startswith("__")})
+        return self.__dict__[name]
+
+
+native = _Native()
 
 
 def last_error():

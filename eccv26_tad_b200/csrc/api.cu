@@ -159,16 +159,16 @@ extern "C" int svtad_conv_dgrad(const void* gy, const int32_t* nbr, const void* 
     return rc;
 }
 
-extern "C" int svtad_conv_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb,
-                                int64_t n, int cin, int cout, int kk, int tokens_per_batch,
-                                int dtype, void* workspace, size_t workspace_bytes, void* stream) {
+static int conv_wgrad_typed(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin,
+                            int cout, int kk, int tokens_per_batch, int dtype, int grad_dtype, void* workspace,
+                            size_t workspace_bytes, void* stream) {
     int rc = check_common("svtad_conv_wgrad", n, cin, cout, kk, tokens_per_batch, dtype);
     if (rc) return rc;
     SV_CHECK_ARG(gw != nullptr, "svtad_conv_wgrad: gw is null");
     cudaStream_t s = (cudaStream_t)stream;
     if (n == 0) {
-        SV_CUDA(cudaMemsetAsync(gw, 0, (size_t)kk * cin * cout * dtype_size(dtype), s));
-        if (gb) SV_CUDA(cudaMemsetAsync(gb, 0, (size_t)cout * dtype_size(dtype), s));
+        SV_CUDA(cudaMemsetAsync(gw, 0, (size_t)kk * cin * cout * dtype_size(grad_dtype), s));
+        if (gb) SV_CUDA(cudaMemsetAsync(gb, 0, (size_t)cout * dtype_size(grad_dtype), s));
         return SVTAD_OK;
     }
     SV_CHECK_ARG(gy && x && nbr, "svtad_conv_wgrad: null pointer");
@@ -176,23 +176,40 @@ extern "C" int svtad_conv_wgrad(const void* gy, const void* x, const int32_t* nb
                  "svtad_conv_wgrad: gy, x, nbr, gw and gb must be 16-byte aligned");
     SV_CHECK_ARG(workspace != nullptr && aligned(workspace, 256), "svtad_conv_wgrad: workspace is null or not 256-byte aligned");
     if (use_tc(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype))
-        return tc_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, workspace, workspace_bytes, s);
+        return tc_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace, workspace_bytes, s);
     if (forced_path() == 2)
         return set_error(SVTAD_ERR_UNSUPPORTED, "svtad_conv_wgrad: tensor-core path forced but shape/dtype unsupported");
-    return simt_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, workspace, workspace_bytes, s);
+    return simt_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace, workspace_bytes, s);
+}
+
+extern "C" int svtad_conv_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb,
+                                int64_t n, int cin, int cout, int kk, int tokens_per_batch,
+                                int dtype, void* workspace, size_t workspace_bytes, void* stream) {
+    return conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, dtype, workspace,
+                            workspace_bytes, stream);
 }
 
 extern "C" int svtad_conv_bwd(const void* gy, const void* x, const int32_t* nbr, const void* w, void* gx,
                               void* gw, void* gb, int64_t n, int cin, int cout, int kk,
                               int tokens_per_batch, int dtype, const int32_t* table_status,
                               void* workspace, size_t workspace_bytes, void* stream) {
+    return svtad_conv_bwd_typed(gy, x, nbr, w, gx, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, dtype,
+                                table_status, workspace, workspace_bytes, stream);
+}
+
+extern "C" int svtad_conv_bwd_typed(const void* gy, const void* x, const int32_t* nbr, const void* w, void* gx,
+                                    void* gw, void* gb, int64_t n, int cin, int cout, int kk,
+                                    int tokens_per_batch, int dtype, int grad_dtype, const int32_t* table_status,
+                                    void* workspace, size_t workspace_bytes, void* stream) {
+    SV_CHECK_ARG(grad_dtype == dtype || grad_dtype == SVTAD_F32,
+                 "svtad_conv_bwd: weight gradients come in the features' type or in float32, not in type %d", grad_dtype);
     SV_CHECK_ARG(gx != nullptr || gw != nullptr, "svtad_conv_bwd: neither gx nor gw requested");
     SV_CHECK_ARG(gb == nullptr || gw != nullptr, "svtad_conv_bwd: gb needs gw");
     if (gw == nullptr)
         return svtad_conv_dgrad(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, table_status,
                                 workspace, workspace_bytes, stream);
     if (gx == nullptr)
-        return svtad_conv_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, workspace,
+        return conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace,
                                 workspace_bytes, stream);
     // workspace = [weight-gradient part | input-gradient part (scatter form, only with a status word)]
     const size_t w_part = align_up(svtad_workspace_bytes(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype), 256);
@@ -205,7 +222,8 @@ extern "C" int svtad_conv_bwd(const void* gy, const void* x, const int32_t* nbr,
     int dev = 0;
     SV_CUDA(cudaGetDevice(&dev));
     if (!overlap_backward() || n == 0 || dev >= MAX_DEVICES) {
-        int rc = svtad_conv_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, workspace, w_part, s);
+        int rc = conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace,
+                                  w_part, s);
         if (rc) return rc;
         return svtad_conv_dgrad(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, table_status, ws_d, d_part, s);
     }
@@ -222,8 +240,8 @@ extern "C" int svtad_conv_bwd(const void* gy, const void* x, const int32_t* nbr,
     // fork: the side stream starts where the caller's stream stands
     SV_CUDA(cudaEventRecord(lane.fork, s));
     SV_CUDA(cudaStreamWaitEvent(lane.stream, lane.fork, 0));
-    int rc_w = svtad_conv_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, workspace, w_part,
-                                lane.stream);
+    int rc_w = conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace,
+                                w_part, lane.stream);
     int rc_d = svtad_conv_dgrad(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, table_status, ws_d,
                                 d_part, s);
     // join, also after an error: whatever was launched on the side stream is ordered before the caller's next work

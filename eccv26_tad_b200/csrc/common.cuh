@@ -53,14 +53,14 @@ int simt_fwd_f32(const ConvArgs& p, cudaStream_t s);
 int simt_dgrad_gather(const ConvArgs& p, const int32_t* status, cudaStream_t s);
 int simt_dgrad_scatter(const ConvArgs& p, const int32_t* status, float* ws, cudaStream_t s);
 int simt_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n,
-               int cin, int cout, int kk, int tpb, int dtype, void* ws, size_t ws_bytes,
+               int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes,
                cudaStream_t s);
 size_t simt_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk);
 // shared pieces of the weight-gradient path (also used by the tensor-core path)
 int bias_partial_launch(const void* gy, float* partial, int64_t n, int cout, int dtype, int splits,
                         cudaStream_t s);
 int wgrad_finalize_launch(const float* ws_w, int splits_w, const float* ws_b, int splits_b,
-                          void* gw, void* gb, int64_t n_w, int cout, int dtype, cudaStream_t s);
+                          void* gw, void* gb, int64_t n_w, int cout, int dtype, int grad_dtype, cudaStream_t s);
 int bias_splits_for(int64_t n);
 
 // tcgen05 kernels (conv_tc.cu)
@@ -68,7 +68,7 @@ bool tc_supported(int op, int64_t n, int cin, int cout, int kk, int dtype);
 int tc_fwd(const ConvArgs& p, cudaStream_t s);
 int tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s);
 int tc_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n,
-             int cin, int cout, int kk, int tpb, int dtype, void* ws, size_t ws_bytes,
+             int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes,
              cudaStream_t s);
 size_t tc_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk);
 int tc_read_error(int32_t* code_out);
@@ -81,7 +81,8 @@ int tc_set_share_floor(int n);
     int prefix##_fwd(const ConvArgs& p, cudaStream_t s);                                                    \
     int prefix##_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s);                           \
     int prefix##_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n,    \
-                       int cin, int cout, int kk, int tpb, int dtype, void* ws, size_t ws_bytes,            \
+                       int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws,             \
+                       size_t ws_bytes,                                                                     \
                        cudaStream_t s);
 SV_DECLARE_TC_FAMILY(hybrid)
 // forward / dgrad on CTA pairs (conv_tc_pair.cu)
@@ -100,6 +101,7 @@ template <> struct Cvt<float> {
         *reinterpret_cast<float4*>(p) = v;
     }
     static __device__ __forceinline__ void store1(float* p, float v) { *p = v; }
+    static __device__ __forceinline__ float value(float v) { return v; }
 };
 template <> struct Cvt<__nv_bfloat16> {
     static __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
@@ -125,6 +127,7 @@ template <> struct Cvt<__nv_bfloat16> {
     static __device__ __forceinline__ void store1(__nv_bfloat16* p, float v) {
         *p = __float2bfloat16_rn(v);
     }
+    static __device__ __forceinline__ float value(__nv_bfloat16 v) { return __bfloat162float(v); }
 };
 template <> struct Cvt<__half> {
     static __device__ __forceinline__ float4 load4(const __half* p) {
@@ -144,6 +147,7 @@ template <> struct Cvt<__half> {
         *reinterpret_cast<uint2*>(p) = r;
     }
     static __device__ __forceinline__ void store1(__half* p, float v) { *p = __float2half_rn(v); }
+    static __device__ __forceinline__ float value(__half v) { return __half2float(v); }
 };
 #endif  // __CUDACC__
 

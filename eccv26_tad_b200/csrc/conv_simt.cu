@@ -376,21 +376,27 @@ bias_partial_kernel(const T* __restrict__ gy, float* __restrict__ partial, long 
     }
 }
 
-// fixed-order reduction of the per-split partials, one rounding to T
-template <typename T>
+// fixed-order reduction of the per-split partials, one rounding to T, written as U (T, or fp32 for the gradient of an
+// fp32 master parameter)
+template <typename T, typename U>
 __global__ void wgrad_finalize_kernel(const float* __restrict__ ws_w, int splits_w,
                                       const float* __restrict__ ws_b, int splits_b,
-                                      T* __restrict__ gw, T* __restrict__ gb, long n_w, int cout) {
+                                      U* __restrict__ gw, U* __restrict__ gb, long n_w, int cout) {
+    auto put = [](U* p, float v) {
+        T t;
+        Cvt<T>::store1(&t, v);
+        Cvt<U>::store1(p, Cvt<T>::value(t));
+    };
     long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (e < n_w) {
         float sum = 0.f;
         for (int s = 0; s < splits_w; ++s) sum += ws_w[(long)s * n_w + e];
-        Cvt<T>::store1(gw + e, sum);
+        put(gw + e, sum);
     } else if (gb != nullptr && e < n_w + cout) {
         int co = (int)(e - n_w);
         float sum = 0.f;
         for (int s = 0; s < splits_b; ++s) sum += ws_b[(long)s * cout + co];
-        Cvt<T>::store1(gb + co, sum);
+        put(gb + co, sum);
     }
 }
 
@@ -413,13 +419,23 @@ int bias_partial_launch(const void* gy, float* partial, int64_t n, int cout, int
 }
 
 int wgrad_finalize_launch(const float* ws_w, int splits_w, const float* ws_b, int splits_b, void* gw,
-                          void* gb, int64_t n_w, int cout, int dtype, cudaStream_t s) {
+                          void* gb, int64_t n_w, int cout, int dtype, int grad_dtype, cudaStream_t s) {
     long total = n_w + (gb ? cout : 0);
     unsigned grid = (unsigned)((total + 255) / 256);
+    auto go = [&](auto kern, auto* as) {
+        kern<<<grid, 256, 0, s>>>(ws_w, splits_w, ws_b, splits_b, static_cast<decltype(as)>(gw), static_cast<decltype(as)>(gb), (long)n_w, cout);
+    };
+    const bool out32 = grad_dtype == SVTAD_F32;
     switch (dtype) {
-        case SVTAD_F32: wgrad_finalize_kernel<float><<<grid, 256, 0, s>>>(ws_w, splits_w, ws_b, splits_b, (float*)gw, (float*)gb, (long)n_w, cout); break;
-        case SVTAD_BF16: wgrad_finalize_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(ws_w, splits_w, ws_b, splits_b, (__nv_bfloat16*)gw, (__nv_bfloat16*)gb, (long)n_w, cout); break;
-        default: wgrad_finalize_kernel<__half><<<grid, 256, 0, s>>>(ws_w, splits_w, ws_b, splits_b, (__half*)gw, (__half*)gb, (long)n_w, cout); break;
+        case SVTAD_F32: go(wgrad_finalize_kernel<float, float>, (float*)nullptr); break;
+        case SVTAD_BF16:
+            if (out32) go(wgrad_finalize_kernel<__nv_bfloat16, float>, (float*)nullptr);
+            else go(wgrad_finalize_kernel<__nv_bfloat16, __nv_bfloat16>, (__nv_bfloat16*)nullptr);
+            break;
+        default:
+            if (out32) go(wgrad_finalize_kernel<__half, float>, (float*)nullptr);
+            else go(wgrad_finalize_kernel<__half, __half>, (__half*)nullptr);
+            break;
     }
     SV_LAUNCH_CHECK("wgrad_finalize_kernel");
     return SVTAD_OK;
@@ -442,7 +458,7 @@ size_t simt_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk) {
 }
 
 int simt_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n,
-               int cin, int cout, int kk, int tpb, int dtype, void* ws, size_t ws_bytes,
+               int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes,
                cudaStream_t s) {
     if (ws_bytes < simt_wgrad_ws_bytes(n, cin, cout, kk))
         return set_error(SVTAD_ERR_WORKSPACE, "svtad_conv_wgrad: workspace %zu < %zu bytes", ws_bytes,
@@ -467,7 +483,7 @@ int simt_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void
         int rc = bias_partial_launch(gy, ws_b, n, cout, dtype, splits_b, s);
         if (rc) return rc;
     }
-    return wgrad_finalize_launch(ws_w, splits, ws_b, splits_b, gw, gb, n_w, cout, dtype, s);
+    return wgrad_finalize_launch(ws_w, splits, ws_b, splits_b, gw, gb, n_w, cout, dtype, grad_dtype, s);
 }
 
 }  // namespace svtad

@@ -246,7 +246,35 @@ static WgradPlan wgrad_plan_for(int64_t n, int cin, int cout, int kk, long sms) 
     return best;
 }
 
-WgradPlan tc_wgrad_plan(int64_t n, int cin, int cout, int kk) { return wgrad_plan_for(n, cin, cout, kk, tc_plan_sms()); }
+// The search above costs the host 1-20 us; the last few answers are kept per thread (a training step asks for the same
+// few problems again and again).  `sms` = 0 stands for the workspace size that covers every hint.
+struct PlanMemo {
+    int64_t n = -1;
+    int cin, cout, kk;
+    long sms;
+    WgradPlan plan;
+    size_t bytes;
+};
+static PlanMemo& plan_slot(int64_t n, int cin, int cout, int kk, long sms) {
+    constexpr unsigned SLOTS = 64;
+    static thread_local PlanMemo memo[SLOTS];
+    const uint64_t h = ((uint64_t)n * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)cin << 40) ^ ((uint64_t)cout << 20) ^ (uint64_t)(kk * 256 + sms);
+    return memo[(h ^ (h >> 29) ^ (h >> 47)) % SLOTS];
+}
+static bool plan_known(const PlanMemo& m, int64_t n, int cin, int cout, int kk, long sms) {
+    return m.n == n && m.cin == cin && m.cout == cout && m.kk == kk && m.sms == sms && getenv("SVTAD_TC_WGRAD_BN") == nullptr &&
+           getenv("SVTAD_TC_WGRAD_SPLITS") == nullptr;
+}
+
+WgradPlan tc_wgrad_plan(int64_t n, int cin, int cout, int kk) {
+    const long sms = tc_plan_sms();
+    PlanMemo& m = plan_slot(n, cin, cout, kk, sms);
+    if (plan_known(m, n, cin, cout, kk, sms)) return m.plan;
+    const WgradPlan pl = wgrad_plan_for(n, cin, cout, kk, sms);
+    if (getenv("SVTAD_TC_WGRAD_BN") == nullptr && getenv("SVTAD_TC_WGRAD_SPLITS") == nullptr)
+        m = PlanMemo{n, cin, cout, kk, sms, pl, 0};
+    return pl;
+}
 
 static size_t plan_bytes(const WgradPlan& pl, int64_t n, int cin, int cout, int kk) {
     size_t w = (size_t)pl.splits * kk * cin * cout * sizeof(float);
@@ -264,6 +292,8 @@ size_t tc_wgrad_plan_ws_bytes(int64_t n, int cin, int cout, int kk) {
 // sized once stays valid when the hint changes (a leaner plan usually has fewer token splits, but the waves'
 // rounding can go the other way: 18 880 rows at C=192, 5x5 takes 3 splits planned for 148 SMs and 5 for 74).
 size_t tc_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk) {
+    PlanMemo& m = plan_slot(n, cin, cout, kk, 0);
+    if (plan_known(m, n, cin, cout, kk, 0)) return m.bytes;
     size_t need = 0;
     const int sms = tc_num_sms();
     for (int share = 1; share <= 16; ++share) {
@@ -272,23 +302,28 @@ size_t tc_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk) {
         const size_t b = plan_bytes(wgrad_plan_for(n, cin, cout, kk, v), n, cin, cout, kk);
         if (b > need) need = b;
     }
+    if (getenv("SVTAD_TC_WGRAD_BN") == nullptr && getenv("SVTAD_TC_WGRAD_SPLITS") == nullptr)
+        m = PlanMemo{n, cin, cout, kk, 0, WgradPlan{}, need};
     return need;
 }
 
 
-// fixed-order reduction of the per-split partials (4 elements per thread), one rounding
+// fixed-order reduction of the per-split partials (4 elements per thread), one rounding; OUT32: the rounded values are
+// written as fp32 (the gradient of an fp32 master parameter), which saves a pass over the gradient
+template <bool OUT32>
 __global__ void __launch_bounds__(256)
 wgrad_reduce4_kernel(const float* __restrict__ ws_w, int splits, const float* __restrict__ ws_b, int splits_b,
-                     uint16_t* __restrict__ gw, uint16_t* __restrict__ gb, long n_w, int cout, int fp16) {
+                     void* __restrict__ gw, void* __restrict__ gb, long n_w, int cout, int fp16) {
     long e = (blockIdx.x * (long)blockDim.x + threadIdx.x) * 4;
     const float* src;
-    uint16_t* dst;
+    void* base;
+    long at;
     long stride;
     int cnt;
     if (e < n_w) {
-        src = ws_w + e; dst = gw + e; stride = n_w; cnt = splits;
+        src = ws_w + e; base = gw; at = e; stride = n_w; cnt = splits;
     } else if (gb != nullptr && e - n_w < cout) {
-        src = ws_b + (e - n_w); dst = gb + (e - n_w); stride = cout; cnt = splits_b;
+        src = ws_b + (e - n_w); base = gb; at = e - n_w; stride = cout; cnt = splits_b;
     } else {
         return;
     }
@@ -301,15 +336,21 @@ wgrad_reduce4_kernel(const float* __restrict__ ws_w, int splits, const float* __
     uint2 o;
     o.x = pack2(acc.x, acc.y, fp16 != 0);
     o.y = pack2(acc.z, acc.w, fp16 != 0);
-    *reinterpret_cast<uint2*>(dst) = o;
+    if (OUT32) {
+        auto wide = [&](uint32_t v) { return widen(static_cast<uint16_t>(v & 0xffffu), fp16 != 0); };
+        *reinterpret_cast<float4*>(static_cast<float*>(base) + at) = make_float4(wide(o.x), wide(o.x >> 16), wide(o.y), wide(o.y >> 16));
+    } else {
+        *reinterpret_cast<uint2*>(static_cast<uint16_t*>(base) + at) = o;
+    }
 }
 
 
 int tc_wgrad_reduce_launch(const float* ws_w, int splits, const float* ws_b, int splits_b, void* gw, void* gb,
-                           long n_w, int cout, int fp16, cudaStream_t s) {
+                           long n_w, int cout, int fp16, bool out32, cudaStream_t s) {
     long total4 = (n_w + (gb ? cout : 0) + 3) / 4;
-    SV_CUDA(tc_launch(wgrad_reduce4_kernel, dim3((unsigned)((total4 + 255) / 256)), dim3(256), 0, s, ws_w, splits, ws_b,
-                      splits_b, (uint16_t*)gw, (uint16_t*)gb, n_w, cout, fp16));
+    SV_CUDA(tc_launch(out32 ? wgrad_reduce4_kernel<true> : wgrad_reduce4_kernel<false>,
+                      dim3((unsigned)((total4 + 255) / 256)), dim3(256), 0, s, ws_w, splits, ws_b, splits_b, gw, gb, n_w,
+                      cout, fp16));
     return SVTAD_OK;
 }
 
@@ -343,8 +384,8 @@ int tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
 }
 
 int tc_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin, int cout,
-             int kk, int tpb, int dtype, void* ws, size_t ws_bytes, cudaStream_t s) {
-    return hybrid_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tpb, dtype, ws, ws_bytes, s);
+             int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes, cudaStream_t s) {
+    return hybrid_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tpb, dtype, grad_dtype, ws, ws_bytes, s);
 }
 
 }  // namespace svtad

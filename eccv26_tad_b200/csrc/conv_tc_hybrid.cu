@@ -634,7 +634,7 @@ static int launch_wgrad_hybrid(const void* gy, const void* x, const int32_t* nbr
 }
 
 int hybrid_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin, int cout,
-                 int kk, int tpb, int dtype, void* ws, size_t ws_bytes, cudaStream_t s) {
+                 int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes, cudaStream_t s) {
     size_t need = tc_wgrad_plan_ws_bytes(n, cin, cout, kk);
     if (ws_bytes < need)
         return set_error(SVTAD_ERR_WORKSPACE, "svtad_conv_wgrad: workspace %zu < %zu bytes", ws_bytes, need);
@@ -664,7 +664,7 @@ int hybrid_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, vo
             if (rc) return rc;
         }
     }
-    return tc_wgrad_reduce_launch(ws_w, pl.splits, ws_b, splits_b, gw, gb, n_w, cout, fp16, s);
+    return tc_wgrad_reduce_launch(ws_w, pl.splits, ws_b, splits_b, gw, gb, n_w, cout, fp16, grad_dtype == SVTAD_F32, s);
 }
 
 }  // namespace svtad

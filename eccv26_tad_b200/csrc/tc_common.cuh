@@ -293,6 +293,6 @@ size_t tc_wgrad_plan_ws_bytes(int64_t n, int cin, int cout, int kk);
 
 // fixed-order reduction of per-split fp32 partials into the 16-bit gradient tensors
 int tc_wgrad_reduce_launch(const float* ws_w, int splits, const float* ws_b, int splits_b, void* gw, void* gb,
-                           long n_w, int cout, int fp16, cudaStream_t s);
+                           long n_w, int cout, int fp16, bool out32, cudaStream_t s);
 
 }  // namespace svtad

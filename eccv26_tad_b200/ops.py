@@ -5,9 +5,9 @@ torch's caching allocator (so they are ordered on the current stream), picking t
 stream and device, and translating status codes to exceptions.
 """
 import torch
-from torch.utils.weak import WeakIdKeyDictionary
 
 from . import _lib
+from ._lib import native as _native
 
 _DTYPES = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}
 
@@ -97,97 +97,48 @@ def _workspace(op, n, cin, cout, kk, code, device):
 
 # ----------------------------------------------------------------------------- table
 # Tables this module built itself are symmetric by construction (entry (i, k) = j  <=>  entry (j, KK-1-k) = i):
-# a full grid, a top-k subset of one, or a subset of a symmetric table.  They are remembered here (by tensor
-# object and version, weakly) so that the backward can use the gather form of the input gradient without the
+# a full grid, a top-k subset of one, or a subset of a symmetric table.  They are remembered by the extension (by
+# tensor object and version, weakly) so that the backward can use the gather form of the input gradient without the
 # device-side validation pass and without the scatter-form fallback launches.
-_symmetric = WeakIdKeyDictionary()
-
-
 def mark_symmetric(table):
     """Declare ``table`` symmetric (valid until the tensor is written to)."""
-    _symmetric[table] = table._version
+    _native.mark_symmetric(table)
     return table
 
 
 def is_known_symmetric(table):
     """True for tables built by this module (or marked by the caller) and views of them, unmodified since."""
-    for t in (table, getattr(table, "_base", None)):
-        if t is not None and _symmetric.get(t) == t._version:
-            return True
-    return False
+    return _native.is_known_symmetric(table)
 
 
 def table_init(B, T, h, w, ksize=3, device="cuda"):
-    out = torch.empty((B, T * h * w, ksize * ksize), dtype=torch.int32, device=device)
-    with _on(out.device):
-        _lib.check(_lib.load().svtad_table_init(B, T, h, w, ksize, _ptr(out), _stream()))
-    return mark_symmetric(out)
+    if device.__class__ is not torch.device:
+        device = torch.device(device)
+    if device.type != "cuda":
+        raise ValueError("SparseConv2D tensors must live on a CUDA device (there is no CPU path)")
+    index = device.index
+    return _native.table_init(B, T, h, w, ksize, torch.cuda.current_device() if index is None else index)
 
 
 def table_build(scores, k_keep, h, w, ksize=3):
     """scores float32 [n_seg, seg_len] -> (kept_idx int32 [n_seg, k], table int32 [n_seg*k, ksize^2])."""
-    _require_cuda(scores)
-    if scores.dtype != torch.float32:
-        scores = scores.float()
-    scores = scores.contiguous()
-    n_seg, seg_len = scores.shape
-    kept = torch.empty((n_seg, k_keep), dtype=torch.int32, device=scores.device)
-    table = torch.empty((n_seg * k_keep, ksize * ksize), dtype=torch.int32, device=scores.device)
-    with _on(scores.device):
-        _lib.check(_lib.load().svtad_table_build(_ptr(scores), n_seg, seg_len, k_keep, h, w, ksize,
-                                                 _ptr(kept), _ptr(table), _stream()))
-    return kept, mark_symmetric(table)
+    return _native.table_build(scores, k_keep, h, w, ksize)
 
 
 def topk_select(scores, k_keep):
     """scores float32 [B, L] -> idx int64 [B, k], ascending (torch.topk + sort with a fixed tie rule)."""
-    _require_cuda(scores)
-    if scores.dtype != torch.float32:
-        scores = scores.float()
-    scores = scores.contiguous()
-    B, L = scores.shape
-    idx = torch.empty((B, k_keep), dtype=torch.int64, device=scores.device)
-    with _on(scores.device):
-        _lib.check(_lib.load().svtad_topk_select(_ptr(scores), B, L, k_keep, _ptr(idx), _stream()))
-    return idx
+    return _native.topk_select(scores, k_keep)
 
 
 def table_remap(table, idx, scratch=None):
     """table int32 [B, N_prev, KK], idx int64 [B, N_new] -> int32 [B, N_new, KK]."""
-    _require_cuda(table, idx)
-    sym = is_known_symmetric(table)
-    table = _i32_table(table)
-    idx = idx.to(torch.int64).contiguous()
-    B, n_prev, kk = table.shape
-    n_new = idx.shape[1]
-    if scratch is None or scratch.numel() < B * n_prev:
-        scratch = torch.empty(B * n_prev, dtype=torch.int32, device=table.device)
-    out = torch.empty((B, n_new, kk), dtype=torch.int32, device=table.device)
-    with _on(table.device):
-        _lib.check(_lib.load().svtad_table_remap(_ptr(table), _ptr(idx), B, n_prev, n_new, kk,
-                                                 _ptr(scratch), _ptr(out), _stream()))
-    return mark_symmetric(out) if sym else out
+    return _native.table_remap(table, idx, scratch)
 
 
 def table_select_remap(scores, table, k_keep):
     """One later pruning round in one kernel: scores float32 [B, N_prev], table int32 [B, N_prev, KK] ->
     (idx int64 [B, k], table int32 [B, k, KK])."""
-    _require_cuda(scores, table)
-    if scores.dtype != torch.float32:
-        scores = scores.float()
-    scores = scores.contiguous()
-    sym = is_known_symmetric(table)
-    table = _i32_table(table)
-    B, n_prev, kk = table.shape
-    if tuple(scores.shape) != (B, n_prev):
-        raise ValueError(f"table_select_remap: scores {tuple(scores.shape)} do not match the table's {(B, n_prev)}")
-    kept = torch.empty((B, k_keep), dtype=torch.int32, device=table.device)
-    idx = torch.empty((B, k_keep), dtype=torch.int64, device=table.device)
-    out = torch.empty((B, k_keep, kk), dtype=torch.int32, device=table.device)
-    with _on(table.device):
-        _lib.check(_lib.load().svtad_table_select_remap(_ptr(scores), _ptr(table), B, n_prev, k_keep, kk, _ptr(kept),
-                                                        _ptr(idx), _ptr(out), _stream()))
-    return idx, (mark_symmetric(out) if sym else out)
+    return _native.table_select_remap(scores, table, k_keep)
 
 
 def table_check(nbr, tokens_per_batch=0, status=None):

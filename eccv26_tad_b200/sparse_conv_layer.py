@@ -25,9 +25,9 @@ import math
 import torch
 import torch.nn as nn
 from torch.autograd import Function
-from torch.utils.weak import WeakIdKeyDictionary
 
 from . import ops
+from ._lib import native as _native
 
 try:  # torch >= 2.4
     from torch.amp import custom_bwd as _custom_bwd, custom_fwd as _custom_fwd
@@ -39,44 +39,6 @@ try:  # torch >= 2.4
         return _custom_bwd(fn, device_type="cuda")
 except ImportError:  # pragma: no cover
     from torch.cuda.amp import custom_bwd, custom_fwd
-
-
-class _PerTableCache:
-    """Facts about a table tensor, valid while the tensor object lives and is not written to."""
-
-    def __init__(self):
-        self._d = WeakIdKeyDictionary()
-
-    def get(self, t, key, make):
-        ent = self._d.get(t)
-        if ent is None or ent[0] != t._version:
-            ent = (t._version, {})
-            self._d[t] = ent
-        if key not in ent[1]:
-            ent[1][key] = make()
-        return ent[1][key]
-
-
-_table_cache = _PerTableCache()
-
-
-_SYMMETRIC = "symmetric by construction"
-
-
-def _status_for(nbr, tokens_per_batch):
-    """What the backward needs to know about a table: ``_SYMMETRIC`` for tables built by this package (no
-    validation pass, no scatter-form fallback), else the device status word of ``svtad_table_check``."""
-    if tokens_per_batch == 0 and ops.is_known_symmetric(nbr):
-        return _SYMMETRIC
-    return _table_cache.get(nbr, ("status", tokens_per_batch), lambda: ops.table_check(nbr, tokens_per_batch))
-
-
-def _bwd(grad_output, x, nbr, weight, tpb, status, need_x, need_w, need_b):
-    if status is _SYMMETRIC:
-        return ops.conv_bwd(grad_output, x, nbr, weight, tpb, need_x=need_x, need_w=need_w, need_b=need_b,
-                            assume_symmetric=True)
-    return ops.conv_bwd(grad_output, x, nbr, weight, tpb, table_status=status, need_x=need_x, need_w=need_w,
-                        need_b=need_b)
 
 
 class SparseConv2dFunction(Function):
@@ -94,7 +56,7 @@ class SparseConv2dFunction(Function):
         ctx.tokens_per_batch = tokens_per_batch
         ctx.table_status = None
         if any(ctx.needs_input_grad[:1]):
-            ctx.table_status = _status_for(neighbor_indices, tokens_per_batch)
+            ctx.table_status = _native.table_status(neighbor_indices, kk, tokens_per_batch)
         out = ops.conv_fwd(x.reshape(-1, C_in), neighbor_indices.reshape(-1, kk), weight, bias,
                            tokens_per_batch)
         return out
@@ -112,59 +74,17 @@ class SparseConv2dFunction(Function):
         need_x = ctx.needs_input_grad[0]
         if not (need_x or need_w or need_b):
             return None, None, None, None, None, None
-        status = None
-        if need_x:
-            status = ctx.table_status
-            if status is None:
-                status = _status_for(neighbor_indices, tpb)
         # one library call: the two halves of the backward are independent, so the weight gradient runs
         # next to the input gradient (the reference launches them one after the other, :100-117)
-        grad_input, grad_weight, grad_bias = _bwd(grad_output, x.reshape(-1, ctx.C_in), nbr, weight, tpb, status,
-                                                  need_x, need_w, need_b)
+        status = ctx.table_status
+        grad_input, grad_weight, grad_bias = ops.conv_bwd(grad_output, x.reshape(-1, ctx.C_in), nbr, weight, tpb,
+                                                          table_status=status, need_x=need_x, need_w=need_w,
+                                                          need_b=need_b, assume_symmetric=status is None)
         if grad_input is not None and x.dim() == 3:
             grad_input = grad_input.view(x.shape)
         if not need_w:
             grad_weight = None
         return grad_input, None, grad_weight, grad_bias, None, None
-
-
-class _SparseConv2dCastFunction(Function):
-    """``SparseConv2dFunction`` for parameters kept in another dtype than the activations (autocast, or a bf16
-    input to an fp32 layer): the low-precision copies are made by the module (and cached there), the gradients
-    are handed back in the parameters' own dtype.  Same kernels, two autograd nodes fewer per call."""
-
-    @staticmethod
-    def forward(ctx, x, neighbor_indices, weight, bias, weight_c, bias_c, tokens_per_batch):
-        kk, C_in, C_out = weight_c.shape
-        if C_in % 4 != 0:
-            raise ValueError(f"C_in ({C_in}) must be divisible by 4 for optimized kernel.")
-        ctx.save_for_backward(x, neighbor_indices, weight_c)
-        ctx.C_in = C_in
-        ctx.tokens_per_batch = tokens_per_batch
-        ctx.param_dtype = weight.dtype
-        ctx.bias_dtype = bias.dtype if bias is not None else None
-        ctx.table_status = _status_for(neighbor_indices, tokens_per_batch) if ctx.needs_input_grad[0] else None
-        return ops.conv_fwd(x.reshape(-1, C_in), neighbor_indices.reshape(-1, kk), weight_c, bias_c, tokens_per_batch)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        x, neighbor_indices, weight_c = ctx.saved_tensors
-        kk = weight_c.shape[0]
-        tpb = ctx.tokens_per_batch
-        need_x, need_w = ctx.needs_input_grad[0], ctx.needs_input_grad[2]
-        need_b = ctx.bias_dtype is not None and ctx.needs_input_grad[3]
-        if not (need_x or need_w or need_b):
-            return None, None, None, None, None, None, None
-        status = None
-        if need_x:
-            status = ctx.table_status if ctx.table_status is not None else _status_for(neighbor_indices, tpb)
-        gx, gw, gb = _bwd(grad_output, x.reshape(-1, ctx.C_in), neighbor_indices.reshape(-1, kk), weight_c, tpb,
-                          status, need_x, need_w, need_b)
-        if gx is not None and x.dim() == 3:
-            gx = gx.view(x.shape)
-        gw = gw.to(ctx.param_dtype) if (need_w and gw is not None) else None
-        gb = gb.to(ctx.bias_dtype) if (need_b and gb is not None) else None
-        return gx, None, gw, gb, None, None, None
 
 
 class SparseConv2d(nn.Module):
@@ -200,47 +120,17 @@ class SparseConv2d(nn.Module):
             nn.init.uniform_(self.bias, -bound, bound)
 
     def forward(self, x, neighbor_indices, local_indices=None):
-        kk = self.kernel_size * self.kernel_size
-        is_batched = x.dim() == 3
-        tokens_per_batch = 0
-        if is_batched:
-            B, N, C = x.shape
-            if local_indices is None:
-                # reference heuristic (:170-177): indices are local iff max < N; cached per table object
-                if neighbor_indices.numel() > 0:
-                    local_indices = _table_cache.get(
-                        neighbor_indices, ("local", N), lambda: bool(neighbor_indices.max() < N))
-                else:
-                    local_indices = False
-            if local_indices:
-                tokens_per_batch = N
-            x = x.reshape(-1, C)
-        table = neighbor_indices
-        if table.dtype != torch.int32:
-            table = _table_cache.get(neighbor_indices, "int32", lambda: neighbor_indices.to(torch.int32))
-            if ops.is_known_symmetric(neighbor_indices):
-                ops.mark_symmetric(table)
-        if table.dim() == 3:
-            table = _table_cache.get(table, "flat", lambda: table.reshape(-1, kk)) if table.is_contiguous() \
-                else table.reshape(-1, kk)
-
-        weight = self.weight
-        bias = self.bias
-        target_dtype = x.dtype
-        if torch.is_autocast_enabled():
-            target_dtype = torch.get_autocast_dtype("cuda")
-            if x.dtype != target_dtype:
-                x = x.to(target_dtype)
-        if weight.dtype == target_dtype and (bias is None or bias.dtype == target_dtype):
-            output = SparseConv2dFunction.apply(x, table, weight, bias, tokens_per_batch, self.chunk_size)
-        else:
-            # parameters live in another dtype (the usual case under autocast): their low-precision copies are
-            # kept until the parameters change, e.g. across the two forward passes of activation checkpointing
-            weight_c, bias_c = self._cast_params(target_dtype)
-            output = _SparseConv2dCastFunction.apply(x, table, weight, bias, weight_c, bias_c, tokens_per_batch)
-        if is_batched:
-            output = output.view(B, N, -1)
-        return output
+        """x ``[N, C]`` or ``[B, N, C]``; everything else - the local / global reading of the indices
+        (reference :170-177), int32 and autocast conversions, kernels, the autograd node - is one call of the
+        extension."""
+        weight, bias = self.weight, self.bias
+        dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
+        if weight.dtype is dtype and (bias is None or bias.dtype is dtype):
+            return _native.conv(x, neighbor_indices, weight, bias, weight, bias, local_indices)
+        # parameters live in another dtype (the usual case under autocast): their low-precision copies are
+        # kept until the parameters change, e.g. across the two forward passes of activation checkpointing
+        weight_c, bias_c = self._cast_params(dtype)
+        return _native.conv(x, neighbor_indices, weight, bias, weight_c, bias_c, local_indices)
 
     def invalidate_cast_cache(self):
         """Drops the cached low-precision parameter copies.  They are keyed on the parameters' version counters,

@@ -161,6 +161,16 @@ int svtad_conv_bwd(const void* gy, const void* x, const int32_t* nbr, const void
                    const int32_t* table_status, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * svtad_conv_bwd with the type of gw and gb chosen by the caller: grad_dtype is dtype, or SVTAD_F32 for fp32 master
+ * parameters of a 16-bit layer (mixed precision).  The values are the same - one rounding to dtype - and are written
+ * as fp32, which saves the separate conversion of the gradient.
+ */
+int svtad_conv_bwd_typed(const void* gy, const void* x, const int32_t* nbr, const void* w, void* gx, void* gw,
+                         void* gb, int64_t n, int cin, int cout, int kk, int tokens_per_batch, int dtype,
+                         int grad_dtype, const int32_t* table_status, void* workspace, size_t workspace_bytes,
+                         void* stream);
+
+/*
  * svtad_conv_wgrad for callers that cannot allocate device memory (no counterpart in the reference).
  * Who needs it: hosts that must not call cudaMalloc once they are running - servers that gave all
  * device memory to their own arena, plugins whose host forbids allocation after start-up, loops that

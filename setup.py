@@ -21,8 +21,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 class BuildWithLibrary(build_py):
     def run(self):
         sys.path.insert(0, ROOT)
-        from eccv26_tad_b200.build import build_library
+        from eccv26_tad_b200.build import build_library, build_native
         build_library()
+        build_native()
         super().run()
 
 
@@ -32,7 +33,7 @@ setup(
     description="B200-native SparseConv2D (SV-TAD): neighbor tables, sparse forward / backward, drop-in opentad_sparse_ops",
     packages=["eccv26_tad_b200"],
     py_modules=["opentad_sparse_ops"],
-    package_data={"eccv26_tad_b200": ["libsvtad.so"]},
+    package_data={"eccv26_tad_b200": ["libsvtad.so", "_native.so"]},
     include_package_data=True,
     cmdclass={"build_py": BuildWithLibrary},
     python_requires=">=3.9",

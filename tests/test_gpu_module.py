@@ -204,3 +204,43 @@ def test_reference_wrapper_runs_unchanged_on_top_of_the_shim():
     assert oconv.rel_err(f32np(m.weight.grad), egw) < 1e-5 and oconv.rel_err(f32np(m.bias.grad), egb) < 1e-5
     from eccv26_tad_b200 import ops
     assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("kind", ["built", "given", "given_late", "asymmetric", "local"])
+@pytest.mark.parametrize("amp", [False, True])
+def test_extension_path_by_what_is_known_about_the_table(kind, amp):
+    """The module's one extension call against the oracle: a table this package built (no validation), a caller's
+    table before and after its validation has come back to the host, an asymmetric one (scatter form) and one with
+    indices local to each batch row (whose heuristic asks the device)."""
+    from eccv26_tad_b200 import SparseConv2d, build_neighbor_table
+    B, C = 3, 64
+    scores, _, tab = make_table(B * 2, 1, 14, 14, 0.3, 3, 61)
+    N = tab.shape[0] // B
+    x, w, b, gy = make_conv_inputs(B * N, C, 128, 3, torch.bfloat16, 61, bias="random")
+    glob = tab.clone()
+    if kind == "built":
+        table = build_neighbor_table(scores.cuda(), 0.3, 14, 14)[1]
+    elif kind == "local":
+        one = tab[:N]
+        glob = torch.cat([torch.where(one >= 0, one + i * N, one) for i in range(B)])
+        table = one.unsqueeze(0).repeat(B, 1, 1).cuda()
+    else:
+        if kind == "asymmetric":
+            glob[5] = -1
+        table = glob.view(B, N, 9).cuda()
+    m = SparseConv2d(C, 128).cuda()
+    with torch.no_grad():
+        m.weight.copy_(w); m.bias.copy_(b)
+    m = m if amp else m.bfloat16()
+    ey, egx, egw, egb = _oracle_grads(glob, x, w, b, gy)
+    for again in range(2):
+        m.zero_grad()
+        xc = x.view(B, N, C).cuda().requires_grad_(True)
+        with torch.autocast("cuda", dtype=torch.bfloat16, enabled=amp):
+            y = m(xc, table)
+        if kind == "given_late":
+            torch.cuda.synchronize()
+        y.backward(gy.view(B, N, 128).cuda())
+        assert m.weight.grad.dtype == m.weight.dtype and m.bias.grad.dtype == m.bias.dtype
+        for got, ref in ((y, ey), (xc.grad, egx), (m.weight.grad, egw), (m.bias.grad, egb)):
+            assert oconv.rel_err(f32np(got).reshape(ref.shape), ref) < 2e-2
