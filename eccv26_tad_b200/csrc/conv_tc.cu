@@ -185,8 +185,8 @@ int tc_pick_bn(int cn, long m_tiles) {
     int best = 0;
     long best_cost = 0;
     for (int c : cand) {
-        if (cn % c != 0) continue;
-        long ctas = m_tiles * (cn / c);
+        if (c - 64 >= cn) continue;          // no wider than the output rounded up to 64 columns
+        long ctas = m_tiles * ((cn + c - 1) / c);
         long waves = (ctas + sms - 1) / sms;
         long cost = waves * (A_TILE_BYTES + b_tile_bytes_for(c));
         if (best == 0 || cost < best_cost) { best = c; best_cost = cost; }
@@ -195,12 +195,15 @@ int tc_pick_bn(int cn, long m_tiles) {
 }
 
 // wgrad work split: (pairs of 64-channel blocks) x (column blocks of width BN) x (splits over tokens).
+// A bias gradient takes one more half pair: a block of ones, whose rows of D are the column sums of gy - the spare half
+// of the last pair where the block count is odd, else a pair of its own.  (At C = 1024 that pair costs 1.4 % of the
+// kernel; a separate pass over gy plus the reduction of its partials took 86 + 30 us beside a 305 us main kernel.)
 // One CTA runs per SM, so a candidate (BN, splits) costs
 //   (waves over the SMs) x (64-token steps per CTA + fixed cost) x (cycles per step at that BN)
 // plus the trip of the fp32 partials through memory (written by the main kernel, read by the reduction).
 // Cycles per step and the partials' rate are what these kernels were measured at on a B200.
-static WgradPlan wgrad_plan_for(int64_t n, int cin, int cout, int kk, long sms) {
-    const int nblocks = kk * (cin / 64);
+static WgradPlan wgrad_plan_for(int64_t n, int cin, int cout, int kk, bool with_bias, long sms) {
+    const int nblocks = kk * ((cin + 63) / 64);
     long max_by_rows = (n + 2 * STAGE_K - 1) / (2 * STAGE_K);
     if (max_by_rows < 1) max_by_rows = 1;
     if (max_by_rows > 64) max_by_rows = 64;
@@ -217,14 +220,14 @@ static WgradPlan wgrad_plan_for(int64_t n, int cin, int cout, int kk, long sms) 
     double best_cost = 0;
     for (int ci = 0; ci < 4; ++ci) {
         const int bn = cand[ci];
-        if (cout % bn != 0) continue;
-        if (bn < 192 && best.bn != 0 && forced_bn == 0) continue;      // narrow blocks only when no wide one divides cout
+        if (bn - 64 >= cout) continue;                                   // no wider than cout rounded up to 64 columns
+        if (bn < 192 && best.bn != 0 && forced_bn == 0) continue;      // narrow blocks only when a wide one would be mostly padding
         if (forced_bn > 0 && bn != forced_bn && cout % forced_bn == 0) continue;
         WgradPlan pl;
         pl.bn = bn;
-        pl.n_nblk = cout / bn;
-        pl.n_pairs = (nblocks + 1) / 2;
-        pl.ones_block = nblocks & 1;
+        pl.n_nblk = (cout + bn - 1) / bn;
+        pl.n_pairs = with_bias ? nblocks / 2 + 1 : (nblocks + 1) / 2;
+        pl.ones_block = with_bias;
         const long ctas = (long)pl.n_pairs * pl.n_nblk;
         for (long c = 1; c <= max_by_rows; ++c) {
             if (forced_s > 0 && c != (forced_s < max_by_rows ? forced_s : max_by_rows)) continue;
@@ -247,66 +250,57 @@ static WgradPlan wgrad_plan_for(int64_t n, int cin, int cout, int kk, long sms) 
 }
 
 // The search above costs the host 1-20 us; the last few answers are kept per thread (a training step asks for the same
-// few problems again and again).  `sms` = 0 stands for the workspace size that covers every hint.
+// few problems again and again).  Key 0 stands for the workspace size that covers every hint.
 struct PlanMemo {
     int64_t n = -1;
     int cin, cout, kk;
-    long sms;
+    long key;
     WgradPlan plan;
     size_t bytes;
+    bool is(int64_t n_, int cin_, int cout_, int kk_, long key_) const {
+        return n == n_ && cin == cin_ && cout == cout_ && kk == kk_ && key == key_;
+    }
 };
-static PlanMemo& plan_slot(int64_t n, int cin, int cout, int kk, long sms) {
+static PlanMemo& plan_slot(int64_t n, int cin, int cout, int kk, long key) {
     constexpr unsigned SLOTS = 64;
     static thread_local PlanMemo memo[SLOTS];
-    const uint64_t h = ((uint64_t)n * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)cin << 40) ^ ((uint64_t)cout << 20) ^ (uint64_t)(kk * 256 + sms);
+    const uint64_t h = ((uint64_t)n * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)cin << 40) ^ ((uint64_t)cout << 20) ^ (uint64_t)(kk * 1024 + key);
     return memo[(h ^ (h >> 29) ^ (h >> 47)) % SLOTS];
 }
-static bool plan_known(const PlanMemo& m, int64_t n, int cin, int cout, int kk, long sms) {
-    return m.n == n && m.cin == cin && m.cout == cout && m.kk == kk && m.sms == sms && getenv("SVTAD_TC_WGRAD_BN") == nullptr &&
-           getenv("SVTAD_TC_WGRAD_SPLITS") == nullptr;
+static bool plan_overridden() { return getenv("SVTAD_TC_WGRAD_BN") != nullptr || getenv("SVTAD_TC_WGRAD_SPLITS") != nullptr; }
+
+WgradPlan tc_wgrad_plan(int64_t n, int cin, int cout, int kk, bool with_bias) {
+    const long sms = tc_plan_sms(), key = 2 * sms + with_bias;
+    if (plan_overridden()) return wgrad_plan_for(n, cin, cout, kk, with_bias, sms);
+    PlanMemo& m = plan_slot(n, cin, cout, kk, key);
+    if (!m.is(n, cin, cout, kk, key)) m = PlanMemo{n, cin, cout, kk, key, wgrad_plan_for(n, cin, cout, kk, with_bias, sms), 0};
+    return m.plan;
 }
 
-WgradPlan tc_wgrad_plan(int64_t n, int cin, int cout, int kk) {
-    const long sms = tc_plan_sms();
-    PlanMemo& m = plan_slot(n, cin, cout, kk, sms);
-    if (plan_known(m, n, cin, cout, kk, sms)) return m.plan;
-    const WgradPlan pl = wgrad_plan_for(n, cin, cout, kk, sms);
-    if (getenv("SVTAD_TC_WGRAD_BN") == nullptr && getenv("SVTAD_TC_WGRAD_SPLITS") == nullptr)
-        m = PlanMemo{n, cin, cout, kk, sms, pl, 0};
-    return pl;
-}
-
-static size_t plan_bytes(const WgradPlan& pl, int64_t n, int cin, int cout, int kk) {
-    size_t w = (size_t)pl.splits * kk * cin * cout * sizeof(float);
-    int sb = pl.ones_block ? pl.splits : bias_splits_for(n);
-    size_t b = (size_t)sb * cout * sizeof(float);
+size_t tc_wgrad_plan_bytes(const WgradPlan& pl, int cin, int cout, int kk) {
+    const size_t w = (size_t)pl.splits * kk * cin * cout * sizeof(float);
+    const size_t b = pl.ones_block ? (size_t)pl.splits * cout * sizeof(float) : 0;
     return align_up(w, 256) + align_up(b, 256);
 }
 
-// Workspace of the plan in force at this moment (what a launch checks its workspace against) ...
-size_t tc_wgrad_plan_ws_bytes(int64_t n, int cin, int cout, int kk) {
-    return plan_bytes(tc_wgrad_plan(n, cin, cout, kk), n, cin, cout, kk);
-}
-
-// ... and what callers are told to provide: enough for the plan under every concurrency hint, so that a workspace
+// What callers are told to provide: enough for the plan under every concurrency hint, so that a workspace
 // sized once stays valid when the hint changes (a leaner plan usually has fewer token splits, but the waves'
 // rounding can go the other way: 18 880 rows at C=192, 5x5 takes 3 splits planned for 148 SMs and 5 for 74).
 size_t tc_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk) {
     PlanMemo& m = plan_slot(n, cin, cout, kk, 0);
-    if (plan_known(m, n, cin, cout, kk, 0)) return m.bytes;
+    if (!plan_overridden() && m.is(n, cin, cout, kk, 0)) return m.bytes;
     size_t need = 0;
     const int sms = tc_num_sms();
-    for (int share = 1; share <= 16; ++share) {
-        int v = sms / share;
-        if (v < 8) v = 8;
-        const size_t b = plan_bytes(wgrad_plan_for(n, cin, cout, kk, v), n, cin, cout, kk);
-        if (b > need) need = b;
-    }
-    if (getenv("SVTAD_TC_WGRAD_BN") == nullptr && getenv("SVTAD_TC_WGRAD_SPLITS") == nullptr)
-        m = PlanMemo{n, cin, cout, kk, 0, WgradPlan{}, need};
+    for (int share = 1; share <= 16; ++share)
+        for (int with_bias = 0; with_bias < 2; ++with_bias) {
+            int v = sms / share;
+            if (v < 8) v = 8;
+            const size_t b = tc_wgrad_plan_bytes(wgrad_plan_for(n, cin, cout, kk, with_bias != 0, v), cin, cout, kk);
+            if (b > need) need = b;
+        }
+    if (!plan_overridden()) m = PlanMemo{n, cin, cout, kk, 0, WgradPlan{}, need};
     return need;
 }
-
 
 // fixed-order reduction of the per-split partials (4 elements per thread), one rounding; OUT32: the rounded values are
 // written as fp32 (the gradient of an fp32 master parameter), which saves a pass over the gradient
@@ -357,7 +351,8 @@ int tc_wgrad_reduce_launch(const float* ws_w, int splits, const float* ws_b, int
 bool tc_supported(int op, int64_t n, int cin, int cout, int kk, int dtype) {
     if (dtype != SVTAD_BF16 && dtype != SVTAD_F16) return false;
     if (n <= 0 || kk > 49) return false;
-    if (cin % 64 != 0 || cout % 64 != 0) return false;
+    // 32: the epilogue's column chunk; a row of 32 channels is 64 bytes, so rows stay 16-byte aligned for the copies
+    if (cin % 32 != 0 || cout % 32 != 0) return false;
     (void)op;
     return true;
 }

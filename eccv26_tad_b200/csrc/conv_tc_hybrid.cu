@@ -5,7 +5,7 @@
 //             transposed) - the gather form of the input gradient, valid for symmetric tables
 //   wgrad     D[128 = two 64-channel blocks of (tap, ci), BN] += A(MN-major: gathered x rows, 64 tokens
 //             per stage) . B(MN-major: gy rows); split over tokens, fp32 partials to the workspace;
-//             an all-ones spare block turns the bias gradient into one more row of D
+//             a block of ones turns the bias gradient into one more row of D
 //
 // Operand feed.  Gathered rows are irregular, so four producer warps copy them with 16-byte cp.async
 // straight into the 128-byte-swizzled layout the UMMA descriptors describe (nothing gathered is ever
@@ -86,7 +86,9 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t stage_base = smem_u32(smem);
     const int tiles_total = m_tiles * n_blks;
-    const int kchunks = cred / STAGE_K;
+    // 64-channel chunks of the reduction; the last one may be partial (channel counts are multiples of 32): its missing
+    // channels are zero-filled in both operands and the MMA steps over them are left out
+    const int kchunks = (cred + STAGE_K - 1) / STAGE_K;
     const int stages_per_tile = kk * kchunks;
     // With RB = 2, two 64-deep buffers form one barrier round (a 128-deep K step): the MMA thread's per-round
     // work (wait, fences, commit) is spent once per eight instructions instead of once per four - worth it when
@@ -209,13 +211,14 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
                         jrow[4 * q4] = v.x; jrow[4 * q4 + 1] = v.y; jrow[4 * q4 + 2] = v.z; jrow[4 * q4 + 3] = v.w;
                     }
                     // A: 8 consecutive lanes cover one row's 128 B (8 chunks of 16 B)
-                    const uint16_t* abase = a + c0 + sub * 8;
+                    const bool there = c0 + sub * 8 < cred;
+                    const uint16_t* abase = a + (there ? c0 + sub * 8 : 0);
 #pragma unroll
                     for (int itr = 0; itr < FW_ITR; ++itr) {
                         const int j = jrow[itr];
                         const int r7 = ((itr & 1) << 2) | rg;            // (row & 7) for row = (FW_ITR * part + itr) * 4 + rg
                         const uint32_t dst = a_tile + ((FW_ITR * part + itr) * 4 + rg) * 128 + ((sub ^ r7) << 4);
-                        cp_async16(dst, abase + (long)(j < 0 ? 0 : j) * cred, j < 0 ? 0u : 16u);
+                        cp_async16(dst, abase + (long)(j < 0 ? 0 : j) * cred, j < 0 || !there ? 0u : 16u);
                     }
                     cp_async_arrive_noinc(bar);
                 }
@@ -235,8 +238,10 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             const uint32_t idesc = make_idesc(fp16 ? 0 : 1, 0, DGRAD ? 0 : 1, TILE_M, BN);
             constexpr uint32_t desc_hi = smem_desc_hi(1024);
             bool alive = true;
-            int local = 0, s = 0;
+            int local = 0, s = 0, kc = 0;
             uint32_t ph = 0;
+            const int last_ks = (cred - (kchunks - 1) * STAGE_K + 15) / 16;     // 16-channel MMA steps of the last chunk
+            const bool whole = last_ks == STAGE_K / 16;
             for (int tile = blockIdx.x; tile < tiles_total && alive; tile += gridDim.x, ++local) {
                 const int buf = local & 1;
                 if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((local >> 1) & 1) ^ 1, s_abort, err, 42)) { alive = false; break; }
@@ -255,14 +260,20 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
                         for (int h = 0; h < halves; ++h) {
                             const uint32_t b_lo = (a_lo + (A_TILE_BYTES >> 4)) | (DGRAD ? 0u : smem_desc_lbo_bits(8192));
                             umma_f16_lh(d_tmem, a_lo, desc_hi, b_lo, desc_hi, idesc, (st | h) != 0 ? 1u : 0u);
+                            if (whole || (kc + h) % kchunks != kchunks - 1) {
 #pragma unroll
-                            for (int ks = 1; ks < STAGE_K / 16; ++ks)
-                                umma_f16_lh_acc(d_tmem, a_lo + ks * 2, desc_hi, b_lo + ks * (DGRAD ? 2 : 128), desc_hi, idesc);
+                                for (int ks = 1; ks < STAGE_K / 16; ++ks)
+                                    umma_f16_lh_acc(d_tmem, a_lo + ks * 2, desc_hi, b_lo + ks * (DGRAD ? 2 : 128), desc_hi, idesc);
+                            } else {
+                                for (int ks = 1; ks < last_ks; ++ks)
+                                    umma_f16_lh_acc(d_tmem, a_lo + ks * 2, desc_hi, b_lo + ks * (DGRAD ? 2 : 128), desc_hi, idesc);
+                            }
                             a_lo += STAGE_BYTES >> 4;
                         }
                         umma_commit(smem_u32(&tail->empty[s]));
                     }
                     __syncwarp();
+                    if (!whole) { kc += halves; if (kc >= kchunks) kc -= kchunks; }
                     if (++s == nbig) { s = 0; ph ^= 1u; }
                 }
                 if (!alive) break;
@@ -284,7 +295,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             // the tile's bias goes to shared memory while the main loop is still running
             float* sb = s_bias + buf * 256;
             for (int t = et; t < BN; t += 128)
-                sb[t] = (!DGRAD && bias != nullptr) ? widen(__ldg(bias + n0 + t), fp16 != 0) : 0.f;
+                sb[t] = (!DGRAD && bias != nullptr && n0 + t < cn) ? widen(__ldg(bias + n0 + t), fp16 != 0) : 0.f;
             named_bar_sync(2, 128);
             if (!warp_wait(smem_u32(&tail->accum_full[buf]), (local >> 1) & 1, s_abort, err, 44, lane)) break;
             tc_fence_after();
@@ -298,7 +309,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
                 uint32_t (&v)[32] = (c & 1) ? vb : va;
                 tmem_ld_wait();
                 if (c + 1 < NC) tmem_ld32(t_addr + (c + 1) * 32, (c & 1) ? va : vb);
-                if (row < n) store_row_chunk32(orow + c * 32, v, sb + c * 32, fp16 != 0, out_al32 != 0);
+                if (row < n && n0 + c * 32 < cn) store_row_chunk32(orow + c * 32, v, sb + c * 32, fp16 != 0, out_al32 != 0);
             }
             tc_fence_before();
             mbar_arrive(smem_u32(&tail->accum_empty[buf]));
@@ -335,14 +346,15 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int pair = blockIdx.x / n_nblk;
     const int n0 = (blockIdx.x % n_nblk) * BN;
-    const int cblocks = cin / 64;
+    const int cblocks = (cin + 63) / 64;      // the last 64-channel block of a tap may be partial
     const int nblocks = kk * cblocks;
     const long i_begin = (long)blockIdx.y * tokens_per_split;
     const long i_end = n < i_begin + tokens_per_split ? n : i_begin + tokens_per_split;
     const int total_stages = i_end > i_begin ? (int)((i_end - i_begin + STAGE_K - 1) / STAGE_K) : 0;
     const uint32_t stage_base = smem_u32(smem);
-    const bool second_real = pair * 2 + 1 < nblocks;
-    // second block of the last pair when the block count is odd: all ones, so its rows of D are sum_i gy[i,:]
+    const bool first_real = pair * 2 < nblocks, second_real = pair * 2 + 1 < nblocks;
+    // the block behind the last real one, when the bias gradient is asked for: all ones, so its rows of D are
+    // sum_i gy[i,:] (where the block count is even it has a pair of its own, whose first block stays zero)
     const bool ones_here = ones_block && !second_real;
 
     // A producer warp owns every n_prod-th 64-token step.  The A tile of a step has 128 slots (slot = block * 64 +
@@ -375,7 +387,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
                 const int slot = lane + 32 * j;
                 const int h = j >> 1, t = slot & 63;
                 const long i = i0 + t;
-                const bool ok = (h == 0 || second_real) && i < i_end;
+                const bool ok = (h == 0 ? first_real : second_real) && i < i_end;
                 const int32_t* src = nbr + (ok ? i * kk + tap[h] : 0);
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
                              ::"r"(smem_u32(my_ent + (own % WG_PF) * 128 + slot)), "l"(src), "r"(ok ? 4u : 0u) : "memory");
@@ -387,7 +399,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
     if (warp < n_prod) {
 #pragma unroll
         for (int own = 0; own < WG_PF; ++own) load_entries(own);
-        if (lane == 31 && warp < total_stages) {
+        if (lane == 31 && warp < total_stages && first_real) {
             const long i0 = i_begin + (long)src_stage(warp) * STAGE_K;
             l2_prefetch_rows(x, i0 - 64, i0 + STAGE_K + 64, n, cin);
         }
@@ -428,6 +440,15 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
         int s = warp % nstage;
         uint32_t ph = ((warp / nstage) & 1) ^ 1;
         const int rows_n = second_real ? 32 : 16;            // slots 64..127 belong to the second block
+        // this lane's 16 bytes of a row, per block; nothing is read behind the channels of a partial block
+        const uint16_t* xh[2];
+        uint32_t bytes[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const bool there = ch0[h] + sub * 8 < cin;
+            xh[h] = x + (there ? ch0[h] + sub * 8 : 0);
+            bytes[h] = there ? 16u : 0u;
+        }
         int own = 0;
         for (int it = warp; it < total_stages && warp < n_prod; it += n_prod, ++own) {
             // this own step's entries have landed (the WG_PF - 1 younger groups may still be in flight)
@@ -440,7 +461,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
                 const int h = j >> 1, t = slot & 63;
                 const long i = i0 + t;
                 v[j] = -1;
-                if ((h == 0 || second_real) && i < i_end) {
+                if ((h == 0 ? first_real : second_real) && i < i_end) {
                     const int raw = my_ent[(own % WG_PF) * 128 + slot];
                     const long jj = (long)raw + (tpb > 0 ? (i / tpb) * (long)tpb : 0);
                     if (raw >= 0 && jj < n) v[j] = (int)jj;
@@ -468,8 +489,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
                     const int j = jrow[itr];
                     const int r7 = ((itr & 1) << 2) | rg;
                     const uint32_t dst = a_tile + r * 128 + ((sub ^ r7) << 4);
-                    const uint16_t* src = x + (long)(j < 0 ? 0 : j) * cin + ch0[itr >> 4] + sub * 8;
-                    cp_async16(dst, src, j < 0 ? 0u : 16u);
+                    cp_async16(dst, xh[itr >> 4] + (long)(j < 0 ? 0 : j) * cin, j < 0 ? 0u : bytes[itr >> 4]);
                 }
             }
             cp_async_arrive_noinc(bar);
@@ -513,9 +533,10 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
             const int blk = pair * 2 + (q >> 1);
             float* dstrow = nullptr;
             if (blk < nblocks) {
-                const long grow = (long)(blk / cblocks) * cin + (blk % cblocks) * 64 + (q & 1) * 32 + lane;
-                dstrow = ws_w + ((long)blockIdx.y * kk * cin + grow) * cout + n0;
-            } else if (ones_here && q == 2 && lane == 0 && ws_b != nullptr) {
+                const int ch = (blk % cblocks) * 64 + (q & 1) * 32 + lane;
+                const long grow = (long)(blk / cblocks) * cin + ch;
+                if (ch < cin) dstrow = ws_w + ((long)blockIdx.y * kk * cin + grow) * cout + n0;
+            } else if (ones_here && q == 2 && lane == 0) {
                 dstrow = ws_b + (long)blockIdx.y * cout + n0;
             }
             constexpr int NC = BN / 32;
@@ -532,7 +553,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = 0u;
                 }
-                if (dstrow != nullptr) {
+                if (dstrow != nullptr && n0 + c * 32 < cout) {
                     // 32 bytes (one whole sector) per store: the workspace is 256-byte aligned, rows are cout * 4 bytes
                     float* dst = dstrow + c * 32;
 #pragma unroll
@@ -578,7 +599,7 @@ static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStre
     auto kern = two ? conv_hybrid_kernel<BN, DGRAD, 2> : conv_hybrid_kernel<BN, DGRAD, 1>;
     { int rc_s = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem); if (rc_s) return rc_s; }
     const int m_tiles = (int)((p.n + TILE_M - 1) / TILE_M);
-    const int n_blks = cn / BN;
+    const int n_blks = (cn + BN - 1) / BN;
     long tiles = (long)m_tiles * n_blks;
     // persistent CTAs.  (Evening the tiles out - 135 tiles as 45 CTAs of 3 instead of 49 CTAs of 3 or 2 - was
     // measured slower inside a step of concurrent kernels: 0.0907 against 0.0858 ms.)
@@ -635,36 +656,24 @@ static int launch_wgrad_hybrid(const void* gy, const void* x, const int32_t* nbr
 
 int hybrid_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin, int cout,
                  int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes, cudaStream_t s) {
-    size_t need = tc_wgrad_plan_ws_bytes(n, cin, cout, kk);
+    const WgradPlan pl = tc_wgrad_plan(n, cin, cout, kk, gb != nullptr);
+    const size_t need = tc_wgrad_plan_bytes(pl, cin, cout, kk);
     if (ws_bytes < need)
         return set_error(SVTAD_ERR_WORKSPACE, "svtad_conv_wgrad: workspace %zu < %zu bytes", ws_bytes, need);
-    WgradPlan pl = tc_wgrad_plan(n, cin, cout, kk);
     const int fp16 = dtype == SVTAD_F16 ? 1 : 0;
     const long n_w = (long)kk * cin * cout;
     float* ws_w = static_cast<float*>(ws);
     float* ws_b = reinterpret_cast<float*>(static_cast<char*>(ws) + align_up((size_t)pl.splits * n_w * sizeof(float), 256));
-    const bool bias_in_kernel = gb != nullptr && pl.ones_block;
-    float* kb = bias_in_kernel ? ws_b : nullptr;
     int rc;
     switch (pl.bn) {
-        case 64: rc = launch_wgrad_hybrid<64>(gy, x, nbr, ws_w, kb, n, cin, cout, kk, tpb, fp16, pl, s); break;
-        case 128: rc = launch_wgrad_hybrid<128>(gy, x, nbr, ws_w, kb, n, cin, cout, kk, tpb, fp16, pl, s); break;
-        case 192: rc = launch_wgrad_hybrid<192>(gy, x, nbr, ws_w, kb, n, cin, cout, kk, tpb, fp16, pl, s); break;
-        case 256: rc = launch_wgrad_hybrid<256>(gy, x, nbr, ws_w, kb, n, cin, cout, kk, tpb, fp16, pl, s); break;
+        case 64: rc = launch_wgrad_hybrid<64>(gy, x, nbr, ws_w, ws_b, n, cin, cout, kk, tpb, fp16, pl, s); break;
+        case 128: rc = launch_wgrad_hybrid<128>(gy, x, nbr, ws_w, ws_b, n, cin, cout, kk, tpb, fp16, pl, s); break;
+        case 192: rc = launch_wgrad_hybrid<192>(gy, x, nbr, ws_w, ws_b, n, cin, cout, kk, tpb, fp16, pl, s); break;
+        case 256: rc = launch_wgrad_hybrid<256>(gy, x, nbr, ws_w, ws_b, n, cin, cout, kk, tpb, fp16, pl, s); break;
         default: return set_error(SVTAD_ERR_UNSUPPORTED, "tensor-core wgrad: no column block for width %d", cout);
     }
     if (rc) return rc;
-    int splits_b = 0;
-    if (gb != nullptr) {
-        if (bias_in_kernel) {
-            splits_b = pl.splits;
-        } else {
-            splits_b = bias_splits_for(n);
-            rc = bias_partial_launch(gy, ws_b, n, cout, dtype, splits_b, s);
-            if (rc) return rc;
-        }
-    }
-    return tc_wgrad_reduce_launch(ws_w, pl.splits, ws_b, splits_b, gw, gb, n_w, cout, fp16, grad_dtype == SVTAD_F32, s);
+    return tc_wgrad_reduce_launch(ws_w, pl.splits, ws_b, gb ? pl.splits : 0, gw, gb, n_w, cout, fp16, grad_dtype == SVTAD_F32, s);
 }
 
 }  // namespace svtad

@@ -139,7 +139,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
     const int cid = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
     const uint32_t stage_base = smem_u32(smem);
     const int items_total = m_pairs * n_blks;
-    const int kchunks = cred / STAGE_K;
+    const int kchunks = (cred + STAGE_K - 1) / STAGE_K;      // the last 64-channel chunk may be partial (see the one-CTA kernel)
     const int stages_per_tile = kk * kchunks;
     // Two 64-deep buffers form one barrier round (a 128-deep K step): the MMA thread's per-round work (wait,
     // fences, commits) is spent once per eight instructions instead of once per four.  A tile with an odd
@@ -241,7 +241,8 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                             tma_load_3d(b_tile, &map_w, c0, n0, wtap, bar);
                         }
                     }
-                    const uint16_t* abase = a + c0 + sub * 8;
+                    const bool there = c0 + sub * 8 < cred;
+                    const uint16_t* abase = a + (there ? c0 + sub * 8 : 0);
                     const int4* trow = reinterpret_cast<const int4*>(xf + (k << 7) + (rg << 5));
                     int jrow[32];
 #pragma unroll
@@ -254,7 +255,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                         const int j = jrow[itr];
                         const int r7 = ((itr & 1) << 2) | rg;
                         const uint32_t dst = a_tile + (itr * 4 + rg) * 128 + ((sub ^ r7) << 4);
-                        cp_async16(dst, abase + (long)(j < 0 ? 0 : j) * cred, j < 0 ? 0u : 16u);
+                        cp_async16(dst, abase + (long)(j < 0 ? 0 : j) * cred, j < 0 || !there ? 0u : 16u);
                     }
                     cp_async_arrive_noinc(bar);
                 }
@@ -271,8 +272,10 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
             // the whole warp walks the loop and waits; one elected lane (the same every time) issues and commits
             const uint32_t idesc = make_idesc(fp16 ? 0 : 1, 0, DGRAD ? 0 : 1, 2 * TILE_M, BN);
             bool alive = true;
-            int local = 0, s = 0;
+            int local = 0, s = 0, kc = 0;
             uint32_t ph = 0;
+            const int last_ks = (cred - (kchunks - 1) * STAGE_K + 15) / 16;     // 16-channel MMA steps of the last chunk
+            const bool whole = last_ks == STAGE_K / 16;
             // distance from one of this CTA's shared-memory addresses to the same location in the odd CTA
             const uint32_t to_peer = map_to_cta(stage_base, 1) - stage_base;
             for (int item = cid; item < items_total && alive; item += n_clusters, ++local) {
@@ -295,10 +298,16 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                         constexpr uint32_t b_hi = DGRAD ? smem_desc_hi(1024) : (((512u >> 4) & 0x3FFFu) | (1u << 14) | (4u << 29));
                         for (int h = 0; h < halves; ++h) {
                             const uint32_t b_lo = (a_lo + (A_TILE_BYTES >> 4)) | (DGRAD ? 0u : smem_desc_lbo_bits(4096));
+                            if (whole || (kc + h) % kchunks != kchunks - 1) {
 #pragma unroll
-                            for (int ks = 0; ks < STAGE_K / 16; ++ks)
-                                umma_pair_f16_lh(d_tmem, a_lo + ks * 2, a_hi, b_lo + ks * (DGRAD ? 2 : 64), b_hi, idesc,
-                                                 ks != 0 ? 1u : ((st | h) != 0 ? 1u : 0u));
+                                for (int ks = 0; ks < STAGE_K / 16; ++ks)
+                                    umma_pair_f16_lh(d_tmem, a_lo + ks * 2, a_hi, b_lo + ks * (DGRAD ? 2 : 64), b_hi, idesc,
+                                                     ks != 0 ? 1u : ((st | h) != 0 ? 1u : 0u));
+                            } else {
+                                for (int ks = 0; ks < last_ks; ++ks)
+                                    umma_pair_f16_lh(d_tmem, a_lo + ks * 2, a_hi, b_lo + ks * (DGRAD ? 2 : 64), b_hi, idesc,
+                                                     ks != 0 ? 1u : ((st | h) != 0 ? 1u : 0u));
+                            }
                             a_lo += STAGE_BYTES >> 4;
                         }
                         const uint32_t e_local = smem_u32(&tail->empty[s]);
@@ -306,6 +315,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                         umma_pair_commit(e_local + to_peer);
                     }
                     __syncwarp();
+                    if (!whole) { kc += halves; if (kc >= kchunks) kc -= kchunks; }
                     if (++s == nbig) { s = 0; ph ^= 1u; }
                 }
                 if (!alive) break;
@@ -341,7 +351,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
             const int n0 = (item % n_blks) * BN;
             float* sb = s_bias + buf * 256;
             for (int t = et; t < BN; t += 128)
-                sb[t] = (!DGRAD && bias != nullptr) ? widen(__ldg(bias + n0 + t), fp16 != 0) : 0.f;
+                sb[t] = (!DGRAD && bias != nullptr && n0 + t < cn) ? widen(__ldg(bias + n0 + t), fp16 != 0) : 0.f;
             named_bar_sync(2, 128);
             if (!warp_wait_pair(smem_u32(&tail->accum_full[buf]), (local >> 1) & 1, s_abort, err, 55, lane)) break;
             tc_fence_after();
@@ -354,7 +364,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                 uint32_t (&v)[32] = (c & 1) ? vb : va;
                 tmem_ld_wait();
                 if (c + 1 < NC) tmem_ld32(t_addr + (c + 1) * 32, (c & 1) ? va : vb);
-                if (row < n) store_row_chunk32(orow + c * 32, v, sb + c * 32, fp16 != 0, out_al32 != 0);
+                if (row < n && n0 + c * 32 < cn) store_row_chunk32(orow + c * 32, v, sb + c * 32, fp16 != 0, out_al32 != 0);
             }
             tc_fence_before();
             __syncwarp();
@@ -405,7 +415,7 @@ static int launch_conv_pair(const ConvArgs& p, const int32_t* status, cudaStream
     { int rc_s = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem); if (rc_s) return rc_s; }
     const long m_tiles = (p.n + TILE_M - 1) / TILE_M;
     const int m_pairs = (int)((m_tiles + 1) / 2);
-    const int n_blks = cn / BN;
+    const int n_blks = (cn + BN - 1) / BN;
     const long items = (long)m_pairs * n_blks;
     const long max_clusters = tc_num_sms() / 2;
     const int clusters = (int)(items < max_clusters ? items : max_clusters);
@@ -427,7 +437,8 @@ static int launch_conv_pair(const ConvArgs& p, const int32_t* status, cudaStream
     return SVTAD_OK;
 }
 
-// widest column block that divides the output width (a pair needs one CTA per row tile whatever the width)
+// The column block with the least padding over the output width, the widest of equals (a pair needs one CTA per row
+// tile whatever the width).
 static int pair_pick_bn(int cn) {
     const int cand[4] = {256, 192, 128, 64};
     const char* e = getenv("SVTAD_TC_BN");
@@ -436,9 +447,12 @@ static int pair_pick_bn(int cn) {
         for (int c : cand)
             if (v == c && cn % v == 0) return v;
     }
-    for (int c : cand)
-        if (cn % c == 0) return c;
-    return 0;
+    int best = 0, padded = 0;
+    for (int c : cand) {
+        const int p = (cn + c - 1) / c * c;
+        if (best == 0 || p < padded) { best = c; padded = p; }
+    }
+    return best;
 }
 
 template <bool DGRAD>

@@ -288,8 +288,8 @@ struct WgradPlan {
     int bn, n_nblk, n_pairs, splits, ones_block;
     long tokens_per_split;
 };
-WgradPlan tc_wgrad_plan(int64_t n, int cin, int cout, int kk);
-size_t tc_wgrad_plan_ws_bytes(int64_t n, int cin, int cout, int kk);
+WgradPlan tc_wgrad_plan(int64_t n, int cin, int cout, int kk, bool with_bias);
+size_t tc_wgrad_plan_bytes(const WgradPlan& pl, int cin, int cout, int kk);
 
 // fixed-order reduction of per-split fp32 partials into the 16-bit gradient tensors
 int tc_wgrad_reduce_launch(const float* ws_w, int splits, const float* ws_b, int splits_b, void* gw, void* gb,

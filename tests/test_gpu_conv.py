@@ -259,6 +259,26 @@ def test_default_dispatch_on_both_sides_of_the_pair_switch(n):
     assert oconv.rel_err(f32np(outs[1])[tail], oconv.dgrad_rows(gf, tn, wf, tail)) < 2e-2
 
 
+@pytest.mark.parametrize("cin,cout,dtype", [(32, 96, torch.bfloat16), (96, 96, torch.bfloat16), (96, 32, torch.float16),
+                                            (160, 352, torch.bfloat16), (320, 224, torch.float16)])
+@pytest.mark.parametrize("n", [131, 2000, 148 * 128 + 5])
+def test_channel_counts_that_leave_partial_blocks(cin, cout, dtype, n):
+    """Multiples of 32 that are no multiples of 64: partial last chunks of the reduction, partial column blocks and
+    partial weight-gradient blocks, on single CTAs and on CTA pairs, with an even and an odd number of blocks."""
+    ops = _ops()
+    assert ops.path_for(0, n, cin, cout, 9, dtype) == "tc"
+    table = _chain_table(n)
+    x, w, b, gy = make_conv_inputs(n, cin, cout, 3, dtype, n % 1000, bias="random")
+    outs = _run_all(table, x, w, b, gy)
+    if n < 10000:
+        _check_all(table, x, w, b, gy, outs, 2e-2)
+    else:
+        _check_sampled(table, x, w, b, gy, outs, 2e-2, row_step=16, n_ci=16)
+    # the weight gradient without the bias gradient takes a plan of its own
+    gw, gb = ops.conv_wgrad(gy.cuda(), x.cuda(), table.cuda(), 9, with_bias=False)
+    assert gb is None and oconv.rel_err(f32np(gw), f32np(outs[2])) < 2e-2
+
+
 def test_geometric_tables_on_both_sides_of_the_pair_switch():
     """Same with tables from the builder: 18 880 rows (148 row tiles, single CTAs) and 19 520 rows (153 tiles, pairs)."""
     for keep, rows in ((0.30, 18880), (0.31, 19520)):
