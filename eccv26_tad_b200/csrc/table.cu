@@ -5,6 +5,8 @@
 // :913-977 gather + remap); the algorithms do not: selection is an exact k-th-key search on
 // order-preserving integer keys, compaction is a ballot/popc prefix scan, and the table is
 // emitted straight from the kept set without materialising the old-to-new map in HBM.
+#include <atomic>
+
 #include "common.cuh"
 
 namespace svtad {
@@ -194,146 +196,311 @@ table_build_warp_kernel(const float* __restrict__ scores, int n_seg, int L, int 
 }
 
 // ------------------------------------------------------------------------------------------
-// build: one CTA per segment (any seg_len whose rank array fits in shared memory)
+// build: a thread-block cluster per segment (seg_len > 256: a clip, or a long batch row)
 // ------------------------------------------------------------------------------------------
-constexpr int BLK = 1024;
+// What bounds it: latency.  A clip of 15 680 scores is 60 KB and its table 340 KB, but every step of the selection
+// (four radix passes, two prefix sums) waits for the one before.  One CTA per clip took 115 us for 15 680 -> 9 408
+// tokens, most of it in 83 dependent trips to memory per thread while the rows were written out by two SMs of 148.
+// So G CTAs (one per 2048 tokens, at most 8) share a segment:
+//   * scores are read once and stay in registers as order-preserving keys;
+//   * per radix pass the CTAs count their own keys and add the G histograms up through distributed shared memory, each
+//     for itself, so a pass costs one cluster barrier;
+//   * what is kept travels as one bit per token: every CTA gets the whole bit set (6.4 KB at the longest segment) and
+//     scans it, after which rank(token) is a word, a mask and a popcount in its own shared memory;
+//   * the rows of a word's kept tokens are contiguous in the output: a warp writes them with coalesced stores.
+constexpr int SEG_THREADS = 1024, SEG_MAX = 51200, SEG_WORDS = SEG_MAX / 32;
 
-__device__ __forceinline__ int block_excl_scan_flag(bool flag, int* s_w, int& total) {
-    // exclusive prefix count of `flag` over the block in thread order; all threads call it
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    unsigned m = __ballot_sync(0xffffffffu, flag);
-    __syncthreads();               // s_w free for reuse
-    if (lane == 0) s_w[wid] = __popc(m);
-    __syncthreads();
-    int before = 0, all = 0;
-#pragma unroll
-    for (int i = 0; i < BLK / 32; ++i) {
-        int c = s_w[i];
-        before += (i < wid) ? c : 0;
-        all += c;
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t in_cta(uint32_t saddr, int cta) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
+    return r;
+}
+template <int G>
+__device__ __forceinline__ void cluster_sync() {
+    if constexpr (G == 1) {
+        __syncthreads();
+    } else {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
-    total = all;
-    return before + __popc(m & ((1u << lane) - 1u));
+}
+// exclusive prefix sum of v over the block in thread order
+__device__ __forceinline__ int block_excl_scan(int v, int* s_w) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += t;
+    }
+    __syncthreads();               // s_w free for reuse
+    if (lane == 31) s_w[wid] = incl;
+    __syncthreads();
+    int w = s_w[lane];             // SEG_THREADS / 32 = 32 warps
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, w, d);
+        if (lane >= d) w += t;
+    }
+    const int before = __shfl_sync(0xffffffffu, w, (wid + 31) & 31);
+    return (wid > 0 ? before : 0) + incl - v;
 }
 
-__global__ void __launch_bounds__(BLK)
-table_build_block_kernel(const float* __restrict__ scores, int n_seg, int L, int k, int h, int w,
-                         int ksize, int32_t* __restrict__ kept_idx, int32_t* __restrict__ table,
-                         int64_t* __restrict__ idx64, const int32_t* __restrict__ table_in, int kk_in) {
-    extern __shared__ int32_t s_rank[];          // [L]
-    __shared__ int s_hist[256];
-    __shared__ int s_w[BLK / 32];
-    __shared__ uint32_t s_prefix;
-    __shared__ int s_need;
-    const int seg = blockIdx.x;
+// ITEMS = words of 32 tokens a warp holds; table_in: rows to renumber (a later pruning round), else the grid's own
+template <int G, int ITEMS>
+__global__ void __launch_bounds__(SEG_THREADS)
+table_build_segment_kernel(const float* __restrict__ scores, int L, int k, int h, int w, int ksize, uint32_t magic_w,
+                           uint32_t magic_hw, uint32_t magic_ks, int kk,
+                           int32_t* __restrict__ kept_idx, int32_t* __restrict__ table, int64_t* __restrict__ idx64,
+                           const int32_t* __restrict__ table_in, int staged) {
+    extern __shared__ __align__(16) int32_t s_rows[];     // this CTA's rows of table_in, if they fit
+    __shared__ int s_hist[4][256];
+    __shared__ int s_found[3];
+    __shared__ uint32_t s_keep[SEG_WORDS], s_eq[SEG_WORDS];
+    __shared__ uint2 s_rank[SEG_WORDS];               // a word's kept bits and the output row of its first kept token
+    __shared__ uint32_t s_list[SEG_THREADS / 32][32]; // per warp: its word's kept tokens, lane | y << 8 | x << 16
+    __shared__ int s_w[SEG_THREADS / 32];
+    const int seg = blockIdx.x / G, cta = blockIdx.x % G;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int n_words = (L + 31) >> 5, per_cta = (n_words + G - 1) / G;
+    const int w_begin = cta * per_cta, w_end = min(n_words, w_begin + per_cta);
     const float* sc = scores + (long)seg * L;
 
-    // (1) radix select of the k-th largest key, one byte per pass, most significant first
-    if (tid == 0) { s_prefix = 0; s_need = k; }
-    uint32_t mask = 0;
-    for (int pass = 3; pass >= 0; --pass) {
-        if (tid < 256) s_hist[tid] = 0;
-        __syncthreads();
-        const uint32_t prefix = s_prefix;
-        for (int e = tid; e < L; e += BLK) {
-            uint32_t key = score_key(__ldg(sc + e));
-            if ((key & mask) == prefix) atomicAdd(&s_hist[(key >> (8 * pass)) & 255], 1);
-        }
-        __syncthreads();
-        if (wid == 0) {
-            // lane l owns bins 255-8l .. 248-8l (descending); find the bin holding the need-th key
-            int need = s_need;
-            int cnt[8], sum = 0;
+    uint32_t key[ITEMS];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { cnt[i] = s_hist[255 - 8 * lane - i]; sum += cnt[i]; }
-            int incl = sum;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                int t = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += t;
-            }
-            unsigned hit = __ballot_sync(0xffffffffu, incl >= need);
-            int owner = __ffs(hit) - 1;      // always found: total matching keys >= need
-            if (lane == owner) {
-                int above = incl - sum;      // keys in strictly higher bins
-                int i = 0;
-                while (i < 7 && above + cnt[i] < need) { above += cnt[i]; ++i; }
-                s_prefix = prefix | ((uint32_t)(255 - 8 * lane - i) << (8 * pass));
-                s_need = need - above;
-            }
-        }
-        mask |= 0xFFu << (8 * pass);
-        __syncthreads();
+    for (int j = 0; j < ITEMS; ++j) {
+        const int word = w_begin + wid + 32 * j, e = word * 32 + lane;
+        key[j] = word < w_end && e < L ? score_key(__ldg(sc + e)) : 0u;     // 0 is below every real key
     }
-    const uint32_t T = s_prefix;
-    const int need_ties = s_need;
-
-    // (2) ordered compaction: tie ranks, keep flags, new ranks
-    int32_t* pos_out = kept_idx + (long)seg * k;      // kept positions, read back in (3)
-    int run_tie = 0, run_keep = 0;
-    for (int c0 = 0; c0 < L; c0 += BLK) {
-        int e = c0 + tid;
-        bool valid = e < L;
-        uint32_t key = valid ? score_key(__ldg(sc + e)) : 0u;
-        bool eq = valid && key == T;
-        bool g = valid && key > T;
-        int tot_tie, tot_keep;
-        int tie_rank = run_tie + block_excl_scan_flag(eq, s_w, tot_tie);
-        bool keep = g || (eq && tie_rank < need_ties);
-        int rank = run_keep + block_excl_scan_flag(keep, s_w, tot_keep);
-        if (valid) s_rank[e] = keep ? rank : -1;
-        if (keep) {
-            if (kept_idx != nullptr) pos_out[rank] = e;
-            if (idx64 != nullptr) idx64[(long)seg * k + rank] = e;
-        }
-        run_tie += tot_tie;
-        run_keep += tot_keep;
+    s_hist[tid >> 8][tid & 255] = 0;
+    // the rows this CTA may have to renumber start their trip now and are in shared memory when the selection is done
+    const int row_begin = w_begin * 32, n_rows = max(0, min(L, w_end * 32) - row_begin);
+    const int32_t* rows_in = table_in != nullptr ? table_in + ((long)seg * L + row_begin) * kk : nullptr;
+    const int shift = (int)((reinterpret_cast<uintptr_t>(rows_in) >> 2) & 3);     // keeps source and target equally aligned
+    if (staged) {
+        const int total = n_rows * kk, lead = min(total, (4 - shift) & 3), vec = (total - lead) >> 2;
+        auto copy = [&](int f, int bytes) {
+            const uint32_t dst = smem_addr(s_rows + shift + f);
+            if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(rows_in + f) : "memory");
+            else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(rows_in + f) : "memory");
+        };
+        if (tid < lead) copy(tid, 4);
+        for (int v = tid; v < vec; v += SEG_THREADS) copy(lead + 4 * v, 16);
+        for (int f = lead + 4 * vec + tid; f < total; f += SEG_THREADS) copy(f, 4);
     }
     __syncthreads();
-    if (table == nullptr) return;
 
-    const long base = (long)seg * k;
-    if (table_in != nullptr) {
-        // (3') later pruning round: the kept rows of the previous table, renumbered through the rank array
-        const long total_in = (long)k * kk_in;
-        const long seg0 = (long)seg * L;
-        int32_t* out_r = table + base * kk_in;
-        for (long f = tid; f < total_in; f += BLK) {
-            int r = (int)(f / kk_in);
-            int tap = (int)(f - (long)r * kk_in);
-            int p = __ldcg(pos_out + r);
-            int32_t old = __ldg(table_in + (seg0 + p) * kk_in + tap);
-            int32_t v = -1;
-            long loc = (long)old - seg0;
-            if (old >= 0 && loc >= 0 && loc < L) {
-                int rk = s_rank[loc];
-                if (rk >= 0) v = (int32_t)(base + rk);
+    // (1) radix select of the k-th largest key, one byte per pass, most significant first
+    uint32_t T = 0, mask = 0;
+    int need = k, at_T = 0;
+#pragma unroll 1
+    for (int pass = 3; pass >= 0; --pass) {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const int word = w_begin + wid + 32 * j;
+            const bool in = word < w_end && word * 32 + lane < L && (key[j] & mask) == T;
+            const int bin = (key[j] >> (8 * pass)) & 255;
+            if (pass == 3) {
+                // sign and exponent fall into a handful of bins: one add per bin and warp
+                const unsigned same = __match_any_sync(0xffffffffu, in ? bin : 256);
+                if (in && (same & lt) == 0) atomicAdd(&s_hist[3][bin], __popc(same));
+            } else if (in) {
+                atomicAdd(&s_hist[pass][bin], 1);
             }
-            out_r[f] = v;
         }
-        return;
+        cluster_sync<G>();
+        // thread t adds up bin 255 - t; an inclusive scan over the bins in descending order names the one that holds
+        // the need-th key (always found: matching keys >= need)
+        int c = 0, incl = 0;
+        if (tid < 256) {
+            if constexpr (G == 1) {
+                c = s_hist[pass][255 - tid];
+            } else {
+                const uint32_t mine = smem_addr(&s_hist[pass][255 - tid]);
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    int v;
+                    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(in_cta(mine, g)) : "memory");
+                    c += v;
+                }
+            }
+            incl = c;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += t;
+            }
+            if (lane == 31) s_w[wid] = incl;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            for (int q = 0; q < wid; ++q) incl += s_w[q];
+            if (incl >= need && incl - c < need) {
+                s_found[0] = 255 - tid;
+                s_found[1] = need - (incl - c);
+                s_found[2] = c;
+            }
+        }
+        __syncthreads();
+        T |= (uint32_t)s_found[0] << (8 * pass);
+        need = s_found[1];
+        at_T = s_found[2];
+        mask |= 0xFFu << (8 * pass);
     }
 
-    // (3) emit table rows
-    const int KK = ksize * ksize, hw = h * w, r0 = ksize >> 1;
-    int32_t* out = table + base * KK;
-    const long total = (long)k * KK;
-    for (long f = tid; f < total; f += BLK) {
-        int r = (int)(f / KK);
-        int tap = (int)(f - (long)r * KK);
-        int dy = tap / ksize - r0, dx = tap % ksize - r0;
-        int p = __ldcg(pos_out + r);
-        int q = p % hw;
-        int y = q / w, x = q - y * w;
-        int yy = y + dy, xx = x + dx;
-        int32_t v = -1;
-        if ((unsigned)yy < (unsigned)h && (unsigned)xx < (unsigned)w) {
-            int rk = s_rank[p + dy * w + dx];
-            if (rk >= 0) v = (int32_t)(base + rk);
+    // (2) kept bits: keys above T, and of those equal to T the first `need`
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const int word = w_begin + wid + 32 * j;
+        const bool valid = word < w_end && word * 32 + lane < L;
+        const uint32_t gt = __ballot_sync(0xffffffffu, valid && key[j] > T);
+        const uint32_t eq = __ballot_sync(0xffffffffu, valid && key[j] == T);
+        if (word < w_end) {
+            if constexpr (G == 1) {
+                if (lane == 0) { s_keep[word] = gt; s_eq[word] = eq; }
+            } else if (lane < G) {
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_cta(smem_addr(&s_keep[word]), lane)), "r"(gt) : "memory");
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_cta(smem_addr(&s_eq[word]), lane)), "r"(eq) : "memory");
+            }
         }
-        out[f] = v;
     }
+    cluster_sync<G>();                 // also the last access to another CTA's shared memory
+    constexpr int WPT = (SEG_WORDS + SEG_THREADS - 1) / SEG_THREADS;     // words per thread in the scans
+    {
+        int ties = 0;
+        if (at_T != need) {            // not every key equal to T is kept: lower tokens first
+            int c = 0;
+#pragma unroll
+            for (int q = 0; q < WPT; ++q)
+                if (tid * WPT + q < n_words) c += __popc(s_eq[tid * WPT + q]);
+            ties = block_excl_scan(c, s_w);
+        }
+        uint32_t kw[WPT];
+        int c = 0;
+#pragma unroll
+        for (int q = 0; q < WPT; ++q) {
+            const int word = tid * WPT + q;
+            kw[q] = 0;
+            if (word < n_words) {
+                uint32_t eq = s_eq[word];
+                int room = at_T != need ? max(0, need - ties) : 32;
+                ties += __popc(eq);
+                while (__popc(eq) > room) eq &= ~(0x80000000u >> __clz(eq));     // drop the highest
+                kw[q] = s_keep[word] | eq;
+                c += __popc(kw[q]);
+            }
+        }
+        int before = block_excl_scan(c, s_w);
+#pragma unroll
+        for (int q = 0; q < WPT; ++q) {
+            const int word = tid * WPT + q;
+            if (word < n_words) { s_rank[word] = make_uint2(kw[q], seg * k + before); before += __popc(kw[q]); }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+
+    // (3) a word's kept positions and table rows
+    const int seg0 = seg * L;          // row numbers fit 31 bits
+    const int hw = h * w, r0 = ksize >> 1;
+    auto renumbered = [&](unsigned loc) -> int32_t {
+        const uint2 rk = s_rank[loc >> 5];
+        const uint32_t below = rk.x << (31 - (loc & 31));       // the token's own bit on top
+        return below >> 31 ? (int32_t)(rk.y + __popc(below) - 1) : -1;
+    };
+    const int d_row = 32 / kk, d_tap = 32 - d_row * kk;           // from one of a lane's entries to the next
+    const int row_of_lane = lane / kk, tap_of_lane = lane - row_of_lane * kk;
+    for (int word = w_begin + wid; word < w_end; word += SEG_THREADS / 32) {
+        const uint2 rk = s_rank[word];
+        const int e = word * 32 + lane;
+        if ((rk.x >> lane) & 1u) {
+            const int r = __popc(rk.x & lt);
+            if (kept_idx != nullptr) kept_idx[rk.y + r] = e;
+            if (idx64 != nullptr) idx64[rk.y + r] = e;
+            const int p = hw == 1 ? 0 : e - div_magic(e, magic_hw) * hw;
+            const int y = w == 1 ? p : div_magic(p, magic_w), x = p - y * w;
+            s_list[wid][r] = (uint32_t)lane | (uint32_t)(y & 0xFF) << 8 | (uint32_t)(x & 0xFF) << 16;
+        }
+        if (table == nullptr) continue;
+        __syncwarp();
+        const int entries = __popc(rk.x) * kk;
+        int32_t* out = table + (long)rk.y * kk;
+        int r = row_of_lane, tap = tap_of_lane;
+        auto advance = [&] {
+            r += d_row;
+            tap += d_tap;
+            if (tap >= kk) { tap -= kk; ++r; }
+        };
+        if (table_in != nullptr) {
+            // later round: the kept rows of the previous table, renumbered
+            const int32_t* in = staged ? s_rows + shift + (word - w_begin) * 32 * kk : rows_in + (word - w_begin) * 32 * (long)kk;
+#pragma unroll 4
+            for (int f = lane; f < entries; f += 32) {
+                const int32_t old = in[(int)(s_list[wid][r] & 31u) * kk + tap];
+                const unsigned loc = (unsigned)(old - seg0);
+                out[f] = old >= 0 && loc < (unsigned)L ? renumbered(loc) : -1;
+                advance();
+            }
+        } else {
+            for (int f = lane; f < entries; f += 32) {
+                const int ty = ksize == 1 ? tap : div_magic(tap, magic_ks);
+                const int dy = ty - r0, dx = tap - ty * ksize - r0;
+                const uint32_t it = s_list[wid][r];
+                const int y = (int)(it >> 8 & 0xFFu) + dy, x = (int)(it >> 16) + dx;
+                out[f] = (unsigned)y < (unsigned)h && (unsigned)x < (unsigned)w
+                             ? renumbered(word * 32 + (int)(it & 31u) + dy * w + dx) : -1;
+                advance();
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// floor(e / d) = umulhi(e, magic) for e < 65536 (see div_magic)
+static uint32_t magic_of(int d) { return (uint32_t)((0x100000000ull + d - 1) / d); }
+
+template <int G, int ITEMS>
+static int segment_launch_as(const float* scores, int n_seg, int L, int k, int h, int w, int ksize, int kk, int32_t* kept_idx,
+                             int32_t* table, int64_t* idx64, const int32_t* table_in, cudaStream_t s) {
+    auto kern = table_build_segment_kernel<G, ITEMS>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n_seg * G));
+    cfg.blockDim = dim3(SEG_THREADS);
+    cfg.stream = s;
+    // rows of the previous table wait in shared memory while they leave room for it
+    const size_t rows = (size_t)(((L + 31) / 32 + G - 1) / G) * 32 * kk * sizeof(int32_t) + 16;
+    const int staged = table_in != nullptr && rows <= 180 * 1024;
+    if (staged) {
+        cfg.dynamicSmemBytes = rows;
+        static std::atomic<uint64_t> ready{0};     // devices on which this kernel may use that much
+        int dev = 0;
+        SV_CUDA(cudaGetDevice(&dev));
+        const uint64_t bit = 1ull << (dev & 63);
+        if (!(ready.load() & bit)) {
+            SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 180 * 1024));
+            ready.fetch_or(bit);
+        }
+    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = G;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = G > 1 ? 1 : 0;
+    SV_CUDA(cudaLaunchKernelEx(&cfg, kern, scores, L, k, h, w, ksize, magic_of(w), magic_of(h * w), magic_of(ksize),
+                               kk, kept_idx, table, idx64, table_in, staged));
+    return SVTAD_OK;
+}
+
+static int segment_launch(const float* scores, int n_seg, int L, int k, int h, int w, int ksize, int kk, int32_t* kept_idx,
+                          int32_t* table, int64_t* idx64, const int32_t* table_in, cudaStream_t s) {
+    // two words (64 tokens) per warp: a CTA per 2048 tokens while a portable cluster covers the segment
+    auto as = L <= 2048 ? segment_launch_as<1, 2> : L <= 4096 ? segment_launch_as<2, 2> : L <= 8192 ? segment_launch_as<4, 2>
+              : L <= 16384 ? segment_launch_as<8, 2> : segment_launch_as<8, 7>;
+    return as(scores, n_seg, L, k, h, w, ksize, kk, kept_idx, table, idx64, table_in, s);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -444,21 +611,10 @@ static int table_build_impl(const float* scores, int n_seg, int seg_len, int k, 
         SV_LAUNCH_CHECK("table_build_warp_kernel");
         return SVTAD_OK;
     }
-    // CTA-per-segment path needs the kept positions in global memory between its phases
     SV_CHECK_ARG(table == nullptr || kept_idx != nullptr, "%s: kept_idx is required with a table", who);
-    size_t smem = (size_t)seg_len * sizeof(int32_t);
-    if (smem > 200 * 1024)
-        return set_error(SVTAD_ERR_UNSUPPORTED, "%s: seg_len=%d exceeds the %d-token segment limit", who, seg_len, 200 * 1024 / 4);
-    static thread_local int attr_dev = -1;
-    int dev = 0;
-    SV_CUDA(cudaGetDevice(&dev));
-    if (attr_dev != dev) {
-        SV_CUDA(cudaFuncSetAttribute(table_build_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr_dev = dev;
-    }
-    table_build_block_kernel<<<n_seg, BLK, smem, s>>>(scores, n_seg, seg_len, k, h, w, ksize, kept_idx, table, idx64, nullptr, 0);
-    SV_LAUNCH_CHECK("table_build_block_kernel");
-    return SVTAD_OK;
+    if (seg_len > SEG_MAX)
+        return set_error(SVTAD_ERR_UNSUPPORTED, "%s: seg_len=%d exceeds the %d-token segment limit", who, seg_len, SEG_MAX);
+    return segment_launch(scores, n_seg, seg_len, k, h, w, ksize, ksize * ksize, kept_idx, table, idx64, nullptr, s);
 }
 
 extern "C" int svtad_table_build(const float* scores, int n_seg, int seg_len, int k_keep, int h,
@@ -486,14 +642,9 @@ extern "C" int svtad_table_select_remap(const float* scores, const int32_t* tabl
     SV_CHECK_ARG((long)B * n_prev < (1l << 31), "svtad_table_select_remap: row count does not fit int32 indices");
     if (B == 0 || k_keep == 0) return SVTAD_OK;
     SV_CHECK_ARG(scores && table_in && kept_idx && table_out, "svtad_table_select_remap: null pointer");
-    size_t smem = (size_t)n_prev * sizeof(int32_t);
-    if (smem > 200 * 1024)
-        return set_error(SVTAD_ERR_UNSUPPORTED, "svtad_table_select_remap: n_prev=%d exceeds the %d-token limit", n_prev, 200 * 1024 / 4);
-    SV_CUDA(cudaFuncSetAttribute(table_build_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    table_build_block_kernel<<<B, BLK, smem, (cudaStream_t)stream>>>(scores, B, n_prev, k_keep, n_prev, 1, 1, kept_idx,
-                                                                     table_out, idx, table_in, kk);
-    SV_LAUNCH_CHECK("table_build_block_kernel");
-    return SVTAD_OK;
+    if (n_prev > SEG_MAX)
+        return set_error(SVTAD_ERR_UNSUPPORTED, "svtad_table_select_remap: n_prev=%d exceeds the %d-token limit", n_prev, SEG_MAX);
+    return segment_launch(scores, B, n_prev, k_keep, n_prev, 1, 1, kk, kept_idx, table_out, idx, table_in, (cudaStream_t)stream);
 }
 
 extern "C" int svtad_table_remap(const int32_t* table_in, const int64_t* idx, int B, int n_prev,

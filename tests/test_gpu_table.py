@@ -177,3 +177,28 @@ def test_public_table_api_names():
     t2 = pkg.update_neighbor_indices(t, idx)
     kept, tab = pkg.build_neighbor_table(scores, 0.6, 14, 14)
     np.testing.assert_array_equal(t2.reshape(-1, 9).cpu().numpy(), tab.cpu().numpy())
+
+
+@pytest.mark.parametrize("L,hw", [(257, None), (2048, (16, 16)), (2049, None), (4096, (8, 16)), (8190, (9, 13)), (8193, None),
+                                  (16384, (16, 16)), (16390, (10, 11)), (51200, (16, 16))])
+@pytest.mark.parametrize("ties", [False, True])
+def test_long_segments_on_both_sides_of_every_cluster_size(L, hw, ties):
+    """One CTA per 2048 tokens, at most eight: selection, table and renumbering at the edges of each cluster size, with
+    distinct scores and with ties that straddle CTAs and words."""
+    ops = _ops()
+    rng = np.random.default_rng(L)
+    s = rng.integers(-2, 3, size=(2, L)).astype(np.float32) if ties else rng.standard_normal((2, L)).astype(np.float32)
+    sc = torch.from_numpy(s).cuda()
+    for k in (1, L // 3, L - 1, L):
+        ekept = otab.select_topk(s, k)
+        np.testing.assert_array_equal(ops.topk_select(sc, k).cpu().numpy(), ekept)
+        if hw is not None and L % (hw[0] * hw[1]) == 0:
+            h, w = hw
+            kept, table = ops.table_build(sc, k, h, w, 3)
+            etable = otab.build_table(s, k, h, w, 3)[1]
+            np.testing.assert_array_equal(kept.cpu().numpy(), ekept)
+            np.testing.assert_array_equal(table.cpu().numpy(), etable)
+            t0 = otab.initial_table(h, w, L // (h * w), 2, 3)
+            idx, tab = ops.table_select_remap(sc, torch.from_numpy(t0).cuda(), k)
+            np.testing.assert_array_equal(idx.cpu().numpy(), ekept)
+            np.testing.assert_array_equal(tab.reshape(-1, 9).cpu().numpy(), etable)
