@@ -47,21 +47,20 @@ struct ConvArgs {
 
 // CUDA-core kernels (conv_simt.cu)
 int simt_fwd(const ConvArgs& p, cudaStream_t s);
-// fp32 forward tuned for the FFMA rate (conv_simt_fwd.cu)
-bool simt_fwd_f32_supported(const ConvArgs& p);
-int simt_fwd_f32(const ConvArgs& p, cudaStream_t s);
 int simt_dgrad_gather(const ConvArgs& p, const int32_t* status, cudaStream_t s);
 int simt_dgrad_scatter(const ConvArgs& p, const int32_t* status, float* ws, cudaStream_t s);
 int simt_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n,
                int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes,
                cudaStream_t s);
 size_t simt_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk);
-// shared pieces of the weight-gradient path (also used by the tensor-core path)
-int bias_partial_launch(const void* gy, float* partial, int64_t n, int cout, int dtype, int splits,
-                        cudaStream_t s);
-int wgrad_finalize_launch(const float* ws_w, int splits_w, const float* ws_b, int splits_b,
-                          void* gw, void* gb, int64_t n_w, int cout, int dtype, int grad_dtype, cudaStream_t s);
-int bias_splits_for(int64_t n);
+
+// fp32 kernels over compacted pairs (conv_f32.cu); channel counts are multiples of 4
+bool f32_supported(int cin, int cout, int kk, int dtype);
+int f32_fwd(const ConvArgs& p, cudaStream_t s);
+int f32_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s);
+int f32_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin, int cout, int kk,
+              int tpb, void* ws, size_t ws_bytes, cudaStream_t s);
+size_t f32_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk);
 
 // tcgen05 kernels (conv_tc.cu)
 bool tc_supported(int op, int64_t n, int cin, int cout, int kk, int dtype);

@@ -1,5 +1,5 @@
-// CUDA-core (FFMA) SparseConv2D kernels: fp32 tensors at any width, 16-bit tensors whose shape the
-// tensor-core path does not take, and the asymmetric-table dgrad.  Strict fp32 FMA accumulation in
+// Generic CUDA-core (FFMA) SparseConv2D kernels: widths that neither the tensor-core path nor the fp32 kernels over
+// compacted pairs (conv_f32.cu) take, and the asymmetric-table dgrad.  Strict fp32 FMA accumulation in
 // (tap, channel) ascending order - the order of the reference's tiled forward
 // (opentad/models/bricks/2d_sparse_v3.cu:574-629) - so fp32 results stay within 1e-5 relative.
 //
@@ -241,11 +241,12 @@ static int dispatch_conv_simt(const ConvArgs& p, const int32_t* status, float* w
 }
 
 int simt_fwd(const ConvArgs& p, cudaStream_t s) {
-    if (simt_fwd_f32_supported(p) && getenv("SVTAD_SIMT_FWD_GENERIC") == nullptr) return simt_fwd_f32(p, s);
+    if (f32_supported(p.cin, p.cout, p.kk, p.dtype) && getenv("SVTAD_SIMT_FWD_GENERIC") == nullptr) return f32_fwd(p, s);
     return dispatch_conv_simt<MODE_FWD>(p, nullptr, nullptr, s);
 }
 
 int simt_dgrad_gather(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
+    if (f32_supported(p.cin, p.cout, p.kk, p.dtype)) return f32_dgrad(p, status, s);
     return dispatch_conv_simt<MODE_DGATHER>(p, status, nullptr, s);
 }
 
@@ -400,12 +401,12 @@ __global__ void wgrad_finalize_kernel(const float* __restrict__ ws_w, int splits
     }
 }
 
-int bias_splits_for(int64_t n) {
+static int bias_splits_for(int64_t n) {
     long s = (n + 127) / 128;
     return (int)(s < 1 ? 1 : (s > 296 ? 296 : s));
 }
 
-int bias_partial_launch(const void* gy, float* partial, int64_t n, int cout, int dtype, int splits,
+static int bias_partial_launch(const void* gy, float* partial, int64_t n, int cout, int dtype, int splits,
                         cudaStream_t s) {
     long rps = (n + splits - 1) / splits;
     if (rps < 1) rps = 1;
@@ -418,7 +419,7 @@ int bias_partial_launch(const void* gy, float* partial, int64_t n, int cout, int
     return SVTAD_OK;
 }
 
-int wgrad_finalize_launch(const float* ws_w, int splits_w, const float* ws_b, int splits_b, void* gw,
+static int wgrad_finalize_launch(const float* ws_w, int splits_w, const float* ws_b, int splits_b, void* gw,
                           void* gb, int64_t n_w, int cout, int dtype, int grad_dtype, cudaStream_t s) {
     long total = n_w + (gb ? cout : 0);
     unsigned grid = (unsigned)((total + 255) / 256);
@@ -454,12 +455,15 @@ static int simt_wgrad_splits(int64_t n, int cin, int cout, int kk) {
 size_t simt_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk) {
     size_t w = (size_t)simt_wgrad_splits(n, cin, cout, kk) * kk * cin * cout * sizeof(float);
     size_t b = (size_t)bias_splits_for(n) * cout * sizeof(float);
-    return align_up(w, 256) + align_up(b, 256);
+    const size_t generic = align_up(w, 256) + align_up(b, 256);
+    const size_t f32 = f32_supported(cin, cout, kk, SVTAD_F32) ? f32_wgrad_ws_bytes(n, cin, cout, kk) : 0;
+    return f32 > generic ? f32 : generic;
 }
 
 int simt_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n,
                int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes,
                cudaStream_t s) {
+    if (f32_supported(cin, cout, kk, dtype)) return f32_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tpb, ws, ws_bytes, s);
     if (ws_bytes < simt_wgrad_ws_bytes(n, cin, cout, kk))
         return set_error(SVTAD_ERR_WORKSPACE, "svtad_conv_wgrad: workspace %zu < %zu bytes", ws_bytes,
                          simt_wgrad_ws_bytes(n, cin, cout, kk));

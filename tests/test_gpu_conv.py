@@ -279,6 +279,25 @@ def test_channel_counts_that_leave_partial_blocks(cin, cout, dtype, n):
     assert gb is None and oconv.rel_err(f32np(gw), f32np(outs[2])) < 2e-2
 
 
+@pytest.mark.parametrize("B,T,h,w,keep,ks,cin,cout", [
+    (1, 1, 1, 1, 1.0, 3, 4, 4),              # one pair in all
+    (1, 1, 9, 7, 1.0, 3, 36, 68),            # full lists of 63 pairs, partial chunk and column block
+    (1, 4, 14, 14, 0.1, 3, 64, 64),          # a cluster of eight per tile, nearly empty lists
+    (2, 20, 14, 14, 0.5, 3, 100, 192),       # a cluster of two
+    (1, 30, 14, 14, 0.4, 5, 128, 64),        # 25 taps
+    (4, 80, 14, 14, 1.0, 3, 8, 12),          # 128-row tiles, lists of two blocks
+    (1, 2, 10, 10, 0.6, 7, 20, 20),          # 49 taps
+])
+def test_fp32_kernels_over_compacted_pairs(B, T, h, w, keep, ks, cin, cout):
+    _, _, table = make_table(B, T, h, w, keep, ks, 77)
+    n = table.shape[0]
+    x, wt, b, gy = make_conv_inputs(n, cin, cout, ks, torch.float32, 77, bias="random")
+    outs = _run_all(table, x, wt, b, gy, sym=True)
+    _check_all(table, x, wt, b, gy, outs, 1e-5)
+    gw, gb = _ops().conv_wgrad(gy.cuda(), x.cuda(), table.cuda(), ks * ks, with_bias=False)
+    assert gb is None and torch.equal(gw, outs[2])
+
+
 def test_geometric_tables_on_both_sides_of_the_pair_switch():
     """Same with tables from the builder: 18 880 rows (148 row tiles, single CTAs) and 19 520 rows (153 tiles, pairs)."""
     for keep, rows in ((0.30, 18880), (0.31, 19520)):
