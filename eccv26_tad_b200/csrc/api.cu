@@ -101,6 +101,10 @@ extern "C" size_t svtad_workspace_bytes(int op, int64_t n, int cin, int cout, in
         case SVTAD_OP_WGRAD: {
             size_t a = simt_wgrad_ws_bytes(n, cin, cout, kk);
             size_t b = tc_supported(op, n, cin, cout, kk, dtype) ? tc_wgrad_ws_bytes(n, cin, cout, kk) : 0;
+            if (b > 0 && pairs_wgrad_wanted(cin, kk)) {
+                const size_t c = pairs_wgrad_ws_bytes(cout);
+                b = b > c ? b : c;
+            }
             return a > b ? a : b;
         }
         case SVTAD_OP_BWD:   // both halves run at the same time: the two workspaces sit side by side
@@ -110,27 +114,45 @@ extern "C" size_t svtad_workspace_bytes(int op, int64_t n, int cin, int cout, in
     return 0;
 }
 
+// Which parts of a plan shorten a layer's kernels by more than the plan takes to make (16-20 us of GPU time, once per
+// table): bit 0 the row order and tile masks (forward, input gradient), bit 1 the pair lists (weight gradient).  density =
+// pairs per row and tap, negative where it is not known: then the sparse case is assumed.
+// Measured at 18 880 rows: C = 512, 3x3 (89 GFLOP dense): forward 64 -> 41 us at density 0.34, 67 -> 51 at 0.58, 220 -> 230
+// (61 760 rows) at 0.87; weight gradient 81 -> 67, 82 -> 92, 280 -> 410.  Below 25 GFLOP a layer is a single wave of tiles
+// and as long as its longest one.
+extern "C" int svtad_plan_wanted(int64_t n, int cin, int cout, int kk, int dtype, double density) {
+    if (svtad_plan_bytes(n, kk) == 0 || kk < 2) return 0;
+    const double work = 2.0 * (double)n * kk * cin * cout;
+    if (!use_tc(SVTAD_OP_FWD, n, cin, cout, kk, dtype) || work < 25e9) return 0;
+    return (density < 0.75 ? 1 : 0) | (density < 0.45 && pairs_wgrad_wanted(cin, kk) ? 2 : 0);
+}
+
 extern "C" int svtad_conv_fwd(const void* x, const int32_t* nbr, const void* w, const void* bias,
                               void* y, int64_t n, int cin, int cout, int kk, int tokens_per_batch,
                               int dtype, void* workspace, size_t workspace_bytes, void* stream) {
     (void)workspace; (void)workspace_bytes;
+    return svtad_conv_fwd_planned(x, nbr, w, bias, y, n, cin, cout, kk, tokens_per_batch, dtype, nullptr, stream);
+}
+
+extern "C" int svtad_conv_fwd_planned(const void* x, const int32_t* nbr, const void* w, const void* bias,
+                                      void* y, int64_t n, int cin, int cout, int kk, int tokens_per_batch,
+                                      int dtype, const void* plan, void* stream) {
     int rc = check_common("svtad_conv_fwd", n, cin, cout, kk, tokens_per_batch, dtype);
     if (rc) return rc;
     if (n == 0) return SVTAD_OK;
     SV_CHECK_ARG(x && nbr && w && y, "svtad_conv_fwd: null pointer");
     SV_CHECK_ARG(aligned(x, 16) && aligned(w, 16) && aligned(y, 16) && aligned(nbr, 16) && aligned(bias, 16),
                  "svtad_conv_fwd: x, nbr, w, bias and y must be 16-byte aligned");
-    ConvArgs p{x, nbr, w, bias, y, n, cin, cout, kk, tokens_per_batch, dtype};
+    ConvArgs p{x, nbr, w, bias, y, n, cin, cout, kk, tokens_per_batch, dtype, plan};
     if (use_tc(SVTAD_OP_FWD, n, cin, cout, kk, dtype)) return tc_fwd(p, (cudaStream_t)stream);
     if (forced_path() == 2)
         return set_error(SVTAD_ERR_UNSUPPORTED, "svtad_conv_fwd: tensor-core path forced but shape/dtype unsupported");
     return simt_fwd(p, (cudaStream_t)stream);
 }
 
-extern "C" int svtad_conv_dgrad(const void* gy, const int32_t* nbr, const void* w, void* gx,
-                                int64_t n, int cin, int cout, int kk, int tokens_per_batch,
-                                int dtype, const int32_t* table_status, void* workspace,
-                                size_t workspace_bytes, void* stream) {
+static int conv_dgrad_planned(const void* gy, const int32_t* nbr, const void* w, void* gx, int64_t n, int cin, int cout,
+                              int kk, int tokens_per_batch, int dtype, const void* plan, const int32_t* table_status,
+                              void* workspace, size_t workspace_bytes, void* stream) {
     int rc = check_common("svtad_conv_dgrad", n, cin, cout, kk, tokens_per_batch, dtype);
     if (rc) return rc;
     if (n == 0) return SVTAD_OK;
@@ -140,7 +162,7 @@ extern "C" int svtad_conv_dgrad(const void* gy, const int32_t* nbr, const void* 
     if (cout % 4 != 0)
         return set_error(SVTAD_ERR_UNSUPPORTED, "svtad_conv_dgrad: C_out (%d) must be divisible by 4", cout);
     cudaStream_t s = (cudaStream_t)stream;
-    ConvArgs p{gy, nbr, w, nullptr, gx, n, cin, cout, kk, tokens_per_batch, dtype};
+    ConvArgs p{gy, nbr, w, nullptr, gx, n, cin, cout, kk, tokens_per_batch, dtype, plan};
     if (use_tc(SVTAD_OP_DGRAD, n, cin, cout, kk, dtype)) {
         rc = tc_dgrad(p, table_status, s);
     } else {
@@ -159,9 +181,17 @@ extern "C" int svtad_conv_dgrad(const void* gy, const int32_t* nbr, const void* 
     return rc;
 }
 
+extern "C" int svtad_conv_dgrad(const void* gy, const int32_t* nbr, const void* w, void* gx,
+                                int64_t n, int cin, int cout, int kk, int tokens_per_batch,
+                                int dtype, const int32_t* table_status, void* workspace,
+                                size_t workspace_bytes, void* stream) {
+    return conv_dgrad_planned(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, nullptr, table_status, workspace,
+                              workspace_bytes, stream);
+}
+
 static int conv_wgrad_typed(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin,
-                            int cout, int kk, int tokens_per_batch, int dtype, int grad_dtype, void* workspace,
-                            size_t workspace_bytes, void* stream) {
+                            int cout, int kk, int tokens_per_batch, int dtype, int grad_dtype, const void* plan,
+                            void* workspace, size_t workspace_bytes, void* stream) {
     int rc = check_common("svtad_conv_wgrad", n, cin, cout, kk, tokens_per_batch, dtype);
     if (rc) return rc;
     SV_CHECK_ARG(gw != nullptr, "svtad_conv_wgrad: gw is null");
@@ -175,8 +205,11 @@ static int conv_wgrad_typed(const void* gy, const void* x, const int32_t* nbr, v
     SV_CHECK_ARG(aligned(gy, 16) && aligned(x, 16) && aligned(gw, 16) && aligned(nbr, 16) && aligned(gb, 16),
                  "svtad_conv_wgrad: gy, x, nbr, gw and gb must be 16-byte aligned");
     SV_CHECK_ARG(workspace != nullptr && aligned(workspace, 256), "svtad_conv_wgrad: workspace is null or not 256-byte aligned");
-    if (use_tc(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype))
+    if (use_tc(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype)) {
+        if (plan != nullptr && pairs_wgrad_wanted(cin, kk))
+            return pairs_wgrad(gy, x, plan, gw, gb, n, cin, cout, kk, dtype, grad_dtype, workspace, workspace_bytes, s);
         return tc_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace, workspace_bytes, s);
+    }
     if (forced_path() == 2)
         return set_error(SVTAD_ERR_UNSUPPORTED, "svtad_conv_wgrad: tensor-core path forced but shape/dtype unsupported");
     return simt_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace, workspace_bytes, s);
@@ -185,7 +218,7 @@ static int conv_wgrad_typed(const void* gy, const void* x, const int32_t* nbr, v
 extern "C" int svtad_conv_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb,
                                 int64_t n, int cin, int cout, int kk, int tokens_per_batch,
                                 int dtype, void* workspace, size_t workspace_bytes, void* stream) {
-    return conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, dtype, workspace,
+    return conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, dtype, nullptr, workspace,
                             workspace_bytes, stream);
 }
 
@@ -193,24 +226,27 @@ extern "C" int svtad_conv_bwd(const void* gy, const void* x, const int32_t* nbr,
                               void* gw, void* gb, int64_t n, int cin, int cout, int kk,
                               int tokens_per_batch, int dtype, const int32_t* table_status,
                               void* workspace, size_t workspace_bytes, void* stream) {
-    return svtad_conv_bwd_typed(gy, x, nbr, w, gx, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, dtype,
+    return svtad_conv_bwd_typed(gy, x, nbr, w, gx, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, dtype, nullptr, 0,
                                 table_status, workspace, workspace_bytes, stream);
 }
 
 extern "C" int svtad_conv_bwd_typed(const void* gy, const void* x, const int32_t* nbr, const void* w, void* gx,
                                     void* gw, void* gb, int64_t n, int cin, int cout, int kk,
-                                    int tokens_per_batch, int dtype, int grad_dtype, const int32_t* table_status,
-                                    void* workspace, size_t workspace_bytes, void* stream) {
+                                    int tokens_per_batch, int dtype, int grad_dtype, const void* plan,
+                                    int plan_use, const int32_t* table_status, void* workspace,
+                                    size_t workspace_bytes, void* stream) {
     SV_CHECK_ARG(grad_dtype == dtype || grad_dtype == SVTAD_F32,
                  "svtad_conv_bwd: weight gradients come in the features' type or in float32, not in type %d", grad_dtype);
+    const void* rows_plan = plan_use & 1 ? plan : nullptr;
+    const void* pairs_plan = plan_use & 2 ? plan : nullptr;
     SV_CHECK_ARG(gx != nullptr || gw != nullptr, "svtad_conv_bwd: neither gx nor gw requested");
     SV_CHECK_ARG(gb == nullptr || gw != nullptr, "svtad_conv_bwd: gb needs gw");
     if (gw == nullptr)
-        return svtad_conv_dgrad(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, table_status,
-                                workspace, workspace_bytes, stream);
+        return conv_dgrad_planned(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, rows_plan, table_status,
+                                  workspace, workspace_bytes, stream);
     if (gx == nullptr)
-        return conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace,
-                                workspace_bytes, stream);
+        return conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, pairs_plan,
+                                workspace, workspace_bytes, stream);
     // workspace = [weight-gradient part | input-gradient part (scatter form, only with a status word)]
     const size_t w_part = align_up(svtad_workspace_bytes(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype), 256);
     const size_t d_part = table_status != nullptr ? svtad_workspace_bytes(SVTAD_OP_DGRAD, n, cin, cout, kk, dtype) : 0;
@@ -222,28 +258,34 @@ extern "C" int svtad_conv_bwd_typed(const void* gy, const void* x, const int32_t
     int dev = 0;
     SV_CUDA(cudaGetDevice(&dev));
     if (!overlap_backward() || n == 0 || dev >= MAX_DEVICES) {
-        int rc = conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace,
-                                  w_part, s);
+        int rc = conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, pairs_plan,
+                                  workspace, w_part, s);
         if (rc) return rc;
-        return svtad_conv_dgrad(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, table_status, ws_d, d_part, s);
+        return conv_dgrad_planned(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, rows_plan, table_status, ws_d,
+                                  d_part, s);
     }
     SideLane& lane = g_lane[dev];
     std::lock_guard<std::mutex> hold(lane.mu);
     int rc = lane_ready(lane);
     if (rc) return rc;
-    // the two kernels share the GPU: each is planned for half of it unless the caller's hint already says more
+    // The two kernels share the GPU: each is planned for half of it unless the caller's hint already says more.  With pair
+    // lists both are persistent and balanced over all SMs, so there the second one moves in as the first one's CTAs leave.
     struct FloorGuard {
         int old;
-        FloorGuard() : old(tc_set_share_floor(2)) {}
+        explicit FloorGuard(int floor) : old(tc_set_share_floor(floor)) {}
         ~FloorGuard() { tc_set_share_floor(old); }
-    } floor_guard;
+    } floor_guard(pairs_plan != nullptr ? 1 : 2);
     // fork: the side stream starts where the caller's stream stands
     SV_CUDA(cudaEventRecord(lane.fork, s));
     SV_CUDA(cudaStreamWaitEvent(lane.stream, lane.fork, 0));
-    int rc_w = conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace,
+    int rc_w = SVTAD_OK, rc_d = SVTAD_OK;
+    auto wgrad = [&] {
+        rc_w = conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, pairs_plan, workspace,
                                 w_part, lane.stream);
-    int rc_d = svtad_conv_dgrad(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, table_status, ws_d,
-                                d_part, s);
+    };
+    if (pairs_plan == nullptr) wgrad();
+    rc_d = conv_dgrad_planned(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, rows_plan, table_status, ws_d, d_part, s);
+    if (pairs_plan != nullptr) wgrad();
     // join, also after an error: whatever was launched on the side stream is ordered before the caller's next work
     cudaError_t e1 = cudaEventRecord(lane.join, lane.stream);
     cudaError_t e2 = cudaStreamWaitEvent(s, lane.join, 0);

@@ -43,6 +43,7 @@ struct ConvArgs {
     void* out;
     int64_t n;
     int cin, cout, kk, tpb, dtype;
+    const void* plan = nullptr;   // the table's work plan, if the call brings one
 };
 
 // CUDA-core kernels (conv_simt.cu)
@@ -87,6 +88,12 @@ SV_DECLARE_TC_FAMILY(hybrid)
 // forward / dgrad on CTA pairs (conv_tc_pair.cu)
 int pair_fwd(const ConvArgs& p, cudaStream_t s);
 int pair_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s);
+
+// weight gradient over the pairs of a plan (conv_tc_pairs.cu)
+bool pairs_wgrad_wanted(int cin, int kk);
+size_t pairs_wgrad_ws_bytes(int cout);
+int pairs_wgrad(const void* gy, const void* x, const void* plan, void* gw, void* gb, int64_t n, int cin, int cout, int kk,
+                int dtype, int grad_dtype, void* ws, size_t ws_bytes, cudaStream_t s);
 
 #ifdef __CUDACC__
 // ---- device helpers ----

@@ -194,6 +194,24 @@ int tc_pick_bn(int cn, long m_tiles) {
     return best;
 }
 
+// The column block with the least padding over the output width, the widest of equals (for kernels whose tiles fill the
+// GPU whatever the width).
+int tc_widest_bn(int cn) {
+    const int cand[4] = {256, 192, 128, 64};
+    const char* e = getenv("SVTAD_TC_BN");
+    if (e != nullptr && *e) {
+        int v = atoi(e);
+        for (int c : cand)
+            if (v == c && cn % v == 0) return v;
+    }
+    int best = 0, padded = 0;
+    for (int c : cand) {
+        const int p = (cn + c - 1) / c * c;
+        if (best == 0 || p < padded) { best = c; padded = p; }
+    }
+    return best;
+}
+
 // wgrad work split: (pairs of 64-channel blocks) x (column blocks of width BN) x (splits over tokens).
 // A bias gradient takes one more half pair: a block of ones, whose rows of D are the column sums of gy - the spare half
 // of the last pair where the block count is odd, else a pair of its own.  (At C = 1024 that pair costs 1.4 % of the
@@ -369,12 +387,12 @@ static bool use_pair(int64_t n) {
 }
 
 int tc_fwd(const ConvArgs& p, cudaStream_t s) {
-    if (use_pair(p.n)) return pair_fwd(p, s);
+    if (p.plan == nullptr && use_pair(p.n)) return pair_fwd(p, s);
     return hybrid_fwd(p, s);
 }
 
 int tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
-    if (use_pair(p.n)) return pair_dgrad(p, status, s);
+    if (p.plan == nullptr && use_pair(p.n)) return pair_dgrad(p, status, s);
     return hybrid_dgrad(p, status, s);
 }
 

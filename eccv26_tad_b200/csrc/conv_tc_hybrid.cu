@@ -27,6 +27,7 @@
 // (conv_tc_pair.cu).
 #include <cstdlib>
 
+#include "plan.cuh"
 #include "tc_common.cuh"
 
 namespace svtad {
@@ -63,12 +64,16 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 // forward / dgrad
 // ---------------------------------------------------------------------------------------------
 // RB = 64-deep buffers per barrier round (1 or 2).
-template <int BN, bool DGRAD, int RB>
+// PLAN: rows, tiles and taps as the table's plan says (plan.cuh): a tile's rows are plan.order's, only the taps of its
+// mask are worked through, and the CTAs take the tiles, longest first, in alternating directions (CTA c gets items c,
+// 2 G - 1 - c, 2 G + c, ...), so that their sums come out even.
+template <int BN, bool DGRAD, int RB, bool PLAN>
 __global__ void __launch_bounds__(FW_THREADS, 1)
 conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __restrict__ a,
                    const int32_t* __restrict__ nbr, const uint16_t* __restrict__ bias,
                    uint16_t* __restrict__ out, const int32_t* __restrict__ status, long n, int cred, int cn,
-                   int kk, int tpb, int nstage, int fp16, int m_tiles, int n_blks, int out_al32, int* __restrict__ err) {
+                   int kk, int tpb, int nstage, int fp16, int m_tiles, int n_blks, int out_al32, PlanView plan,
+                   int* __restrict__ err) {
     if (DGRAD && status != nullptr && (__ldg(status) & SVTAD_TABLE_ASYMMETRIC)) return;
     constexpr int B_TILE_BYTES = b_tile_bytes_for(BN);
     constexpr int B_TX_BYTES = DGRAD ? BN * 128 : B_TILE_BYTES;
@@ -82,6 +87,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
     // current tile's final row numbers in the order the producer lanes read them (16-byte loads)
     int* s_tab = reinterpret_cast<int*>(tail + 1);
     volatile int* s_abort = &tail->abort_flag;
+    int* s_row = s_tab + 2 * TILE_M * kk + 2 * 256;      // PLAN: row of each of the next tile's slots (behind the bias)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t stage_base = smem_u32(smem);
@@ -89,12 +95,23 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
     // 64-channel chunks of the reduction; the last one may be partial (channel counts are multiples of 32): its missing
     // channels are zero-filled in both operands and the MMA steps over them are left out
     const int kchunks = (cred + STAGE_K - 1) / STAGE_K;
-    const int stages_per_tile = kk * kchunks;
+    const uint64_t all_taps = (1ull << kk) - 1;
+    // the CTA's local-th item: its tile and column block; false behind the last one
+    auto item = [&](int local, int& tile, int& blk) {
+        const int turn = PLAN && (local & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
+        const int it = local * (int)gridDim.x + turn;
+        if (it >= tiles_total) return false;
+        tile = it / n_blks;
+        blk = it - tile * n_blks;
+        if (PLAN) tile = __ldg(plan.seq + tile);
+        return true;
+    };
+    auto taps_of = [&](int tile) { return PLAN ? __ldg(plan.mask + tile) : all_taps; };
     // With RB = 2, two 64-deep buffers form one barrier round (a 128-deep K step): the MMA thread's per-round
     // work (wait, fences, commit) is spent once per eight instructions instead of once per four - worth it when
     // at least three rounds fit in shared memory.  A tile with an odd number of 64-deep steps gets an empty last
     // half: its owner only arrives on the barrier.
-    const int sp_pad = RB == 2 ? ((stages_per_tile + 1) & ~1) : stages_per_tile;
+    auto padded = [](int steps) { return RB == 2 ? ((steps + 1) & ~1) : steps; };
     const int nbig = nstage / RB;             // nstage (number of 64-deep buffers) is a multiple of RB
     constexpr int RSH = RB == 2 ? 1 : 0;      // buffer -> barrier round
     const int tab_ints = TILE_M * kk;
@@ -103,11 +120,21 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
     // of the rows the tile will gather: for tables built on a grid they lie within a few dozen rows of the tile's
     // own, so the gathers that follow the table's trip to memory do not have to make a second one.
     auto load_table = [&](int tile) {
-        const long row0 = (long)(tile / n_blks) * TILE_M;
+        const uint32_t dst = smem_u32(s_tab);
+        if constexpr (PLAN) {
+            // a row per thread, four bytes at a time: the rows lie anywhere
+            const int i = __ldg(plan.order + (long)tile * TILE_M + tid);
+            s_row[tid] = i;
+            const int32_t* src = nbr + (long)(i < 0 ? 0 : i) * kk;
+            for (int k = 0; k < kk; ++k)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (tid * kk + k) * 4), "l"(src + k) : "memory");
+            cp_async_commit();
+            return;
+        }
+        const long row0 = (long)tile * TILE_M;
         const long rows = (n - row0) < TILE_M ? (n - row0) : TILE_M;
         const int valid_bytes = (int)rows * kk * 4;
         const char* src = reinterpret_cast<const char*>(nbr + row0 * kk);
-        const uint32_t dst = smem_u32(s_tab);
         for (int c = tid; c * 16 < tab_ints * 4; c += FW_A_THREADS) {
             int left = valid_bytes - c * 16;
             uint32_t nb = left >= 16 ? 16u : (left > 0 ? (uint32_t)left : 0u);
@@ -117,7 +144,10 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
         if (tid == FW_A_THREADS - 1) l2_prefetch_rows(a, row0 - 64, row0 + TILE_M + 64, n, cred);
     };
     // the first tile's rows start their trip before anything else is set up
-    if (warp < FW_A_WARPS && (int)blockIdx.x < tiles_total) load_table(blockIdx.x);
+    {
+        int tile, blk;
+        if (warp < FW_A_WARPS && item(0, tile, blk)) load_table(tile);
+    }
     if (warp == FW_A_WARPS) {
         tmem_alloc(smem_u32(&tail->tmem_slot), TM_COLS);
         tmem_relinquish();
@@ -150,10 +180,13 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
         // where the parity of the empty barrier looks the same as "free", and refill a buffer in use.
         const int grp = warp / FW_NPW, part = warp % FW_NPW;
         const int n_own = nstage < FW_GROUPS ? nstage : FW_GROUPS;
-        int local = 0;
-        for (int tile = blockIdx.x; tile < tiles_total; tile += gridDim.x, ++local) {
-            const long row0 = (long)(tile / n_blks) * TILE_M;
-            const int n0 = (tile % n_blks) * BN;
+        int it0 = 0;                    // K steps of the tiles before this one
+        int tile, blk;
+        for (int local = 0; item(local, tile, blk); ++local) {
+            const long row0 = (long)tile * TILE_M;
+            const int n0 = blk * BN;
+            const uint64_t taps = taps_of(tile);
+            const int steps = PLAN ? __popcll(taps) * kchunks : kk * kchunks, sp_pad = padded(steps);
             int* xf = s_tab + tab_ints;
             // this tile's table rows have landed (only table copies are ever committed to a group); the first
             // barrier also says that every producer warp is done reading the previous tile's row numbers
@@ -163,27 +196,34 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             // stored as [tap][row & 3][row >> 2], the order in which a lane group walks a stage's rows
             for (int d = tid; d < tab_ints; d += FW_A_THREADS) {
                 const int k = d >> 7, r = ((d & 31) << 2) | ((d >> 5) & 3);
-                long i = row0 + r;
+                long i = PLAN ? (long)s_row[r] : row0 + r;
                 int raw = s_tab[r * kk + k];
                 long jj = (long)raw + (tpb > 0 ? (i / tpb) * (long)tpb : 0);
-                xf[d] = (i < n && raw >= 0 && jj < n) ? (int)jj : -1;
+                xf[d] = ((PLAN ? i >= 0 : i < n) && raw >= 0 && jj < n) ? (int)jj : -1;
             }
             named_bar_sync(1, FW_A_THREADS);
-            if (tile + (int)gridDim.x < tiles_total) load_table(tile + gridDim.x);
+            int next, next_blk;
+            if (item(local + 1, next, next_blk)) load_table(next);
+            const int it1 = it0;
+            it0 += sp_pad;
             if (!alive || grp >= n_own) continue;   // keep taking part in the barriers above
-            const int it0 = local * sp_pad;
             // first step of this tile that this warp's group owns; then every n_own-th one.  Buffer, phase and
             // (tap, chunk) advance incrementally: no division in the loop.
-            int st = ((grp - it0) % n_own + n_own) % n_own;
-            int s = (it0 + st) % nstage;                         // 64-deep buffer; its barrier round is s >> RSH
-            uint32_t ph = (((it0 + st) / nstage) & 1) ^ 1;
+            int st = ((grp - it1) % n_own + n_own) % n_own;
+            int s = (it1 + st) % nstage;                         // 64-deep buffer; its barrier round is s >> RSH
+            uint32_t ph = (((it1 + st) / nstage) & 1) ^ 1;
             int k = st / kchunks, kc = st - k * kchunks;
+            uint64_t left = taps;                                // PLAN: the current tap is the lowest bit
+            if (PLAN) {
+                for (; k > 0; --k) left &= left - 1;
+                k = left != 0 ? __ffsll(left) - 1 : 0;
+            }
             for (; st < sp_pad; st += n_own) {
                 if (!warp_wait(smem_u32(&tail->empty[s >> RSH]), ph, s_abort, err, 41, lane)) { alive = false; break; }
                 const uint32_t a_tile = stage_base + (uint32_t)s * STAGE_BYTES;
                 const uint32_t bar = smem_u32(&tail->full[s >> RSH]);
                 const bool tma_turn = lane == 0 && part == 0;
-                if (RB == 2 && st >= stages_per_tile) {
+                if (RB == 2 && st >= steps) {
                     // the empty half of the tile's last round: same number of arrivals, nothing to copy
                     mbar_arrive(bar);
                     if (tma_turn) mbar_arrive(bar);
@@ -225,7 +265,15 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
                 s += n_own;
                 while (s >= nstage) { s -= nstage; ph ^= 1u; }
                 kc += n_own;
-                while (kc >= kchunks) { kc -= kchunks; if (++k == kk) k = 0; }
+                while (kc >= kchunks) {
+                    kc -= kchunks;
+                    if (PLAN) {
+                        left &= left - 1;
+                        k = left != 0 ? __ffsll(left) - 1 : 0;
+                    } else if (++k == kk) {
+                        k = 0;
+                    }
+                }
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -242,7 +290,9 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             uint32_t ph = 0;
             const int last_ks = (cred - (kchunks - 1) * STAGE_K + 15) / 16;     // 16-channel MMA steps of the last chunk
             const bool whole = last_ks == STAGE_K / 16;
-            for (int tile = blockIdx.x; tile < tiles_total && alive; tile += gridDim.x, ++local) {
+            int tile, blk;
+            for (; alive && item(local, tile, blk); ++local) {
+                const int steps = PLAN ? __popcll(taps_of(tile)) * kchunks : kk * kchunks, sp_pad = padded(steps);
                 const int buf = local & 1;
                 if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((local >> 1) & 1) ^ 1, s_abort, err, 42)) { alive = false; break; }
                 tc_fence_after();
@@ -252,7 +302,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
                     fence_proxy_async();   // cp.async (generic proxy) writes -> tcgen05.mma (async proxy) reads
                     tc_fence_after();
                     const uint32_t a_tile = stage_base + (uint32_t)(RB * s) * STAGE_BYTES;
-                    const int halves = (RB == 2 && st + 1 < stages_per_tile) ? 2 : 1;
+                    const int halves = (RB == 2 && st + 1 < steps) ? 2 : 1;
                     if (elect_one_sync()) {
                         // descriptor low words: start address >> 4 (shared memory is below 256 KB, so adding a K step's
                         // offset never carries into the LBO field above it)
@@ -287,11 +337,12 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
         const int q = warp & 3;
         const int et = tid - (FW_A_WARPS + 1) * 32;          // 0..127 among the epilogue threads
         float* s_bias = reinterpret_cast<float*>(s_tab + 2 * tab_ints);   // [2][256]
-        int local = 0;
-        for (int tile = blockIdx.x; tile < tiles_total; tile += gridDim.x, ++local) {
+        int tile, blk;
+        for (int local = 0; item(local, tile, blk); ++local) {
             const int buf = local & 1;
-            const long row = (long)(tile / n_blks) * TILE_M + q * 32 + lane;
-            const int n0 = (tile % n_blks) * BN;
+            const long slot = (long)tile * TILE_M + q * 32 + lane;
+            const long row = PLAN ? (long)__ldg(plan.order + slot) : slot;
+            const int n0 = blk * BN;
             // the tile's bias goes to shared memory while the main loop is still running
             float* sb = s_bias + buf * 256;
             for (int t = et; t < BN; t += 128)
@@ -309,7 +360,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
                 uint32_t (&v)[32] = (c & 1) ? vb : va;
                 tmem_ld_wait();
                 if (c + 1 < NC) tmem_ld32(t_addr + (c + 1) * 32, (c & 1) ? va : vb);
-                if (row < n && n0 + c * 32 < cn) store_row_chunk32(orow + c * 32, v, sb + c * 32, fp16 != 0, out_al32 != 0);
+                if ((PLAN ? row >= 0 : row < n) && n0 + c * 32 < cn) store_row_chunk32(orow + c * 32, v, sb + c * 32, fp16 != 0, out_al32 != 0);
             }
             tc_fence_before();
             mbar_arrive(smem_u32(&tail->accum_empty[buf]));
@@ -574,7 +625,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
-template <int BN, bool DGRAD>
+template <int BN, bool DGRAD, bool PLAN>
 static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
     const int cred = DGRAD ? p.cout : p.cin;
     const int cn = DGRAD ? p.cin : p.cout;
@@ -587,7 +638,8 @@ static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStre
         if (rc) return rc;
     }
     const size_t stage = A_TILE_BYTES + b_tile_bytes_for(BN);
-    const size_t extra = sizeof(TmaTail) + 2 * (size_t)TILE_M * p.kk * sizeof(int) + 2 * 256 * sizeof(float);
+    const size_t extra = sizeof(TmaTail) + 2 * (size_t)TILE_M * p.kk * sizeof(int) + 2 * 256 * sizeof(float) +
+                         (PLAN ? TILE_M * sizeof(int) : 0);
     int nstage = (int)((TC_SMEM_LIMIT - 1024 - extra) / stage);
     if (nstage > 16) nstage = 16;
     if (nstage < 2)
@@ -596,31 +648,41 @@ static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStre
     const bool two = nstage >= 6;
     if (two) nstage &= ~1;
     const size_t smem = 1024 + nstage * stage + extra;
-    auto kern = two ? conv_hybrid_kernel<BN, DGRAD, 2> : conv_hybrid_kernel<BN, DGRAD, 1>;
+    auto kern = two ? conv_hybrid_kernel<BN, DGRAD, 2, PLAN> : conv_hybrid_kernel<BN, DGRAD, 1, PLAN>;
     { int rc_s = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem); if (rc_s) return rc_s; }
     const int m_tiles = (int)((p.n + TILE_M - 1) / TILE_M);
     const int n_blks = (cn + BN - 1) / BN;
     long tiles = (long)m_tiles * n_blks;
     // persistent CTAs.  (Evening the tiles out - 135 tiles as 45 CTAs of 3 instead of 49 CTAs of 3 or 2 - was
     // measured slower inside a step of concurrent kernels: 0.0907 against 0.0858 ms.)
-    const long plan = tc_plan_sms();
-    int grid = (int)(tiles < plan ? tiles : plan);
+    const long sms = tc_plan_sms();
+    int grid = (int)(tiles < sms ? tiles : sms);
+    PlanView view{};
+    if (PLAN) plan_layout(p.n, p.kk, p.plan, &view);
     SV_CUDA(tc_launch(kern, dim3(grid), dim3(FW_THREADS), smem, s, map_w, (const uint16_t*)p.a, p.nbr,
                       (const uint16_t*)p.bias, (uint16_t*)p.out, status, (long)p.n, cred, cn, p.kk, p.tpb, nstage, fp16,
-                      m_tiles, n_blks, (reinterpret_cast<uintptr_t>(p.out) % 32 == 0) ? 1 : 0, tc_error_ptr()));
+                      m_tiles, n_blks, (reinterpret_cast<uintptr_t>(p.out) % 32 == 0) ? 1 : 0, view, tc_error_ptr()));
     return SVTAD_OK;
 }
 
 template <bool DGRAD>
 static int dispatch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
     const int cn = DGRAD ? p.cin : p.cout;
+    if (p.plan != nullptr) {
+        switch (tc_widest_bn(cn)) {
+            case 64: return launch_conv_hybrid<64, DGRAD, true>(p, status, s);
+            case 128: return launch_conv_hybrid<128, DGRAD, true>(p, status, s);
+            case 192: return launch_conv_hybrid<192, DGRAD, true>(p, status, s);
+            default: return launch_conv_hybrid<256, DGRAD, true>(p, status, s);
+        }
+    }
     int bn = tc_pick_bn(cn, (p.n + TILE_M - 1) / TILE_M);
     switch (bn) {
-        case 64: return launch_conv_hybrid<64, DGRAD>(p, status, s);
-        case 96: return launch_conv_hybrid<96, DGRAD>(p, status, s);
-        case 128: return launch_conv_hybrid<128, DGRAD>(p, status, s);
-        case 192: return launch_conv_hybrid<192, DGRAD>(p, status, s);
-        case 256: return launch_conv_hybrid<256, DGRAD>(p, status, s);
+        case 64: return launch_conv_hybrid<64, DGRAD, false>(p, status, s);
+        case 96: return launch_conv_hybrid<96, DGRAD, false>(p, status, s);
+        case 128: return launch_conv_hybrid<128, DGRAD, false>(p, status, s);
+        case 192: return launch_conv_hybrid<192, DGRAD, false>(p, status, s);
+        case 256: return launch_conv_hybrid<256, DGRAD, false>(p, status, s);
     }
     return set_error(SVTAD_ERR_UNSUPPORTED, "tensor-core conv: no column block for width %d", cn);
 }

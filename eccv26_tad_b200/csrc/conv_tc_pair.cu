@@ -437,28 +437,10 @@ static int launch_conv_pair(const ConvArgs& p, const int32_t* status, cudaStream
     return SVTAD_OK;
 }
 
-// The column block with the least padding over the output width, the widest of equals (a pair needs one CTA per row
-// tile whatever the width).
-static int pair_pick_bn(int cn) {
-    const int cand[4] = {256, 192, 128, 64};
-    const char* e = getenv("SVTAD_TC_BN");
-    if (e != nullptr && *e) {
-        int v = atoi(e);
-        for (int c : cand)
-            if (v == c && cn % v == 0) return v;
-    }
-    int best = 0, padded = 0;
-    for (int c : cand) {
-        const int p = (cn + c - 1) / c * c;
-        if (best == 0 || p < padded) { best = c; padded = p; }
-    }
-    return best;
-}
-
 template <bool DGRAD>
 static int dispatch_conv_pair(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
     const int cn = DGRAD ? p.cin : p.cout;
-    switch (pair_pick_bn(cn)) {
+    switch (tc_widest_bn(cn)) {
         case 64: return launch_conv_pair<64, DGRAD>(p, status, s);
         case 128: return launch_conv_pair<128, DGRAD>(p, status, s);
         case 192: return launch_conv_pair<192, DGRAD>(p, status, s);

@@ -1,0 +1,404 @@
+// Weight gradient over the pairs of a table's plan: tcgen05 / TMEM, 16-bit tensors, fp32 accumulate.
+//
+//   gw[k] = sum over the pairs (i, j) of tap k of x[j]^T . gy[i]
+//
+// The kernel without a plan (wgrad_hybrid_kernel) walks all tokens for every tap and multiplies zero rows where a
+// neighbor is pruned; here a tap's reduction runs over its list, 64 pairs per step: a third of the steps at keep 30 %,
+// a quarter with a 5x5 stencil.  Work unit = (tap, 128 input channels, BN output channels), and one more row of units,
+// fed with ones instead of x and walking all rows, for the column sums of gy: the bias gradient.  The list lengths are
+// on the device and very uneven (the centre tap has every row for a pair), so the units are laid end to end and each
+// persistent CTA takes an equal run of steps, whatever units it cuts: whole units are rounded and stored directly, the
+// cut ones leave their fp32 pieces, at most two per CTA, to a second launch that adds them up in a fixed order.  (Whole
+// units dealt out in turn left a quarter of the SMs' time idle.)  A unit's accumulator is drained while the next unit's
+// main loop fills the other one.
+//
+// Both operands are gathered rows in the MN-major 128-byte-swizzled layout (64 tokens x 64 channels = 8 KB blocks), so a
+// step of 128 x 256 copies 48 KB; what bounds the loop is the SM's path to L2 (48 KB in ~ 700 cycles against 512 cycles
+// of tensor work).
+#include "plan.cuh"
+#include "tc_common.cuh"
+
+namespace svtad {
+
+// Two warps fill a buffer, 32 of its 64 tokens each.  A warp gets a 512-byte cp.async out every 40 cycles or so however
+// many bytes are in flight (measured: 25 / 49 / 70 bytes per cycle and SM with 2 / 4 / 8 warps), so with four producers
+// a step of 48 KB took 1 780 cycles.
+constexpr int WP_A_WARPS = 8, WP_PER_BUF = 2, WP_GROUPS = WP_A_WARPS / WP_PER_BUF;
+constexpr int WP_THREADS = (WP_A_WARPS + 5) * 32;      // then the MMA warp (TMEM owner) and four epilogue warps
+constexpr int WP_MAX_KK = 49;
+constexpr int WP_MIN_RUN = 20;             // steps that pay for a CTA's start and its piece's trip through memory
+
+struct WgradUnits {
+    int m_blks, n_blks;                    // 128-channel blocks of x, BN-channel blocks of gy
+    int taps, bias;                        // bias: whether the bias gradient is asked for
+    int runs;                              // CTAs of the main launch
+};
+
+// the units' lengths and places in the end-to-end order, from the lists' lengths; made by every block (all threads call)
+struct UnitMap {
+    int len[WP_MAX_KK + 1];                // steps of a unit of the tap; [taps]: bias units
+    long base[WP_MAX_KK + 2];              // first step of the tap's units
+    int runs;                              // of about equal length, none below MIN_RUN steps
+    long run_len, run_rest;
+
+    __device__ void make(const WgradUnits& u, const PlanView& plan, long n) {
+        const int t = threadIdx.x;
+        if (t <= u.taps) len[t] = (int)(((t < u.taps ? (long)__ldg(plan.count + t) : u.bias ? n : 0) + STAGE_K - 1) / STAGE_K);
+        __syncthreads();
+        if (t <= u.taps + 1) {
+            long at = 0;
+            for (int k = 0; k < t; ++k) at += (long)len[k] * (k < u.taps ? u.m_blks * u.n_blks : u.n_blks);
+            base[t] = at;
+            if (t == u.taps + 1) {
+                runs = (int)(at / WP_MIN_RUN < 1 ? 1 : at / WP_MIN_RUN < u.runs ? at / WP_MIN_RUN : u.runs);
+                run_len = at / runs;
+                run_rest = at - run_len * runs;
+            }
+        }
+        __syncthreads();
+    }
+    // first step of a run; runs behind the last one are empty
+    __device__ long run_begin(int run) const { return run >= runs ? run_len * runs + run_rest : run * run_len + (run < run_rest ? run : run_rest); }
+    // the unit that step `pos` belongs to
+    __device__ void at(const WgradUnits& u, long pos, int& tap, int& unit, int& step) const {
+        int k = 0;
+        while (pos >= base[k + 1]) ++k;    // pos < total
+        const int off = (int)(pos - base[k]);
+        tap = k;
+        unit = off / len[k];
+        step = off - unit * len[k];
+    }
+};
+
+// four rounded values (two packed words) of a gradient, in 16 bits or as fp32
+__device__ __forceinline__ void store_quad(void* base, long at, uint32_t a, uint32_t b, bool fp16, bool out32) {
+    if (out32)
+        *reinterpret_cast<float4*>(static_cast<float*>(base) + at) =
+            make_float4(widen((uint16_t)(a & 0xffffu), fp16), widen((uint16_t)(a >> 16), fp16), widen((uint16_t)(b & 0xffffu), fp16),
+                        widen((uint16_t)(b >> 16), fp16));
+    else
+        *reinterpret_cast<uint2*>(static_cast<uint16_t*>(base) + at) = make_uint2(a, b);
+}
+
+template <int BN>
+__global__ void __launch_bounds__(WP_THREADS, 1)
+wgrad_pairs_kernel(const uint16_t* __restrict__ gy, const uint16_t* __restrict__ x, PlanView plan, void* __restrict__ gw,
+                   void* __restrict__ gb, float* __restrict__ pieces, long n, int cin, int cout, WgradUnits units, int nstage,
+                   int fp16, int out32, int* __restrict__ err) {
+    constexpr int B_TILE_BYTES = BN * 128;                 // 64 tokens x BN channels
+    constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
+    constexpr int TM_COLS = tmem_cols2_for(BN);
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    TmaTail* tail = reinterpret_cast<TmaTail*>(smem + (size_t)nstage * STAGE_BYTES);
+    __shared__ UnitMap map;
+    volatile int* s_abort = &tail->abort_flag;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t stage_base = smem_u32(smem);
+
+    if (warp == WP_A_WARPS) {
+        tmem_alloc(smem_u32(&tail->tmem_slot), TM_COLS);
+        tmem_relinquish();
+    }
+    if (tid == 0) {
+        for (int s = 0; s < nstage; ++s) {
+            mbar_init(smem_u32(&tail->full[s]), 32 * WP_PER_BUF);      // the copies of the warps that fill it
+            mbar_init(smem_u32(&tail->empty[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&tail->accum_full[b]), 1);
+            mbar_init(smem_u32(&tail->accum_empty[b]), 128);
+        }
+        tail->abort_flag = 0;
+        fence_mbar_init();
+    }
+    tc_fence_before();
+    map.make(units, plan, n);
+    tc_fence_after();
+    const uint32_t tmem_base = tail->tmem_slot;
+
+    // the CTA's run of steps, piece by piece: steps [s0, s1) of a unit
+    long pos = map.run_begin(blockIdx.x);
+    const long run_end = map.run_begin(blockIdx.x + 1);
+    int tap, m, nb, s0, s1;
+    auto next_piece = [&] {
+        if (pos >= run_end) return false;
+        int unit;
+        map.at(units, pos, tap, unit, s0);
+        m = tap < units.taps ? unit / units.n_blks : 0;
+        nb = unit - m * units.n_blks;
+        s1 = (int)(run_end - pos < map.len[tap] - s0 ? s0 + (run_end - pos) : map.len[tap]);
+        pos += s1 - s0;
+        return true;
+    };
+
+    if (warp < WP_A_WARPS) {
+        // ------------------------------------------------------------------ producers: two warps per step, groups in turn
+        const int sub = lane & 7, rg = lane >> 3;
+        const int grp = warp / WP_PER_BUF, part = warp % WP_PER_BUF;
+        const int n_prod = nstage < WP_GROUPS ? nstage : WP_GROUPS;      // never more groups than buffers (see the forward kernel)
+        bool alive = true;
+        int it0 = 0;
+        // the lane's place in the buffers: token itr * 4 + rg of the warp's 32, 16-byte chunk sub of each 64-channel block
+        const uint32_t lane_dst[2] = {(uint32_t)(part * 4096 + rg * 128 + ((sub ^ rg) << 4)), (uint32_t)(part * 4096 + rg * 128 + ((sub ^ (4 | rg)) << 4))};
+        while (alive && grp < n_prod && next_piece()) {
+            const bool ones = tap == units.taps;
+            const int count = ones ? (int)n : __ldg(plan.count + tap), steps = s1 - s0;
+            const int32_t* li = plan.pair_i + (long)tap * n + s0 * STAGE_K;
+            const int32_t* lj = plan.pair_j + (long)tap * n + s0 * STAGE_K;
+            const int left = count - s0 * STAGE_K;
+            // nothing is read behind the channels of a partial block
+            const uint16_t* xa = x + m * 128 + sub * 8;
+            const uint16_t* gb0 = gy + nb * BN + sub * 8;
+            const int x_left = cin - (m * 128 + sub * 8), g_left = cout - (nb * BN + sub * 8);
+            int st = ((grp - it0) % n_prod + n_prod) % n_prod;
+            int s = (it0 + st) % nstage;
+            uint32_t ph = (((it0 + st) / nstage) & 1) ^ 1;
+            it0 += steps;
+            int vi, vj;
+            auto entries = [&](int step) {                 // this lane's pair of a coming step
+                const int p = step * STAGE_K + part * 32 + lane;
+                const bool in = step < steps && p < left;
+                vi = in ? (ones ? s0 * STAGE_K + p : __ldg(li + p)) : -1;
+                vj = in && !ones ? __ldg(lj + p) : -1;
+            };
+            entries(st);
+            for (; st < steps; st += n_prod) {
+                int ri[8], rj[8];                           // the rows this lane's copies take
+#pragma unroll
+                for (int itr = 0; itr < 8; ++itr) {
+                    ri[itr] = __shfl_sync(0xffffffffu, vi, itr * 4 + rg);
+                    rj[itr] = __shfl_sync(0xffffffffu, vj, itr * 4 + rg);
+                }
+                entries(st + n_prod);
+                int ok = 1;
+                if (lane == 0) ok = mbar_wait(smem_u32(&tail->empty[s]), ph, s_abort, err, 61) ? 1 : 0;
+                if (!__shfl_sync(0xffffffffu, ok, 0)) { alive = false; break; }
+                __syncwarp();
+                const uint32_t a_tile = stage_base + (uint32_t)s * STAGE_BYTES;
+                const uint32_t bar = smem_u32(&tail->full[s]);
+                if (ones) {
+                    const uint32_t one = fp16 ? 0x3C003C00u : 0x3F803F80u;
+                    for (int c = lane; c < 512; c += 32)
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(a_tile + part * 4096 + (c & 255) * 16 + (c >> 8) * 8192), "r"(one) : "memory");
+                    fence_proxy_async();
+                } else if (x_left > 64) {
+#pragma unroll
+                    for (int itr = 0; itr < 8; ++itr) {
+                        const int j = rj[itr];
+                        const uint16_t* src = xa + (long)max(j, 0) * cin;
+                        const uint32_t dst = a_tile + lane_dst[itr & 1] + itr * 512, bytes = j < 0 ? 0u : 16u;
+                        cp_async16(dst, src, bytes);
+                        cp_async16(dst + 8192, src + 64, bytes);
+                    }
+                } else {
+#pragma unroll
+                    for (int itr = 0; itr < 8; ++itr) {
+                        const int j = x_left > 0 ? rj[itr] : -1;
+                        const uint32_t dst = a_tile + lane_dst[itr & 1] + itr * 512;
+                        cp_async16(dst, x_left > 0 ? xa + (long)max(j, 0) * cin : x, j < 0 ? 0u : 16u);
+                        cp_async16(dst + 8192, x, 0u);
+                    }
+                }
+#pragma unroll
+                for (int itr = 0; itr < 8; ++itr) {
+                    const int i = ri[itr];
+                    const uint32_t dst = a_tile + A_TILE_BYTES + lane_dst[itr & 1] + itr * 512, bytes = i < 0 ? 0u : 16u;
+                    const uint16_t* src = gb0 + (long)max(i, 0) * cout;
+                    if (g_left > BN - 64) {
+#pragma unroll
+                        for (int b = 0; b < BN / 64; ++b) cp_async16(dst + b * 8192, src + b * 64, bytes);
+                    } else {
+#pragma unroll
+                        for (int b = 0; b < BN / 64; ++b) cp_async16(dst + b * 8192, g_left > b * 64 ? src + b * 64 : gy, g_left > b * 64 ? bytes : 0u);
+                    }
+                }
+                cp_async_arrive_noinc(bar);
+                s += n_prod;
+                while (s >= nstage) { s -= nstage; ph ^= 1u; }
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp == WP_A_WARPS) {
+        // ------------------------------------------------------------------ MMA issuer (whole warp waits, one lane issues)
+        const uint32_t idesc = make_idesc(fp16 ? 0 : 1, 1, 1, TILE_M, BN);
+        bool alive = true;
+        int s = 0;
+        uint32_t ph = 0;
+        for (int local = 0; alive && next_piece(); ++local) {
+            const int buf = local & 1, steps = s1 - s0;
+            if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((local >> 1) & 1) ^ 1, s_abort, err, 62)) break;
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + buf * BN;
+            for (int st = 0; st < steps; ++st) {
+                if (!mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 63)) { alive = false; break; }
+                fence_proxy_async();       // cp.async (generic proxy) writes -> tcgen05.mma (async proxy) reads
+                tc_fence_after();
+                const uint32_t a_tile = stage_base + (uint32_t)s * STAGE_BYTES;
+                if (elect_one_sync()) {
+                    // both operands MN-major: 16 tokens per step = 2048 B, 64-channel blocks 8192 B apart
+                    const uint32_t a_lo = ((a_tile & 0x3FFFFu) >> 4) | smem_desc_lbo_bits(8192);
+                    const uint32_t b_lo = a_lo + (A_TILE_BYTES >> 4);
+                    umma_f16_lh(d_tmem, a_lo, smem_desc_hi(1024), b_lo, smem_desc_hi(1024), idesc, st != 0 ? 1u : 0u);
+#pragma unroll
+                    for (int ks = 1; ks < STAGE_K / 16; ++ks)
+                        umma_f16_lh_acc(d_tmem, a_lo + ks * 128, smem_desc_hi(1024), b_lo + ks * 128, smem_desc_hi(1024), idesc);
+                    umma_commit(smem_u32(&tail->empty[s]));
+                }
+                __syncwarp();
+                if (++s == nstage) { s = 0; ph ^= 1u; }
+            }
+            if (!alive) break;
+            if (elect_one_sync()) umma_commit(smem_u32(&tail->accum_full[buf]));
+            __syncwarp();
+        }
+    } else {
+        // ------------------------------------------------------------------ epilogue (the last four warps)
+        constexpr int NC = BN / 32;
+        const int q = warp & 3;
+        for (int local = 0; next_piece(); ++local) {
+            const int buf = local & 1;
+            int ok = 1;
+            if (lane == 0) ok = mbar_wait(smem_u32(&tail->accum_full[buf]), (local >> 1) & 1, s_abort, err, 64) ? 1 : 0;
+            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+            __syncwarp();
+            tc_fence_after();
+            const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN;
+            const int row = q * 32 + lane, ci = m * 128 + row, n0 = nb * BN;
+            const bool bias = tap == units.taps;
+            const bool mine = bias ? row == 0 : ci < cin;
+            // a whole unit goes to the gradient, a piece of a cut one to its place: 0 begins inside a unit, 1 ends there
+            float* part = nullptr;
+            if (s0 > 0 || s1 < map.len[tap])
+                part = pieces + (((long)blockIdx.x * 2 + (s0 > 0 ? 0 : 1)) * TILE_M + row) * BN;
+            void* out = bias ? gb : gw;
+            const long at = (bias ? 0 : ((long)tap * cin + ci) * cout) + n0;
+            uint32_t va[32], vb[32];
+            tmem_ld32(t_addr, va);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                uint32_t (&v)[32] = (c & 1) ? vb : va;
+                tmem_ld_wait();
+                if (c + 1 < NC) tmem_ld32(t_addr + (c + 1) * 32, (c & 1) ? va : vb);
+                if (!mine || n0 + c * 32 >= cout) continue;
+                if (part != nullptr) {
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) st_global_v8(part + c * 32 + g * 8, &v[g * 8]);
+                } else {
+                    uint32_t o[16];
+#pragma unroll
+                    for (int g = 0; g < 16; ++g) o[g] = pack2(__uint_as_float(v[2 * g]), __uint_as_float(v[2 * g + 1]), fp16 != 0);
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) store_quad(out, at + c * 32 + g * 4, o[2 * g], o[2 * g + 1], fp16 != 0, out32 != 0);
+                }
+            }
+            tc_fence_before();
+            mbar_arrive(smem_u32(&tail->accum_empty[buf]));
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == WP_A_WARPS) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc(tmem_base, TM_COLS);
+    }
+}
+
+constexpr int WP_STRIP = 4;
+
+// The cut units: grid.x = the boundaries between the runs; the first boundary inside a unit adds its pieces up in the
+// order of the runs, with one rounding.  grid.y = strips of WP_STRIP rows of the unit.  Blocks behind the boundaries clear
+// the gradient of taps that have no pair at all.
+template <int BN>
+__global__ void __launch_bounds__(256)
+wgrad_pairs_sum_kernel(const float* __restrict__ pieces, PlanView plan, void* __restrict__ gw, void* __restrict__ gb, long n,
+                       int cin, int cout, WgradUnits units, int fp16, int out32) {
+    __shared__ UnitMap map;
+    map.make(units, plan, n);
+    if ((int)blockIdx.x >= units.runs - 1) {
+        const int tap = (int)blockIdx.x - (units.runs - 1);
+        if (map.len[tap] > 0) return;
+        const long plane = (long)cin * cout;
+        for (long e = (blockIdx.y * 256l + threadIdx.x) * 4; e < plane; e += gridDim.y * 1024l)
+            store_quad(gw, tap * plane + e, 0u, 0u, fp16 != 0, out32 != 0);
+        return;
+    }
+    const int run = (int)blockIdx.x;
+    if (run + 1 >= map.runs) return;
+    const long cut = map.run_begin(run + 1);
+    int tap, unit, step;
+    map.at(units, cut, tap, unit, step);
+    if (step == 0) return;                                          // between two units
+    const long begin = cut - step, end = begin + map.len[tap];
+    if (begin < map.run_begin(run)) return;                         // an earlier boundary lies inside this unit, too
+    int parts = 2;
+    while (run + parts < map.runs && map.run_begin(run + parts) < end) ++parts;
+    const int m = tap < units.taps ? unit / units.n_blks : 0, nb = unit - m * units.n_blks;
+    const bool bias = tap == units.taps;
+    constexpr int QUADS = WP_STRIP * BN / 4;
+    for (int e = threadIdx.x; e < QUADS; e += 256) {
+        const int row = blockIdx.y * WP_STRIP + e / (BN / 4), col = (e % (BN / 4)) * 4, co = nb * BN + col;
+        if (co >= cout || (bias ? row > 0 : m * 128 + row >= cin)) continue;
+        // the first run ends in this unit (its second place), the others begin in it
+        const float* src = pieces + ((long)run * 2 * TILE_M + row) * BN + col;
+        float4 sum = __ldcg(reinterpret_cast<const float4*>(src + TILE_M * BN));
+#pragma unroll 8
+        for (int r = 1; r < parts; ++r) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(src + (long)r * 2 * TILE_M * BN));
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+        }
+        store_quad(bias ? gb : gw, (bias ? 0 : ((long)tap * cin + m * 128 + row) * cout) + co, pack2(sum.x, sum.y, fp16 != 0),
+                   pack2(sum.z, sum.w, fp16 != 0), fp16 != 0, out32 != 0);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------
+static WgradUnits pairs_units(int cin, int cout, int kk, bool with_bias) {
+    const int bn = tc_widest_bn(cout);
+    return WgradUnits{(cin + 127) / 128, (cout + bn - 1) / bn, kk, with_bias ? 1 : 0, tc_num_sms()};
+}
+
+size_t pairs_wgrad_ws_bytes(int cout) { return (size_t)tc_num_sms() * 2 * TILE_M * tc_widest_bn(cout) * sizeof(float); }
+
+// Worth it where the lists' third of the steps outweighs gathering gy's rows as well and padding the input channels to
+// blocks of 128 (C = 192 loses a quarter of each MMA).
+bool pairs_wgrad_wanted(int cin, int kk) { return kk >= 2 && (cin + 127) / 128 * 128 * 4 <= cin * 5; }
+
+template <int BN>
+static int launch_pairs(const void* gy, const void* x, const PlanView& plan, void* gw, void* gb, float* pieces, int64_t n, int cin,
+                        int cout, int kk, int fp16, int out32, cudaStream_t s) {
+    const WgradUnits u = pairs_units(cin, cout, kk, gb != nullptr);
+    const size_t stage = A_TILE_BYTES + (size_t)BN * 128;
+    int nstage = (int)((TC_SMEM_LIMIT - 1024 - sizeof(TmaTail) - sizeof(UnitMap) - 64) / stage);
+    if (nstage > 8) nstage = 8;
+    const size_t smem = 1024 + nstage * stage + sizeof(TmaTail);
+    auto kern = wgrad_pairs_kernel<BN>;
+    int rc = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem);
+    if (rc) return rc;
+    SV_CUDA(tc_launch(kern, dim3((unsigned)u.runs), dim3(WP_THREADS), smem, s, (const uint16_t*)gy, (const uint16_t*)x, plan, gw, gb,
+                      pieces, (long)n, cin, cout, u, nstage, fp16, out32, tc_error_ptr()));
+    SV_CUDA(tc_launch(wgrad_pairs_sum_kernel<BN>, dim3((unsigned)(u.runs - 1 + kk), TILE_M / WP_STRIP), dim3(256), 0, s, pieces, plan, gw,
+                      gb, (long)n, cin, cout, u, fp16, out32));
+    return SVTAD_OK;
+}
+
+int pairs_wgrad(const void* gy, const void* x, const void* plan, void* gw, void* gb, int64_t n, int cin, int cout, int kk,
+                int dtype, int grad_dtype, void* ws, size_t ws_bytes, cudaStream_t s) {
+    const size_t need = pairs_wgrad_ws_bytes(cout);
+    if (ws_bytes < need) return set_error(SVTAD_ERR_WORKSPACE, "svtad_conv_wgrad: workspace %zu < %zu bytes", ws_bytes, need);
+    PlanView view;
+    plan_layout(n, kk, plan, &view);
+    const int fp16 = dtype == SVTAD_F16, out32 = grad_dtype == SVTAD_F32;
+    float* pieces = static_cast<float*>(ws);
+    switch (tc_widest_bn(cout)) {
+        case 64: return launch_pairs<64>(gy, x, view, gw, gb, pieces, n, cin, cout, kk, fp16, out32, s);
+        case 128: return launch_pairs<128>(gy, x, view, gw, gb, pieces, n, cin, cout, kk, fp16, out32, s);
+        case 192: return launch_pairs<192>(gy, x, view, gw, gb, pieces, n, cin, cout, kk, fp16, out32, s);
+        default: return launch_pairs<256>(gy, x, view, gw, gb, pieces, n, cin, cout, kk, fp16, out32, s);
+    }
+}
+
+}  // namespace svtad

@@ -8,7 +8,7 @@
 // library's one-call backward without touching the interpreter.
 //
 // What is known about a neighbor table (symmetric by construction, indices local to a batch row or not, the device
-// status word of svtad_table_check, an int32 copy) is kept per tensor object and version; entries of dead tables are
+// status word of svtad_table_check, an int32 copy, the work plan of svtad_plan_build) is kept per tensor object and version; entries of dead tables are
 // swept whenever a new table is entered.
 #include <ATen/ATen.h>
 #include <ATen/autocast_mode.h>
@@ -72,8 +72,9 @@ void* mptr(Tensor& t) { return t.defined() && t.numel() ? t.data_ptr() : nullptr
 const int32_t* iptr(const Tensor& t) { return static_cast<const int32_t*>(ptr(t)); }
 
 // ------------------------------------------------------------------------------------------------ table facts
-// Landing places in pinned memory for status words on their way to the host: one page, allocated at the first use
-// (pinning memory takes milliseconds, so not once per table).  A place whose copy is still under way when its table
+// Landing places in pinned memory for what the device finds out about a table (a status word, the lengths of a plan's
+// lists) on its way to the host: one block, allocated at the first use (pinning memory takes milliseconds, so not once
+// per table).  A place whose copy is still under way when its table
 // dies is handed out again only after the copy has landed; when all are taken the caller does without.
 class HostWords {
   public:
@@ -103,15 +104,15 @@ class HostWords {
 
   private:
     bool make_page() {
-        constexpr int PLACES = 64;
-        if (cudaHostAlloc(&page_, PLACES * 64, cudaHostAllocPortable) != cudaSuccess) {
+        constexpr int PLACES = 128, BYTES = 256;
+        if (cudaHostAlloc(&page_, PLACES * BYTES, cudaHostAllocPortable) != cudaSuccess) {
             (void)cudaGetLastError();
             page_ = nullptr;
             return false;
         }
         for (int i = 0; i < PLACES; ++i) {
             Place p;
-            p.word = reinterpret_cast<volatile int32_t*>(static_cast<char*>(page_) + 64 * i);
+            p.word = reinterpret_cast<volatile int32_t*>(static_cast<char*>(page_) + BYTES * i);
             if (cudaEventCreateWithFlags(&p.copied, cudaEventDisableTiming) == cudaSuccess) free_.push_back(p);
         }
         return true;
@@ -138,11 +139,18 @@ struct Facts {
     Tensor status;               // device word of svtad_table_check
     HostWords::Place host;       // where its copy on the host arrives
     Tensor i32;                  // contiguous, aligned int32 form of a table of another kind
+    int64_t plan_tpb = -1;       // tokens_per_batch the plan below belongs to
+    void* plan_stream = nullptr;
+    HostWords::Place plan_host;  // where the lengths of its lists arrive on the host
+    double density = -1;         // pairs per row and tap, once they have arrived
+    bool full_grid = false;      // svtad_table_init's: hardly a neighbor missing
+    Tensor plan;                 // svtad_plan_build's, shared by the layers that use the table on that stream
     std::mutex mu;               // guards everything below `version`
 
     explicit Facts(const Tensor& t) : owner(t.getIntrusivePtr()), version(t._version()), device(t.get_device()) {}
     ~Facts() {
         if (host.word) host_words(device).give_back(host);
+        if (plan_host.word) host_words(device).give_back(plan_host);
     }
 };
 
@@ -175,10 +183,11 @@ FactStore& store() {
     return *s;
 }
 
-void mark_symmetric(const Tensor& t, bool built) {
+void mark_symmetric(const Tensor& t, bool built, bool full_grid = false) {
     if (auto f = store().find(t, true)) {
         f->symmetric = true;
         f->built = built;
+        f->full_grid = full_grid;
     }
 }
 
@@ -253,6 +262,54 @@ Tensor int32_table(const Tensor& table) {
     return f->i32;
 }
 
+// The table's work plan for a layer that wants one, else an undefined tensor, and which parts of it the layer should use.
+// Made once per table; under graph capture it belongs to the call (its contents are there only when the graph runs).  How
+// many neighbors are there is known to the host only once the lists' lengths have come back: the call that makes a plan
+// takes the sparse case for granted.
+constexpr int USE_ROWS = 1, USE_PAIRS = 2;
+struct Plan {
+    Tensor data;
+    int use = 0;
+};
+Plan plan_for(const Tensor& table, const Tensor& nbr, int64_t n, int cin, int cout, int kk, int code, int64_t tpb, void* stream) {
+    Plan p;
+    const int wanted = svtad_plan_wanted(n, cin, cout, kk, code, -1.0);
+    if (!wanted) return p;
+    auto make = [&] {
+        Tensor plan = empty_on({static_cast<int64_t>(svtad_plan_bytes(n, kk))}, at::kByte, nbr.device());
+        check(svtad_plan_build(iptr(nbr), n, kk, static_cast<int>(tpb), plan.data_ptr(), stream));
+        return plan;
+    };
+    auto f = store().find(table, true);
+    if (!f) return Plan{make(), wanted};
+    if (auto s = symmetric_facts(table); s && s->full_grid) return p;
+    std::lock_guard<std::mutex> hold(f->mu);
+    if (!(f->plan_tpb == tpb && f->plan_stream == stream && f->plan.defined())) {
+        Tensor plan = make();
+        if (capturing(stream)) return Plan{plan, wanted};
+        f->plan = plan;
+        f->plan_stream = stream;
+        f->plan_tpb = tpb;
+        f->density = -1;
+        if (f->plan_host.word || host_words(f->device).take(f->plan_host)) {
+            C10_CUDA_CHECK(cudaMemcpyAsync(const_cast<int32_t*>(f->plan_host.word), svtad_plan_counts(plan.data_ptr(), n, kk),
+                                           kk * sizeof(int32_t), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)));
+            C10_CUDA_CHECK(cudaEventRecord(f->plan_host.copied, static_cast<cudaStream_t>(stream)));
+        }
+    } else if (f->density < 0 && f->plan_host.word && !capturing(stream)) {
+        if (cudaEventQuery(f->plan_host.copied) == cudaSuccess) {
+            double pairs = 0;
+            for (int k = 0; k < kk; ++k) pairs += f->plan_host.word[k];
+            f->density = pairs / (static_cast<double>(n) * kk);
+        } else {
+            (void)cudaGetLastError();
+        }
+    }
+    p.use = svtad_plan_wanted(n, cin, cout, kk, code, f->density);
+    if (p.use) p.data = f->plan;
+    return p;
+}
+
 // tokens_per_batch of a call on [B, N, C] features: N when the table's indices are local to each batch row, else 0.
 // Reference heuristic (sparse_conv_layer.py:170-177): local iff max(table) < N.  It needs the table's values, so it is
 // evaluated once per table object; with one batch row the two readings agree, and a table this package built over all
@@ -297,6 +354,7 @@ struct SparseConvBackward : public torch::autograd::Node {
     Dims d;
     at::ScalarType w_dtype, b_dtype;                     // of the parameters
     Tensor status;
+    Plan plan;
     bool released = false;
 
     std::string name() const override { return "SparseConv2dBackward"; }
@@ -306,6 +364,7 @@ struct SparseConvBackward : public torch::autograd::Node {
         x.reset_data();
         table.reset_data();
         weight.reset_data();
+        plan = Plan();
         released = true;
     }
 
@@ -342,7 +401,8 @@ struct SparseConvBackward : public torch::autograd::Node {
         const size_t bytes = need_w || st.defined() ? svtad_workspace_bytes(op, d.n, d.cin, d.cout, d.kk, code) : 0;
         if (bytes) ws = empty_on({static_cast<int64_t>(bytes)}, at::kByte, dev);
         check(svtad_conv_bwd_typed(ptr(gy), ptr(xc), iptr(nbr), ptr(wc), mptr(gx), mptr(gw), mptr(gb), d.n, d.cin, d.cout,
-                                   d.kk, static_cast<int>(d.tpb), code, dtype_code(gdt), iptr(st), mptr(ws), bytes, stream));
+                                   d.kk, static_cast<int>(d.tpb), code, dtype_code(gdt), ptr(plan.data), plan.use, iptr(st),
+                                   mptr(ws), bytes, stream));
         out[0] = gx;
         if (task_should_compute_output(1)) out[1] = gw.scalar_type() == w_dtype ? gw : gw.to(w_dtype);
         if (need_b) out[2] = gb.scalar_type() == b_dtype ? gb : gb.to(b_dtype);
@@ -374,6 +434,7 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
     const bool grad = at::GradMode::is_enabled() &&
                       (x.requires_grad() || weight.requires_grad() || (bias.defined() && bias.requires_grad()));
     Tensor y, nbr, status;
+    Plan plan;
     {
         at::NoGradGuard no_grad;
         d.tpb = batched ? tokens_per_batch(table, x.size(0), x.size(1), d.kk, local) : 0;
@@ -386,8 +447,9 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
             y = empty_on({d.n, d.cout}, dt, dev);
         }
         if (grad && x.requires_grad()) status = status_for(table, nbr, d.n, d.kk, d.tpb, stream);
-        check(svtad_conv_fwd(ptr(xc), iptr(nbr), ptr(wc), ptr(bc), mptr(y), d.n, d.cin, d.cout, d.kk,
-                             static_cast<int>(d.tpb), code, nullptr, 0, stream));
+        plan = plan_for(table, nbr, d.n, d.cin, d.cout, d.kk, code, d.tpb, stream);
+        check(svtad_conv_fwd_planned(ptr(xc), iptr(nbr), ptr(wc), ptr(bc), mptr(y), d.n, d.cin, d.cout, d.kk,
+                                     static_cast<int>(d.tpb), code, plan.use & USE_ROWS ? ptr(plan.data) : nullptr, stream));
     }
     if (grad) {
         auto node = std::shared_ptr<SparseConvBackward>(new SparseConvBackward(), torch::autograd::deleteNode);
@@ -396,6 +458,7 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
         node->w_dtype = weight.scalar_type();
         node->b_dtype = bias.defined() ? bias.scalar_type() : dt;
         node->status = status;
+        node->plan = plan;
         node->x = torch::autograd::SavedVariable(x, false);
         node->table = torch::autograd::SavedVariable(table, false);
         node->weight = torch::autograd::SavedVariable(weight_c, false);
@@ -415,7 +478,7 @@ Tensor table_init(int64_t B, int64_t T, int64_t h, int64_t w, int64_t ksize, at:
     Tensor out = empty_on({B, T * h * w, ksize * ksize}, at::kInt, dev);
     check(svtad_table_init(static_cast<int>(B), static_cast<int>(T), static_cast<int>(h), static_cast<int>(w),
                            static_cast<int>(ksize), static_cast<int32_t*>(mptr(out)), stream_of(dev)));
-    mark_symmetric(out, true);
+    mark_symmetric(out, true, true);
     return out;
 }
 

@@ -284,6 +284,7 @@ int tc_make_map_sw(CUtensorMap* map, int rank, const void* base, const uint64_t*
                    int swizzle_bytes);
 // column-block width of a forward / dgrad CTA for an output of `cn` columns and `m_tiles` row tiles
 int tc_pick_bn(int cn, long m_tiles);
+int tc_widest_bn(int cn);
 struct WgradPlan {
     int bn, n_nblk, n_pairs, splits, ones_block;
     long tokens_per_split;
