@@ -517,20 +517,9 @@ static int launch_conv_f32(const ConvArgs& p, const int32_t* status, int bm, int
     if (rc) return rc;
     const int cn = DGRAD ? p.cin : p.cout, cred = DGRAD ? p.cout : p.cin;
     const int tiles_m = (int)((p.n + bm - 1) / bm), tiles_n = (cn + F_BN - 1) / F_BN;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles_m * tiles_n * G));
-    cfg.blockDim = dim3(F_THREADS);
-    cfg.dynamicSmemBytes = conv_f32_smem(bm, p.kk);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = G;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = G > 1 ? 1 : 0;
-    SV_CUDA(cudaLaunchKernelEx(&cfg, kern, (const float*)p.a, p.nbr, (const float*)p.w, (const float*)p.bias, (float*)p.out,
-                               status, (long)p.n, cred, cn, p.cin, p.cout, p.kk, p.tpb, tiles_n, bm, G));
+    SV_CUDA(launch_plain(kern, dim3((unsigned)(tiles_m * tiles_n * G)), dim3(F_THREADS), conv_f32_smem(bm, p.kk), s, G,
+                         (const float*)p.a, p.nbr, (const float*)p.w, (const float*)p.bias, (float*)p.out, status, (long)p.n, cred,
+                         cn, p.cin, p.cout, p.kk, p.tpb, tiles_n, bm, G));
     return SVTAD_OK;
 }
 

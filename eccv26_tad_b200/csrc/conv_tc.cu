@@ -326,6 +326,8 @@ template <bool OUT32>
 __global__ void __launch_bounds__(256)
 wgrad_reduce4_kernel(const float* __restrict__ ws_w, int splits, const float* __restrict__ ws_b, int splits_b,
                      void* __restrict__ gw, void* __restrict__ gb, long n_w, int cout, int fp16) {
+    pdl_wait();
+    pdl_trigger();
     long e = (blockIdx.x * (long)blockDim.x + threadIdx.x) * 4;
     const float* src;
     void* base;
@@ -360,8 +362,8 @@ wgrad_reduce4_kernel(const float* __restrict__ ws_w, int splits, const float* __
 int tc_wgrad_reduce_launch(const float* ws_w, int splits, const float* ws_b, int splits_b, void* gw, void* gb,
                            long n_w, int cout, int fp16, bool out32, cudaStream_t s) {
     long total4 = (n_w + (gb ? cout : 0) + 3) / 4;
-    SV_CUDA(tc_launch(out32 ? wgrad_reduce4_kernel<true> : wgrad_reduce4_kernel<false>,
-                      dim3((unsigned)((total4 + 255) / 256)), dim3(256), 0, s, ws_w, splits, ws_b, splits_b, gw, gb, n_w,
+    SV_CUDA(launch_pdl(out32 ? wgrad_reduce4_kernel<true> : wgrad_reduce4_kernel<false>,
+                      dim3((unsigned)((total4 + 255) / 256)), dim3(256), 0, s, 1, ws_w, splits, ws_b, splits_b, gw, gb, n_w,
                       cout, fp16));
     return SVTAD_OK;
 }

@@ -36,15 +36,8 @@ constexpr int HY_THREADS = 288;    // warps 0-3 producers, warp 4 MMA + TMEM own
 constexpr int A_WARPS = 4;
 constexpr int A_THREADS = A_WARPS * 32;
 // forward / dgrad: producer warps, then the MMA warp, then four epilogue warps
-#ifndef SV_FW_A_WARPS
-#define SV_FW_A_WARPS 4
-#endif
-constexpr int FW_A_WARPS = SV_FW_A_WARPS;
-// warps that share the fill of one buffer
-#ifndef SV_FW_NPW
-#define SV_FW_NPW 1
-#endif
-constexpr int FW_NPW = SV_FW_NPW;
+constexpr int FW_A_WARPS = 8;
+constexpr int FW_NPW = 2;                    // warps that share the fill of one buffer (four by themselves: 1 to 3 % slower)
 constexpr int FW_GROUPS = FW_A_WARPS / FW_NPW;
 constexpr int FW_ITR = 32 / FW_NPW;          // 4-row copy iterations per lane and buffer
 constexpr int FW_A_THREADS = FW_A_WARPS * 32;
@@ -74,7 +67,10 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
                    uint16_t* __restrict__ out, const int32_t* __restrict__ status, long n, int cred, int cn,
                    int kk, int tpb, int nstage, int fp16, int m_tiles, int n_blks, int out_al32, PlanView plan,
                    int* __restrict__ err) {
-    if (DGRAD && status != nullptr && (__ldg(status) & SVTAD_TABLE_ASYMMETRIC)) return;
+    if (DGRAD && status != nullptr) {
+        pdl_wait();
+        if (__ldg(status) & SVTAD_TABLE_ASYMMETRIC) return;
+    }
     constexpr int B_TILE_BYTES = b_tile_bytes_for(BN);
     constexpr int B_TX_BYTES = DGRAD ? BN * 128 : B_TILE_BYTES;
     constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
@@ -123,11 +119,13 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
         const uint32_t dst = smem_u32(s_tab);
         if constexpr (PLAN) {
             // a row per thread, four bytes at a time: the rows lie anywhere
-            const int i = __ldg(plan.order + (long)tile * TILE_M + tid);
-            s_row[tid] = i;
-            const int32_t* src = nbr + (long)(i < 0 ? 0 : i) * kk;
-            for (int k = 0; k < kk; ++k)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (tid * kk + k) * 4), "l"(src + k) : "memory");
+            if (tid < TILE_M) {
+                const int i = __ldg(plan.order + (long)tile * TILE_M + tid);
+                s_row[tid] = i;
+                const int32_t* src = nbr + (long)(i < 0 ? 0 : i) * kk;
+                for (int k = 0; k < kk; ++k)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (tid * kk + k) * 4), "l"(src + k) : "memory");
+            }
             cp_async_commit();
             return;
         }
@@ -143,16 +141,17 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
         cp_async_commit();
         if (tid == FW_A_THREADS - 1) l2_prefetch_rows(a, row0 - 64, row0 + TILE_M + 64, n, cred);
     };
-    // the first tile's rows start their trip before anything else is set up
-    {
+    // the first tile's rows start their trip while the MMA warp sets the rest up
+    if (warp < FW_A_WARPS) {
         int tile, blk;
-        if (warp < FW_A_WARPS && item(0, tile, blk)) load_table(tile);
+        pdl_wait();
+        if (item(0, tile, blk)) load_table(tile);
     }
     if (warp == FW_A_WARPS) {
         tmem_alloc(smem_u32(&tail->tmem_slot), TM_COLS);
         tmem_relinquish();
     }
-    if (tid == 0) {
+    if (tid == FW_A_WARPS * 32) {
         for (int b = 0; b < nbig; ++b) {
             mbar_init(smem_u32(&tail->full[b]), (FW_NPW * 32 + 1) * RB);    // per buffer: the copies of the lanes that fill it + the TMA byte-count arrival
             mbar_init(smem_u32(&tail->empty[b]), 1);
@@ -169,6 +168,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tail->tmem_slot;
+    pdl_trigger();
 
     if (warp < FW_A_WARPS) {
         // ------------------------------------------------------------------ producers
@@ -446,7 +446,8 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
         }
         cp_async_commit();     // one group per own step, empty or not: the wait below counts groups
     };
-    // the first steps' entries start their trip before anything else is set up
+    // the first steps' entries start their trip while the MMA warp sets the rest up
+    if (warp < A_WARPS) pdl_wait();
     if (warp < n_prod) {
 #pragma unroll
         for (int own = 0; own < WG_PF; ++own) load_entries(own);
@@ -459,7 +460,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
         tmem_alloc(smem_u32(&tail->tmem_slot), TM_COLS);
         tmem_relinquish();
     }
-    if (tid == 0) {
+    if (tid == 4 * 32) {
         for (int s = 0; s < nstage; ++s) {
             mbar_init(smem_u32(&tail->full[s]), 33);     // the owning warp's 32 copy arrivals + the TMA byte count
             mbar_init(smem_u32(&tail->empty[s]), 1);
@@ -473,6 +474,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tail->tmem_slot;
+    pdl_trigger();
 
     if (warp < A_WARPS) {
         // ------------------------------------------------------------------ producers
@@ -659,7 +661,7 @@ static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStre
     int grid = (int)(tiles < sms ? tiles : sms);
     PlanView view{};
     if (PLAN) plan_layout(p.n, p.kk, p.plan, &view);
-    SV_CUDA(tc_launch(kern, dim3(grid), dim3(FW_THREADS), smem, s, map_w, (const uint16_t*)p.a, p.nbr,
+    SV_CUDA(launch_pdl(kern, dim3(grid), dim3(FW_THREADS), smem, s, 1, map_w, (const uint16_t*)p.a, p.nbr,
                       (const uint16_t*)p.bias, (uint16_t*)p.out, status, (long)p.n, cred, cn, p.kk, p.tpb, nstage, fp16,
                       m_tiles, n_blks, (reinterpret_cast<uintptr_t>(p.out) % 32 == 0) ? 1 : 0, view, tc_error_ptr()));
     return SVTAD_OK;
@@ -711,7 +713,7 @@ static int launch_wgrad_hybrid(const void* gy, const void* x, const int32_t* nbr
     dim3 grid((unsigned)(pl.n_pairs * pl.n_nblk), (unsigned)pl.splits);
     auto kern = wgrad_hybrid_kernel<BN>;
     { int rc_s = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem); if (rc_s) return rc_s; }
-    SV_CUDA(tc_launch(kern, grid, dim3(HY_THREADS), smem, s, map_gy, (const uint16_t*)x, nbr, ws_w, ws_b, (long)n, cin, cout, kk, tpb, pl.tokens_per_split,
+    SV_CUDA(launch_pdl(kern, grid, dim3(HY_THREADS), smem, s, 1, map_gy, (const uint16_t*)x, nbr, ws_w, ws_b, (long)n, cin, cout, kk, tpb, pl.tokens_per_split,
                       pl.n_nblk, nstage, fp16, pl.ones_block, tc_error_ptr()));
     return SVTAD_OK;
 }

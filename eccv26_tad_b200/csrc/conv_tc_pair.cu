@@ -120,7 +120,10 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                  uint16_t* __restrict__ out, const int32_t* __restrict__ status, long n, int cred, int cn,
                  int kk, int tpb, int nstage, int fp16, int m_pairs, int n_blks, int out_al32, int* __restrict__ err) {
     // uniform over the whole grid, so both CTAs of a pair leave together
-    if (DGRAD && status != nullptr && (__ldg(status) & SVTAD_TABLE_ASYMMETRIC)) return;
+    if (DGRAD && status != nullptr) {
+        pdl_wait();
+        if (__ldg(status) & SVTAD_TABLE_ASYMMETRIC) return;
+    }
     constexpr int HALF = BN / 2;                  // columns of B this CTA stages
     constexpr int B_BYTES = HALF * 128;           // 64 K x HALF columns x 2 bytes, either layout
     constexpr int STAGE_BYTES = A_TILE_BYTES + B_BYTES;
@@ -168,13 +171,16 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
         // L2 prefetch of the rows this tile will gather (see the one-CTA kernel)
         if (tid == PR_A_THREADS - 1) l2_prefetch_rows(a, row0 - 64, row0 + TILE_M + 64, n, cred);
     };
-    // the first tile's rows start their trip before anything else is set up
-    if (warp < PR_A_WARPS && cid < items_total) load_table(cid);
+    // the first tile's rows start their trip while the MMA warp sets the rest up
+    if (warp < PR_A_WARPS) {
+        pdl_wait();
+        if (cid < items_total) load_table(cid);
+    }
     if (warp == 4) {
         tmem_alloc_pair(smem_u32(&tail->tmem_slot), TM_COLS);
         tmem_relinquish_pair();
     }
-    if (tid == 0) {
+    if (tid == 4 * 32) {
         for (int b = 0; b < nbig; ++b) {
             mbar_init(smem_u32(&tail->full[b]), rank == 0 ? 67 : 66);   // two halves x (32 copies + TMA), + the relay
             mbar_init(smem_u32(&tail->empty[b]), 1);
@@ -192,6 +198,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
     cluster_barrier();          // both CTAs' barriers exist before anyone arrives on the other's
     tc_fence_after();
     const uint32_t tmem_base = tail->tmem_slot;
+    pdl_trigger();
 
     if (warp < PR_A_WARPS) {
         // ------------------------------------------------------------------ producers (both CTAs)
@@ -419,21 +426,9 @@ static int launch_conv_pair(const ConvArgs& p, const int32_t* status, cudaStream
     const long items = (long)m_pairs * n_blks;
     const long max_clusters = tc_num_sms() / 2;
     const int clusters = (int)(items < max_clusters ? items : max_clusters);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(2 * clusters));
-    cfg.blockDim = dim3(PR_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    SV_CUDA(cudaLaunchKernelEx(&cfg, kern, map_w, (const uint16_t*)p.a, p.nbr, (const uint16_t*)p.bias,
-                               (uint16_t*)p.out, status, (long)p.n, cred, cn, p.kk, p.tpb, nstage, fp16, m_pairs,
-                               n_blks, (reinterpret_cast<uintptr_t>(p.out) % 32 == 0) ? 1 : 0, tc_error_ptr()));
+    SV_CUDA(launch_pdl(kern, dim3((unsigned)(2 * clusters)), dim3(PR_THREADS), smem, s, 2, map_w, (const uint16_t*)p.a, p.nbr,
+                       (const uint16_t*)p.bias, (uint16_t*)p.out, status, (long)p.n, cred, cn, p.kk, p.tpb, nstage, fp16, m_pairs,
+                       n_blks, (reinterpret_cast<uintptr_t>(p.out) % 32 == 0) ? 1 : 0, tc_error_ptr()));
     return SVTAD_OK;
 }
 

@@ -113,9 +113,11 @@ wgrad_pairs_kernel(const uint16_t* __restrict__ gy, const uint16_t* __restrict__
         fence_mbar_init();
     }
     tc_fence_before();
+    pdl_wait();
     map.make(units, plan, n);
     tc_fence_after();
     const uint32_t tmem_base = tail->tmem_slot;
+    pdl_trigger();
 
     // the CTA's run of steps, piece by piece: steps [s0, s1) of a unit
     long pos = map.run_begin(blockIdx.x);
@@ -315,6 +317,8 @@ __global__ void __launch_bounds__(256)
 wgrad_pairs_sum_kernel(const float* __restrict__ pieces, PlanView plan, void* __restrict__ gw, void* __restrict__ gb, long n,
                        int cin, int cout, WgradUnits units, int fp16, int out32) {
     __shared__ UnitMap map;
+    pdl_wait();
+    pdl_trigger();
     map.make(units, plan, n);
     if ((int)blockIdx.x >= units.runs - 1) {
         const int tap = (int)blockIdx.x - (units.runs - 1);
@@ -378,9 +382,9 @@ static int launch_pairs(const void* gy, const void* x, const PlanView& plan, voi
     auto kern = wgrad_pairs_kernel<BN>;
     int rc = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem);
     if (rc) return rc;
-    SV_CUDA(tc_launch(kern, dim3((unsigned)u.runs), dim3(WP_THREADS), smem, s, (const uint16_t*)gy, (const uint16_t*)x, plan, gw, gb,
+    SV_CUDA(launch_pdl(kern, dim3((unsigned)u.runs), dim3(WP_THREADS), smem, s, 1, (const uint16_t*)gy, (const uint16_t*)x, plan, gw, gb,
                       pieces, (long)n, cin, cout, u, nstage, fp16, out32, tc_error_ptr()));
-    SV_CUDA(tc_launch(wgrad_pairs_sum_kernel<BN>, dim3((unsigned)(u.runs - 1 + kk), TILE_M / WP_STRIP), dim3(256), 0, s, pieces, plan, gw,
+    SV_CUDA(launch_pdl(wgrad_pairs_sum_kernel<BN>, dim3((unsigned)(u.runs - 1 + kk), TILE_M / WP_STRIP), dim3(256), 0, s, 1, pieces, plan, gw,
                       gb, (long)n, cin, cout, u, fp16, out32));
     return SVTAD_OK;
 }

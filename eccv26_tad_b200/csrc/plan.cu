@@ -204,6 +204,8 @@ plan_kernel(const int32_t* __restrict__ nbr, long n, int kk, int tpb, PlanRing r
     extern __shared__ __align__(16) unsigned char p_smem[];
     __shared__ int s_w[PLAN_WARPS + 1];
     const int job = blockIdx.x / PLAN_G;
+    pdl_wait();
+    pdl_trigger();
     if (job == 0) sort_rows(nbr, n, kk, ring, o, *reinterpret_cast<SortSmem*>(p_smem), s_w);      // the longest first
     else list_tap(nbr, n, kk, tpb, job - 1, o, s_w);
 }
@@ -249,18 +251,7 @@ extern "C" int svtad_plan_build(const int32_t* nbr, int64_t n, int kk, int token
         SV_CUDA(cudaFuncSetAttribute(plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem)));
         ready.fetch_or(bit);
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((kk + 1) * PLAN_G));
-    cfg.blockDim = dim3(PLAN_THREADS);
-    cfg.dynamicSmemBytes = sizeof(SortSmem);
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = PLAN_G;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    SV_CUDA(cudaLaunchKernelEx(&cfg, plan_kernel, nbr, (long)n, kk, tokens_per_batch, ring, o));
+    SV_CUDA(launch_pdl(plan_kernel, dim3((unsigned)((kk + 1) * PLAN_G)), dim3(PLAN_THREADS), sizeof(SortSmem),
+                       (cudaStream_t)stream, PLAN_G, nbr, (long)n, kk, tokens_per_batch, ring, o));
     return SVTAD_OK;
 }

@@ -20,11 +20,18 @@ __device__ __forceinline__ uint32_t score_key(float f) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
+// a score with that key (the canonical one of those that share it)
+__device__ __forceinline__ float key_score(uint32_t key) {
+    return __uint_as_float((key & 0x80000000u) ? key & 0x7FFFFFFFu : ~key);
+}
+
 // ------------------------------------------------------------------------------------------
 // init
 // ------------------------------------------------------------------------------------------
 __global__ void table_init_kernel(int32_t* __restrict__ table, long total, int hw, int h, int w,
                                   int ksize, int kk) {
+    pdl_wait();
+    pdl_trigger();
     long f0 = (long)(blockIdx.x * (long)blockDim.x + threadIdx.x) * 4;
     if (f0 >= total) return;
     int r = ksize >> 1;
@@ -74,7 +81,7 @@ table_build_warp_kernel(const float* __restrict__ scores, int n_seg, int L, int 
     constexpr int CAP = ITEMS * 32;
     constexpr int KKMAX = (KS > 0) ? KS * KS : 49;
     __shared__ int16_t s_rank[WARPS][CAP];
-    __shared__ uint32_t s_pos[WARPS][CAP];
+    __shared__ int16_t s_pos[WARPS][CAP];
     constexpr int RR = (KS > 0 && KS <= 5) ? 32 : 8;   // kept tokens whose rows are staged per round
     __shared__ int32_t s_out[WARPS][RR * KKMAX];     // staged table rows, written out with coalesced stores
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -89,59 +96,93 @@ table_build_warp_kernel(const float* __restrict__ scores, int n_seg, int L, int 
         int e = j * 32 + lane;
         key[j] = (e < L) ? score_key(__ldg(sc + e)) : 0u;   // 0 is below every real key
     }
-    // Threshold search, bit by bit from the top: T grows while count(key >= T) >= k.  As soon as the count
-    // is exactly k the kept set {key >= T} is decided and the remaining bits are skipped; if it never is
-    // (ties at the boundary) all 32 bits are walked and T ends as the k-th largest key.
+    // Threshold search between lo (at least k keys are >= lo) and hi (fewer are >= hi).  Of four candidates two come by
+    // interpolation between the counts on the scores' own scale, one halves the interval on that scale and one on the
+    // keys', which bounds the search for any input: 8 rounds for N(0,1) scores, 11 for softmax-like ones, where bit by
+    // bit took 19.  Once a candidate splits off exactly k keys the kept set {key >= lo} is decided; if none does
+    // (ties at the boundary) lo ends as the k-th largest key.
     uint32_t T = 0;
+    bool decided = L == k;
     if (L != k) {
-#pragma unroll 1
-        for (int bit = 31; bit >= 0; --bit) {
-            uint32_t cand = T | (1u << bit);
+        uint32_t lo = 0, hi = 0xFFFFFFFFu, mx = 0;
+        int n_lo = L, n_hi = 0;
+        {
+            uint32_t mn = 0xFFFFFFFFu;
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) {
+                mx = max(mx, key[j]);
+                if (j * 32 + lane < L) mn = min(mn, key[j]);
+            }
+            lo = __reduce_min_sync(0xffffffffu, mn);
+            mx = __reduce_max_sync(0xffffffffu, mx);
+        }
+        if (mx == 0xFFFFFFFFu) {          // NaNs: they are kept first
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) n_hi += key[j] == mx;
+            n_hi = __reduce_add_sync(0xffffffffu, n_hi);
+            if (n_hi >= k) lo = mx;
+        } else {
+            hi = mx + 1;
+        }
+        for (int round = 0; hi - lo > 1; ++round) {
+            uint32_t cand = lo + (hi - lo) / 2;
+            if ((round & 3) != 3) {
+                const float f_lo = key_score(lo), f_hi = key_score(hi);
+                const float at = (round & 3) == 2 ? 0.5f : __fdividef((float)(n_lo - k) + 0.5f, (float)(n_lo - n_hi));
+                const uint32_t by_value = score_key(f_lo + (f_hi - f_lo) * at);
+                if (by_value > lo && by_value < hi) cand = by_value;       // not for an infinite or NaN value
+            }
             int c = 0;
 #pragma unroll
             for (int j = 0; j < ITEMS; ++j) c += (key[j] >= cand);
             c = __reduce_add_sync(0xffffffffu, c);
-            if (c >= k) {
-                T = cand;
-                if (c == k) break;
-            }
+            if (c >= k) { lo = cand; n_lo = c; } else { hi = cand; n_hi = c; }
+            if (c == k) { decided = true; break; }
         }
+        T = lo;
     }
-    int gt = 0;
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) gt += (key[j] > T);
-    gt = __reduce_add_sync(0xffffffffu, gt);
-    const int need_ties = k - gt;   // >= 1 ties at the threshold are kept, lowest index first
 
-    const int hw = h * w;
-    int run_tie = 0, run_keep = 0;
+    int run_keep = 0;
+    if (decided) {
+        unsigned km[ITEMS];
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        int e = j * 32 + lane;
-        bool valid = e < L;
-        bool eq = valid && key[j] == T;
-        bool g = valid && key[j] > T;
-        unsigned eqm = __ballot_sync(0xffffffffu, eq);
-        int tie_rank = run_tie + __popc(eqm & lt);
-        bool keep = g || (eq && tie_rank < need_ties);
-        unsigned km = __ballot_sync(0xffffffffu, keep);
-        int rank = run_keep + __popc(km & lt);
-        if (valid) s_rank[wid][e] = keep ? (int16_t)rank : (int16_t)-1;
-        if (keep) {
-            int p = (hw == 1) ? 0 : e - div_magic(e, magic_hw) * hw;
-            int y = (w == 1) ? p : div_magic(p, magic_w), x = p - y * w;
-            s_pos[wid][rank] = (uint32_t)e | ((uint32_t)y << 16) | ((uint32_t)x << 24);
+        for (int j = 0; j < ITEMS; ++j) km[j] = __ballot_sync(0xffffffffu, j * 32 + lane < L && key[j] >= T);
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const int e = j * 32 + lane, rank = run_keep + __popc(km[j] & lt);
+            const bool keep = (km[j] >> lane) & 1u;
+            if (e < L) s_rank[wid][e] = keep ? (int16_t)rank : (int16_t)-1;
+            if (keep) s_pos[wid][rank] = (int16_t)e;
+            run_keep += __popc(km[j]);
         }
-        run_tie += __popc(eqm);
-        run_keep += __popc(km);
+    } else {
+        int gt = 0;
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) gt += (key[j] > T);
+        const int need_ties = k - __reduce_add_sync(0xffffffffu, gt);   // >= 1 ties at the threshold are kept, lowest index first
+        int run_tie = 0;
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const int e = j * 32 + lane;
+            const bool valid = e < L, eq = valid && key[j] == T;
+            const unsigned eqm = __ballot_sync(0xffffffffu, eq);
+            const bool keep = (valid && key[j] > T) || (eq && run_tie + __popc(eqm & lt) < need_ties);
+            const unsigned km = __ballot_sync(0xffffffffu, keep);
+            const int rank = run_keep + __popc(km & lt);
+            if (valid) s_rank[wid][e] = keep ? (int16_t)rank : (int16_t)-1;
+            if (keep) s_pos[wid][rank] = (int16_t)e;
+            run_tie += __popc(eqm);
+            run_keep += __popc(km);
+        }
     }
     __syncwarp();
+    const int hw = h * w;
 
     const long base = (long)seg * k;
     if (kept_idx != nullptr)
-        for (int r = lane; r < k; r += 32) kept_idx[base + r] = (int32_t)(s_pos[wid][r] & 0xFFFFu);
+        for (int r = lane; r < k; r += 32) kept_idx[base + r] = s_pos[wid][r];
     if (idx64 != nullptr)
-        for (int r = lane; r < k; r += 32) idx64[base + r] = (int64_t)(s_pos[wid][r] & 0xFFFFu);
+        for (int r = lane; r < k; r += 32) idx64[base + r] = s_pos[wid][r];
     if (table == nullptr) return;
 
     // one lane per kept token computes its K*K entries into shared memory; the warp then writes the
@@ -151,8 +192,8 @@ table_build_warp_kernel(const float* __restrict__ scores, int n_seg, int L, int 
     for (int r0 = 0; r0 < k; r0 += RR) {
         const int r = r0 + lane;
         if (lane < RR && r < k) {
-            const uint32_t pk = s_pos[wid][r];
-            const int p = (int)(pk & 0xFFFFu), y = (int)((pk >> 16) & 0xFFu), x = (int)(pk >> 24);
+            const int p = s_pos[wid][r], q = hw == 1 ? 0 : p - div_magic(p, magic_hw) * hw;
+            const int y = w == 1 ? q : div_magic(q, magic_w), x = q - y * w;
             if (KS > 0) {
 #pragma unroll
                 for (int tap = 0; tap < KS * KS; ++tap) {
@@ -267,6 +308,8 @@ table_build_segment_kernel(const float* __restrict__ scores, int L, int k, int h
     const int n_words = (L + 31) >> 5, per_cta = (n_words + G - 1) / G;
     const int w_begin = cta * per_cta, w_end = min(n_words, w_begin + per_cta);
     const float* sc = scores + (long)seg * L;
+    pdl_wait();
+    pdl_trigger();
 
     uint32_t key[ITEMS];
 #pragma unroll
@@ -465,15 +508,10 @@ template <int G, int ITEMS>
 static int segment_launch_as(const float* scores, int n_seg, int L, int k, int h, int w, int ksize, int kk, int32_t* kept_idx,
                              int32_t* table, int64_t* idx64, const int32_t* table_in, cudaStream_t s) {
     auto kern = table_build_segment_kernel<G, ITEMS>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(n_seg * G));
-    cfg.blockDim = dim3(SEG_THREADS);
-    cfg.stream = s;
     // rows of the previous table wait in shared memory while they leave room for it
     const size_t rows = (size_t)(((L + 31) / 32 + G - 1) / G) * 32 * kk * sizeof(int32_t) + 16;
     const int staged = table_in != nullptr && rows <= 180 * 1024;
     if (staged) {
-        cfg.dynamicSmemBytes = rows;
         static std::atomic<uint64_t> ready{0};     // devices on which this kernel may use that much
         int dev = 0;
         SV_CUDA(cudaGetDevice(&dev));
@@ -483,15 +521,8 @@ static int segment_launch_as(const float* scores, int n_seg, int L, int k, int h
             ready.fetch_or(bit);
         }
     }
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = G;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = G > 1 ? 1 : 0;
-    SV_CUDA(cudaLaunchKernelEx(&cfg, kern, scores, L, k, h, w, ksize, magic_of(w), magic_of(h * w), magic_of(ksize),
-                               kk, kept_idx, table, idx64, table_in, staged));
+    SV_CUDA(launch_pdl(kern, dim3((unsigned)(n_seg * G)), dim3(SEG_THREADS), staged ? rows : 0, s, G, scores, L, k, h, w, ksize,
+                       magic_of(w), magic_of(h * w), magic_of(ksize), kk, kept_idx, table, idx64, table_in, staged));
     return SVTAD_OK;
 }
 
@@ -576,9 +607,8 @@ extern "C" int svtad_table_init(int B, int T, int h, int w, int ksize, int32_t* 
     SV_CHECK_ARG(table != nullptr, "svtad_table_init: table is null");
     long total = rows * ksize * ksize;
     long threads = (total + 3) / 4;
-    table_init_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        table, total, h * w, h, w, ksize, ksize * ksize);
-    SV_LAUNCH_CHECK("table_init_kernel");
+    SV_CUDA(launch_pdl(table_init_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, 1, table,
+                       total, h * w, h, w, ksize, ksize * ksize));
     return SVTAD_OK;
 }
 
@@ -602,13 +632,8 @@ static int table_build_impl(const float* scores, int n_seg, int seg_len, int k, 
     if (seg_len <= 256) {
         unsigned grid = (unsigned)((n_seg + 7) / 8);
         const uint32_t mw = (uint32_t)((0x100000000ull + w - 1) / w), mhw = (uint32_t)((0x100000000ull + h * w - 1) / (h * w));
-        if (ksize == 3)
-            table_build_warp_kernel<8, 3><<<grid, 256, 0, s>>>(scores, n_seg, seg_len, k, h, w, ksize, mw, mhw, kept_idx, table, idx64);
-        else if (ksize == 5)
-            table_build_warp_kernel<8, 5><<<grid, 256, 0, s>>>(scores, n_seg, seg_len, k, h, w, ksize, mw, mhw, kept_idx, table, idx64);
-        else
-            table_build_warp_kernel<8, 0><<<grid, 256, 0, s>>>(scores, n_seg, seg_len, k, h, w, ksize, mw, mhw, kept_idx, table, idx64);
-        SV_LAUNCH_CHECK("table_build_warp_kernel");
+        auto kern = ksize == 3 ? table_build_warp_kernel<8, 3> : ksize == 5 ? table_build_warp_kernel<8, 5> : table_build_warp_kernel<8, 0>;
+        SV_CUDA(launch_plain(kern, dim3(grid), dim3(256), 0, s, 1, scores, n_seg, seg_len, k, h, w, ksize, mw, mhw, kept_idx, table, idx64));
         return SVTAD_OK;
     }
     SV_CHECK_ARG(table == nullptr || kept_idx != nullptr, "%s: kept_idx is required with a table", who);

@@ -261,15 +261,6 @@ constexpr int tmem_cols2_for(int bn) { return 2 * bn <= 64 ? 64 : 2 * bn <= 128 
 
 
 // ---- host helpers shared by the tensor-core translation units (defined in conv_tc.cu) ----
-template <typename... KArgs, typename... Args>
-inline cudaError_t tc_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
-}
 constexpr size_t TC_SMEM_LIMIT = 227 * 1024;
 int tc_num_sms();
 int tc_plan_sms();          // SMs a kernel is planned for: all of them divided by the caller's concurrency hint

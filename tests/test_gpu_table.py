@@ -202,3 +202,22 @@ def test_long_segments_on_both_sides_of_every_cluster_size(L, hw, ties):
             idx, tab = ops.table_select_remap(sc, torch.from_numpy(t0).cuda(), k)
             np.testing.assert_array_equal(idx.cpu().numpy(), ekept)
             np.testing.assert_array_equal(tab.reshape(-1, 9).cpu().numpy(), etable)
+
+
+@pytest.mark.parametrize("dist", ["normal", "exp", "wide", "one_outlier", "subnormal", "few_values", "inf", "nan_some"])
+def test_threshold_search_of_short_segments(dist):
+    """The per-slice builder's search by interpolation: score distributions that it converges on fast, slowly and not at
+    all (ties, infinities, NaNs), every k."""
+    ops = _ops()
+    rng = np.random.default_rng(11)
+    n, L = 40, 196
+    s = rng.standard_normal((n, L))
+    s = {"normal": s, "exp": np.exp(4 * s), "wide": np.sign(s) * 10.0 ** (30 * np.abs(s) / 3 - 15), "one_outlier": np.where(s > 2.9, 1e30, s),
+         "subnormal": s * 1e-42, "few_values": np.round(s), "inf": np.where(s > 1, np.inf, np.where(s < -1, -np.inf, s)),
+         "nan_some": np.where(s > 0.8, np.nan, s)}[dist].astype(np.float32)
+    sc = torch.from_numpy(s).cuda()
+    for k in (1, 2, 20, 49, 97, 150, L - 1, L):
+        kept, table = ops.table_build(sc, k, 14, 14, 3)
+        ekept, etable = otab.build_table(s, k, 14, 14, 3)
+        np.testing.assert_array_equal(kept.cpu().numpy(), ekept)
+        np.testing.assert_array_equal(table.cpu().numpy(), etable)
