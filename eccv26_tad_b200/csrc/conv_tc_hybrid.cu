@@ -60,12 +60,14 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 // PLAN: rows, tiles and taps as the table's plan says (plan.cuh): a tile's rows are plan.order's, only the taps of its
 // mask are worked through, and the CTAs take the tiles, longest first, in alternating directions (CTA c gets items c,
 // 2 G - 1 - c, 2 G + c, ...), so that their sums come out even.
-template <int BN, bool DGRAD, int RB, bool PLAN>
+// SPLIT: a cluster of G CTAs shares one item: each takes G-th of its K steps, parks its sums in the shared memory that the
+// ring has left, and finishes its share of the rows and columns from all CTAs' sums, in the order of the CTAs.
+template <int BN, bool DGRAD, int RB, bool PLAN, bool SPLIT>
 __global__ void __launch_bounds__(FW_THREADS, 1)
 conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __restrict__ a,
                    const int32_t* __restrict__ nbr, const uint16_t* __restrict__ bias,
                    uint16_t* __restrict__ out, const int32_t* __restrict__ status, long n, int cred, int cn,
-                   int kk, int tpb, int nstage, int fp16, int m_tiles, int n_blks, int out_al32, PlanView plan,
+                   int kk, int tpb, int nstage, int fp16, int m_tiles, int n_blks, int out_al32, int G, PlanView plan,
                    int* __restrict__ err) {
     if (DGRAD && status != nullptr) {
         pdl_wait();
@@ -75,6 +77,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
     constexpr int B_TX_BYTES = DGRAD ? BN * 128 : B_TILE_BYTES;
     constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
     constexpr int TM_COLS = tmem_cols2_for(BN);
+    constexpr int PARK = BN + 4;             // floats per row of the parked sums (SPLIT)
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -95,13 +98,16 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
     // the CTA's local-th item: its tile and column block; false behind the last one
     auto item = [&](int local, int& tile, int& blk) {
         const int turn = PLAN && (local & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
-        const int it = local * (int)gridDim.x + turn;
-        if (it >= tiles_total) return false;
+        const int it = SPLIT ? turn / G : local * (int)gridDim.x + turn;
+        if (SPLIT ? local > 0 : it >= tiles_total) return false;
         tile = it / n_blks;
         blk = it - tile * n_blks;
         if (PLAN) tile = __ldg(plan.seq + tile);
         return true;
     };
+    // SPLIT: this CTA's K steps [k_lo, k_hi) of the item
+    const int share = SPLIT ? (int)blockIdx.x % G : 0;
+    const int k_lo = SPLIT ? kk * kchunks * share / G : 0, k_hi = SPLIT ? kk * kchunks * (share + 1) / G : kk * kchunks;
     auto taps_of = [&](int tile) { return PLAN ? __ldg(plan.mask + tile) : all_taps; };
     // With RB = 2, two 64-deep buffers form one barrier round (a 128-deep K step): the MMA thread's per-round
     // work (wait, fences, commit) is spent once per eight instructions instead of once per four - worth it when
@@ -186,7 +192,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             const long row0 = (long)tile * TILE_M;
             const int n0 = blk * BN;
             const uint64_t taps = taps_of(tile);
-            const int steps = PLAN ? __popcll(taps) * kchunks : kk * kchunks, sp_pad = padded(steps);
+            const int steps = PLAN ? __popcll(taps) * kchunks : k_hi - k_lo, sp_pad = padded(steps);
             int* xf = s_tab + tab_ints;
             // this tile's table rows have landed (only table copies are ever committed to a group); the first
             // barrier also says that every producer warp is done reading the previous tile's row numbers
@@ -212,7 +218,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             int st = ((grp - it1) % n_own + n_own) % n_own;
             int s = (it1 + st) % nstage;                         // 64-deep buffer; its barrier round is s >> RSH
             uint32_t ph = (((it1 + st) / nstage) & 1) ^ 1;
-            int k = st / kchunks, kc = st - k * kchunks;
+            int k = (k_lo + st) / kchunks, kc = k_lo + st - k * kchunks;
             uint64_t left = taps;                                // PLAN: the current tap is the lowest bit
             if (PLAN) {
                 for (; k > 0; --k) left &= left - 1;
@@ -286,13 +292,13 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             const uint32_t idesc = make_idesc(fp16 ? 0 : 1, 0, DGRAD ? 0 : 1, TILE_M, BN);
             constexpr uint32_t desc_hi = smem_desc_hi(1024);
             bool alive = true;
-            int local = 0, s = 0, kc = 0;
+            int local = 0, s = 0, kc = SPLIT ? k_lo % kchunks : 0;
             uint32_t ph = 0;
             const int last_ks = (cred - (kchunks - 1) * STAGE_K + 15) / 16;     // 16-channel MMA steps of the last chunk
             const bool whole = last_ks == STAGE_K / 16;
             int tile, blk;
             for (; alive && item(local, tile, blk); ++local) {
-                const int steps = PLAN ? __popcll(taps_of(tile)) * kchunks : kk * kchunks, sp_pad = padded(steps);
+                const int steps = PLAN ? __popcll(taps_of(tile)) * kchunks : k_hi - k_lo, sp_pad = padded(steps);
                 const int buf = local & 1;
                 if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((local >> 1) & 1) ^ 1, s_abort, err, 42)) { alive = false; break; }
                 tc_fence_after();
@@ -351,6 +357,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             if (!warp_wait(smem_u32(&tail->accum_full[buf]), (local >> 1) & 1, s_abort, err, 44, lane)) break;
             tc_fence_after();
             const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN;
+            if constexpr (SPLIT) break;              // drained below
             uint16_t* orow = out + row * cn + n0;
             // two 32-column chunks in flight: the next tcgen05.ld runs while this chunk is converted and stored
             uint32_t va[32], vb[32];
@@ -364,6 +371,55 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             }
             tc_fence_before();
             mbar_arrive(smem_u32(&tail->accum_empty[buf]));
+        }
+    }
+    if constexpr (SPLIT) {
+        cluster_barrier();          // every CTA's MMAs are done: nothing is left in the rings, which take the sums now
+        int tile, blk;
+        item(0, tile, blk);
+        const int per = (TILE_M + G - 1) / G;                   // rows that a CTA finishes: [share * per, ...)
+        const uint32_t park = smem_u32(smem);                   // [CTA the sums come from][row][PARK]
+        if (warp > FW_A_WARPS) {
+            const int r = (warp & 3) * 32 + lane, owner = r / per;
+            const uint32_t dst = map_to_cta(park + ((share * per + r - owner * per) * PARK) * 4, owner);
+            const uint32_t t_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+            uint32_t va[32], vb[32];
+            tc_fence_after();
+            tmem_ld32(t_addr, va);
+#pragma unroll
+            for (int c = 0; c < BN / 32; ++c) {
+                uint32_t (&v)[32] = (c & 1) ? vb : va;
+                tmem_ld_wait();
+                if (c + 1 < BN / 32) tmem_ld32(t_addr + (c + 1) * 32, (c & 1) ? va : vb);
+#pragma unroll
+                for (int g = 0; g < 8; ++g)
+                    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
+                                 ::"r"(dst + (c * 32 + g * 4) * 4), "r"(v[4 * g]), "r"(v[4 * g + 1]), "r"(v[4 * g + 2]), "r"(v[4 * g + 3]) : "memory");
+            }
+        }
+        cluster_barrier();
+        // eight columns of a row per thread, the CTAs' sums in their order
+        const float* sums = reinterpret_cast<const float*>(smem);
+        const long row0 = (long)tile * TILE_M + share * per;
+        const int rows = share * per + per <= TILE_M ? per : TILE_M - share * per;
+        for (int e = tid; e < rows * (BN / 8); e += FW_THREADS) {
+            const int r = e / (BN / 8), c = (e % (BN / 8)) * 8, col = blk * BN + c;
+            if (row0 + r >= n || col >= cn) continue;
+            float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for (int p = 0; p < G; ++p) {
+                const float4* src = reinterpret_cast<const float4*>(sums + (p * per + r) * PARK + c);
+                const float4 u = src[0], v = src[1];
+                sum[0] += u.x; sum[1] += u.y; sum[2] += u.z; sum[3] += u.w;
+                sum[4] += v.x; sum[5] += v.y; sum[6] += v.z; sum[7] += v.w;
+            }
+            uint32_t o[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float b0 = 0.f, b1 = 0.f;
+                if (!DGRAD && bias != nullptr) { b0 = widen(__ldg(bias + col + 2 * q), fp16 != 0); b1 = widen(__ldg(bias + col + 2 * q + 1), fp16 != 0); }
+                o[q] = pack2(sum[2 * q] + b0, sum[2 * q + 1] + b1, fp16 != 0);
+            }
+            *reinterpret_cast<uint4*>(out + (row0 + r) * cn + col) = make_uint4(o[0], o[1], o[2], o[3]);
         }
     }
     tc_fence_before();
@@ -627,8 +683,8 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
-template <int BN, bool DGRAD, bool PLAN>
-static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
+template <int BN, bool DGRAD, bool PLAN, bool SPLIT>
+static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, int G, cudaStream_t s) {
     const int cred = DGRAD ? p.cout : p.cin;
     const int cn = DGRAD ? p.cin : p.cout;
     const int fp16 = p.dtype == SVTAD_F16 ? 1 : 0;
@@ -650,7 +706,7 @@ static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStre
     const bool two = nstage >= 6;
     if (two) nstage &= ~1;
     const size_t smem = 1024 + nstage * stage + extra;
-    auto kern = two ? conv_hybrid_kernel<BN, DGRAD, 2, PLAN> : conv_hybrid_kernel<BN, DGRAD, 1, PLAN>;
+    auto kern = two ? conv_hybrid_kernel<BN, DGRAD, 2, PLAN, SPLIT> : conv_hybrid_kernel<BN, DGRAD, 1, PLAN, SPLIT>;
     { int rc_s = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem); if (rc_s) return rc_s; }
     const int m_tiles = (int)((p.n + TILE_M - 1) / TILE_M);
     const int n_blks = (cn + BN - 1) / BN;
@@ -658,13 +714,41 @@ static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStre
     // persistent CTAs.  (Evening the tiles out - 135 tiles as 45 CTAs of 3 instead of 49 CTAs of 3 or 2 - was
     // measured slower inside a step of concurrent kernels: 0.0907 against 0.0858 ms.)
     const long sms = tc_plan_sms();
-    int grid = (int)(tiles < sms ? tiles : sms);
+    const int grid = SPLIT ? (int)tiles * G : (int)(tiles < sms ? tiles : sms);
     PlanView view{};
     if (PLAN) plan_layout(p.n, p.kk, p.plan, &view);
-    SV_CUDA(launch_pdl(kern, dim3(grid), dim3(FW_THREADS), smem, s, 1, map_w, (const uint16_t*)p.a, p.nbr,
+    SV_CUDA(launch_pdl(kern, dim3(grid), dim3(FW_THREADS), smem, s, SPLIT ? G : 1, map_w, (const uint16_t*)p.a, p.nbr,
                       (const uint16_t*)p.bias, (uint16_t*)p.out, status, (long)p.n, cred, cn, p.kk, p.tpb, nstage, fp16,
-                      m_tiles, n_blks, (reinterpret_cast<uintptr_t>(p.out) % 32 == 0) ? 1 : 0, view, tc_error_ptr()));
+                      m_tiles, n_blks, (reinterpret_cast<uintptr_t>(p.out) % 32 == 0) ? 1 : 0, G, view, tc_error_ptr()));
     return SVTAD_OK;
+}
+
+// Few row tiles and a long reduction leave most SMs idle: column block and cluster size for the K split, or 0 where it does
+// not pay.  A K step takes what a CTA was measured to need at that width; sharing an item out costs 2 to 6 us more than
+// finishing it alone (cluster launch, two cluster barriers, the sums' trip between SMs).  Clusters of three and more do not
+// pack a GPC's SMs completely, hence the limits on the grid.  1 180 rows, C = 1024: 41.6 -> 31.1 us; 2 360 rows, C = 512,
+// 5x5: 56 -> 38 us; 2 208 rows, C = 256: 11.9 -> 10.3 us.  The choice must not depend on the concurrency hint: the sums'
+// order would.
+static int pick_split(int cn, long m_tiles, int steps, int& G) {
+    if (getenv("SVTAD_TC_BN") != nullptr) return 0;
+    const int width[4] = {64, 128, 192, 256};
+    const double step_us[4] = {0.19, 0.23, 0.28, 0.344}, sharing_us[4] = {1.9, 3.5, 4.0, 6.0};
+    const int sizes[5] = {2, 3, 4, 5, 8}, limit[5] = {148, 120, 120, 112, 112};
+    const long sms = tc_num_sms();
+    double alone = 1e30, best = 1e30;
+    int bn = 0;
+    for (int i = 0; i < 4; ++i) {
+        if (width[i] - 64 >= cn) continue;
+        const long tiles = m_tiles * ((cn + width[i] - 1) / width[i]);
+        const double t = (double)((tiles + sms - 1) / sms) * steps * step_us[i];
+        if (t < alone) alone = t;
+        for (int g = 0; g < 5; ++g) {
+            if (tiles * sizes[g] * 148 > limit[g] * sms) continue;
+            const double u = (steps + sizes[g] - 1) / sizes[g] * step_us[i] + sharing_us[i];
+            if (u < best) { best = u; bn = width[i]; G = sizes[g]; }
+        }
+    }
+    return best + 0.6 < alone ? bn : 0;
 }
 
 template <bool DGRAD>
@@ -672,19 +756,27 @@ static int dispatch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaSt
     const int cn = DGRAD ? p.cin : p.cout;
     if (p.plan != nullptr) {
         switch (tc_widest_bn(cn)) {
-            case 64: return launch_conv_hybrid<64, DGRAD, true>(p, status, s);
-            case 128: return launch_conv_hybrid<128, DGRAD, true>(p, status, s);
-            case 192: return launch_conv_hybrid<192, DGRAD, true>(p, status, s);
-            default: return launch_conv_hybrid<256, DGRAD, true>(p, status, s);
+            case 64: return launch_conv_hybrid<64, DGRAD, true, false>(p, status, 1, s);
+            case 128: return launch_conv_hybrid<128, DGRAD, true, false>(p, status, 1, s);
+            case 192: return launch_conv_hybrid<192, DGRAD, true, false>(p, status, 1, s);
+            default: return launch_conv_hybrid<256, DGRAD, true, false>(p, status, 1, s);
         }
+    }
+    int G = 1;
+    const int split_bn = pick_split(cn, (p.n + TILE_M - 1) / TILE_M, p.kk * (((DGRAD ? p.cout : p.cin) + STAGE_K - 1) / STAGE_K), G);
+    switch (split_bn) {
+        case 64: return launch_conv_hybrid<64, DGRAD, false, true>(p, status, G, s);
+        case 128: return launch_conv_hybrid<128, DGRAD, false, true>(p, status, G, s);
+        case 192: return launch_conv_hybrid<192, DGRAD, false, true>(p, status, G, s);
+        case 256: return launch_conv_hybrid<256, DGRAD, false, true>(p, status, G, s);
     }
     int bn = tc_pick_bn(cn, (p.n + TILE_M - 1) / TILE_M);
     switch (bn) {
-        case 64: return launch_conv_hybrid<64, DGRAD, false>(p, status, s);
-        case 96: return launch_conv_hybrid<96, DGRAD, false>(p, status, s);
-        case 128: return launch_conv_hybrid<128, DGRAD, false>(p, status, s);
-        case 192: return launch_conv_hybrid<192, DGRAD, false>(p, status, s);
-        case 256: return launch_conv_hybrid<256, DGRAD, false>(p, status, s);
+        case 64: return launch_conv_hybrid<64, DGRAD, false, false>(p, status, 1, s);
+        case 96: return launch_conv_hybrid<96, DGRAD, false, false>(p, status, 1, s);
+        case 128: return launch_conv_hybrid<128, DGRAD, false, false>(p, status, 1, s);
+        case 192: return launch_conv_hybrid<192, DGRAD, false, false>(p, status, 1, s);
+        case 256: return launch_conv_hybrid<256, DGRAD, false, false>(p, status, 1, s);
     }
     return set_error(SVTAD_ERR_UNSUPPORTED, "tensor-core conv: no column block for width %d", cn);
 }

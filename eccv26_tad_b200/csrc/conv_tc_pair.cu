@@ -7,9 +7,9 @@
 // weight tile is halved (12 KB written + 12 KB read instead of 24 + 24 at BN = 192), which is what bounds the
 // one-CTA kernels, and a problem of m row tiles needs m CTAs whatever BN is.
 //
-// Roles per CTA (288 threads): warps 0-3 producers (cp.async gathers + lane 0's TMA of the B half, arriving on
-// the CTA's own full barrier), warp 4: in the even CTA the MMA issuer, in the odd CTA a relay that forwards
-// "my stage is full" to the even CTA's barrier; warps 5-8 epilogue of the CTA's own accumulator.
+// Roles per CTA (416 threads): warps 0-7 producers (cp.async gathers + lane 0's TMA of the B half, arriving on
+// the CTA's own full barrier), warp 8: in the even CTA the MMA issuer, in the odd CTA a relay that forwards
+// "my stage is full" to the even CTA's barrier; warps 9-12 epilogue of the CTA's own accumulator.
 // The even CTA's MMA thread commits to the empty / accumulator barriers of both CTAs.  No TMA load uses
 // cluster multicast.  Every wait is bounded (device error word), and both CTAs meet at a cluster barrier before
 // tensor memory is freed, so neither leaves while the other may still read its shared memory.
@@ -23,21 +23,12 @@
 
 namespace svtad {
 
-constexpr int PR_THREADS = 288;
-constexpr int PR_A_WARPS = 4;
+// Two producer warps share the fill of a 64-deep buffer (64 rows each), as in the one-CTA kernel.
+constexpr int PR_A_WARPS = 8, PR_NPW = 2, PR_GROUPS = PR_A_WARPS / PR_NPW;
+constexpr int PR_ITR = 32 / PR_NPW;          // 4-row copy iterations per lane and buffer
 constexpr int PR_A_THREADS = PR_A_WARPS * 32;
+constexpr int PR_THREADS = (PR_A_WARPS + 5) * 32;
 
-__device__ __forceinline__ uint32_t cluster_cta_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// address of the same shared-memory location in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-    return r;
-}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -65,10 +56,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
             }
         }
     }
-}
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t slot_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(ncols) : "memory");
@@ -149,9 +136,9 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
     // number of 64-deep steps gets an empty last half: its owner only arrives on the barrier.
     const int sp_pad = (stages_per_tile + 1) & ~1;
     const int nbig = nstage >> 1;             // nstage (number of 64-deep buffers) is even
-    // never more producer warps than buffers: a warp that is not held back by its own previous use of a buffer
+    // never more producer groups than buffers: a group that is not held back by its own previous use of a buffer
     // could run two rounds ahead of the consumer, where the empty barrier's parity reads as "free"
-    const int n_prod = nstage < PR_A_WARPS ? nstage : PR_A_WARPS;
+    const int n_prod = nstage < PR_GROUPS ? nstage : PR_GROUPS;
     const int tab_ints = TILE_M * kk;
     float* s_bias = reinterpret_cast<float*>(s_tab + 2 * tab_ints);   // [2][256]
 
@@ -176,13 +163,14 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
         pdl_wait();
         if (cid < items_total) load_table(cid);
     }
-    if (warp == 4) {
+    if (warp == PR_A_WARPS) {
         tmem_alloc_pair(smem_u32(&tail->tmem_slot), TM_COLS);
         tmem_relinquish_pair();
     }
-    if (tid == 4 * 32) {
+    if (tid == PR_A_WARPS * 32) {
         for (int b = 0; b < nbig; ++b) {
-            mbar_init(smem_u32(&tail->full[b]), rank == 0 ? 67 : 66);   // two halves x (32 copies + TMA), + the relay
+            // two buffers x (the copies of the lanes that fill it + TMA), + the relay
+            mbar_init(smem_u32(&tail->full[b]), 2 * (PR_NPW * 32 + 1) + (rank == 0 ? 1 : 0));
             mbar_init(smem_u32(&tail->empty[b]), 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -203,6 +191,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
     if (warp < PR_A_WARPS) {
         // ------------------------------------------------------------------ producers (both CTAs)
         const int sub = lane & 7, rg = lane >> 3;
+        const int grp = warp / PR_NPW, part = warp % PR_NPW;
         bool alive = true;
         int local = 0;
         for (int item = cid; item < items_total; item += n_clusters, ++local) {
@@ -220,9 +209,9 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
             }
             named_bar_sync(1, PR_A_THREADS);
             if (item + n_clusters < items_total) load_table(item + n_clusters);
-            if (!alive || warp >= n_prod) continue;
+            if (!alive || grp >= n_prod) continue;
             const int it0 = local * sp_pad;
-            int st = ((warp - it0) % n_prod + n_prod) % n_prod;
+            int st = ((grp - it0) % n_prod + n_prod) % n_prod;
             int s = (it0 + st) % nstage;                         // 64-deep buffer; its barrier round is s >> 1
             uint32_t ph = (((it0 + st) / nstage) & 1) ^ 1;
             int k = st / kchunks, kc = st - k * kchunks;
@@ -233,10 +222,10 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                 if (st >= stages_per_tile) {
                     // the empty half of the tile's last round: same number of arrivals, nothing to copy
                     mbar_arrive(bar);
-                    if (lane == 0) mbar_arrive(bar);
+                    if (lane == 0 && part == 0) mbar_arrive(bar);
                 } else {
                     const int c0 = kc * STAGE_K;
-                    if (lane == 0) {
+                    if (lane == 0 && part == 0) {
                         const uint32_t b_tile = a_tile + A_TILE_BYTES;
                         const int wtap = DGRAD ? (kk - 1 - k) : k;
                         mbar_expect_tx(bar, B_BYTES);
@@ -250,18 +239,18 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                     }
                     const bool there = c0 + sub * 8 < cred;
                     const uint16_t* abase = a + (there ? c0 + sub * 8 : 0);
-                    const int4* trow = reinterpret_cast<const int4*>(xf + (k << 7) + (rg << 5));
-                    int jrow[32];
+                    const int4* trow = reinterpret_cast<const int4*>(xf + (k << 7) + (rg << 5) + PR_ITR * part);
+                    int jrow[PR_ITR];
 #pragma unroll
-                    for (int q4 = 0; q4 < 8; ++q4) {
+                    for (int q4 = 0; q4 < PR_ITR / 4; ++q4) {
                         const int4 v = trow[q4];
                         jrow[4 * q4] = v.x; jrow[4 * q4 + 1] = v.y; jrow[4 * q4 + 2] = v.z; jrow[4 * q4 + 3] = v.w;
                     }
 #pragma unroll
-                    for (int itr = 0; itr < 32; ++itr) {
+                    for (int itr = 0; itr < PR_ITR; ++itr) {
                         const int j = jrow[itr];
                         const int r7 = ((itr & 1) << 2) | rg;
-                        const uint32_t dst = a_tile + (itr * 4 + rg) * 128 + ((sub ^ r7) << 4);
+                        const uint32_t dst = a_tile + ((PR_ITR * part + itr) * 4 + rg) * 128 + ((sub ^ r7) << 4);
                         cp_async16(dst, abase + (long)(j < 0 ? 0 : j) * cred, j < 0 || !there ? 0u : 16u);
                     }
                     cp_async_arrive_noinc(bar);
@@ -273,7 +262,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-    } else if (warp == 4) {
+    } else if (warp == PR_A_WARPS) {
         if (rank == 0) {
             // ------------------------------------------------------------------ MMA issuer (even CTA)
             // the whole warp walks the loop and waits; one elected lane (the same every time) issues and commits
@@ -348,7 +337,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
             }
         }
     } else {
-        // ------------------------------------------------------------------ epilogue (warps 5..8, both CTAs)
+        // ------------------------------------------------------------------ epilogue (the last four warps, both CTAs)
         const int q = warp & 3;
         const int et = tid - (PR_A_WARPS + 1) * 32;
         int local = 0;
@@ -384,7 +373,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
     tc_fence_before();
     __syncthreads();
     cluster_barrier();          // nobody frees tensor memory or leaves while the other CTA's work may still touch it
-    if (warp == 4) {
+    if (warp == PR_A_WARPS) {
         __syncwarp();
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, TM_COLS);

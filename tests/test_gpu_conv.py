@@ -298,6 +298,29 @@ def test_fp32_kernels_over_compacted_pairs(B, T, h, w, keep, ks, cin, cout):
     assert gb is None and torch.equal(gw, outs[2])
 
 
+@pytest.mark.parametrize("n,cin,cout,ks,dtype", [
+    (5, 512, 96, 3, torch.bfloat16),        # one tile, clusters of eight, a partial column block
+    (1180, 1024, 1024, 3, torch.bfloat16),  # clusters of three, 43 + 43 + 42 rows
+    (700, 352, 512, 5, torch.float16),      # 25 taps, a partial last chunk
+    (2208, 256, 256, 3, torch.bfloat16),    # clusters of two
+    (300, 768, 192, 3, torch.bfloat16),
+])
+def test_k_steps_shared_by_a_cluster(n, cin, cout, ks, dtype):
+    """Few row tiles and a long reduction: the K steps of a tile split over a thread-block cluster."""
+    table = -np.ones((n, ks * ks), dtype=np.int32)
+    for k in range(ks * ks):                             # shifts along a line, a third of them pruned
+        shift = k - ks * ks // 2
+        j = np.arange(n) + shift
+        keep = (j >= 0) & (j < n) & ((np.arange(n) + j) % 3 > 0) if shift else np.ones(n, bool)
+        table[keep, k] = j[keep]
+    table = torch.from_numpy(table)
+    x, w, b, gy = make_conv_inputs(n, cin, cout, ks, dtype, n, bias="random")
+    outs = _run_all(table, x, w, b, gy, sym=True)
+    _check_sampled(table, x, w, b, gy, outs, 2e-2, row_step=7, n_ci=8)
+    again = _run_all(table, x, w, b, gy, sym=True)
+    assert all(torch.equal(u, v) for u, v in zip(outs, again))
+
+
 def test_geometric_tables_on_both_sides_of_the_pair_switch():
     """Same with tables from the builder: 18 880 rows (148 row tiles, single CTAs) and 19 520 rows (153 tiles, pairs)."""
     for keep, rows in ((0.30, 18880), (0.31, 19520)):
