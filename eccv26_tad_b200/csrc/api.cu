@@ -268,13 +268,16 @@ extern "C" int svtad_conv_bwd_typed(const void* gy, const void* x, const int32_t
     std::lock_guard<std::mutex> hold(lane.mu);
     int rc = lane_ready(lane);
     if (rc) return rc;
-    // The two kernels share the GPU: each is planned for half of it unless the caller's hint already says more.  With pair
-    // lists both are persistent and balanced over all SMs, so there the second one moves in as the first one's CTAs leave.
+    // The two kernels share the GPU.  While one of them cannot fill it, each is planned for half of it (unless the caller's
+    // hint already says more): 8 084 rows, C = 256 (9.5 GFLOP a pass): 30 us against 32.5 planned for all of it.  From 18
+    // GFLOP on both are planned for all of it and the second moves in as the first one's CTAs leave: 6 132 rows, C = 1024:
+    // 249 -> 200 us; 3 744 rows, C = 320, 5x5: 74 -> 59 us.  With pair lists both are persistent and balanced over all SMs.
+    const bool whole_gpu = pairs_plan != nullptr || 2.0 * (double)n * kk * cin * cout >= 18e9;
     struct FloorGuard {
         int old;
         explicit FloorGuard(int floor) : old(tc_set_share_floor(floor)) {}
         ~FloorGuard() { tc_set_share_floor(old); }
-    } floor_guard(pairs_plan != nullptr ? 1 : 2);
+    } floor_guard(whole_gpu ? 1 : 2);
     // fork: the side stream starts where the caller's stream stands
     SV_CUDA(cudaEventRecord(lane.fork, s));
     SV_CUDA(cudaStreamWaitEvent(lane.stream, lane.fork, 0));

@@ -233,6 +233,7 @@ static WgradPlan wgrad_plan_for(int64_t n, int cin, int cout, int kk, bool with_
     const double step_cycles[4] = {650.0, 584.0, 450.0, 400.0};
     // partials are written once and read once: from L2 while they fit beside the operands, else from memory
     const double partial_cycles_l2 = 2.0 * 1.9e9 / 12.0e12, partial_cycles_mem = 2.0 * 1.9e9 / 4.0e12;
+    const double second_launch = 3000.0;
     WgradPlan best;
     best.bn = 0;
     double best_cost = 0;
@@ -253,8 +254,9 @@ static WgradPlan wgrad_plan_for(int64_t n, int cin, int cout, int kk, bool with_
             const long splits = (n + tps - 1) / tps;
             const long waves = (ctas * splits + sms - 1) / sms;
             const double steps = (double)tps / STAGE_K + 12.0;          // + set-up, first operands, drain
-            const double partial_bytes = (double)splits * kk * cin * cout * sizeof(float);
-            const double cost = (double)waves * steps * step_cycles[ci] +
+            // one split needs no partials and no second launch
+            const double partial_bytes = splits > 1 ? (double)splits * kk * cin * cout * sizeof(float) : 0.0;
+            const double cost = (double)waves * steps * step_cycles[ci] + (splits > 1 ? second_launch : 0.0) +
                                 partial_bytes * (partial_bytes < 48e6 ? partial_cycles_l2 : partial_cycles_mem);
             if (best.bn == 0 || cost < best_cost * 0.98) {
                 best = pl;

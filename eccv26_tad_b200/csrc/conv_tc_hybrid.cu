@@ -437,7 +437,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
 template <int BN>
 __global__ void __launch_bounds__(HY_THREADS, 1)
 wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* __restrict__ x,
-                    const int32_t* __restrict__ nbr, float* __restrict__ ws_w, float* __restrict__ ws_b,
+                    const int32_t* __restrict__ nbr, void* __restrict__ ws_w, void* __restrict__ ws_b, int direct, int out32,
                     long n, int cin, int cout, int kk, int tpb, long tokens_per_split, int n_nblk,
                     int nstage, int fp16, int ones_block, int* __restrict__ err) {
     constexpr int B_TILE_BYTES = b_tile_bytes_for(BN);
@@ -633,20 +633,23 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
         if (alive && total_stages > 0 && elect_one_sync()) umma_commit(smem_u32(&tail->accum_full[0]));
         __syncwarp();
     } else {
-        // epilogue: fp32 partial tile -> ws_w[split][(tap, ci)][co]; the all-ones block -> ws_b[split][co]
+        // epilogue: fp32 partial tile -> ws_w[split][(tap, ci)][co]; the all-ones block -> ws_b[split][co].  direct: there
+        // is one split, and the rounded values go to the gradients themselves (ws_w, ws_b are gw, gb)
         bool have = true;
         if (total_stages > 0) have = mbar_wait(smem_u32(&tail->accum_full[0]), 0, s_abort, err, 53);
         tc_fence_after();
         if (have) {
             const int q = warp & 3;
             const int blk = pair * 2 + (q >> 1);
-            float* dstrow = nullptr;
+            long at = -1;
+            void* base = ws_w;
             if (blk < nblocks) {
                 const int ch = (blk % cblocks) * 64 + (q & 1) * 32 + lane;
                 const long grow = (long)(blk / cblocks) * cin + ch;
-                if (ch < cin) dstrow = ws_w + ((long)blockIdx.y * kk * cin + grow) * cout + n0;
+                if (ch < cin) at = ((long)blockIdx.y * kk * cin + grow) * cout + n0;
             } else if (ones_here && q == 2 && lane == 0) {
-                dstrow = ws_b + (long)blockIdx.y * cout + n0;
+                at = (long)blockIdx.y * cout + n0;
+                base = ws_b;
             }
             constexpr int NC = BN / 32;
             const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
@@ -662,9 +665,24 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = 0u;
                 }
-                if (dstrow != nullptr && n0 + c * 32 < cout) {
+                if (at < 0 || n0 + c * 32 >= cout) continue;
+                if (direct) {
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        uint32_t o[4];
+#pragma unroll
+                        for (int q4 = 0; q4 < 4; ++q4)
+                            o[q4] = pack2(__uint_as_float(v[g * 8 + 2 * q4]), __uint_as_float(v[g * 8 + 2 * q4 + 1]), fp16 != 0);
+                        if (out32) {
+                            store_quad(base, at + c * 32 + g * 8, o[0], o[1], fp16 != 0, true);
+                            store_quad(base, at + c * 32 + g * 8 + 4, o[2], o[3], fp16 != 0, true);
+                        } else {
+                            *reinterpret_cast<uint4*>(static_cast<uint16_t*>(base) + at + c * 32 + g * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+                        }
+                    }
+                } else {
                     // 32 bytes (one whole sector) per store: the workspace is 256-byte aligned, rows are cout * 4 bytes
-                    float* dst = dstrow + c * 32;
+                    float* dst = static_cast<float*>(base) + at + c * 32;
 #pragma unroll
                     for (int g = 0; g < 4; ++g) st_global_v8(dst + g * 8, &v[g * 8]);
                 }
@@ -723,32 +741,45 @@ static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, int G, c
     return SVTAD_OK;
 }
 
-// Few row tiles and a long reduction leave most SMs idle: column block and cluster size for the K split, or 0 where it does
+// Few row tiles and a long reduction leave most SMs idle: cluster size and column block for the K split, or 0 where it does
 // not pay.  A K step takes what a CTA was measured to need at that width; sharing an item out costs 2 to 6 us more than
 // finishing it alone (cluster launch, two cluster barriers, the sums' trip between SMs).  Clusters of three and more do not
 // pack a GPC's SMs completely, hence the limits on the grid.  1 180 rows, C = 1024: 41.6 -> 31.1 us; 2 360 rows, C = 512,
-// 5x5: 56 -> 38 us; 2 208 rows, C = 256: 11.9 -> 10.3 us.  The choice must not depend on the concurrency hint: the sums'
-// order would.
+// 5x5: 56 -> 38 us; 2 208 rows, C = 256: 11.9 -> 10.3 us.
+// The order of the sums depends on the cluster size alone, so that is chosen for the whole GPU whatever the concurrency
+// hint says.  The column block is then chosen for the SMs the kernel may count on: next to a weight gradient, narrow blocks
+// over the whole GPU would make one kernel wait for the other (1 834 rows, C = 320: 27.9 against 20 us).
 static int pick_split(int cn, long m_tiles, int steps, int& G) {
     if (getenv("SVTAD_TC_BN") != nullptr) return 0;
     const int width[4] = {64, 128, 192, 256};
     const double step_us[4] = {0.19, 0.23, 0.28, 0.344}, sharing_us[4] = {1.9, 3.5, 4.0, 6.0};
     const int sizes[5] = {2, 3, 4, 5, 8}, limit[5] = {148, 120, 120, 112, 112};
-    const long sms = tc_num_sms();
+    const long sms = tc_num_sms(), mine = tc_plan_sms();
+    auto tiles_of = [&](int i) { return m_tiles * ((cn + width[i] - 1) / width[i]); };
     double alone = 1e30, best = 1e30;
-    int bn = 0;
+    int pick = -1;
     for (int i = 0; i < 4; ++i) {
         if (width[i] - 64 >= cn) continue;
-        const long tiles = m_tiles * ((cn + width[i] - 1) / width[i]);
+        const long tiles = tiles_of(i);
         const double t = (double)((tiles + sms - 1) / sms) * steps * step_us[i];
         if (t < alone) alone = t;
         for (int g = 0; g < 5; ++g) {
             if (tiles * sizes[g] * 148 > limit[g] * sms) continue;
             const double u = (steps + sizes[g] - 1) / sizes[g] * step_us[i] + sharing_us[i];
-            if (u < best) { best = u; bn = width[i]; G = sizes[g]; }
+            if (u < best) { best = u; pick = g; }
         }
     }
-    return best + 0.6 < alone ? bn : 0;
+    if (pick < 0 || best + 0.6 >= alone) return 0;
+    G = sizes[pick];
+    int bn = 0;
+    best = 1e30;
+    for (int i = 0; i < 4; ++i) {
+        if (width[i] - 64 >= cn) continue;
+        const long waves = (tiles_of(i) * G * 148 + limit[pick] * mine - 1) / (limit[pick] * mine);
+        const double u = waves * ((steps + G - 1) / G * step_us[i] + sharing_us[i] + (waves > 1 ? 6.0 : 0.0));
+        if (u < best) { best = u; bn = width[i]; }
+    }
+    return bn;
 }
 
 template <bool DGRAD>
@@ -786,7 +817,7 @@ int hybrid_fwd(const ConvArgs& p, cudaStream_t s) { return dispatch_conv_hybrid<
 int hybrid_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) { return dispatch_conv_hybrid<true>(p, status, s); }
 
 template <int BN>
-static int launch_wgrad_hybrid(const void* gy, const void* x, const int32_t* nbr, float* ws_w, float* ws_b, int64_t n, int cin, int cout, int kk, int tpb, int fp16,
+static int launch_wgrad_hybrid(const void* gy, const void* x, const int32_t* nbr, void* ws_w, void* ws_b, int direct, int out32, int64_t n, int cin, int cout, int kk, int tpb, int fp16,
                                const WgradPlan& pl, cudaStream_t s) {
     CUtensorMap map_gy;
     {
@@ -805,7 +836,7 @@ static int launch_wgrad_hybrid(const void* gy, const void* x, const int32_t* nbr
     dim3 grid((unsigned)(pl.n_pairs * pl.n_nblk), (unsigned)pl.splits);
     auto kern = wgrad_hybrid_kernel<BN>;
     { int rc_s = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem); if (rc_s) return rc_s; }
-    SV_CUDA(launch_pdl(kern, grid, dim3(HY_THREADS), smem, s, 1, map_gy, (const uint16_t*)x, nbr, ws_w, ws_b, (long)n, cin, cout, kk, tpb, pl.tokens_per_split,
+    SV_CUDA(launch_pdl(kern, grid, dim3(HY_THREADS), smem, s, 1, map_gy, (const uint16_t*)x, nbr, ws_w, ws_b, direct, out32, (long)n, cin, cout, kk, tpb, pl.tokens_per_split,
                       pl.n_nblk, nstage, fp16, pl.ones_block, tc_error_ptr()));
     return SVTAD_OK;
 }
@@ -820,16 +851,20 @@ int hybrid_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, vo
     const long n_w = (long)kk * cin * cout;
     float* ws_w = static_cast<float*>(ws);
     float* ws_b = reinterpret_cast<float*>(static_cast<char*>(ws) + align_up((size_t)pl.splits * n_w * sizeof(float), 256));
+    // one split: the main kernel's own sums are the gradients
+    const int direct = pl.splits == 1, out32 = grad_dtype == SVTAD_F32;
+    void* to_w = direct ? gw : ws_w;
+    void* to_b = direct ? gb : ws_b;
     int rc;
     switch (pl.bn) {
-        case 64: rc = launch_wgrad_hybrid<64>(gy, x, nbr, ws_w, ws_b, n, cin, cout, kk, tpb, fp16, pl, s); break;
-        case 128: rc = launch_wgrad_hybrid<128>(gy, x, nbr, ws_w, ws_b, n, cin, cout, kk, tpb, fp16, pl, s); break;
-        case 192: rc = launch_wgrad_hybrid<192>(gy, x, nbr, ws_w, ws_b, n, cin, cout, kk, tpb, fp16, pl, s); break;
-        case 256: rc = launch_wgrad_hybrid<256>(gy, x, nbr, ws_w, ws_b, n, cin, cout, kk, tpb, fp16, pl, s); break;
+        case 64: rc = launch_wgrad_hybrid<64>(gy, x, nbr, to_w, to_b, direct, out32, n, cin, cout, kk, tpb, fp16, pl, s); break;
+        case 128: rc = launch_wgrad_hybrid<128>(gy, x, nbr, to_w, to_b, direct, out32, n, cin, cout, kk, tpb, fp16, pl, s); break;
+        case 192: rc = launch_wgrad_hybrid<192>(gy, x, nbr, to_w, to_b, direct, out32, n, cin, cout, kk, tpb, fp16, pl, s); break;
+        case 256: rc = launch_wgrad_hybrid<256>(gy, x, nbr, to_w, to_b, direct, out32, n, cin, cout, kk, tpb, fp16, pl, s); break;
         default: return set_error(SVTAD_ERR_UNSUPPORTED, "tensor-core wgrad: no column block for width %d", cout);
     }
-    if (rc) return rc;
-    return tc_wgrad_reduce_launch(ws_w, pl.splits, ws_b, gb ? pl.splits : 0, gw, gb, n_w, cout, fp16, grad_dtype == SVTAD_F32, s);
+    if (rc || direct) return rc;
+    return tc_wgrad_reduce_launch(ws_w, pl.splits, ws_b, gb ? pl.splits : 0, gw, gb, n_w, cout, fp16, out32 != 0, s);
 }
 
 }  // namespace svtad

@@ -70,16 +70,6 @@ struct UnitMap {
     }
 };
 
-// four rounded values (two packed words) of a gradient, in 16 bits or as fp32
-__device__ __forceinline__ void store_quad(void* base, long at, uint32_t a, uint32_t b, bool fp16, bool out32) {
-    if (out32)
-        *reinterpret_cast<float4*>(static_cast<float*>(base) + at) =
-            make_float4(widen((uint16_t)(a & 0xffffu), fp16), widen((uint16_t)(a >> 16), fp16), widen((uint16_t)(b & 0xffffu), fp16),
-                        widen((uint16_t)(b >> 16), fp16));
-    else
-        *reinterpret_cast<uint2*>(static_cast<uint16_t*>(base) + at) = make_uint2(a, b);
-}
-
 template <int BN>
 __global__ void __launch_bounds__(WP_THREADS, 1)
 wgrad_pairs_kernel(const uint16_t* __restrict__ gy, const uint16_t* __restrict__ x, PlanView plan, void* __restrict__ gw,

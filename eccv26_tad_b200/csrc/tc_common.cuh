@@ -212,6 +212,16 @@ __device__ __forceinline__ void store_row_chunk32(uint16_t* dst, const uint32_t 
     }
 }
 
+// four rounded values (two packed words) of a gradient, in 16 bits or as fp32
+__device__ __forceinline__ void store_quad(void* base, long at, uint32_t a, uint32_t b, bool fp16, bool out32) {
+    if (out32)
+        *reinterpret_cast<float4*>(static_cast<float*>(base) + at) =
+            make_float4(widen((uint16_t)(a & 0xffffu), fp16), widen((uint16_t)(a >> 16), fp16), widen((uint16_t)(b & 0xffffu), fp16),
+                        widen((uint16_t)(b >> 16), fp16));
+    else
+        *reinterpret_cast<uint2*>(static_cast<uint16_t*>(base) + at) = make_uint2(a, b);
+}
+
 // bytes of one B stage: MN-major tiles are whole 64-column blocks of 8 KB, K-major tiles BN rows of 128 B
 constexpr int b_tile_bytes_for(int bn) { return ((bn + 63) / 64) * 8192; }
 constexpr int tmem_cols_for(int bn) { return bn <= 32 ? 32 : bn <= 64 ? 64 : bn <= 128 ? 128 : 256; }
