@@ -102,7 +102,7 @@ extern "C" size_t svtad_workspace_bytes(int op, int64_t n, int cin, int cout, in
             size_t a = simt_wgrad_ws_bytes(n, cin, cout, kk);
             size_t b = tc_supported(op, n, cin, cout, kk, dtype) ? tc_wgrad_ws_bytes(n, cin, cout, kk) : 0;
             if (b > 0 && pairs_wgrad_wanted(cin, kk)) {
-                const size_t c = pairs_wgrad_ws_bytes(cout);
+                const size_t c = pairs_wgrad_ws_bytes(cin, cout);
                 b = b > c ? b : c;
             }
             return a > b ? a : b;

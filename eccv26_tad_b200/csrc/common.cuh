@@ -91,7 +91,7 @@ int pair_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s);
 
 // weight gradient over the pairs of a plan (conv_tc_pairs.cu)
 bool pairs_wgrad_wanted(int cin, int kk);
-size_t pairs_wgrad_ws_bytes(int cout);
+size_t pairs_wgrad_ws_bytes(int cin, int cout);
 int pairs_wgrad(const void* gy, const void* x, const void* plan, void* gw, void* gb, int64_t n, int cin, int cout, int kk,
                 int dtype, int grad_dtype, void* ws, size_t ws_bytes, cudaStream_t s);
 
