@@ -258,13 +258,14 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
                     }
                     // A: 8 consecutive lanes cover one row's 128 B (8 chunks of 16 B)
                     const bool there = c0 + sub * 8 < cred;
+                    const uint32_t abytes = there ? 16u : 0u;
                     const uint16_t* abase = a + (there ? c0 + sub * 8 : 0);
 #pragma unroll
                     for (int itr = 0; itr < FW_ITR; ++itr) {
                         const int j = jrow[itr];
                         const int r7 = ((itr & 1) << 2) | rg;            // (row & 7) for row = (FW_ITR * part + itr) * 4 + rg
                         const uint32_t dst = a_tile + ((FW_ITR * part + itr) * 4 + rg) * 128 + ((sub ^ r7) << 4);
-                        cp_async16(dst, abase + (long)(j < 0 ? 0 : j) * cred, j < 0 || !there ? 0u : 16u);
+                        cp_async16(dst, row_at(abase, j, (uint32_t)cred * 2), j < 0 ? 0u : abytes);
                     }
                     cp_async_arrive_noinc(bar);
                 }
@@ -598,7 +599,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
                     const int j = jrow[itr];
                     const int r7 = ((itr & 1) << 2) | rg;
                     const uint32_t dst = a_tile + r * 128 + ((sub ^ r7) << 4);
-                    cp_async16(dst, xh[itr >> 4] + (long)(j < 0 ? 0 : j) * cin, j < 0 ? 0u : bytes[itr >> 4]);
+                    cp_async16(dst, row_at(xh[itr >> 4], j, (uint32_t)cin * 2), j < 0 ? 0u : bytes[itr >> 4]);
                 }
             }
             cp_async_arrive_noinc(bar);

@@ -238,6 +238,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                         }
                     }
                     const bool there = c0 + sub * 8 < cred;
+                    const uint32_t abytes = there ? 16u : 0u;
                     const uint16_t* abase = a + (there ? c0 + sub * 8 : 0);
                     const int4* trow = reinterpret_cast<const int4*>(xf + (k << 7) + (rg << 5) + PR_ITR * part);
                     int jrow[PR_ITR];
@@ -251,7 +252,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                         const int j = jrow[itr];
                         const int r7 = ((itr & 1) << 2) | rg;
                         const uint32_t dst = a_tile + ((PR_ITR * part + itr) * 4 + rg) * 128 + ((sub ^ r7) << 4);
-                        cp_async16(dst, abase + (long)(j < 0 ? 0 : j) * cred, j < 0 || !there ? 0u : 16u);
+                        cp_async16(dst, row_at(abase, j, (uint32_t)cred * 2), j < 0 ? 0u : abytes);
                     }
                     cp_async_arrive_noinc(bar);
                 }

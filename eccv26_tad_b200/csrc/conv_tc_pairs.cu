@@ -196,7 +196,7 @@ wgrad_pairs_kernel(const uint16_t* __restrict__ gy, const uint16_t* __restrict__
 #pragma unroll
                     for (int itr = 0; itr < ITS; ++itr) {
                         const int j = rj[itr];
-                        const uint16_t* src = xa + (long)max(j, 0) * cin;
+                        const uint16_t* src = static_cast<const uint16_t*>(row_at(xa, j, (uint32_t)cin * 2));
                         const uint32_t dst = a_tile + lane_dst[itr & 1] + itr * 512, bytes = j < 0 ? 0u : 16u;
 #pragma unroll
                         for (int b = 0; b < 2 * MH; ++b) cp_async16(dst + b * BLK, src + b * 64, bytes);
@@ -217,7 +217,7 @@ wgrad_pairs_kernel(const uint16_t* __restrict__ gy, const uint16_t* __restrict__
                 for (int itr = 0; itr < ITS; ++itr) {
                     const int i = ri[itr];
                     const uint32_t dst = a_tile + A_BYTES + lane_dst[itr & 1] + itr * 512, bytes = i < 0 ? 0u : 16u;
-                    const uint16_t* src = gb0 + (long)max(i, 0) * cout;
+                    const uint16_t* src = static_cast<const uint16_t*>(row_at(gb0, i, (uint32_t)cout * 2));
                     if (g_left > BN - 64) {
 #pragma unroll
                         for (int b = 0; b < BN / 64; ++b) cp_async16(dst + b * BLK, src + b * 64, bytes);
