@@ -118,13 +118,20 @@ extern "C" size_t svtad_workspace_bytes(int op, int64_t n, int cin, int cout, in
 // table): bit 0 the row order and tile masks (forward, input gradient), bit 1 the pair lists (weight gradient).  density =
 // pairs per row and tap, negative where it is not known: then the sparse case is assumed.
 // Measured at 18 880 rows: C = 512, 3x3 (89 GFLOP dense): forward 64 -> 41 us at density 0.34, 67 -> 51 at 0.58, 220 -> 230
-// (61 760 rows) at 0.87; weight gradient 81 -> 67, 82 -> 92, 280 -> 410.  Below 25 GFLOP a layer is a single wave of tiles
-// and as long as its longest one.
+// (61 760 rows) at 0.87; weight gradient 81 -> 67, 82 -> 92, 280 -> 410.
+// 15 to 25 GFLOP: the rows' order pays while there are tiles enough to share out (9 440 rows, C = 320: forward 20.2 -> 16.8 us,
+// backward 60 -> 47; 20 944 rows, C = 256, density 0.60: 33 -> 23 and 58 -> 50; 1 475 rows, C = 768: 22 -> 27), the lists do not
+// (18 880 rows, C = 256: backward 39 -> 48 us with them).  Below, a layer is a single wave of tiles and as long as its longest one.
+// Stencils beyond 3 x 3: the order is by the eight nearest neighbors, and a tile needs nearly all of the others (19.9 of 25 taps at
+// density 0.28, 22.4 at 0.61), so it takes more work to pay (18 880 rows, C = 256: 44 -> 42.5; 2 688 rows, C = 512: 29 -> 46), while
+// the lists gain the more (3 200 rows, C = 384, density 0.12: backward 63 -> 40 us).
 extern "C" int svtad_plan_wanted(int64_t n, int cin, int cout, int kk, int dtype, double density) {
     if (svtad_plan_bytes(n, kk) == 0 || kk < 2) return 0;
     const double work = 2.0 * (double)n * kk * cin * cout;
-    if (!use_tc(SVTAD_OP_FWD, n, cin, cout, kk, dtype) || work < 25e9) return 0;
-    return (density < 0.75 ? 1 : 0) | (density < 0.45 && pairs_wgrad_wanted(cin, kk) ? 2 : 0);
+    if (!use_tc(SVTAD_OP_FWD, n, cin, cout, kk, dtype)) return 0;
+    const bool rows = kk > 9 ? density < 0.45 && work >= 50e9 : density < 0.75 && (work >= 25e9 || (work >= 15e9 && n >= 2560));
+    const bool pairs = density < 0.45 && work >= (kk > 9 && density < 0.2 ? 15e9 : 25e9) && pairs_wgrad_wanted(cin, kk);
+    return (rows ? 1 : 0) | (pairs ? 2 : 0);
 }
 
 extern "C" int svtad_conv_fwd(const void* x, const int32_t* nbr, const void* w, const void* bias,

@@ -783,11 +783,33 @@ static int pick_split(int cn, long m_tiles, int steps, int& G) {
     return bn;
 }
 
+// Column block of the forward by a plan (the input gradient, which shares the GPU with the weight gradient, takes the widest: with
+// these 131 us instead of 117 for 5 900 rows, C = 1024).  The tiles come longest first, and some tile needs every tap, so few
+// tiles wait for that one: narrower blocks shorten it until the blocks' number times what each costs (its steps, half of the 3 x 3
+// taps and all the others on average, + 2.4 us for a further block of a CTA) fills the SMs for longer.  4 160 rows, C = 768: 42.6 us
+// with blocks of 256, 31.7 with 128; 5 900 rows, C = 512: 30.5 and 23.4; 18 880 rows, C = 1024: 129 and 173.
+static int pick_planned(int cn, long m_tiles, int kk, int chunks) {
+    if (getenv("SVTAD_TC_BN") != nullptr) return tc_widest_bn(cn);
+    const int width[4] = {64, 128, 192, 256};
+    const double step_us[4] = {0.19, 0.23, 0.28, 0.344}, taps = kk > 9 ? kk - 4.5 : kk * 0.5;
+    int bn = 0;
+    double best = 1e30;
+    for (int i = 3; i >= 0; --i) {
+        if (width[i] - 64 >= cn) continue;
+        const long items = m_tiles * ((cn + width[i] - 1) / width[i]), sms = tc_plan_sms();
+        const double longest = kk * chunks * step_us[i];
+        const double work = items <= sms ? 0 : (double)items / sms * (taps * chunks * step_us[i] + 2.4);
+        const double t = longest > work ? longest : work;
+        if (t < best * 0.95) { best = t; bn = width[i]; }
+    }
+    return bn;
+}
+
 template <bool DGRAD>
 static int dispatch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
     const int cn = DGRAD ? p.cin : p.cout;
     if (p.plan != nullptr) {
-        switch (tc_widest_bn(cn)) {
+        switch (DGRAD ? tc_widest_bn(cn) : pick_planned(cn, (p.n + TILE_M - 1) / TILE_M, p.kk, (p.cin + STAGE_K - 1) / STAGE_K)) {
             case 64: return launch_conv_hybrid<64, DGRAD, true, false>(p, status, 1, s);
             case 128: return launch_conv_hybrid<128, DGRAD, true, false>(p, status, 1, s);
             case 192: return launch_conv_hybrid<192, DGRAD, true, false>(p, status, 1, s);

@@ -271,9 +271,9 @@ struct Plan {
     Tensor data;
     int use = 0;
 };
-Plan plan_for(const Tensor& table, const Tensor& nbr, int64_t n, int cin, int cout, int kk, int code, int64_t tpb, void* stream) {
+Plan plan_for(const Tensor& table, const Tensor& nbr, int64_t n, int cin, int cout, int kk, int code, int64_t tpb, int parts, void* stream) {
     Plan p;
-    const int wanted = svtad_plan_wanted(n, cin, cout, kk, code, -1.0);
+    const int wanted = svtad_plan_wanted(n, cin, cout, kk, code, -1.0) & parts;
     if (!wanted) return p;
     auto make = [&] {
         Tensor plan = empty_on({static_cast<int64_t>(svtad_plan_bytes(n, kk))}, at::kByte, nbr.device());
@@ -305,7 +305,7 @@ Plan plan_for(const Tensor& table, const Tensor& nbr, int64_t n, int cin, int co
             (void)cudaGetLastError();
         }
     }
-    p.use = svtad_plan_wanted(n, cin, cout, kk, code, f->density);
+    p.use = svtad_plan_wanted(n, cin, cout, kk, code, f->density) & parts;
     if (p.use) p.data = f->plan;
     return p;
 }
@@ -447,7 +447,7 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
             y = empty_on({d.n, d.cout}, dt, dev);
         }
         if (grad && x.requires_grad()) status = status_for(table, nbr, d.n, d.kk, d.tpb, stream);
-        plan = plan_for(table, nbr, d.n, d.cin, d.cout, d.kk, code, d.tpb, stream);
+        plan = plan_for(table, nbr, d.n, d.cin, d.cout, d.kk, code, d.tpb, grad ? USE_ROWS | USE_PAIRS : USE_ROWS, stream);
         check(svtad_conv_fwd_planned(ptr(xc), iptr(nbr), ptr(wc), ptr(bc), mptr(y), d.n, d.cin, d.cout, d.kk,
                                      static_cast<int>(d.tpb), code, plan.use & USE_ROWS ? ptr(plan.data) : nullptr, stream));
     }

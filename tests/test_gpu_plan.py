@@ -100,6 +100,7 @@ def _planned(table, x, w, b, gy, tpb=0, grad_fp32=False):
     (1, 60, 0.5, 5, 160, 320, torch.bfloat16),         # partial chunks and column blocks, taps outside the sorted ring
     (4, 80, 0.6, 3, 64, 512, torch.bfloat16),          # one chunk per tap, two column blocks
     (1, 40, 1.0, 3, 96, 96, torch.bfloat16),           # the full grid
+    (4, 18, 0.3, 3, 768, 768, torch.bfloat16),         # few tiles: the forward takes narrower column blocks than the input gradient
     (4, 40, 0.3, 3, 480, 96, torch.float16),           # weight gradient by blocks of 256 input channels, the last one partial
     (1, 20, 0.3, 3, 512, 288, torch.bfloat16),         # ... whole units and cut ones, a partial column block
 ])
