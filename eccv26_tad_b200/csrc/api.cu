@@ -121,7 +121,9 @@ extern "C" size_t svtad_workspace_bytes(int op, int64_t n, int cin, int cout, in
 // (61 760 rows) at 0.87; weight gradient 81 -> 67, 82 -> 92, 280 -> 410.
 // 15 to 25 GFLOP: the rows' order pays while there are tiles enough to share out (9 440 rows, C = 320: forward 20.2 -> 16.8 us,
 // backward 60 -> 47; 20 944 rows, C = 256, density 0.60: 33 -> 23 and 58 -> 50; 1 475 rows, C = 768: 22 -> 27), the lists do not
-// (18 880 rows, C = 256: backward 39 -> 48 us with them).  Below, a layer is a single wave of tiles and as long as its longest one.
+// (18 880 rows, C = 256: backward 39 -> 48 us with them).  10 to 15 GFLOP: with more tiles than SMs, where the order saves most of
+// the second wave (19 600 rows, C = 192, density 0.51: forward 24.1 -> 14.1 us, backward 37 -> 32; 43 200 rows, C = 128, 0.55: 22.1 ->
+// 17.6 and 40.3 -> 39.6), which three layers on a table pay the plan with.  Below, a layer is a single wave of tiles and as long as its longest one.
 // Stencils beyond 3 x 3: the order is by the eight nearest neighbors, and a tile needs nearly all of the others (19.9 of 25 taps at
 // density 0.28, 22.4 at 0.61), so it takes more work to pay (18 880 rows, C = 256: 44 -> 42.5; 2 688 rows, C = 512: 29 -> 46), while
 // the lists gain the more (3 200 rows, C = 384, density 0.12: backward 63 -> 40 us).
@@ -129,7 +131,7 @@ extern "C" int svtad_plan_wanted(int64_t n, int cin, int cout, int kk, int dtype
     if (svtad_plan_bytes(n, kk) == 0 || kk < 2) return 0;
     const double work = 2.0 * (double)n * kk * cin * cout;
     if (!use_tc(SVTAD_OP_FWD, n, cin, cout, kk, dtype)) return 0;
-    const bool rows = kk > 9 ? density < 0.45 && work >= 50e9 : density < 0.75 && (work >= 25e9 || (work >= 15e9 && n >= 2560));
+    const bool rows = kk > 9 ? density < 0.45 && work >= 50e9 : density < 0.75 && (work >= 25e9 || (work >= 15e9 && n >= 2560) || (work >= 10e9 && n > 148 * 128));
     const bool pairs = density < 0.45 && work >= (kk > 9 && density < 0.2 ? 15e9 : 25e9) && pairs_wgrad_wanted(cin, kk);
     return (rows ? 1 : 0) | (pairs ? 2 : 0);
 }
