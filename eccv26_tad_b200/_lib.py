@@ -38,8 +38,10 @@ SIGNATURES = {
     "svtad_plan_counts": (c_p, [c_p, c_i64, c_int]),
     "svtad_plan_bytes": (c_sz, [c_i64, c_int]),
     "svtad_plan_build": (c_int, [c_p, c_i64, c_int, c_int, c_p, c_p]),
+    "svtad_plan_build_parts": (c_int, [c_p, c_i64, c_int, c_int, c_int, c_p, c_p]),
     "svtad_conv_fwd_planned": (c_int, [c_p, c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_p, c_p]),
     "svtad_conv_bwd_typed": (c_int, [c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_int, c_p, c_int, c_p, c_p, c_sz, c_p]),
+    "svtad_conv_bwd_planned": (c_int, [c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_int, c_p, c_int, c_int, c_p, c_p, c_sz, c_p]),
     "svtad_static_workspace_bytes": (c_sz, []),
     "svtad_conv_wgrad_static": (c_int, [c_p, c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_p]),
     "svtad_allreduce_stage_bytes": (c_sz, [c_i64]),

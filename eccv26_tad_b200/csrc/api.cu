@@ -114,26 +114,32 @@ extern "C" size_t svtad_workspace_bytes(int op, int64_t n, int cin, int cout, in
     return 0;
 }
 
-// Which parts of a plan shorten a layer's kernels by more than the plan takes to make (16-20 us of GPU time, once per
-// table): bit 0 the row order and tile masks (forward, input gradient), bit 1 the pair lists (weight gradient).  density =
-// pairs per row and tap, negative where it is not known: then the sparse case is assumed.
-// Measured at 18 880 rows: C = 512, 3x3 (89 GFLOP dense): forward 64 -> 41 us at density 0.34, 67 -> 51 at 0.58, 220 -> 230
-// (61 760 rows) at 0.87; weight gradient 81 -> 67, 82 -> 92, 280 -> 410.
-// 15 to 25 GFLOP: the rows' order pays while there are tiles enough to share out (9 440 rows, C = 320: forward 20.2 -> 16.8 us,
-// backward 60 -> 47; 20 944 rows, C = 256, density 0.60: 33 -> 23 and 58 -> 50; 1 475 rows, C = 768: 22 -> 27), the lists do not
-// (18 880 rows, C = 256: backward 39 -> 48 us with them).  10 to 15 GFLOP: with more tiles than SMs, where the order saves most of
-// the second wave (19 600 rows, C = 192, density 0.51: forward 24.1 -> 14.1 us, backward 37 -> 32; 43 200 rows, C = 128, 0.55: 22.1 ->
-// 17.6 and 40.3 -> 39.6), which three layers on a table pay the plan with.  Below, a layer is a single wave of tiles and as long as its longest one.
-// Stencils beyond 3 x 3: the order is by the eight nearest neighbors, and a tile needs nearly all of the others (19.9 of 25 taps at
-// density 0.28, 22.4 at 0.61), so it takes more work to pay (18 880 rows, C = 256: 44 -> 42.5; 2 688 rows, C = 512: 29 -> 46), while
-// the lists gain the more (3 200 rows, C = 384, density 0.12: backward 63 -> 40 us).
+// Which parts of a plan gain a layer more than it costs to make them for this one layer and call: the row order (forward,
+// input gradient) takes 10 us up to 7 000 rows, 16 at 18 880, 30 at 60 000, the pair lists (weight gradient; 3 x 3) 4 to 9,
+// next to the input gradient.  What they save goes by the products that are not there, work * (1 - density); on what a plan
+// costs the line rises with the rows.  Measured, us of a training pass (forward + backward) without a plan and with one made
+// for it, by the products left out:
+//   4 720 rows, C = 512, density 0.35 (14 GFLOP): 75 -> 82             9 440, C = 512, 0.59 (18): 110 -> 127
+//   2 400, C = 768, 0.27 (19): 111 -> 84                              11 800, C = 384, 0.35 (20): 110 -> 83
+//   4 720, C = 768, 0.35 (32): 153 -> 116                             6 400, C = 512, 0.19 (24): 100 -> 80
+//   18 880, C = 256, 0.35 (14): 67 -> 83                              18 880, C = 384, 0.35 (32): 144 -> 102
+//   37 760, C = 256, 0.59 (18): 116 -> 126                            37 760, C = 384, 0.59 (41): 260 -> 234
+//   50 240, C = 384, 0.75 (33): 367 -> 376                            50 240, C = 512, 0.75 (59): 619 -> 570
+//   18 880, C = 1024, 0.35 (232): 870 -> 430                          15 680, C = 1024, 0.91 (27): 817 -> 657
+// Up to sixteen tiles the kernels without a plan share a tile's K steps over a cluster, and the longest tile, which needs
+// nearly every tap, is all that matters: 1 770, C = 1024, 0.35 (22): 118 -> 128.
+// Stencils beyond 3 x 3: the order is by the eight nearest neighbors, and a tile needs nearly all of the others (19.9 of 25
+// taps at density 0.28, 22.4 at 0.61): 2 360 rows, C = 512: forward 38 -> 78 us; 18 880, C = 256: 44 -> 43.  So these take the
+// lists alone, which take 8 to 19 us (backward with the lists' making): 4 720 rows, C = 384, 0.28 (25 GFLOP): 97 -> 76; 9 440,
+// C = 256, 0.28 (22): 69 -> 75; 18 880, C = 256, 0.28 (45): 109 -> 97; 9 440, C = 384, 0.52 (33): 156 -> 122.
+// density = pairs per row and tap; negative: not known, the sparse case (0.35) is assumed.
 extern "C" int svtad_plan_wanted(int64_t n, int cin, int cout, int kk, int dtype, double density) {
     if (svtad_plan_bytes(n, kk) == 0 || kk < 2) return 0;
-    const double work = 2.0 * (double)n * kk * cin * cout;
-    if (!use_tc(SVTAD_OP_FWD, n, cin, cout, kk, dtype)) return 0;
-    const bool rows = kk > 9 ? density < 0.45 && work >= 50e9 : density < 0.75 && (work >= 25e9 || (work >= 15e9 && n >= 2560) || (work >= 10e9 && n > 148 * 128));
-    const bool pairs = density < 0.45 && work >= (kk > 9 && density < 0.2 ? 15e9 : 25e9) && pairs_wgrad_wanted(cin, kk);
-    return (rows ? 1 : 0) | (pairs ? 2 : 0);
+    const double there = density < 0 ? 0.35 : density < 1 ? density : 1;
+    const double saved = 2e-9 * (double)n * kk * cin * cout * (1 - there);
+    const bool near = kk <= 9;
+    if (saved < (near ? 15.0 : 23.0) + (double)n / 2500 || !use_tc(SVTAD_OP_FWD, n, cin, cout, kk, dtype)) return 0;
+    return (near && n > 2048 ? SVTAD_PLAN_ROWS : 0) | ((!near || n > 2048) && pairs_wgrad_wanted(cin, kk) ? SVTAD_PLAN_PAIRS : 0);
 }
 
 extern "C" int svtad_conv_fwd(const void* x, const int32_t* nbr, const void* w, const void* bias,
@@ -244,18 +250,35 @@ extern "C" int svtad_conv_bwd_typed(const void* gy, const void* x, const int32_t
                                     int tokens_per_batch, int dtype, int grad_dtype, const void* plan,
                                     int plan_use, const int32_t* table_status, void* workspace,
                                     size_t workspace_bytes, void* stream) {
+    return svtad_conv_bwd_planned(gy, x, nbr, w, gx, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype,
+                                  const_cast<void*>(plan), plan_use, 0, table_status, workspace, workspace_bytes, stream);
+}
+
+extern "C" int svtad_conv_bwd_planned(const void* gy, const void* x, const int32_t* nbr, const void* w, void* gx,
+                                      void* gw, void* gb, int64_t n, int cin, int cout, int kk,
+                                      int tokens_per_batch, int dtype, int grad_dtype, void* plan, int plan_use,
+                                      int plan_make, const int32_t* table_status, void* workspace,
+                                      size_t workspace_bytes, void* stream) {
     SV_CHECK_ARG(grad_dtype == dtype || grad_dtype == SVTAD_F32,
                  "svtad_conv_bwd: weight gradients come in the features' type or in float32, not in type %d", grad_dtype);
-    const void* rows_plan = plan_use & 1 ? plan : nullptr;
-    const void* pairs_plan = plan_use & 2 ? plan : nullptr;
+    SV_CHECK_ARG((plan_make & ~SVTAD_PLAN_PAIRS) == 0, "svtad_conv_bwd: only the pair lists are made here, not parts %d", plan_make);
+    const void* rows_plan = plan_use & SVTAD_PLAN_ROWS ? plan : nullptr;
+    const void* pairs_plan = plan_use & SVTAD_PLAN_PAIRS ? plan : nullptr;
+    // where the lists are to be made, in front of the weight gradient on its stream
+    auto make_lists = [&](cudaStream_t on) {
+        if (plan_make == 0 || pairs_plan == nullptr || gw == nullptr || n == 0) return SVTAD_OK;
+        return svtad_plan_build_parts(nbr, n, kk, tokens_per_batch, SVTAD_PLAN_PAIRS, plan, on);
+    };
     SV_CHECK_ARG(gx != nullptr || gw != nullptr, "svtad_conv_bwd: neither gx nor gw requested");
     SV_CHECK_ARG(gb == nullptr || gw != nullptr, "svtad_conv_bwd: gb needs gw");
     if (gw == nullptr)
         return conv_dgrad_planned(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, rows_plan, table_status,
                                   workspace, workspace_bytes, stream);
-    if (gx == nullptr)
+    if (gx == nullptr) {
+        if (int rc = make_lists((cudaStream_t)stream)) return rc;
         return conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, pairs_plan,
                                 workspace, workspace_bytes, stream);
+    }
     // workspace = [weight-gradient part | input-gradient part (scatter form, only with a status word)]
     const size_t w_part = align_up(svtad_workspace_bytes(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype), 256);
     const size_t d_part = table_status != nullptr ? svtad_workspace_bytes(SVTAD_OP_DGRAD, n, cin, cout, kk, dtype) : 0;
@@ -267,7 +290,9 @@ extern "C" int svtad_conv_bwd_typed(const void* gy, const void* x, const int32_t
     int dev = 0;
     SV_CUDA(cudaGetDevice(&dev));
     if (!overlap_backward() || n == 0 || dev >= MAX_DEVICES) {
-        int rc = conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, pairs_plan,
+        int rc = make_lists(s);
+        if (rc) return rc;
+        rc = conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, pairs_plan,
                                   workspace, w_part, s);
         if (rc) return rc;
         return conv_dgrad_planned(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, rows_plan, table_status, ws_d,
@@ -296,8 +321,9 @@ extern "C" int svtad_conv_bwd_typed(const void* gy, const void* x, const int32_t
                                 w_part, lane.stream);
     };
     if (pairs_plan == nullptr) wgrad();
+    else rc_w = make_lists(lane.stream);
     rc_d = conv_dgrad_planned(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, rows_plan, table_status, ws_d, d_part, s);
-    if (pairs_plan != nullptr) wgrad();
+    if (pairs_plan != nullptr && rc_w == SVTAD_OK) wgrad();
     // join, also after an error: whatever was launched on the side stream is ordered before the caller's next work
     cudaError_t e1 = cudaEventRecord(lane.join, lane.stream);
     cudaError_t e2 = cudaStreamWaitEvent(s, lane.join, 0);

@@ -8,8 +8,10 @@
 // library's one-call backward without touching the interpreter.
 //
 // What is known about a neighbor table (symmetric by construction, indices local to a batch row or not, the device
-// status word of svtad_table_check, an int32 copy, the work plan of svtad_plan_build) is kept per tensor object and version; entries of dead tables are
-// swept whenever a new table is entered.
+// status word of svtad_table_check, an int32 copy, how many of its entries are there) is kept per tensor object and
+// version; entries of dead tables are swept whenever a new table is entered.  A table's work plan is not: a table can be
+// written to without its version moving (a replayed graph that holds the selection, the C ABI, a raw pointer), so a
+// layer makes its plan from what the table holds when its kernels run, every time.
 #include <ATen/ATen.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
@@ -23,6 +25,8 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <algorithm>
+#include <cstdlib>
 #include <memory>
 #include <mutex>
 #include <unordered_map>
@@ -72,9 +76,8 @@ void* mptr(Tensor& t) { return t.defined() && t.numel() ? t.data_ptr() : nullptr
 const int32_t* iptr(const Tensor& t) { return static_cast<const int32_t*>(ptr(t)); }
 
 // ------------------------------------------------------------------------------------------------ table facts
-// Landing places in pinned memory for what the device finds out about a table (a status word, the lengths of a plan's
-// lists) on its way to the host: one block, allocated at the first use (pinning memory takes milliseconds, so not once
-// per table).  A place whose copy is still under way when its table
+// Landing places in pinned memory for a table's status word on its way to the host: one block, allocated at the first
+// use (pinning memory takes milliseconds, so not once per table).  A place whose copy is still under way when its table
 // dies is handed out again only after the copy has landed; when all are taken the caller does without.
 class HostWords {
   public:
@@ -139,31 +142,26 @@ struct Facts {
     Tensor status;               // device word of svtad_table_check
     HostWords::Place host;       // where its copy on the host arrives
     Tensor i32;                  // contiguous, aligned int32 form of a table of another kind
-    int64_t plan_tpb = -1;       // tokens_per_batch the plan below belongs to
-    void* plan_stream = nullptr;
-    HostWords::Place plan_host;  // where the lengths of its lists arrive on the host
-    double density = -1;         // pairs per row and tap, once they have arrived
-    bool full_grid = false;      // svtad_table_init's: hardly a neighbor missing
-    Tensor plan;                 // svtad_plan_build's, shared by the layers that use the table on that stream
+    double density = -1;         // pairs per row and tap, as far as the host knows (only speed hangs on it)
     std::mutex mu;               // guards everything below `version`
 
-    explicit Facts(const Tensor& t) : owner(t.getIntrusivePtr()), version(t._version()), device(t.get_device()) {}
+    static int64_t version_of(const Tensor& t) { return t.is_inference() ? -1 : static_cast<int64_t>(t._version()); }
+    explicit Facts(const Tensor& t) : owner(t.getIntrusivePtr()), version(version_of(t)), device(t.get_device()) {}
     ~Facts() {
         if (host.word) host_words(device).give_back(host);
-        if (plan_host.word) host_words(device).give_back(plan_host);
     }
 };
 
 class FactStore {
   public:
     // facts of this very tensor object at its present version, entered if `make`; null otherwise.  Tensors made in
-    // inference mode have no version counter, so nothing can be remembered about them.
-    std::shared_ptr<Facts> find(const Tensor& t, bool make) {
-        if (t.is_inference()) return nullptr;
+    // inference mode have no version counter, so only what speed hangs on can be remembered about them (`hint`).
+    std::shared_ptr<Facts> find(const Tensor& t, bool make, bool hint = false) {
+        if (t.is_inference() && !hint) return nullptr;
         std::lock_guard<std::mutex> hold(mu_);
         auto it = map_.find(t.unsafeGetTensorImpl());
         if (it != map_.end()) {
-            if (!it->second->owner.expired() && it->second->version == static_cast<int64_t>(t._version())) return it->second;
+            if (!it->second->owner.expired() && it->second->version == Facts::version_of(t)) return it->second;
             map_.erase(it);
         }
         if (!make) return nullptr;
@@ -183,12 +181,45 @@ FactStore& store() {
     return *s;
 }
 
-void mark_symmetric(const Tensor& t, bool built, bool full_grid = false) {
+void mark_symmetric(const Tensor& t, bool built, double density = -1) {
     if (auto f = store().find(t, true)) {
         f->symmetric = true;
         f->built = built;
-        f->full_grid = full_grid;
     }
+    if (density < 0) return;
+    auto f = store().find(t, true, true);
+    std::lock_guard<std::mutex> hold(f->mu);
+    f->density = density;
+}
+
+// the table's density, where it or the tensor it looks into has one
+double density_of(const Tensor& t) {
+    auto known = [](const Tensor& u) {
+        auto f = store().find(u, false, true);
+        if (!f) return -1.0;
+        std::lock_guard<std::mutex> hold(f->mu);
+        return f->density;
+    };
+    const double d = known(t);
+    return d >= 0 || !t.is_view() ? d : known(Tensor(at::TensorBase(t._base())));
+}
+
+// Expected pairs per row and tap of a table whose segments of `len` tokens, of an h x w grid per slice, keep k each.
+double expected_density(int64_t len, int64_t k, int64_t h, int64_t w, int64_t ksize) {
+    if (ksize < 1 || h < 1 || w < 1) return -1;
+    const double share = len > 1 ? static_cast<double>(k - 1) / static_cast<double>(len - 1) : 0;
+    double inside = 0;      // neighbors that lie on the grid, per token
+    for (int64_t d = -(ksize / 2); d <= ksize / 2; ++d)
+        for (int64_t e = -(ksize / 2); e <= ksize / 2; ++e)
+            if (d != 0 || e != 0)
+                inside += static_cast<double>(std::max<int64_t>(0, h - std::abs(d)) * std::max<int64_t>(0, w - std::abs(e))) / static_cast<double>(h * w);
+    return (1 + inside * share) / static_cast<double>(ksize * ksize);
+}
+// ... and of a table of that density, n_prev rows per batch row, of which k are kept
+double pruned_density(double density, int64_t kk, int64_t n_prev, int64_t k) {
+    if (density < 0 || kk < 1) return -1;
+    const double share = n_prev > 1 ? static_cast<double>(k - 1) / static_cast<double>(n_prev - 1) : 0;
+    return (1 + std::max(0.0, density * static_cast<double>(kk) - 1) * share) / static_cast<double>(kk);
 }
 
 // the table's own facts or, for a view, those of the tensor it looks into
@@ -262,52 +293,21 @@ Tensor int32_table(const Tensor& table) {
     return f->i32;
 }
 
-// The table's work plan for a layer that wants one, else an undefined tensor, and which parts of it the layer should use.
-// Made once per table; under graph capture it belongs to the call (its contents are there only when the graph runs).  How
-// many neighbors are there is known to the host only once the lists' lengths have come back: the call that makes a plan
-// takes the sparse case for granted.
-constexpr int USE_ROWS = 1, USE_PAIRS = 2;
-struct Plan {
-    Tensor data;
-    int use = 0;
-};
-Plan plan_for(const Tensor& table, const Tensor& nbr, int64_t n, int cin, int cout, int kk, int code, int64_t tpb, int parts, void* stream) {
-    Plan p;
-    const int wanted = svtad_plan_wanted(n, cin, cout, kk, code, -1.0) & parts;
-    if (!wanted) return p;
-    auto make = [&] {
-        Tensor plan = empty_on({static_cast<int64_t>(svtad_plan_bytes(n, kk))}, at::kByte, nbr.device());
-        check(svtad_plan_build(iptr(nbr), n, kk, static_cast<int>(tpb), plan.data_ptr(), stream));
-        return plan;
-    };
-    auto f = store().find(table, true);
-    if (!f) return Plan{make(), wanted};
-    if (auto s = symmetric_facts(table); s && s->full_grid) return p;
-    std::lock_guard<std::mutex> hold(f->mu);
-    if (!(f->plan_tpb == tpb && f->plan_stream == stream && f->plan.defined())) {
-        Tensor plan = make();
-        if (capturing(stream)) return Plan{plan, wanted};
-        f->plan = plan;
-        f->plan_stream = stream;
-        f->plan_tpb = tpb;
-        f->density = -1;
-        if (f->plan_host.word || host_words(f->device).take(f->plan_host)) {
-            C10_CUDA_CHECK(cudaMemcpyAsync(const_cast<int32_t*>(f->plan_host.word), svtad_plan_counts(plan.data_ptr(), n, kk),
-                                           kk * sizeof(int32_t), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)));
-            C10_CUDA_CHECK(cudaEventRecord(f->plan_host.copied, static_cast<cudaStream_t>(stream)));
-        }
-    } else if (f->density < 0 && f->plan_host.word && !capturing(stream)) {
-        if (cudaEventQuery(f->plan_host.copied) == cudaSuccess) {
-            double pairs = 0;
-            for (int k = 0; k < kk; ++k) pairs += f->plan_host.word[k];
-            f->density = pairs / (static_cast<double>(n) * kk);
-        } else {
-            (void)cudaGetLastError();
+// Which parts of a work plan a layer should use: only where the table's density is known, which for a caller's table means
+// that this call, as one that reads the indices' kind from the values (see tokens_per_batch), may ask the device; once per
+// table, and only for layers that a sparse table would bring a plan.  So the kernels that run, and with them the order of
+// their sums, do not hang on when an answer arrives.
+int plan_parts(const Tensor& table, int64_t n, int cin, int cout, int kk, int code, bool may_ask, void* stream) {
+    if (!svtad_plan_wanted(n, cin, cout, kk, code, 0.0)) return 0;
+    double density = density_of(table);
+    if (density < 0 && may_ask && !capturing(stream)) {
+        if (auto f = store().find(table, true)) {
+            density = static_cast<double>(at::ge(table, 0).sum().item<int64_t>()) / static_cast<double>(table.numel());
+            std::lock_guard<std::mutex> hold(f->mu);
+            f->density = density;
         }
     }
-    p.use = svtad_plan_wanted(n, cin, cout, kk, code, f->density) & parts;
-    if (p.use) p.data = f->plan;
-    return p;
+    return density < 0 ? 0 : svtad_plan_wanted(n, cin, cout, kk, code, density);
 }
 
 // tokens_per_batch of a call on [B, N, C] features: N when the table's indices are local to each batch row, else 0.
@@ -354,7 +354,8 @@ struct SparseConvBackward : public torch::autograd::Node {
     Dims d;
     at::ScalarType w_dtype, b_dtype;                     // of the parameters
     Tensor status;
-    Plan plan;
+    Tensor plan;                                         // the forward's, with its row order; undefined without one
+    bool lists = false;                                  // the weight gradient goes by pair lists, made by the backward
     bool released = false;
 
     std::string name() const override { return "SparseConv2dBackward"; }
@@ -364,7 +365,7 @@ struct SparseConvBackward : public torch::autograd::Node {
         x.reset_data();
         table.reset_data();
         weight.reset_data();
-        plan = Plan();
+        plan.reset();
         released = true;
     }
 
@@ -400,9 +401,12 @@ struct SparseConvBackward : public torch::autograd::Node {
         const int op = need_w ? (st.defined() ? SVTAD_OP_BWD : SVTAD_OP_WGRAD) : SVTAD_OP_DGRAD;
         const size_t bytes = need_w || st.defined() ? svtad_workspace_bytes(op, d.n, d.cin, d.cout, d.kk, code) : 0;
         if (bytes) ws = empty_on({static_cast<int64_t>(bytes)}, at::kByte, dev);
-        check(svtad_conv_bwd_typed(ptr(gy), ptr(xc), iptr(nbr), ptr(wc), mptr(gx), mptr(gw), mptr(gb), d.n, d.cin, d.cout,
-                                   d.kk, static_cast<int>(d.tpb), code, dtype_code(gdt), ptr(plan.data), plan.use, iptr(st),
-                                   mptr(ws), bytes, stream));
+        const int make = lists && need_w ? SVTAD_PLAN_PAIRS : 0, use = (plan.defined() ? SVTAD_PLAN_ROWS : 0) | make;
+        Tensor pl = plan;
+        if (make && !pl.defined()) pl = empty_on({static_cast<int64_t>(svtad_plan_bytes(d.n, d.kk))}, at::kByte, dev);
+        check(svtad_conv_bwd_planned(ptr(gy), ptr(xc), iptr(nbr), ptr(wc), mptr(gx), mptr(gw), mptr(gb), d.n, d.cin, d.cout,
+                                     d.kk, static_cast<int>(d.tpb), code, dtype_code(gdt), pl.defined() ? mptr(pl) : nullptr, use,
+                                     make, iptr(st), mptr(ws), bytes, stream));
         out[0] = gx;
         if (task_should_compute_output(1)) out[1] = gw.scalar_type() == w_dtype ? gw : gw.to(w_dtype);
         if (need_b) out[2] = gb.scalar_type() == b_dtype ? gb : gb.to(b_dtype);
@@ -433,8 +437,8 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
     void* stream = stream_of(dev);
     const bool grad = at::GradMode::is_enabled() &&
                       (x.requires_grad() || weight.requires_grad() || (bias.defined() && bias.requires_grad()));
-    Tensor y, nbr, status;
-    Plan plan;
+    Tensor y, nbr, status, plan;
+    int parts = 0;
     {
         at::NoGradGuard no_grad;
         d.tpb = batched ? tokens_per_batch(table, x.size(0), x.size(1), d.kk, local) : 0;
@@ -447,9 +451,13 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
             y = empty_on({d.n, d.cout}, dt, dev);
         }
         if (grad && x.requires_grad()) status = status_for(table, nbr, d.n, d.kk, d.tpb, stream);
-        plan = plan_for(table, nbr, d.n, d.cin, d.cout, d.kk, code, d.tpb, grad ? USE_ROWS | USE_PAIRS : USE_ROWS, stream);
+        parts = plan_parts(table, d.n, d.cin, d.cout, d.kk, code, batched && local < 0, stream);
+        if (parts & SVTAD_PLAN_ROWS) {
+            plan = empty_on({static_cast<int64_t>(svtad_plan_bytes(d.n, d.kk))}, at::kByte, dev);
+            check(svtad_plan_build_parts(iptr(nbr), d.n, d.kk, static_cast<int>(d.tpb), SVTAD_PLAN_ROWS, mptr(plan), stream));
+        }
         check(svtad_conv_fwd_planned(ptr(xc), iptr(nbr), ptr(wc), ptr(bc), mptr(y), d.n, d.cin, d.cout, d.kk,
-                                     static_cast<int>(d.tpb), code, plan.use & USE_ROWS ? ptr(plan.data) : nullptr, stream));
+                                     static_cast<int>(d.tpb), code, ptr(plan), stream));
     }
     if (grad) {
         auto node = std::shared_ptr<SparseConvBackward>(new SparseConvBackward(), torch::autograd::deleteNode);
@@ -459,6 +467,7 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
         node->b_dtype = bias.defined() ? bias.scalar_type() : dt;
         node->status = status;
         node->plan = plan;
+        node->lists = (parts & SVTAD_PLAN_PAIRS) != 0;
         node->x = torch::autograd::SavedVariable(x, false);
         node->table = torch::autograd::SavedVariable(table, false);
         node->weight = torch::autograd::SavedVariable(weight_c, false);
@@ -478,7 +487,7 @@ Tensor table_init(int64_t B, int64_t T, int64_t h, int64_t w, int64_t ksize, at:
     Tensor out = empty_on({B, T * h * w, ksize * ksize}, at::kInt, dev);
     check(svtad_table_init(static_cast<int>(B), static_cast<int>(T), static_cast<int>(h), static_cast<int>(w),
                            static_cast<int>(ksize), static_cast<int32_t*>(mptr(out)), stream_of(dev)));
-    mark_symmetric(out, true, true);
+    mark_symmetric(out, true, expected_density(T * h * w, T * h * w, h, w, ksize));
     return out;
 }
 
@@ -491,7 +500,7 @@ std::pair<Tensor, Tensor> table_build(const Tensor& scores_in, int64_t k, int64_
     check(svtad_table_build(static_cast<const float*>(ptr(scores)), static_cast<int>(n_seg), static_cast<int>(L),
                             static_cast<int>(k), static_cast<int>(h), static_cast<int>(w), static_cast<int>(ksize),
                             static_cast<int32_t*>(mptr(kept)), static_cast<int32_t*>(mptr(table)), stream_of(dev)));
-    mark_symmetric(table, true);
+    mark_symmetric(table, true, expected_density(L, k, h, w, ksize));
     return {kept, table};
 }
 
@@ -520,7 +529,7 @@ Tensor table_remap(const Tensor& table_in, const Tensor& idx_in, const Tensor& s
     check(svtad_table_remap(iptr(table), static_cast<const int64_t*>(ptr(idx)), static_cast<int>(B), static_cast<int>(n_prev),
                             static_cast<int>(n_new), static_cast<int>(kk), static_cast<int32_t*>(mptr(scratch)),
                             static_cast<int32_t*>(mptr(out)), stream_of(dev)));
-    if (sym) mark_symmetric(out, sym->built);
+    if (sym) mark_symmetric(out, sym->built, pruned_density(density_of(table_in), kk, n_prev, n_new));
     return out;
 }
 
@@ -539,7 +548,7 @@ std::pair<Tensor, Tensor> table_select_remap(const Tensor& scores_in, const Tens
                                    static_cast<int>(n_prev), static_cast<int>(k), static_cast<int>(kk),
                                    static_cast<int32_t*>(mptr(kept)), static_cast<int64_t*>(mptr(idx)),
                                    static_cast<int32_t*>(mptr(out)), stream_of(dev)));
-    if (sym) mark_symmetric(out, sym->built);
+    if (sym) mark_symmetric(out, sym->built, pruned_density(density_of(table_in), kk, n_prev, k));
     return {idx, out};
 }
 

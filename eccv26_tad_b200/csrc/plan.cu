@@ -9,8 +9,8 @@
 // Any permutation is a correct order, and a row's own sum does not depend on it: taps that a tile skips would have added
 // zeros.
 //
-// One launch of clusters of eight CTAs: cluster k < kk lists tap k, the last one sorts.  Latency bounds it (18 880 rows:
-// a table of 680 KB); every row is looked at twice, the counts meet in distributed shared memory in between.
+// One launch of clusters of eight CTAs: one sorts, one per tap lists.  Latency bounds it (18 880 rows: a table of
+// 680 KB); every row is looked at twice, the counts meet in distributed shared memory in between.
 #include <atomic>
 
 #include "plan.cuh"
@@ -200,10 +200,10 @@ __device__ void sort_rows(const int32_t* __restrict__ nbr, long n, int kk, const
 }
 
 __global__ void __launch_bounds__(PLAN_THREADS)
-plan_kernel(const int32_t* __restrict__ nbr, long n, int kk, int tpb, PlanRing ring, PlanOut o) {
+plan_kernel(const int32_t* __restrict__ nbr, long n, int kk, int tpb, int sorts, PlanRing ring, PlanOut o) {
     extern __shared__ __align__(16) unsigned char p_smem[];
     __shared__ int s_w[PLAN_WARPS + 1];
-    const int job = blockIdx.x / PLAN_G;
+    const int job = blockIdx.x / PLAN_G + (sorts ? 0 : 1);
     pdl_wait();
     pdl_trigger();
     if (job == 0) sort_rows(nbr, n, kk, ring, o, *reinterpret_cast<SortSmem*>(p_smem), s_w);      // the longest first
@@ -225,8 +225,14 @@ extern "C" const int32_t* svtad_plan_counts(const void* plan, int64_t n, int kk)
 }
 
 extern "C" int svtad_plan_build(const int32_t* nbr, int64_t n, int kk, int tokens_per_batch, void* plan, void* stream) {
+    return svtad_plan_build_parts(nbr, n, kk, tokens_per_batch, SVTAD_PLAN_ROWS | SVTAD_PLAN_PAIRS, plan, stream);
+}
+
+extern "C" int svtad_plan_build_parts(const int32_t* nbr, int64_t n, int kk, int tokens_per_batch, int parts, void* plan,
+                                      void* stream) {
     SV_CHECK_ARG(svtad_plan_bytes(n, kk) > 0, "svtad_plan_build: no plan for %lld rows and %d taps", (long long)n, kk);
     SV_CHECK_ARG(nbr != nullptr && plan != nullptr && tokens_per_batch >= 0, "svtad_plan_build: bad argument");
+    SV_CHECK_ARG(parts > 0 && parts <= (SVTAD_PLAN_ROWS | SVTAD_PLAN_PAIRS), "svtad_plan_build: no such parts: %d", parts);
     SV_CHECK_ARG(reinterpret_cast<uintptr_t>(plan) % 256 == 0, "svtad_plan_build: plan is not 256-byte aligned");
     PlanView v;
     plan_layout(n, kk, plan, &v);
@@ -251,7 +257,8 @@ extern "C" int svtad_plan_build(const int32_t* nbr, int64_t n, int kk, int token
         SV_CUDA(cudaFuncSetAttribute(plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem)));
         ready.fetch_or(bit);
     }
-    SV_CUDA(launch_pdl(plan_kernel, dim3((unsigned)((kk + 1) * PLAN_G)), dim3(PLAN_THREADS), sizeof(SortSmem),
-                       (cudaStream_t)stream, PLAN_G, nbr, (long)n, kk, tokens_per_batch, ring, o));
+    const int sorts = parts & SVTAD_PLAN_ROWS ? 1 : 0, lists = parts & SVTAD_PLAN_PAIRS ? kk : 0;
+    SV_CUDA(launch_pdl(plan_kernel, dim3((unsigned)((sorts + lists) * PLAN_G)), dim3(PLAN_THREADS), sorts ? sizeof(SortSmem) : 0,
+                       (cudaStream_t)stream, PLAN_G, nbr, (long)n, kk, tokens_per_batch, sorts, ring, o));
     return SVTAD_OK;
 }

@@ -163,18 +163,22 @@ int svtad_conv_bwd(const void* gy, const void* x, const int32_t* nbr, const void
 /*
  * Work plan of a table (no counterpart in the reference): rows ordered so that those with the same neighbors sit
  * together, and per tap the list of (row, neighbor) pairs that exist, so that the kernels of a large layer skip the
- * neighbors that are not there (at keep 30 % two thirds of a 3x3 stencil).  A plan belongs to one table and one
- * tokens_per_batch and stays valid while the table does; any number of layers may share it.
- *   svtad_plan_wanted  which parts of a plan gain a layer of this size more than making it costs: bit 0 the row order
- *                      (forward, input gradient), bit 1 the pair lists (weight gradient); density = pairs per row and tap
- *                      of the table, negative where it is not known
+ * neighbors that are not there (at keep 30 % two thirds of a 3x3 stencil).  A plan belongs to what the table held when
+ * svtad_plan_build ran on the stream, to its n and kk and to one tokens_per_batch: whoever writes to the table, by whatever
+ * route, makes the plan anew.  Any number of layers may share it until then.
+ *   svtad_plan_wanted  which parts of a plan gain one layer of this size, in one pass, more than making them costs:
+ *                      SVTAD_PLAN_ROWS the row order (forward, input gradient), SVTAD_PLAN_PAIRS the pair lists (weight
+ *                      gradient); density = pairs per row and tap of the table, negative where it is not known
  *   svtad_plan_bytes   size of a plan (0: no plan for such a table: more than 131072 rows)
- *   svtad_plan_build   makes it in `plan` (device memory, 256-byte aligned)
+ *   svtad_plan_build   makes it in `plan` (device memory, 256-byte aligned); _parts: only the parts named
  *   svtad_plan_counts  where in a plan the kk lists' lengths are (int32, device memory)
  */
 int svtad_plan_wanted(int64_t n, int cin, int cout, int kk, int dtype, double density);
+#define SVTAD_PLAN_ROWS 1
+#define SVTAD_PLAN_PAIRS 2
 size_t svtad_plan_bytes(int64_t n, int kk);
 int svtad_plan_build(const int32_t* nbr, int64_t n, int kk, int tokens_per_batch, void* plan, void* stream);
+int svtad_plan_build_parts(const int32_t* nbr, int64_t n, int kk, int tokens_per_batch, int parts, void* plan, void* stream);
 const int32_t* svtad_plan_counts(const void* plan, int64_t n, int kk);
 
 /* svtad_conv_fwd with a plan (NULL: none).  Same results. */
@@ -182,14 +186,20 @@ int svtad_conv_fwd_planned(const void* x, const int32_t* nbr, const void* w, con
                            int cin, int cout, int kk, int tokens_per_batch, int dtype, const void* plan, void* stream);
 
 /*
- * svtad_conv_bwd with a plan (NULL: none), the parts of it to use (bits as svtad_plan_wanted's) and with the type of gw and gb chosen by the caller: grad_dtype is dtype, or
- * SVTAD_F32 for fp32 master parameters of a 16-bit layer (mixed precision).  The values are the same - one rounding to
- * dtype - and are written as fp32, which saves the separate conversion of the gradient.
+ * svtad_conv_bwd with a plan (NULL: none), the parts of it to use (bits as svtad_plan_wanted's) and with the type of gw
+ * and gb chosen by the caller: grad_dtype is dtype, or SVTAD_F32 for fp32 master parameters of a 16-bit layer (mixed
+ * precision).  The values are the same - one rounding to dtype - and are written as fp32, which saves the separate
+ * conversion of the gradient.  svtad_conv_bwd_planned with plan_make = SVTAD_PLAN_PAIRS first makes the pair lists in
+ * `plan`, next to the input gradient.
  */
 int svtad_conv_bwd_typed(const void* gy, const void* x, const int32_t* nbr, const void* w, void* gx, void* gw,
                          void* gb, int64_t n, int cin, int cout, int kk, int tokens_per_batch, int dtype,
                          int grad_dtype, const void* plan, int plan_use, const int32_t* table_status, void* workspace,
                          size_t workspace_bytes, void* stream);
+int svtad_conv_bwd_planned(const void* gy, const void* x, const int32_t* nbr, const void* w, void* gx, void* gw,
+                           void* gb, int64_t n, int cin, int cout, int kk, int tokens_per_batch, int dtype,
+                           int grad_dtype, void* plan, int plan_use, int plan_make, const int32_t* table_status,
+                           void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * svtad_conv_wgrad for callers that cannot allocate device memory (no counterpart in the reference).

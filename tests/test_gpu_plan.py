@@ -148,3 +148,168 @@ def test_module_with_a_layer_that_wants_a_plan(keep, table_kind):
         assert torch.equal(y, ey) and torch.equal(gx, egx)
         assert oconv.rel_err(f32np(gw), f32np(egw)) < 8e-3 and oconv.rel_err(f32np(gb), f32np(egb)) < 8e-3
     assert ops.device_error() == 0
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# The module's plans: made from what the table holds when the kernels run, by a rule that nothing asynchronous enters.
+# C = 512 at 18 880 rows, keep 0.3: a layer whose forward, input gradient and weight gradient go by a plan.
+# ---------------------------------------------------------------------------------------------------------------------
+def _scores(T, seed):
+    return torch.randn(T, 196, device="cuda", generator=torch.Generator("cuda").manual_seed(seed))
+
+
+def _layer(C, ks, n, seed, Co=None):
+    import eccv26_tad_b200 as sv
+    g = torch.Generator("cuda").manual_seed(seed)
+    m = sv.SparseConv2d(C, Co or C, kernel_size=ks).cuda().bfloat16()
+    x = torch.randn(n, C, device="cuda", generator=g).bfloat16().requires_grad_(True)
+    gy = torch.randn(n, Co or C, device="cuda", generator=g).bfloat16()
+    return m, x, gy
+
+
+def _pass(m, x, table, gy):
+    y = m(x, table)
+    return (y.detach().reshape(gy.shape),) + torch.autograd.grad(y, (x, m.weight, m.bias), gy.reshape(y.shape))
+
+
+def _unplanned(m, x, table, gy):
+    from eccv26_tad_b200 import ops
+    w, flat = m.weight.detach(), table.reshape(-1, m.weight.shape[0])
+    xf = x.detach().reshape(-1, x.shape[-1])
+    gw, gb = ops.conv_wgrad(gy, xf, flat, w.shape[0])
+    return ops.conv_fwd(xf, flat, w, m.bias.detach()), ops.conv_dgrad(gy, flat, w, assume_symmetric=True), gw, gb
+
+
+def _close(got, want):
+    for a, b in zip(got, want):
+        # both round the same fp32 sums, made in another order, once: less than one bf16 step apart
+        assert oconv.rel_err(f32np(a).reshape(b.shape), f32np(b)) < 8e-3
+
+
+def _wanted(n, C, kk, density):
+    from eccv26_tad_b200 import _lib
+    return _lib.load().svtad_plan_wanted(n, C, C, kk, _lib.BF16, density)
+
+
+def test_a_table_rewritten_behind_the_version_counter():
+    """The C ABI (or a replayed graph that holds the selection) writes another table into the same memory."""
+    import eccv26_tad_b200 as sv
+    from eccv26_tad_b200 import _lib
+    T = 320
+    kept, table = sv.build_neighbor_table(_scores(T, 1), 0.3, 14, 14)
+    n = table.shape[0]
+    assert _wanted(n, 512, 9, 0.35) == 3
+    m, x, gy = _layer(512, 3, n, 1)
+    for _ in range(2):
+        _close(_pass(m, x, table, gy), _unplanned(m, x, table, gy))
+        torch.cuda.synchronize()
+    other, version = _scores(T, 2), table._version
+    _lib.check(_lib.load().svtad_table_build(other.data_ptr(), T, 196, n // T, 14, 14, 3, kept.data_ptr(), table.data_ptr(),
+                                             torch.cuda.current_stream().cuda_stream))
+    assert table._version == version
+    _close(_pass(m, x, table, gy), _unplanned(m, x, table, gy))
+
+
+def test_graph_captured_behind_a_warm_up_on_the_same_stream():
+    """Warm-up and capture on one stream; between replays the table is refreshed in place, and memory that the warm-up
+    gave back is used by others."""
+    import eccv26_tad_b200 as sv
+    T = 320
+    tables = [sv.build_neighbor_table(_scores(T, s), 0.3, 14, 14)[1] for s in (3, 4, 5)]
+    table = tables[0]
+    m, x, gy = _layer(512, 3, table.shape[0], 2)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        for _ in range(2):
+            _pass(m, x, table, gy)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            out = _pass(m, x, table, gy)
+    torch.cuda.current_stream().wait_stream(s)
+    for new in tables[1:]:
+        table.copy_(new)
+        junk = [torch.full((1 << 20,), -7, dtype=torch.int32, device="cuda") for _ in range(4)]
+        g.replay()
+        torch.cuda.synchronize()
+        _close(out, _unplanned(m, x, new, gy))
+        del junk
+
+
+def test_one_table_serves_layers_of_different_stencils():
+    """225 * m entries are m * 25 rows of 9 taps as well as m * 9 rows of 25: each layer reads the table its own way."""
+    import eccv26_tad_b200 as sv
+    flat = sv.get_initial_neighbor_indices(15, 15, 40, "cuda", 1, 5).reshape(-1)          # 9 000 rows of 25
+    flat = torch.where(torch.rand(flat.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(6)) < 0.3, flat, -1)
+    for C, ks in ((512, 3), (512, 5), (512, 3)):
+        kk = ks * ks
+        n = flat.numel() // kk
+        m, x, gy = _layer(C, ks, n, 3)
+        x3 = x.detach().view(1, n, C).requires_grad_(True)                                 # [B, N, C]: the density is asked for
+        y, gx, gw, gb = _pass(m, x3, flat, gy)
+        ey, _, egw, egb = _unplanned(m, x3, flat, gy)
+        _close((y, gw, gb), (ey, egw, egb))
+        # not a symmetric table: the input gradient is the scatter form's
+        w, egx = m.weight.detach(), torch.zeros(n, C, device="cuda")
+        t = flat.view(n, kk).long()
+        for k in range(kk):
+            i = ((t[:, k] >= 0) & (t[:, k] < n)).nonzero().view(-1)
+            egx.index_add_(0, t[i, k], gy[i].float() @ w[k].float().t())
+        _close((gx.view(n, C),), (egx,))
+
+
+@pytest.mark.parametrize("C,ks,T,keep,given", [(512, 3, 320, 0.3, True), (512, 3, 160, 0.5, True), (512, 3, 160, 0.6, True),
+                                               (512, 3, 80, 1.0, True), (512, 5, 25, 0.38, False), (768, 3, 80, 0.3, False),
+                                               (1024, 3, 30, 0.3, True)])
+def test_passes_repeat_bit_for_bit(C, ks, T, keep, given):
+    """Neither the first pass on a table nor one that follows a synchronisation takes other kernels than the rest."""
+    import eccv26_tad_b200 as sv
+    if keep == 1.0:
+        table = sv.get_initial_neighbor_indices(14, 14, T, "cuda", 1, ks)[0]
+    else:
+        table = sv.build_neighbor_table(_scores(T, 7), keep, 14, 14, ks)[1]
+    n = table.shape[0]
+    table = table.view(1, n, ks * ks)
+    m, x, gy = _layer(C, ks, n, 4)
+    x = x.detach().view(1, n, C).requires_grad_(True)
+    first = None
+    for i in range(6):
+        t = table.clone() if given and i in (0, 3) else (table if first is None or not given else t)
+        got = _pass(m, x, t, gy)
+        if i % 2:
+            torch.cuda.synchronize()
+        first = first or got
+        assert all(torch.equal(a, b) for a, b in zip(got, first))
+    with torch.no_grad():
+        assert torch.equal(m(x, t).view(n, C), first[0])
+    _close(first, _unplanned(m, x, table, gy))
+
+
+def test_two_streams_share_a_table():
+    import eccv26_tad_b200 as sv
+    table = sv.build_neighbor_table(_scores(320, 8), 0.3, 14, 14)[1]
+    layers = [_layer(512, 3, table.shape[0], s) for s in (5, 6)]
+    want = [_unplanned(m, x, table, gy) for m, x, gy in layers]
+    streams = [torch.cuda.Stream() for _ in layers]
+    torch.cuda.synchronize()
+    outs = []
+    for _ in range(3):
+        for s, (m, x, gy) in zip(streams, layers):
+            with torch.cuda.stream(s):
+                outs.append(_pass(m, x, table, gy))
+    torch.cuda.synchronize()
+    for i, got in enumerate(outs):
+        _close(got, want[i % 2])
+
+
+def test_tables_made_in_inference_mode():
+    import eccv26_tad_b200 as sv
+    m, x, _ = _layer(512, 3, 62720, 9)
+    with torch.inference_mode():
+        full = sv.get_initial_neighbor_indices(14, 14, 320, "cuda", 1)
+        sparse = sv.build_neighbor_table(_scores(320, 9), 0.3, 14, 14)[1]
+        for table in (full, sparse):
+            n = table.numel() // 9
+            for _ in range(2):
+                y = m(x[:n], table)
+            assert torch.equal(y, m(x[:n], table.clone()))

@@ -243,3 +243,17 @@ def test_workspace_sizes_do_not_depend_on_the_concurrency_hint():
                 assert got == base[s], (hint, s)
     finally:
         lib.svtad_set_concurrency(start)
+
+
+def test_a_plan_is_wanted_where_one_layer_pays_for_it():
+    """svtad_plan_wanted: what a plan saves one layer in one pass has to exceed what making it takes."""
+    lib = _lib.load()
+
+    def wanted(n, c, kk, density, dtype=_lib.BF16):
+        return lib.svtad_plan_wanted(n, c, c, kk, dtype, density)
+    assert wanted(18880, 1024, 9, 0.35) == 3 and wanted(18880, 512, 9, 0.35) == 3 and wanted(18880, 384, 9, 0.35, _lib.F16) == 3
+    assert wanted(19600, 192, 9, 0.51) == 0 and wanted(43200, 128, 9, 0.55) == 0            # 17 to 25 us for 5 to 15
+    assert wanted(18880, 256, 9, 0.35) == 0 and wanted(1770, 1024, 9, 0.35) == 0
+    assert wanted(62720, 512, 9, 0.91) == 0 and wanted(50240, 384, 9, 0.75) == 0            # hardly a neighbor missing
+    assert wanted(18880, 256, 25, 0.28) == 2 and wanted(2360, 512, 25, 0.52) == 0           # 5x5: the lists alone
+    assert wanted(18880, 1024, 9, 0.35, _lib.F32) == 0 and wanted(140000, 1024, 9, 0.35) == 0 and wanted(18880, 1024, 1, 0.35) == 0
