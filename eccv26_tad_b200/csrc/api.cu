@@ -93,25 +93,34 @@ extern "C" int svtad_device_error(int32_t* code_out) {
     return tc_read_error(code_out);
 }
 
+// weight gradient alone, by a plan's pair lists or not
+static size_t wgrad_ws_bytes(int64_t n, int cin, int cout, int kk, int dtype, bool by_pairs) {
+    if (n <= 0 || cin <= 0 || cout <= 0 || kk <= 0) return 0;
+    const bool tc = tc_supported(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype);
+    if (by_pairs && tc && forced_path() != 1 && pairs_wgrad_wanted(cin, kk)) return pairs_wgrad_ws_bytes(cin, cout);
+    const size_t a = simt_wgrad_ws_bytes(n, cin, cout, kk, dtype), b = tc ? tc_wgrad_ws_bytes(n, cin, cout, kk) : 0;
+    return a > b ? a : b;
+}
+
 extern "C" size_t svtad_workspace_bytes(int op, int64_t n, int cin, int cout, int kk, int dtype) {
     if (n <= 0 || cin <= 0 || cout <= 0 || kk <= 0) return 0;
     switch (op) {
         case SVTAD_OP_FWD: return 0;
         case SVTAD_OP_DGRAD: return align_up((size_t)n * cin * sizeof(float), 256);   // scatter form only
-        case SVTAD_OP_WGRAD: {
-            size_t a = simt_wgrad_ws_bytes(n, cin, cout, kk);
-            size_t b = tc_supported(op, n, cin, cout, kk, dtype) ? tc_wgrad_ws_bytes(n, cin, cout, kk) : 0;
-            if (b > 0 && pairs_wgrad_wanted(cin, kk)) {
-                const size_t c = pairs_wgrad_ws_bytes(cin, cout);
-                b = b > c ? b : c;
-            }
+        case SVTAD_OP_WGRAD: return wgrad_ws_bytes(n, cin, cout, kk, dtype, false);
+        case SVTAD_OP_BWD: {  // with or without a plan
+            const size_t a = svtad_bwd_workspace_bytes(n, cin, cout, kk, dtype, 0, 1);
+            const size_t b = svtad_bwd_workspace_bytes(n, cin, cout, kk, dtype, SVTAD_PLAN_PAIRS, 1);
             return a > b ? a : b;
         }
-        case SVTAD_OP_BWD:   // both halves run at the same time: the two workspaces sit side by side
-            return align_up(svtad_workspace_bytes(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype), 256) +
-                   svtad_workspace_bytes(SVTAD_OP_DGRAD, n, cin, cout, kk, dtype);
     }
     return 0;
+}
+
+extern "C" size_t svtad_bwd_workspace_bytes(int64_t n, int cin, int cout, int kk, int dtype, int plan_use, int scatter) {
+    // both halves run at the same time: the two workspaces sit side by side
+    return align_up(wgrad_ws_bytes(n, cin, cout, kk, dtype, (plan_use & SVTAD_PLAN_PAIRS) != 0), 256) +
+           (scatter ? svtad_workspace_bytes(SVTAD_OP_DGRAD, n, cin, cout, kk, dtype) : 0);
 }
 
 // Which parts of a plan gain a layer more than it costs to make them for this one layer and call: the row order (forward,
@@ -206,7 +215,7 @@ extern "C" int svtad_conv_dgrad(const void* gy, const int32_t* nbr, const void* 
 
 static int conv_wgrad_typed(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin,
                             int cout, int kk, int tokens_per_batch, int dtype, int grad_dtype, const void* plan,
-                            void* workspace, size_t workspace_bytes, void* stream) {
+                            void* workspace, size_t workspace_bytes, void* stream, bool fit = false) {
     int rc = check_common("svtad_conv_wgrad", n, cin, cout, kk, tokens_per_batch, dtype);
     if (rc) return rc;
     SV_CHECK_ARG(gw != nullptr, "svtad_conv_wgrad: gw is null");
@@ -223,11 +232,22 @@ static int conv_wgrad_typed(const void* gy, const void* x, const int32_t* nbr, v
     if (use_tc(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype)) {
         if (plan != nullptr && pairs_wgrad_wanted(cin, kk))
             return pairs_wgrad(gy, x, plan, gw, gb, n, cin, cout, kk, dtype, grad_dtype, workspace, workspace_bytes, s);
-        return tc_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace, workspace_bytes, s);
+        return tc_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace, workspace_bytes, fit, s);
     }
     if (forced_path() == 2)
         return set_error(SVTAD_ERR_UNSUPPORTED, "svtad_conv_wgrad: tensor-core path forced but shape/dtype unsupported");
     return simt_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, workspace, workspace_bytes, s);
+}
+
+size_t svtad::wgrad_least_ws_bytes(int64_t n, int cin, int cout, int kk, int dtype, bool with_bias) {
+    if (n <= 0 || cin <= 0 || cout <= 0 || kk <= 0) return 0;
+    return use_tc(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype) ? tc_wgrad_partials(1, with_bias, cin, cout, kk)
+                                                           : simt_wgrad_ws_bytes(n, cin, cout, kk, dtype);
+}
+
+int svtad::conv_wgrad_fit(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin, int cout,
+                          int kk, int tpb, int dtype, void* ws, size_t ws_bytes, cudaStream_t s) {
+    return conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tpb, dtype, dtype, nullptr, ws, ws_bytes, s, true);
 }
 
 extern "C" int svtad_conv_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb,
@@ -280,7 +300,7 @@ extern "C" int svtad_conv_bwd_planned(const void* gy, const void* x, const int32
                                 workspace, workspace_bytes, stream);
     }
     // workspace = [weight-gradient part | input-gradient part (scatter form, only with a status word)]
-    const size_t w_part = align_up(svtad_workspace_bytes(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype), 256);
+    const size_t w_part = svtad_bwd_workspace_bytes(n, cin, cout, kk, dtype, pairs_plan != nullptr ? plan_use : 0, 0);
     const size_t d_part = table_status != nullptr ? svtad_workspace_bytes(SVTAD_OP_DGRAD, n, cin, cout, kk, dtype) : 0;
     if (n > 0 && (workspace == nullptr || workspace_bytes < w_part + d_part))
         return set_error(SVTAD_ERR_WORKSPACE, "svtad_conv_bwd: workspace %zu < %zu bytes", workspace_bytes,

@@ -53,7 +53,7 @@ int simt_dgrad_scatter(const ConvArgs& p, const int32_t* status, float* ws, cuda
 int simt_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n,
                int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes,
                cudaStream_t s);
-size_t simt_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk);
+size_t simt_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk, int dtype);
 
 // fp32 kernels over compacted pairs (conv_f32.cu); channel counts are multiples of 4
 bool f32_supported(int cin, int cout, int kk, int dtype);
@@ -67,10 +67,16 @@ size_t f32_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk);
 bool tc_supported(int op, int64_t n, int cin, int cout, int kk, int dtype);
 int tc_fwd(const ConvArgs& p, cudaStream_t s);
 int tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s);
+// fit: take no more token splits than the workspace holds the partials of (at least one)
 int tc_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n,
-             int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes,
+             int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes, bool fit,
              cudaStream_t s);
 size_t tc_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk);
+size_t tc_wgrad_partials(long splits, bool with_bias, int cin, int cout, int kk);     // of that many token splits
+// svtad_conv_wgrad in a workspace of a given size: the smallest it can do with, and the call
+size_t wgrad_least_ws_bytes(int64_t n, int cin, int cout, int kk, int dtype, bool with_bias);
+int conv_wgrad_fit(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin, int cout, int kk,
+                   int tpb, int dtype, void* ws, size_t ws_bytes, cudaStream_t s);
 int tc_read_error(int32_t* code_out);
 int tc_set_share(int n);
 int tc_get_share();
@@ -82,8 +88,7 @@ int tc_set_share_floor(int n);
     int prefix##_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s);                           \
     int prefix##_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n,    \
                        int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws,             \
-                       size_t ws_bytes,                                                                     \
-                       cudaStream_t s);
+                       size_t ws_bytes, bool fit, cudaStream_t s);
 SV_DECLARE_TC_FAMILY(hybrid)
 // forward / dgrad on CTA pairs (conv_tc_pair.cu)
 int pair_fwd(const ConvArgs& p, cudaStream_t s);

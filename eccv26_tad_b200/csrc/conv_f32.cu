@@ -547,10 +547,11 @@ int f32_fwd(const ConvArgs& p, cudaStream_t s) { return dispatch_conv_f32<false>
 int f32_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) { return dispatch_conv_f32<true>(p, status, s); }
 
 // Token ranges: about two full loads of the GPU (four CTAs an SM), so that the centre tap's CTAs, which have every token
-// for a pair, do not outlast the rest; each range at least 128 tokens, the partials at most 64 MB.
+// for a pair, do not outlast the rest; each range at least 128 tokens, the partials of several ranges at most 31 MB, which
+// with the bias gradient's fit the built-in workspace of svtad_conv_wgrad_static.
 static int f32_wgrad_splits(int64_t n, int cin, int cout, int kk) {
     const long tiles = (long)kk * ((cin + 63) / 64) * ((cout + 63) / 64);
-    const long by_rows = (n + 127) / 128, by_size = (64l << 20) / ((long)kk * cin * cout * 4);
+    const long by_rows = (n + 127) / 128, by_size = (31l << 20) / ((long)kk * cin * cout * 4);
     long s = (8 * 148 + tiles - 1) / tiles;
     if (s > by_rows) s = by_rows;
     if (s > by_size) s = by_size;

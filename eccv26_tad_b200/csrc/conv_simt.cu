@@ -452,21 +452,20 @@ static int simt_wgrad_splits(int64_t n, int cin, int cout, int kk) {
     return (int)s;
 }
 
-size_t simt_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk) {
+size_t simt_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk, int dtype) {
+    if (f32_supported(cin, cout, kk, dtype)) return f32_wgrad_ws_bytes(n, cin, cout, kk);
     size_t w = (size_t)simt_wgrad_splits(n, cin, cout, kk) * kk * cin * cout * sizeof(float);
     size_t b = (size_t)bias_splits_for(n) * cout * sizeof(float);
-    const size_t generic = align_up(w, 256) + align_up(b, 256);
-    const size_t f32 = f32_supported(cin, cout, kk, SVTAD_F32) ? f32_wgrad_ws_bytes(n, cin, cout, kk) : 0;
-    return f32 > generic ? f32 : generic;
+    return align_up(w, 256) + align_up(b, 256);
 }
 
 int simt_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n,
                int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes,
                cudaStream_t s) {
     if (f32_supported(cin, cout, kk, dtype)) return f32_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tpb, ws, ws_bytes, s);
-    if (ws_bytes < simt_wgrad_ws_bytes(n, cin, cout, kk))
+    if (ws_bytes < simt_wgrad_ws_bytes(n, cin, cout, kk, dtype))
         return set_error(SVTAD_ERR_WORKSPACE, "svtad_conv_wgrad: workspace %zu < %zu bytes", ws_bytes,
-                         simt_wgrad_ws_bytes(n, cin, cout, kk));
+                         simt_wgrad_ws_bytes(n, cin, cout, kk, dtype));
     const int splits = simt_wgrad_splits(n, cin, cout, kk);
     const long n_w = (long)kk * cin * cout;
     float* ws_w = static_cast<float*>(ws);

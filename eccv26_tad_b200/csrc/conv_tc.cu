@@ -220,7 +220,8 @@ int tc_widest_bn(int cn) {
 //   (waves over the SMs) x (64-token steps per CTA + fixed cost) x (cycles per step at that BN)
 // plus the trip of the fp32 partials through memory (written by the main kernel, read by the reduction).
 // Cycles per step and the partials' rate are what these kernels were measured at on a B200.
-static WgradPlan wgrad_plan_for(int64_t n, int cin, int cout, int kk, bool with_bias, long sms) {
+// limit: most bytes the partials of several splits may take (0: any).
+static WgradPlan wgrad_plan_for(int64_t n, int cin, int cout, int kk, bool with_bias, long sms, size_t limit = 0) {
     const int nblocks = kk * ((cin + 63) / 64);
     long max_by_rows = (n + 2 * STAGE_K - 1) / (2 * STAGE_K);
     if (max_by_rows < 1) max_by_rows = 1;
@@ -252,6 +253,7 @@ static WgradPlan wgrad_plan_for(int64_t n, int cin, int cout, int kk, bool with_
             if (forced_s > 0 && c != (forced_s < max_by_rows ? forced_s : max_by_rows)) continue;
             const long tps = ((n + c - 1) / c + STAGE_K - 1) / STAGE_K * STAGE_K;
             const long splits = (n + tps - 1) / tps;
+            if (limit > 0 && splits > 1 && tc_wgrad_partials(splits, with_bias, cin, cout, kk) > limit) continue;
             const long waves = (ctas * splits + sms - 1) / sms;
             const double steps = (double)tps / STAGE_K + 12.0;          // + set-up, first operands, drain
             // one split needs no partials and no second launch
@@ -289,18 +291,24 @@ static PlanMemo& plan_slot(int64_t n, int cin, int cout, int kk, long key) {
 }
 static bool plan_overridden() { return getenv("SVTAD_TC_WGRAD_BN") != nullptr || getenv("SVTAD_TC_WGRAD_SPLITS") != nullptr; }
 
-WgradPlan tc_wgrad_plan(int64_t n, int cin, int cout, int kk, bool with_bias) {
+WgradPlan tc_wgrad_plan(int64_t n, int cin, int cout, int kk, bool with_bias, size_t limit) {
     const long sms = tc_plan_sms(), key = 2 * sms + with_bias;
+    if (limit > 0) {
+        const WgradPlan pl = tc_wgrad_plan(n, cin, cout, kk, with_bias, 0);
+        return tc_wgrad_plan_bytes(pl, cin, cout, kk) <= limit ? pl : wgrad_plan_for(n, cin, cout, kk, with_bias, sms, limit);
+    }
     if (plan_overridden()) return wgrad_plan_for(n, cin, cout, kk, with_bias, sms);
     PlanMemo& m = plan_slot(n, cin, cout, kk, key);
     if (!m.is(n, cin, cout, kk, key)) m = PlanMemo{n, cin, cout, kk, key, wgrad_plan_for(n, cin, cout, kk, with_bias, sms), 0};
     return m.plan;
 }
 
+size_t tc_wgrad_partials(long splits, bool with_bias, int cin, int cout, int kk) {
+    return align_up((size_t)splits * kk * cin * cout * sizeof(float), 256) +
+           (with_bias ? align_up((size_t)splits * cout * sizeof(float), 256) : 0);
+}
 size_t tc_wgrad_plan_bytes(const WgradPlan& pl, int cin, int cout, int kk) {
-    const size_t w = (size_t)pl.splits * kk * cin * cout * sizeof(float);
-    const size_t b = pl.ones_block ? (size_t)pl.splits * cout * sizeof(float) : 0;
-    return align_up(w, 256) + align_up(b, 256);
+    return tc_wgrad_partials(pl.splits, pl.ones_block != 0, cin, cout, kk);
 }
 
 // What callers are told to provide: enough for the plan under every concurrency hint, so that a workspace
@@ -401,8 +409,8 @@ int tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
 }
 
 int tc_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin, int cout,
-             int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes, cudaStream_t s) {
-    return hybrid_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tpb, dtype, grad_dtype, ws, ws_bytes, s);
+             int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes, bool fit, cudaStream_t s) {
+    return hybrid_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tpb, dtype, grad_dtype, ws, ws_bytes, fit, s);
 }
 
 }  // namespace svtad

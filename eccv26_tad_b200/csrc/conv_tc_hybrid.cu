@@ -865,8 +865,8 @@ static int launch_wgrad_hybrid(const void* gy, const void* x, const int32_t* nbr
 }
 
 int hybrid_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin, int cout,
-                 int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes, cudaStream_t s) {
-    const WgradPlan pl = tc_wgrad_plan(n, cin, cout, kk, gb != nullptr);
+                 int kk, int tpb, int dtype, int grad_dtype, void* ws, size_t ws_bytes, bool fit, cudaStream_t s) {
+    const WgradPlan pl = tc_wgrad_plan(n, cin, cout, kk, gb != nullptr, fit ? ws_bytes : 0);
     const size_t need = tc_wgrad_plan_bytes(pl, cin, cout, kk);
     if (ws_bytes < need)
         return set_error(SVTAD_ERR_WORKSPACE, "svtad_conv_wgrad: workspace %zu < %zu bytes", ws_bytes, need);

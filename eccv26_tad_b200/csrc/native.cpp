@@ -398,11 +398,11 @@ struct SparseConvBackward : public torch::autograd::Node {
         }
         if (need_w) gw = empty_on({d.kk, d.cin, d.cout}, gdt, dev);
         if (need_b) gb = empty_on({d.cout}, gdt, dev);
-        const int op = need_w ? (st.defined() ? SVTAD_OP_BWD : SVTAD_OP_WGRAD) : SVTAD_OP_DGRAD;
-        const size_t bytes = need_w || st.defined() ? svtad_workspace_bytes(op, d.n, d.cin, d.cout, d.kk, code) : 0;
-        if (bytes) ws = empty_on({static_cast<int64_t>(bytes)}, at::kByte, dev);
         const int make = lists && need_w ? SVTAD_PLAN_PAIRS : 0, use = (plan.defined() ? SVTAD_PLAN_ROWS : 0) | make;
         Tensor pl = plan;
+        const size_t bytes = need_w ? svtad_bwd_workspace_bytes(d.n, d.cin, d.cout, d.kk, code, use, st.defined())
+                                    : (st.defined() ? svtad_workspace_bytes(SVTAD_OP_DGRAD, d.n, d.cin, d.cout, d.kk, code) : 0);
+        if (bytes) ws = empty_on({static_cast<int64_t>(bytes)}, at::kByte, dev);
         if (make && !pl.defined()) pl = empty_on({static_cast<int64_t>(svtad_plan_bytes(d.n, d.kk))}, at::kByte, dev);
         check(svtad_conv_bwd_planned(ptr(gy), ptr(xc), iptr(nbr), ptr(wc), mptr(gx), mptr(gw), mptr(gb), d.n, d.cin, d.cout,
                                      d.kk, static_cast<int>(d.tpb), code, dtype_code(gdt), pl.defined() ? mptr(pl) : nullptr, use,

@@ -52,7 +52,7 @@ extern "C" size_t svtad_static_workspace_bytes(void) { return SVTAD_STATIC_WS_BY
 extern "C" int svtad_conv_wgrad_static(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb,
                                        int64_t n, int cin, int cout, int kk, int tokens_per_batch, int dtype,
                                        void* stream) {
-    const size_t need = svtad_workspace_bytes(SVTAD_OP_WGRAD, n, cin, cout, kk, dtype);
+    const size_t need = wgrad_least_ws_bytes(n, cin, cout, kk, dtype, gb != nullptr);
     if (need > SVTAD_STATIC_WS_BYTES)
         return set_error(SVTAD_ERR_WORKSPACE,
                          "svtad_conv_wgrad_static: this problem needs a %zu-byte workspace, the built-in one holds "
@@ -65,6 +65,6 @@ extern "C" int svtad_conv_wgrad_static(const void* gy, const void* x, const int3
     }
     // nothing in the workspace has to start at zero: every split writes its whole partial before the
     // reduction reads it, so the previous call's contents are simply overwritten
-    return svtad_conv_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, ws,
-                            SVTAD_STATIC_WS_BYTES, stream);
+    return conv_wgrad_fit(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, ws, SVTAD_STATIC_WS_BYTES,
+                          (cudaStream_t)stream);
 }

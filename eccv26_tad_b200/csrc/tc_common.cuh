@@ -312,7 +312,7 @@ struct WgradPlan {
     int bn, n_nblk, n_pairs, splits, ones_block;
     long tokens_per_split;
 };
-WgradPlan tc_wgrad_plan(int64_t n, int cin, int cout, int kk, bool with_bias);
+WgradPlan tc_wgrad_plan(int64_t n, int cin, int cout, int kk, bool with_bias, size_t limit = 0);
 size_t tc_wgrad_plan_bytes(const WgradPlan& pl, int cin, int cout, int kk);
 
 // fixed-order reduction of per-split fp32 partials into the 16-bit gradient tensors

@@ -113,8 +113,13 @@ int svtad_table_select_remap(const float* scores, const int32_t* table_in, int B
 int svtad_table_check(const int32_t* nbr, int64_t n, int kk, int tokens_per_batch,
                       int32_t* status, void* stream);
 
-/* Workspace size (bytes) that the given op needs for the given problem (0 for the forward). */
+/*
+ * Workspace size (bytes) that the given op needs for the given problem (0 for the forward); for SVTAD_OP_BWD enough
+ * with and without a plan.  svtad_bwd_workspace_bytes: what one call of svtad_conv_bwd_typed / _planned needs with that
+ * plan_use (0: no plan), with (scatter != 0) or without a table status.
+ */
 size_t svtad_workspace_bytes(int op, int64_t n, int cin, int cout, int kk, int dtype);
+size_t svtad_bwd_workspace_bytes(int64_t n, int cin, int cout, int kk, int dtype, int plan_use, int scatter);
 
 /*
  * y[i,co] = bias[co] + sum_k sum_ci x[nbr[i,k]+off(i), ci] * w[k,ci,co]; bias may be NULL.
@@ -209,8 +214,10 @@ int svtad_conv_bwd_planned(const void* gy, const void* x, const int32_t* nbr, co
  * of SVTAD_STATIC_WS_BYTES that is part of the library's device image, so every GPU that loads the
  * library holds that much memory until the process exits.  The call itself allocates nothing
  * (no cudaMalloc / cudaFree, no allocating library routine).
- *   - Limit: problems with svtad_workspace_bytes(SVTAD_OP_WGRAD, ...) > SVTAD_STATIC_WS_BYTES are
- *     refused with SVTAD_ERR_WORKSPACE (C = 192 and 256 at 3x3 fit; C = 1024 does not).
+ *   - Limit: problems of which the array does not hold the smallest workspace (16-bit tensors on the tensor
+ *     cores: one fp32 copy of gw and gb) are refused with SVTAD_ERR_WORKSPACE (C = 192 and 256 at 3x3 fit; C = 1024 does
+ *     not).  Where svtad_workspace_bytes(SVTAD_OP_WGRAD, ...) is more than the array holds, the tokens are split less
+ *     often than in svtad_conv_wgrad.
  *   - "Allocates nothing" holds from the second call of a kind on.  The first call on a device looks the
  *     array's address up (cudaGetSymbolAddress, with that device current), and the first launch of each
  *     kernel variant (one per column-block width and dtype family, plus the reduction) makes the CUDA

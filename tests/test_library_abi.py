@@ -257,3 +257,23 @@ def test_a_plan_is_wanted_where_one_layer_pays_for_it():
     assert wanted(62720, 512, 9, 0.91) == 0 and wanted(50240, 384, 9, 0.75) == 0            # hardly a neighbor missing
     assert wanted(18880, 256, 25, 0.28) == 2 and wanted(2360, 512, 25, 0.52) == 0           # 5x5: the lists alone
     assert wanted(18880, 1024, 9, 0.35, _lib.F32) == 0 and wanted(140000, 1024, 9, 0.35) == 0 and wanted(18880, 1024, 1, 0.35) == 0
+
+
+def test_workspace_sizes_count_the_pair_lists_only_where_a_plan_is_used():
+    """The weight gradient by pair lists parks pieces of its sums (74 MB at C = 256); a call without a plan does not."""
+    lib = _lib.load()
+    mb = 1 << 20
+    for dtype in (_lib.BF16, _lib.F16):
+        for n, most in ((100, 5), (4720, 16), (18880, 19)):
+            assert lib.svtad_workspace_bytes(_lib.OP_WGRAD, n, 256, 256, 9, dtype) < most * mb
+            plain, listed = (lib.svtad_bwd_workspace_bytes(n, 256, 256, 9, dtype, use, 0) for use in (0, 2))
+            assert plain < most * mb < listed
+            assert lib.svtad_bwd_workspace_bytes(n, 256, 256, 9, dtype, 1, 0) == plain             # the row order takes none
+            scatter = lib.svtad_workspace_bytes(_lib.OP_DGRAD, n, 256, 256, 9, dtype)
+            assert lib.svtad_bwd_workspace_bytes(n, 256, 256, 9, dtype, 0, 1) == plain + scatter
+            assert lib.svtad_workspace_bytes(_lib.OP_BWD, n, 256, 256, 9, dtype) == listed + scatter
+        assert lib.svtad_workspace_bytes(_lib.OP_WGRAD, 18880, 192, 192, 9, dtype) <= lib.svtad_static_workspace_bytes()
+    # fp32: several ranges' partials fit the built-in workspace, one range's where they can
+    for c in (64, 192, 256, 320, 384, 512, 704, 768):
+        assert lib.svtad_workspace_bytes(_lib.OP_WGRAD, 18880, c, c, 9, _lib.F32) <= lib.svtad_static_workspace_bytes()
+    assert lib.svtad_bwd_workspace_bytes(0, 256, 256, 9, _lib.BF16, 3, 1) == 0

@@ -61,3 +61,28 @@ def test_static_workspace_rejects_oversized_problems():
     rc = lib.svtad_conv_wgrad_static(dummy.data_ptr(), dummy.data_ptr(), dummy.data_ptr(), dummy.data_ptr(), None,
                                      n, C, C, 9, 0, _lib.BF16, None)
     assert rc == _lib.ERR_WORKSPACE and "built-in" in _lib.last_error()
+
+
+@pytest.mark.parametrize("T,keep,cin,cout,dtype,same", [
+    (80, 0.30, 256, 256, torch.bfloat16, True),      # what the header promises
+    (16, 0.30, 512, 512, torch.float16, True),
+    (160, 0.30, 512, 1024, torch.bfloat16, False),   # the usual two token splits would take 36 MB
+    (40, 0.30, 1024, 768, torch.bfloat16, None),
+])
+def test_static_workspace_takes_what_one_copy_of_the_gradient_fits(T, keep, cin, cout, dtype, same):
+    from eccv26_tad_b200 import _lib, ops
+    lib = _lib.load()
+    table = make_table(1, T, 14, 14, keep, 3, 304)[2]
+    n = table.shape[0]
+    code = _lib.BF16 if dtype == torch.bfloat16 else _lib.F16
+    assert same is None or (lib.svtad_workspace_bytes(_lib.OP_WGRAD, n, cin, cout, 9, code) <= lib.svtad_static_workspace_bytes()) == same
+    x, w, b, gy = make_conv_inputs(n, cin, cout, 3, dtype, 304)
+    tc, xc, gc = table.cuda(), x.cuda(), gy.cuda()
+    ref_gw, ref_gb = ops.conv_wgrad(gc, xc, tc, 9)
+    gw, gb = torch.full_like(ref_gw, float("nan")), torch.full_like(ref_gb, float("nan"))
+    ops.conv_wgrad_static(gc, xc, tc, gw, gb)
+    if same:
+        assert torch.equal(gw, ref_gw) and torch.equal(gb, ref_gb)
+    # the same fp32 sums in another order, rounded once: less than one 16-bit step apart
+    assert oconv.rel_err(f32np(gw), f32np(ref_gw)) < 8e-3 and oconv.rel_err(f32np(gb), f32np(ref_gb)) < 8e-3
+    assert ops.device_error() == 0
