@@ -76,9 +76,22 @@ void* mptr(Tensor& t) { return t.defined() && t.numel() ? t.data_ptr() : nullptr
 const int32_t* iptr(const Tensor& t) { return static_cast<const int32_t*>(ptr(t)); }
 
 // ------------------------------------------------------------------------------------------------ table facts
+// Another thread may be capturing a graph in the mode that forbids calls like these everywhere.
+struct AnyCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AnyCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~AnyCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+bool landed(cudaEvent_t e) {
+    AnyCapture relaxed;
+    if (cudaEventQuery(e) == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return false;
+}
+
 // Landing places in pinned memory for a table's status word on its way to the host: one block, allocated at the first
-// use (pinning memory takes milliseconds, so not once per table).  A place whose copy is still under way when its table
-// dies is handed out again only after the copy has landed; when all are taken the caller does without.
+// use (pinning memory takes milliseconds, so not once per table).  A place takes one copy: it is given back when its table
+// dies or asks anew, and handed out again only after that copy has landed.  When all are taken the caller does without.
 class HostWords {
   public:
     struct Place {
@@ -89,10 +102,7 @@ class HostWords {
         std::lock_guard<std::mutex> hold(mu_);
         if (!page_ && !make_page()) return false;
         for (size_t i = 0; i < free_.size(); ++i) {
-            if (cudaEventQuery(free_[i].copied) != cudaSuccess) {
-                (void)cudaGetLastError();
-                continue;
-            }
+            if (!landed(free_[i].copied)) continue;
             p = free_[i];
             free_[i] = free_.back();
             free_.pop_back();
@@ -107,6 +117,7 @@ class HostWords {
 
   private:
     bool make_page() {
+        AnyCapture relaxed;
         constexpr int PLACES = 128, BYTES = 256;
         if (cudaHostAlloc(&page_, PLACES * BYTES, cudaHostAllocPortable) != cudaSuccess) {
             (void)cudaGetLastError();
@@ -130,26 +141,37 @@ HostWords& host_words(int device) {      // an event belongs to the device it wa
     return h[device % DEVICES];
 }
 
+// What svtad_table_check found for rows of kk taps and a tokens_per_batch.  The word on the device belongs to the stream it
+// was written on: other streams neither wait for it nor keep its memory, so they ask for themselves.
+struct Check {
+    const int kk, device;
+    const int64_t tpb;
+    void* const stream;
+    Tensor word;
+    HostWords::Place host;       // where its copy on the host arrives, if there was a place
+    Check(int kk_, int64_t tpb_, void* stream_, int device_) : kk(kk_), device(device_), tpb(tpb_), stream(stream_) {}
+    ~Check() {
+        if (host.word) host_words(device).give_back(host);
+    }
+};
+constexpr size_t MOST_KEPT = 8;      // forms of one table kept at a time
+
 struct Facts {
     c10::weak_intrusive_ptr<c10::TensorImpl> owner;
     int64_t version;
     int device;
-    bool symmetric = false;      // by construction, or vouched for by the caller
+    bool symmetric = false;      // by construction, or vouched for by the caller, ...
+    int64_t symmetric_kk = 0;    // ... as rows of that many taps (0: not said)
     bool built = false;          // by this package: also batch-global over all of its rows
     int64_t local_n = -1;        // rows per batch row the answer `local` belongs to (-1: not asked yet)
     bool local = false;
-    int64_t status_tpb = -1;     // tokens_per_batch the status word below belongs to
-    Tensor status;               // device word of svtad_table_check
-    HostWords::Place host;       // where its copy on the host arrives
-    Tensor i32;                  // contiguous, aligned int32 form of a table of another kind
+    std::vector<std::shared_ptr<Check>> checks;      // one per reading of the table and stream, the newest last
+    std::vector<std::pair<void*, Tensor>> i32;       // per stream, a contiguous, aligned int32 form of a table of another kind
     double density = -1;         // pairs per row and tap, as far as the host knows (only speed hangs on it)
     std::mutex mu;               // guards everything below `version`
 
     static int64_t version_of(const Tensor& t) { return t.is_inference() ? -1 : static_cast<int64_t>(t._version()); }
     explicit Facts(const Tensor& t) : owner(t.getIntrusivePtr()), version(version_of(t)), device(t.get_device()) {}
-    ~Facts() {
-        if (host.word) host_words(device).give_back(host);
-    }
 };
 
 class FactStore {
@@ -184,6 +206,7 @@ FactStore& store() {
 void mark_symmetric(const Tensor& t, bool built, double density = -1) {
     if (auto f = store().find(t, true)) {
         f->symmetric = true;
+        f->symmetric_kk = t.dim() > 1 ? t.size(-1) : 0;
         f->built = built;
     }
     if (density < 0) return;
@@ -235,7 +258,10 @@ std::shared_ptr<Facts> symmetric_facts(const Tensor& t) {
     return nullptr;
 }
 
-bool is_known_symmetric(const Tensor& t) { return symmetric_facts(t) != nullptr; }
+bool is_known_symmetric(const Tensor& t, int64_t kk) {
+    auto f = symmetric_facts(t);
+    return f && (kk == 0 || f->symmetric_kk == 0 || f->symmetric_kk == kk);
+}
 
 bool capturing(void* stream) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -248,49 +274,59 @@ Tensor table_check(const Tensor& nbr, int64_t n, int kk, int64_t tpb, void* stre
     return status;
 }
 
+std::shared_ptr<Check> kept_check(Facts& f, int kk, int64_t tpb, void* stream) {
+    for (const auto& c : f.checks)
+        if (c->kk == kk && c->tpb == tpb && c->stream == stream) return c;
+    return nullptr;
+}
+
 // What the backward needs to know about a table: an undefined tensor when its entries are known to be symmetric (no
 // validation, no scatter-form fallback), else the status word on the device.  The word is copied to the host behind
-// the check, see found_symmetric().
+// the check, see found_symmetric().  Under graph capture the check belongs to the call: its word is written when the graph
+// runs, in the graph's own memory.
 Tensor status_for(const Tensor& table, const Tensor& nbr, int64_t n, int kk, int64_t tpb, void* stream) {
-    if (tpb == 0 && is_known_symmetric(table)) return Tensor();
-    auto f = store().find(table, true);
+    if (tpb == 0 && is_known_symmetric(table, kk)) return Tensor();
+    auto f = capturing(stream) ? nullptr : store().find(table, true);
     if (!f) return table_check(nbr, n, kk, tpb, stream);
     std::lock_guard<std::mutex> hold(f->mu);
-    if (f->status_tpb == tpb && f->status.defined()) return f->status;
-    f->status = table_check(nbr, n, kk, tpb, stream);
-    f->status_tpb = tpb;
-    if (!capturing(stream) && (f->host.word || host_words(f->device).take(f->host))) {
-        C10_CUDA_CHECK(cudaMemcpyAsync(const_cast<int32_t*>(f->host.word), f->status.const_data_ptr(), sizeof(int32_t),
+    if (auto c = kept_check(*f, kk, tpb, stream)) return c->word;
+    auto c = std::make_shared<Check>(kk, tpb, stream, f->device);
+    c->word = table_check(nbr, n, kk, tpb, stream);
+    if (host_words(f->device).take(c->host)) {
+        C10_CUDA_CHECK(cudaMemcpyAsync(const_cast<int32_t*>(c->host.word), c->word.const_data_ptr(), sizeof(int32_t),
                                        cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)));
-        C10_CUDA_CHECK(cudaEventRecord(f->host.copied, static_cast<cudaStream_t>(stream)));
+        C10_CUDA_CHECK(cudaEventRecord(c->host.copied, static_cast<cudaStream_t>(stream)));
     }
-    return f->status;
+    if (f->checks.size() >= MOST_KEPT) f->checks.erase(f->checks.begin());
+    f->checks.push_back(c);
+    return c->word;
 }
 
 // Whether the validation pass of a table has come back clean.  Never waits: while the word's copy is under way the
 // answer is no and the kernels read the word on the device.  By the time a network's backward reaches the layer the
 // copy has arrived, and the fallback's three launches per backward go away.
-bool found_symmetric(const Tensor& table, int64_t tpb, void* stream) {
-    auto f = store().find(table, false);
+bool found_symmetric(const Tensor& table, int kk, int64_t tpb, void* stream) {
+    auto f = capturing(stream) ? nullptr : store().find(table, false);
     if (!f) return false;
     std::lock_guard<std::mutex> hold(f->mu);
-    if (f->status_tpb != tpb || !f->host.word || capturing(stream)) return false;
-    if (cudaEventQuery(f->host.copied) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    return *f->host.word == 0;
+    const auto c = kept_check(*f, kk, tpb, stream);
+    return c && c->host.word && landed(c->host.copied) && *c->host.word == 0;
 }
 
-Tensor int32_table(const Tensor& table) {
+// A table of another kind is converted once per stream, and again in every captured call.
+Tensor int32_table(const Tensor& table, void* stream) {
     if (table.scalar_type() == at::kInt && table.is_contiguous() &&
         (table.numel() == 0 || reinterpret_cast<uintptr_t>(table.const_data_ptr()) % 16 == 0))
         return table;
-    auto f = store().find(table, true);
+    auto f = capturing(stream) ? nullptr : store().find(table, true);
     if (!f) return c16(table.to(at::kInt));
     std::lock_guard<std::mutex> hold(f->mu);
-    if (!f->i32.defined()) f->i32 = c16(table.to(at::kInt));
-    return f->i32;
+    for (const auto& [on, form] : f->i32)
+        if (on == stream) return form;
+    Tensor form = c16(table.to(at::kInt));
+    if (f->i32.size() >= MOST_KEPT) f->i32.erase(f->i32.begin());
+    f->i32.emplace_back(stream, form);
+    return form;
 }
 
 // Which parts of a work plan a layer should use: only where the table's density is known, which for a caller's table means
@@ -380,7 +416,7 @@ struct SparseConvBackward : public torch::autograd::Node {
         if (!need_x && !need_w) return out;
         auto self = getptr();
         Tensor xs = x.unpack(self), ts = table.unpack(self), w = weight.unpack(self);
-        const Tensor gy = c16(grads[0]), xc = c16(xs), wc = c16(w), nbr = int32_table(ts);
+        const Tensor gy = c16(grads[0]), xc = c16(xs), wc = c16(w), nbr = int32_table(ts, stream_of(ts.device()));
         const at::ScalarType dt = xc.scalar_type();
         TORCH_CHECK_VALUE(gy.scalar_type() == dt && wc.scalar_type() == dt, "grad_output, x and weight must share one dtype");
         TORCH_CHECK_VALUE(gy.numel() == d.n * d.cout, "grad_output has ", gy.numel(), " elements, expected ", d.n, " x ", d.cout);
@@ -394,7 +430,7 @@ struct SparseConvBackward : public torch::autograd::Node {
         Tensor gx, gw, gb, ws, st;
         if (need_x) {
             gx = empty_on(xs.sizes(), dt, dev);
-            if (status.defined() && !found_symmetric(ts, d.tpb, stream)) st = status;
+            if (status.defined() && !found_symmetric(ts, d.kk, d.tpb, stream)) st = status;
         }
         if (need_w) gw = empty_on({d.kk, d.cin, d.cout}, gdt, dev);
         if (need_b) gb = empty_on({d.cout}, gdt, dev);
@@ -442,7 +478,7 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
     {
         at::NoGradGuard no_grad;
         d.tpb = batched ? tokens_per_batch(table, x.size(0), x.size(1), d.kk, local) : 0;
-        nbr = int32_table(table);
+        nbr = int32_table(table, stream);
         require_shapes("conv_fwd", d, nbr, bias_c);
         const Tensor xc = c16(x), wc = c16(weight_c), bc = bias_c.defined() ? c16(bias_c) : Tensor();
         if (batched) {
@@ -519,7 +555,7 @@ Tensor table_remap(const Tensor& table_in, const Tensor& idx_in, const Tensor& s
     require_cuda(table_in);
     require_cuda(idx_in);
     auto sym = symmetric_facts(table_in);
-    const Tensor table = int32_table(table_in), idx = idx_in.to(at::kLong).contiguous();
+    const Tensor table = int32_table(table_in, stream_of(table_in.device())), idx = idx_in.to(at::kLong).contiguous();
     const int64_t B = table.size(0), n_prev = table.size(1), kk = table.size(2), n_new = idx.size(1);
     const at::Device dev = table.device();
     c10::cuda::OptionalCUDAGuard guard(dev);
@@ -537,7 +573,7 @@ std::pair<Tensor, Tensor> table_select_remap(const Tensor& scores_in, const Tens
     require_cuda(table_in);
     const Tensor scores = scores_of(scores_in);
     auto sym = symmetric_facts(table_in);
-    const Tensor table = int32_table(table_in);
+    const Tensor table = int32_table(table_in, stream_of(table_in.device()));
     const int64_t B = table.size(0), n_prev = table.size(1), kk = table.size(2);
     TORCH_CHECK_VALUE(scores.dim() == 2 && scores.size(0) == B && scores.size(1) == n_prev, "table_select_remap: scores ",
                       scores.sizes(), " do not match the table's (", B, ", ", n_prev, ")");
@@ -641,7 +677,7 @@ PyObject* py_mark_symmetric(PyObject*, PyObject* t) {
 
 PyObject* py_is_known_symmetric(PyObject*, PyObject* t) {
     HANDLE_TH_ERRORS
-    return PyBool_FromLong(is_known_symmetric(need_tensor(t, "table")));
+    return PyBool_FromLong(is_known_symmetric(need_tensor(t, "table"), 0));
     END_HANDLE_TH_ERRORS
 }
 
@@ -652,8 +688,8 @@ PyObject* py_table_status(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor table = need_tensor(a[0], "table");
     require_cuda(table);
     const int kk = static_cast<int>(arg_int(a[1]));
-    const Tensor nbr = int32_table(table);
     c10::cuda::OptionalCUDAGuard guard(table.device());
+    const Tensor nbr = int32_table(table, stream_of(table.device()));
     const Tensor st = status_for(table, nbr, nbr.numel() / kk, kk, arg_int(a[2]), stream_of(table.device()));
     if (!st.defined()) Py_RETURN_NONE;
     return THPVariable_Wrap(st);

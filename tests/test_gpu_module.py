@@ -244,3 +244,94 @@ def test_extension_path_by_what_is_known_about_the_table(kind, amp):
         assert m.weight.grad.dtype == m.weight.dtype and m.bias.grad.dtype == m.bias.dtype
         for got, ref in ((y, ey), (xc.grad, egx), (m.weight.grad, egw), (m.bias.grad, egb)):
             assert oconv.rel_err(f32np(got).reshape(ref.shape), ref) < 2e-2
+
+
+def _small_layer(table, C=64, seed=81):
+    """A bf16 layer with inputs for `table` (on the CPU), and what it has to give."""
+    from eccv26_tad_b200 import SparseConv2d
+    n, kk = table.shape
+    ks = int(kk ** 0.5)
+    x, w, b, gy = make_conv_inputs(n, C, C, ks, torch.bfloat16, seed, bias="random")
+    m = SparseConv2d(C, C, kernel_size=ks).cuda().bfloat16()
+    with torch.no_grad():
+        m.weight.copy_(w); m.bias.copy_(b)
+    return m, x.cuda().requires_grad_(True), gy.cuda(), _oracle_grads(table, x, w, b, gy)
+
+
+def _run(m, x, table, gy):
+    y = m(x, table)
+    return (y.detach(),) + torch.autograd.grad(y, (x, m.weight, m.bias), gy)
+
+
+def _check(got, want):
+    for a, b in zip(got, want):
+        assert oconv.rel_err(f32np(a), b) < 2e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+def test_what_one_stream_found_out_about_a_table_is_not_read_by_another_before_it_is_there(dtype):
+    """The int32 form of an int64 table and the status word of an asymmetric one, asked for on a second stream while
+    the first has not got to them yet."""
+    _, _, table = make_table(1, 8, 14, 14, 0.4, 3, 81)
+    table[7] = -1                                                       # asymmetric: the input gradient is the scatter form's
+    m, x, gy, want = _small_layer(table)
+    _check(_run(m, x, table.cuda(), gy), want)                          # kernels loaded
+    t = table.to(dtype).cuda()
+    busy, other = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(40_000_000)                                   # some 20 ms in front of the conversion and the check
+        first = _run(m, x, t, gy)
+    with torch.cuda.stream(other):
+        second = _run(m, x, t, gy)
+    torch.cuda.synchronize()
+    _check(second, want)
+    _check(first, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_a_table_first_met_under_graph_capture(dtype, symmetric):
+    """What a captured call finds out is in the graph's memory and there only when the graph has run: an eager call before
+    the first replay asks anew, and the graph follows its table."""
+    _, _, table = make_table(1, 8, 14, 14, 0.4, 3, 82)
+    if not symmetric:
+        table[9] = -1
+    m, x, gy, want = _small_layer(table)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        for warm in (table.cuda(), table.to(dtype).cuda()):
+            _run(m, x, warm, gy)
+        s.synchronize()
+        t = table.to(dtype).cuda()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            out = _run(m, x, t, gy)
+        _check(_run(m, x, t, gy), want)
+        torch.cuda.synchronize()
+        for seed in (82, 83):
+            _, _, new = make_table(1, 8, 14, 14, 0.4, 3, seed)
+            if seed == 83:
+                new[20] = -1                                            # symmetric no more
+            else:
+                new = table
+            t.copy_(new.to(dtype))
+            junk = torch.full((1 << 20,), -5, dtype=torch.int32, device="cuda")
+            g.replay()
+            torch.cuda.synchronize()
+            _check(out, _oracle_grads(new, *(v.detach().cpu() for v in (x, m.weight, m.bias, gy))))
+            del junk
+
+
+def test_a_symmetric_table_read_with_another_stencil():
+    """Rows of 9 taps that this package built are rows of 25 taps of no symmetry."""
+    from eccv26_tad_b200 import build_neighbor_table
+    scores, _, table = make_table(25, 1, 10, 10, 0.4, 3, 84)            # 1 000 rows of 9 = 360 of 25
+    built = build_neighbor_table(scores.cuda(), 0.4, 10, 10)[1]
+    assert torch.equal(built.cpu(), table)
+    by25 = table.reshape(-1, 25)
+    m, x, gy, want = _small_layer(torch.where(by25 < by25.shape[0], by25, -1))      # entries out of range read as zero
+    _check(_run(m, x, built.reshape(-1, 25), gy), want)
+    m, x, gy, want = _small_layer(table)
+    _check(_run(m, x, built, gy), want)
