@@ -375,12 +375,16 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
         }
     }
     if constexpr (SPLIT) {
+        // a CTA whose wait gave up stops the whole cluster: the others' sums are not finished with what it left behind
+        __syncthreads();
+        if (tid < G && *s_abort) store_to_cta(smem_u32(&tail->abort_flag), tid, 1);
         cluster_barrier();          // every CTA's MMAs are done: nothing is left in the rings, which take the sums now
+        const bool whole = *s_abort == 0;
         int tile, blk;
         item(0, tile, blk);
         const int per = (TILE_M + G - 1) / G;                   // rows that a CTA finishes: [share * per, ...)
         const uint32_t park = smem_u32(smem);                   // [CTA the sums come from][row][PARK]
-        if (warp > FW_A_WARPS) {
+        if (whole && warp > FW_A_WARPS) {
             const int r = (warp & 3) * 32 + lane, owner = r / per;
             const uint32_t dst = map_to_cta(park + ((share * per + r - owner * per) * PARK) * 4, owner);
             const uint32_t t_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
@@ -402,7 +406,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
         // eight columns of a row per thread, the CTAs' sums in their order
         const float* sums = reinterpret_cast<const float*>(smem);
         const long row0 = (long)tile * TILE_M + share * per;
-        const int rows = share * per + per <= TILE_M ? per : TILE_M - share * per;
+        const int rows = !whole ? 0 : share * per + per <= TILE_M ? per : TILE_M - share * per;
         for (int e = tid; e < rows * (BN / 8); e += FW_THREADS) {
             const int r = e / (BN / 8), c = (e % (BN / 8)) * 8, col = blk * BN + c;
             if (row0 + r >= n || col >= cn) continue;

@@ -275,6 +275,10 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
     return r;
 }
+// a word of CTA `rank`'s shared memory, by the address that the same word has here
+__device__ __forceinline__ void store_to_cta(uint32_t saddr, uint32_t rank, int v) {
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(map_to_cta(saddr, rank)), "r"(v) : "memory");
+}
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

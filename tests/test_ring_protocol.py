@@ -52,3 +52,18 @@ def test_no_overwrite_when_producers_do_not_outnumber_buffers():
 def test_overwrite_is_possible_with_more_producers_than_buffers():
     for P, S in [(4, 2), (4, 3), (6, 5), (8, 5)]:
         assert any(run(P, S, steps=40, seed=seed) for seed in range(400)), (P, S)
+
+
+def test_ctas_that_share_a_tile_store_nothing_once_a_wait_gave_up():
+    """The K split's finish (conv_tc_hybrid.cu): no wait can be made to run out here without breaking the kernel, so this
+    reads the order of its steps - every CTA tells its abort to the cluster in front of the barrier, and parks and stores
+    sums only if none had one to tell."""
+    import os
+    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "eccv26_tad_b200", "csrc", "conv_tc_hybrid.cu")
+    text = open(path).read()
+    finish = text[text.index("cluster_barrier();") - 600:text.index("// wgrad\n")]
+    finish = finish[finish.index("if constexpr (SPLIT) {"):]
+    told, barrier = finish.index("if (tid < G && *s_abort) store_to_cta("), finish.index("cluster_barrier();")
+    known, parks = finish.index("const bool whole = *s_abort == 0;"), finish.index("if (whole && warp > FW_A_WARPS)")
+    stores = finish.index("const int rows = !whole ? 0 :")
+    assert finish.index("__syncthreads();") < told < barrier < known < parks < stores
