@@ -9,7 +9,7 @@
 //
 // What is known about a neighbor table (symmetric by construction, indices local to a batch row or not, the device
 // status word of svtad_table_check, an int32 copy, how many of its entries are there) is kept per tensor object and
-// version; entries of dead tables are swept whenever a new table is entered.  A table's work plan is not: a table can be
+// version; entries of dead tables are swept as new tables are entered.  A table's work plan is not: a table can be
 // written to without its version moving (a replayed graph that holds the selection, the C ABI, a raw pointer), so a
 // layer makes its plan from what the table holds when its kernels run, every time.
 #include <ATen/ATen.h>
@@ -27,9 +27,9 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <map>
 #include <memory>
 #include <mutex>
-#include <unordered_map>
 #include <vector>
 
 #include "../../include/svtad.h"
@@ -187,7 +187,13 @@ class FactStore {
             map_.erase(it);
         }
         if (!make) return nullptr;
-        for (auto e = map_.begin(); e != map_.end();) e = e->second->owner.expired() ? map_.erase(e) : std::next(e);
+        // dead tables' entries go a few at a time: all of them while the tables are few, at the same cost where there are many
+        auto e = map_.upper_bound(swept_);
+        for (int i = 0; i < 8 && !map_.empty(); ++i) {
+            if (e == map_.end()) e = map_.begin();
+            swept_ = e->first;
+            e = e->second->owner.expired() ? map_.erase(e) : std::next(e);
+        }
         auto f = std::make_shared<Facts>(t);
         map_[t.unsafeGetTensorImpl()] = f;
         return f;
@@ -195,7 +201,8 @@ class FactStore {
 
   private:
     std::mutex mu_;
-    std::unordered_map<const c10::TensorImpl*, std::shared_ptr<Facts>> map_;
+    const c10::TensorImpl* swept_ = nullptr;
+    std::map<const c10::TensorImpl*, std::shared_ptr<Facts>, std::less<>> map_;
 };
 
 FactStore& store() {
@@ -204,15 +211,14 @@ FactStore& store() {
 }
 
 void mark_symmetric(const Tensor& t, bool built, double density = -1) {
-    if (auto f = store().find(t, true)) {
-        f->symmetric = true;
-        f->symmetric_kk = t.dim() > 1 ? t.size(-1) : 0;
-        f->built = built;
-    }
-    if (density < 0) return;
-    auto f = store().find(t, true, true);
+    auto f = store().find(t, true, density >= 0);
+    if (!f) return;
     std::lock_guard<std::mutex> hold(f->mu);
-    f->density = density;
+    if (density >= 0) f->density = density;
+    if (t.is_inference()) return;
+    f->symmetric = true;
+    f->symmetric_kk = t.dim() > 1 ? t.size(-1) : 0;
+    f->built = built;
 }
 
 // the table's density, where it or the tensor it looks into has one

@@ -277,3 +277,22 @@ def test_workspace_sizes_count_the_pair_lists_only_where_a_plan_is_used():
     for c in (64, 192, 256, 320, 384, 512, 704, 768):
         assert lib.svtad_workspace_bytes(_lib.OP_WGRAD, 18880, c, c, 9, _lib.F32) <= lib.svtad_static_workspace_bytes()
     assert lib.svtad_bwd_workspace_bytes(0, 256, 256, 9, _lib.BF16, 3, 1) == 0
+
+
+def test_entering_a_table_costs_the_same_however_many_tables_are_alive():
+    import time
+    import torch
+    from eccv26_tad_b200 import ops
+
+    def per_table(count):
+        tables = [torch.zeros(1, 9, dtype=torch.int32) for _ in range(count)]
+        t0 = time.perf_counter()
+        for t in tables:
+            ops.mark_symmetric(t)
+        return (time.perf_counter() - t0) / count, tables
+    per_table(200)
+    few, _ = per_table(200)
+    _, alive = per_table(30000)
+    many, more = per_table(2000)
+    assert many < 20 * few + 20e-6          # a look at each of 30 000 would take hundreds of microseconds
+    assert all(ops.is_known_symmetric(t) for t in alive + more)
