@@ -456,6 +456,12 @@ struct SparseConvBackward : public torch::autograd::Node {
     }
 };
 
+// The node below has no forward-mode formula: refused, as a torch.autograd.Function without jvp is.
+void refuse_tangent(const Tensor& t) {
+    TORCH_CHECK_NOT_IMPLEMENTED(!t.defined() || !t._fw_grad(/*level=*/0).defined(),
+                                "SparseConv2d does not support forward mode automatic differentiation");
+}
+
 // weight_c / bias_c: the parameters in the computing dtype (the parameters themselves when it is theirs)
 Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& bias, const Tensor& weight_c,
             const Tensor& bias_c, int local) {
@@ -463,6 +469,9 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
     require_cuda(table);
     require_cuda(weight_c);
     require_cuda(bias_c);
+    refuse_tangent(x);
+    refuse_tangent(weight);
+    refuse_tangent(bias);
     const at::ScalarType dt = weight_c.scalar_type();
     if (x.scalar_type() != dt) x = x.to(dt);          // autocast: recorded by autograd like any cast
     const int code = dtype_code(dt);

@@ -335,3 +335,25 @@ def test_a_symmetric_table_read_with_another_stencil():
     _check(_run(m, x, built.reshape(-1, 25), gy), want)
     m, x, gy, want = _small_layer(table)
     _check(_run(m, x, built, gy), want)
+
+
+def test_forward_mode_differentiation_is_refused():
+    """There is no formula for it: a dual tensor must not come out without its tangent."""
+    import torch.autograd.forward_ad as fwad
+    _, _, table = make_table(1, 2, 14, 14, 0.4, 3, 85)
+    m, x, _, want = _small_layer(table)
+    t, params = table.cuda(), {"weight": m.weight.detach(), "bias": m.bias.detach()}
+    with fwad.dual_level():
+        for name in ("x", "weight", "bias"):
+            v = x.detach() if name == "x" else params[name]
+            dual = fwad.make_dual(v, torch.ones_like(v))
+            with pytest.raises(NotImplementedError, match="forward mode"):
+                torch.func.functional_call(m, {**params, name: dual} if name != "x" else params, (dual if name == "x" else x, t))
+            with pytest.raises(NotImplementedError, match="forward mode"), torch.no_grad():
+                torch.func.functional_call(m, {**params, name: dual} if name != "x" else params, (dual if name == "x" else x, t))
+        assert oconv.rel_err(f32np(m(x, t)), want[0]) < 2e-2
+    for transform in (lambda: torch.func.jvp(lambda v: m(v, t), (x.detach(),), (torch.ones_like(x),)),
+                      lambda: torch.func.vmap(lambda v: m(v, t))(torch.stack([x.detach()] * 2)),
+                      lambda: torch.func.grad(lambda v: m(v, t).sum())(x.detach())):
+        with pytest.raises(RuntimeError):
+            transform()
