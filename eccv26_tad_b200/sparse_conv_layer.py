@@ -29,6 +29,8 @@ from torch.autograd import Function
 from . import ops
 from ._lib import native as _native
 
+_tracing = torch._C._get_tracing_state
+
 try:  # torch >= 2.4
     from torch.amp import custom_bwd as _custom_bwd, custom_fwd as _custom_fwd
 
@@ -124,6 +126,8 @@ class SparseConv2d(nn.Module):
         (reference :170-177), int32 and autocast conversions, kernels, the autograd node - is one call of the
         extension."""
         weight, bias = self.weight, self.bias
+        if _tracing() is not None:
+            return self._forward_by_function(x, neighbor_indices, local_indices)
         dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
         if weight.dtype is dtype and (bias is None or bias.dtype is dtype):
             return _native.conv(x, neighbor_indices, weight, bias, weight, bias, local_indices)
@@ -131,6 +135,23 @@ class SparseConv2d(nn.Module):
         # kept until the parameters change, e.g. across the two forward passes of activation checkpointing
         weight_c, bias_c = self._cast_params(dtype)
         return _native.conv(x, neighbor_indices, weight, bias, weight_c, bias_c, local_indices)
+
+    def _forward_by_function(self, x, neighbor_indices, local_indices):
+        """The same call in operations that ``torch.jit.trace`` can record: an extension call would be a constant to it."""
+        kk = self.kernel_size * self.kernel_size
+        batched, tokens_per_batch = x.dim() == 3, 0
+        if batched:
+            B, N, C = x.shape
+            if B > 1 and N > 0:
+                if local_indices is None:
+                    local_indices = neighbor_indices.numel() > 0 and bool(neighbor_indices.max() < N)
+                tokens_per_batch = int(N) if local_indices else 0
+            x = x.reshape(-1, C)
+        dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
+        bias = self.bias if self.bias is None else self.bias.to(dtype)
+        y = SparseConv2dFunction.apply(x.to(dtype), neighbor_indices.to(torch.int32).reshape(-1, kk), self.weight.to(dtype), bias,
+                                       tokens_per_batch, self.chunk_size)
+        return y.view(B, N, self.out_channels) if batched else y
 
     def invalidate_cast_cache(self):
         """Drops the cached low-precision parameter copies.  They are keyed on the parameters' version counters,

@@ -357,3 +357,33 @@ def test_forward_mode_differentiation_is_refused():
                       lambda: torch.func.grad(lambda v: m(v, t).sum())(x.detach())):
         with pytest.raises(RuntimeError):
             transform()
+
+
+@pytest.mark.parametrize("kind", ["plain", "batched", "local", "amp"])
+@pytest.mark.parametrize("grad", [True, False])
+def test_a_traced_module_follows_its_inputs(kind, grad):
+    """torch.jit.trace records the layer, not the features it was traced with."""
+    from eccv26_tad_b200 import SparseConv2d
+    _, _, table = make_table(2, 2, 14, 14, 0.4, 3, 86)
+    n, C = table.shape[0], 64
+    x, w, b, gy = (t.cuda() for t in make_conv_inputs(n, C, C, 3, torch.float32, 86, bias="random"))
+    t, m = table.cuda(), SparseConv2d(C, C).cuda()
+    with torch.no_grad():
+        m.weight.copy_(w); m.bias.copy_(b)
+    if kind != "plain":
+        x, t = x.view(2, n // 2, C), t.view(2, n // 2, 9)
+    if kind == "local":
+        t = t[:1].repeat(2, 1, 1)
+    other = torch.randn_like(x)
+    with torch.set_grad_enabled(grad), torch.autocast("cuda", dtype=torch.bfloat16, enabled=kind == "amp"):
+        traced = torch.jit.trace(m, (x, t), check_trace=False)
+        for v in (x, other):
+            v.requires_grad_(grad)
+            got, want = traced(v, t), m(v, t)
+            assert got.shape == want.shape and got.dtype == want.dtype and torch.equal(got, want)
+            assert got.requires_grad == grad
+            if grad:
+                g = [torch.autograd.grad(y, (v, m.weight, m.bias), gy.view(y.shape).to(y.dtype)) for y in (got, want)]
+                for a, e in zip(*g):
+                    # under autocast the module rounds each gradient of a parameter once, as the cast in the trace does
+                    assert a.dtype == e.dtype and oconv.rel_err(f32np(a), f32np(e)) < 1e-5
