@@ -530,6 +530,7 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
 // ------------------------------------------------------------------------------------------------ table functions
 Tensor scores_of(const Tensor& scores) {
     require_cuda(scores);
+    TORCH_CHECK_VALUE(scores.dim() == 2, "scores have ", scores.dim(), " dimensions, expected [segments, tokens]");
     return (scores.scalar_type() == at::kFloat ? scores : scores.to(at::kFloat)).contiguous();
 }
 
@@ -569,6 +570,7 @@ Tensor topk_select(const Tensor& scores_in, int64_t k) {
 Tensor table_remap(const Tensor& table_in, const Tensor& idx_in, const Tensor& scratch_in) {
     require_cuda(table_in);
     require_cuda(idx_in);
+    TORCH_CHECK_VALUE(table_in.dim() == 3, "the neighbor table has ", table_in.dim(), " dimensions, expected [batch, rows, taps]");
     auto sym = symmetric_facts(table_in);
     const Tensor table = int32_table(table_in, stream_of(table_in.device())), idx = idx_in.to(at::kLong).contiguous();
     const int64_t B = table.size(0), n_prev = table.size(1), kk = table.size(2), n_new = idx.size(1);
@@ -587,6 +589,7 @@ Tensor table_remap(const Tensor& table_in, const Tensor& idx_in, const Tensor& s
 std::pair<Tensor, Tensor> table_select_remap(const Tensor& scores_in, const Tensor& table_in, int64_t k) {
     require_cuda(table_in);
     const Tensor scores = scores_of(scores_in);
+    TORCH_CHECK_VALUE(table_in.dim() == 3, "the neighbor table has ", table_in.dim(), " dimensions, expected [batch, rows, taps]");
     auto sym = symmetric_facts(table_in);
     const Tensor table = int32_table(table_in, stream_of(table_in.device()));
     const int64_t B = table.size(0), n_prev = table.size(1), kk = table.size(2);

@@ -221,3 +221,22 @@ def test_threshold_search_of_short_segments(dist):
         ekept, etable = otab.build_table(s, k, 14, 14, 3)
         np.testing.assert_array_equal(kept.cpu().numpy(), ekept)
         np.testing.assert_array_equal(table.cpu().numpy(), etable)
+
+
+def test_tensors_of_another_number_of_dimensions_are_refused():
+    import eccv26_tad_b200 as sv
+    scores = torch.randn(2, 196, device="cuda")
+    table = sv.build_neighbor_table(scores, None, 14, 14, num_keep=50)[1]
+    idx = torch.zeros(1, 5, dtype=torch.int64, device="cuda")
+    for bad in (scores[0], scores.unsqueeze(-1), scores.unsqueeze(0)):
+        with pytest.raises(ValueError):
+            sv.build_neighbor_table(bad, None, 14, 14, num_keep=50)
+        with pytest.raises(ValueError):
+            sv.select_topk(bad, 5)
+        with pytest.raises(ValueError):
+            sv.select_and_update(bad, table.view(2, 50, 9), 5)
+    for bad in (table, table.view(1, 1, 100, 9)):
+        with pytest.raises(ValueError):
+            sv.update_neighbor_indices(bad, idx)
+        with pytest.raises(ValueError):
+            sv.select_and_update(torch.randn(1, 100, device="cuda"), bad, 5)
