@@ -188,10 +188,11 @@ table_build_warp_kernel(const float* __restrict__ scores, int n_seg, int L, int 
     // one lane per kept token computes its K*K entries into shared memory; the warp then writes the
     // staged rows (contiguous in the table) with 16-byte stores
     const int KK = (KS > 0) ? KS * KS : ksize * ksize;
+    const int RN = KS > 0 ? RR : min(RR, RR * KKMAX / KK);      // stencils beyond 7 x 7: as many rows as fit (15 x 15: one)
     int32_t* so = s_out[wid];
-    for (int r0 = 0; r0 < k; r0 += RR) {
+    for (int r0 = 0; r0 < k; r0 += RN) {
         const int r = r0 + lane;
-        if (lane < RR && r < k) {
+        if (lane < RN && r < k) {
             const int p = s_pos[wid][r], q = hw == 1 ? 0 : p - div_magic(p, magic_hw) * hw;
             const int y = w == 1 ? q : div_magic(q, magic_w), x = q - y * w;
             if (KS > 0) {
@@ -218,7 +219,7 @@ table_build_warp_kernel(const float* __restrict__ scores, int n_seg, int L, int 
             }
         }
         __syncwarp();
-        const int rows = (k - r0) < RR ? (k - r0) : RR;
+        const int rows = (k - r0) < RN ? (k - r0) : RN;
         const int cnt = rows * KK;
         const long g0 = (base + r0) * KK;                  // first table element of this round
         int32_t* out = table + g0;

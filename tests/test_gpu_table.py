@@ -240,3 +240,15 @@ def test_tensors_of_another_number_of_dimensions_are_refused():
             sv.update_neighbor_indices(bad, idx)
         with pytest.raises(ValueError):
             sv.select_and_update(torch.randn(1, 100, device="cuda"), bad, 5)
+
+
+@pytest.mark.parametrize("ksize", [7, 9, 11, 13, 15])
+@pytest.mark.parametrize("h,w", [(14, 14), (16, 16), (3, 5)])
+def test_wide_stencils_on_short_segments(ksize, h, w):
+    """Rows of up to 225 taps, 24 segments (three blocks of eight warps, whose staging areas lie side by side)."""
+    import eccv26_tad_b200 as sv
+    scores = make_scores(24, h * w, 91)
+    k = otab.num_keep(0.6, h * w)
+    ekept, etable = otab.build_table(scores.numpy(), k, h, w, ksize)
+    kept, table = sv.build_neighbor_table(scores.cuda(), None, h, w, ksize, num_keep=k)
+    assert np.array_equal(kept.cpu().numpy(), ekept) and np.array_equal(table.cpu().numpy(), etable)
