@@ -253,11 +253,11 @@ def conv_bwd(gy, x, nbr, weight, tokens_per_batch=0, table_status=None, need_x=T
             table_status = None
         elif need_x and table_status is None:
             table_status = table_check(nbr, tokens_per_batch)
-        if assume_symmetric:     # no scatter-form part in the workspace
-            op = _lib.OP_WGRAD if need_w else None
+        if need_w:               # without a plan; the scatter form's part only behind a table status
+            nbytes = _lib.load().svtad_bwd_workspace_bytes(n, cin, cout, kk, code, 0, int(need_x and not assume_symmetric))
         else:
-            op = _lib.OP_BWD if (need_x and need_w) else (_lib.OP_WGRAD if need_w else _lib.OP_DGRAD)
-        ws, ws_bytes = _workspace(op, n, cin, cout, kk, code, dev) if op is not None else (None, 0)
+            nbytes = 0 if assume_symmetric else _lib.load().svtad_workspace_bytes(_lib.OP_DGRAD, n, cin, cout, kk, code)
+        ws, ws_bytes = (torch.empty(nbytes, dtype=torch.uint8, device=dev), nbytes) if nbytes else (None, 0)
         _lib.check(_lib.load().svtad_conv_bwd(_ptr(gy), _ptr(x), _ptr(nbr), _ptr(weight), _ptr(gx), _ptr(gw), _ptr(gb),
                                               n, cin, cout, kk, tokens_per_batch, code,
                                               _ptr(table_status) if (need_x and not assume_symmetric) else None,

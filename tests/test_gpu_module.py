@@ -387,3 +387,22 @@ def test_a_traced_module_follows_its_inputs(kind, grad):
                 for a, e in zip(*g):
                     # under autocast the module rounds each gradient of a parameter once, as the cast in the trace does
                     assert a.dtype == e.dtype and oconv.rel_err(f32np(a), f32np(e)) < 1e-5
+
+
+@pytest.mark.parametrize("known", [True, False])
+def test_a_backward_without_a_plan_takes_no_workspace_for_one(known):
+    """C = 256 at some 500 rows: a few MB of partial sums, not the 74 MB of the pair lists' pieces."""
+    from eccv26_tad_b200 import ops
+    _, _, table = make_table(1, 8, 14, 14, 0.3, 3, 87)
+    m, x, gy, want = _small_layer(table, C=256)
+    t = table.cuda()
+    if known:
+        ops.mark_symmetric(t)
+    for run in (lambda: _run(m, x, t, gy)[1:], lambda: ops.conv_bwd(gy, x.detach(), t, m.weight.detach(), assume_symmetric=known)):
+        _check(run(), want[1:])
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        run()
+        torch.cuda.synchronize()
+        assert torch.cuda.max_memory_allocated() - before < 24 << 20
