@@ -80,6 +80,7 @@ int conv_wgrad_fit(const void* gy, const void* x, const int32_t* nbr, void* gw, 
 int tc_read_error(int32_t* code_out);
 int tc_set_share(int n);
 int tc_get_share();
+int tc_num_sms();               // of the current device
 int tc_set_share_floor(int n);
 
 // the single-CTA tensor-core kernels behind tc_* (conv_tc_hybrid.cu)

@@ -531,9 +531,10 @@ template <bool DGRAD>
 static int dispatch_conv_f32(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
     const long tiles_n = ((DGRAD ? p.cin : p.cout) + F_BN - 1) / F_BN;
     const long t128 = (p.n + 127) / 128 * tiles_n, t64 = (p.n + 63) / 64 * tiles_n;
-    const int bm = t128 >= 148 ? 128 : 64;
+    const long sms = tc_num_sms();
+    const int bm = t128 >= sms ? 128 : 64;
     const long tiles = bm == 128 ? t128 : t64;
-    const long three = (3 * 148 + tiles / 2) / tiles, two = (2 * 148 + tiles / 2) / tiles;
+    const long three = (3 * sms + tiles / 2) / tiles, two = (2 * sms + tiles / 2) / tiles;
     long G = three < 3 ? three : 3;
     if (two > G) G = two < 8 ? two : 8;
     return launch_conv_f32<DGRAD>(p, status, bm, G < 1 ? 1 : (int)G, s);
@@ -552,7 +553,7 @@ int f32_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) { return
 static int f32_wgrad_splits(int64_t n, int cin, int cout, int kk) {
     const long tiles = (long)kk * ((cin + 63) / 64) * ((cout + 63) / 64);
     const long by_rows = (n + 127) / 128, by_size = (31l << 20) / ((long)kk * cin * cout * 4);
-    long s = (8 * 148 + tiles - 1) / tiles;
+    long s = (8l * tc_num_sms() + tiles - 1) / tiles;
     if (s > by_rows) s = by_rows;
     if (s > by_size) s = by_size;
     return (int)(s < 1 ? 1 : s);

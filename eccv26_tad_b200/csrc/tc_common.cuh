@@ -298,7 +298,6 @@ constexpr int tmem_cols2_for(int bn) { return 2 * bn <= 64 ? 64 : 2 * bn <= 128 
 
 // ---- host helpers shared by the tensor-core translation units (defined in conv_tc.cu) ----
 constexpr size_t TC_SMEM_LIMIT = 227 * 1024;
-int tc_num_sms();
 int tc_plan_sms();          // SMs a kernel is planned for: all of them divided by the caller's concurrency hint
 int tc_set_share(int n);    // sets the hint, returns the previous one
 int tc_get_share();
