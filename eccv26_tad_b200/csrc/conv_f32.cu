@@ -1,6 +1,6 @@
 // fp32 SparseConv2D on the CUDA cores: forward, input gradient (gather form) and weight gradient.
 //
-// fp32 tensors cannot go through the tensor cores without losing the 1e-5 the reference's fp32 path holds
+// fp32 tensors cannot go through the tensor cores as TF32 without losing the 1e-5 the reference's fp32 path holds
 // (opentad/models/bricks/2d_sparse_v3.cu:545-651, a 32 x 32 shared-memory tile kernel with two __syncthreads per
 // 32-deep step; for C_in >= 128 implicit_gemm_v2.cu:197-300, gather + cuBLAS SGEMM + reduce; backward by atomics,
 // 2d_sparse_v3.cu:656-745).  What bounds these kernels is the FP32 FMA pipe (72 TFLOP/s measured on a B200), so the work

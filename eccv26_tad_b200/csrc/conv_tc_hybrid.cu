@@ -7,10 +7,10 @@
 //             per stage) . B(MN-major: gy rows); split over tokens, fp32 partials to the workspace;
 //             a block of ones turns the bias gradient into one more row of D
 //
-// Operand feed.  Gathered rows are irregular, so four producer warps copy them with 16-byte cp.async
-// straight into the 128-byte-swizzled layout the UMMA descriptors describe (nothing gathered is ever
-// materialised in HBM); each warp owns every fourth pipeline stage, so a stage costs 32 barrier
-// arrivals instead of one per thread.  Regular tiles (weights, gy) come through TMA, issued by lane 0
+// Operand feed.  Gathered rows are irregular, so producer warps copy them with 16-byte cp.async straight into
+// the 128-byte-swizzled layout the UMMA descriptors describe (nothing gathered is ever materialised in HBM).
+// Forward / dgrad: eight warps, two of which fill a buffer together, so that the four pairs own every fourth
+// pipeline stage; wgrad: four warps, a stage each in turn (eight were slower there).  Regular tiles (weights, gy) come through TMA, issued by lane 0
 // of the warp that owns the stage.  One elected thread issues tcgen05.mma; four warps drain the
 // accumulator (tcgen05.ld -> +bias -> one rounding -> 16-byte stores).
 //

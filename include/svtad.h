@@ -186,7 +186,11 @@ int svtad_plan_build(const int32_t* nbr, int64_t n, int kk, int tokens_per_batch
 int svtad_plan_build_parts(const int32_t* nbr, int64_t n, int kk, int tokens_per_batch, int parts, void* plan, void* stream);
 const int32_t* svtad_plan_counts(const void* plan, int64_t n, int kk);
 
-/* svtad_conv_fwd with a plan (NULL: none).  Same results. */
+/*
+ * svtad_conv_fwd with a plan (NULL: none).  A row's sum is the same whatever the order of the rows, so results are the same
+ * bit for bit, except where the call without a plan splits a tile's K steps over a cluster (few rows, long reductions),
+ * which adds the same products up in another order.
+ */
 int svtad_conv_fwd_planned(const void* x, const int32_t* nbr, const void* w, const void* bias, void* y, int64_t n,
                            int cin, int cout, int kk, int tokens_per_batch, int dtype, const void* plan, void* stream);
 
@@ -282,8 +286,8 @@ int svtad_allreduce_sum_emulated(void* const* bufs, int world, int64_t n_elems, 
  * step on a B200: 0.110 ms with the default, 0.086 ms with a hint of 3).  Results do not depend on the hint beyond
  * the summation order of the weight gradient's partials.  The hint is process-wide and read at launch time;
  * svtad_workspace_bytes does not depend on it (it covers the plan under every hint), so a workspace sized once
- * stays valid when the hint changes.  svtad_conv_bwd, whose two
- * kernels run side by side, plans them for half the GPU each even under the default.
+ * stays valid when the hint changes.  svtad_conv_bwd, whose two kernels run side by side, plans them for half the GPU
+ * each even under the default, up to 18 GFLOP a pass; larger ones, and those by pair lists, for all of it.
  * svtad_set_concurrency returns the previous value (values are clamped to [1, 16]); SVTAD_CONCURRENCY in the
  * environment gives the start value.
  */

@@ -122,8 +122,8 @@ def test_planned_kernels_give_the_unplanned_results(B, T, keep, ks, cin, cout, d
 
 @pytest.mark.parametrize("keep,table_kind", [(0.3, "built"), (0.5, "given"), (1.0, "given"), (1.0, "built")])
 def test_module_with_a_layer_that_wants_a_plan(keep, table_kind):
-    """C = 512 at 18 880 / 31 360 / 62 720 rows: the module's plan (first pass: the density is not known yet; later ones go
-    by it), results as without one."""
+    """C = 512 at 18 880 / 31 360 / 62 720 rows: with the module's plan (a table built here that is sparse enough) and without
+    one (the full grid; a caller's table whose density the call does not ask for), results as without one."""
     import eccv26_tad_b200 as sv
     from eccv26_tad_b200 import ops
     B = 4
