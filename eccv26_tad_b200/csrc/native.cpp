@@ -571,7 +571,7 @@ Tensor table_remap(const Tensor& table_in, const Tensor& idx_in, const Tensor& s
     require_cuda(table_in);
     require_cuda(idx_in);
     TORCH_CHECK_VALUE(table_in.dim() == 3, "the neighbor table has ", table_in.dim(), " dimensions, expected [batch, rows, taps]");
-    auto sym = symmetric_facts(table_in);
+    auto sym = is_known_symmetric(table_in, table_in.size(2)) ? symmetric_facts(table_in) : nullptr;
     const Tensor table = int32_table(table_in, stream_of(table_in.device())), idx = idx_in.to(at::kLong).contiguous();
     const int64_t B = table.size(0), n_prev = table.size(1), kk = table.size(2), n_new = idx.size(1);
     const at::Device dev = table.device();
@@ -590,7 +590,7 @@ std::pair<Tensor, Tensor> table_select_remap(const Tensor& scores_in, const Tens
     require_cuda(table_in);
     const Tensor scores = scores_of(scores_in);
     TORCH_CHECK_VALUE(table_in.dim() == 3, "the neighbor table has ", table_in.dim(), " dimensions, expected [batch, rows, taps]");
-    auto sym = symmetric_facts(table_in);
+    auto sym = is_known_symmetric(table_in, table_in.size(2)) ? symmetric_facts(table_in) : nullptr;
     const Tensor table = int32_table(table_in, stream_of(table_in.device()));
     const int64_t B = table.size(0), n_prev = table.size(1), kk = table.size(2);
     TORCH_CHECK_VALUE(scores.dim() == 2 && scores.size(0) == B && scores.size(1) == n_prev, "table_select_remap: scores ",
@@ -695,7 +695,8 @@ PyObject* py_mark_symmetric(PyObject*, PyObject* t) {
 
 PyObject* py_is_known_symmetric(PyObject*, PyObject* t) {
     HANDLE_TH_ERRORS
-    return PyBool_FromLong(is_known_symmetric(need_tensor(t, "table"), 0));
+    const Tensor table = need_tensor(t, "table");
+    return PyBool_FromLong(is_known_symmetric(table, table.dim() > 1 ? table.size(-1) : 0));
     END_HANDLE_TH_ERRORS
 }
 

@@ -296,3 +296,12 @@ def test_entering_a_table_costs_the_same_however_many_tables_are_alive():
     many, more = per_table(2000)
     assert many < 20 * few + 20e-6          # a look at each of 30 000 would take hundreds of microseconds
     assert all(ops.is_known_symmetric(t) for t in alive + more)
+
+
+def test_a_symmetric_table_is_symmetric_in_rows_of_its_own_length():
+    import torch
+    from eccv26_tad_b200 import ops
+    t = ops.mark_symmetric(torch.zeros(100, 9, dtype=torch.int32))
+    assert ops.is_known_symmetric(t) and ops.is_known_symmetric(t.view(4, 25, 9)) and ops.is_known_symmetric(t[:50])
+    assert not ops.is_known_symmetric(t.view(36, 25)) and not ops.is_known_symmetric(t.view(1, 36, 25))
+    assert ops.is_known_symmetric(t.view(-1))           # no row length to go by
