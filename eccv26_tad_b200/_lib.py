@@ -36,6 +36,7 @@ SIGNATURES = {
     "svtad_conv_wgrad": (c_int, [c_p, c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_p, c_sz, c_p]),
     "svtad_conv_bwd": (c_int, [c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i64, c_int, c_int, c_int, c_int, c_int, c_p, c_p, c_sz, c_p]),
     "svtad_plan_wanted": (c_int, [c_i64, c_int, c_int, c_int, c_int, ctypes.c_double]),
+    "svtad_plan_wanted_fwd": (c_int, [c_i64, c_int, c_int, c_int, c_int, ctypes.c_double]),
     "svtad_plan_counts": (c_p, [c_p, c_i64, c_int]),
     "svtad_plan_bytes": (c_sz, [c_i64, c_int]),
     "svtad_plan_build": (c_int, [c_p, c_i64, c_int, c_int, c_p, c_p]),

@@ -124,31 +124,45 @@ extern "C" size_t svtad_bwd_workspace_bytes(int64_t n, int cin, int cout, int kk
 }
 
 // Which parts of a plan gain a layer more than it costs to make them for this one layer and call: the row order (forward,
-// input gradient) takes 10 us up to 7 000 rows, 16 at 18 880, 30 at 60 000, the pair lists (weight gradient; 3 x 3) 4 to 9,
-// next to the input gradient.  What they save goes by the products that are not there, work * (1 - density); on what a plan
-// costs the line rises with the rows.  Measured, us of a training pass (forward + backward) without a plan and with one made
-// for it, by the products left out:
-//   4 720 rows, C = 512, density 0.35 (14 GFLOP): 75 -> 82             9 440, C = 512, 0.59 (18): 110 -> 127
-//   2 400, C = 768, 0.27 (19): 111 -> 84                              11 800, C = 384, 0.35 (20): 110 -> 83
-//   4 720, C = 768, 0.35 (32): 153 -> 116                             6 400, C = 512, 0.19 (24): 100 -> 80
-//   18 880, C = 256, 0.35 (14): 67 -> 83                              18 880, C = 384, 0.35 (32): 144 -> 102
-//   37 760, C = 256, 0.59 (18): 116 -> 126                            37 760, C = 384, 0.59 (41): 260 -> 234
-//   50 240, C = 384, 0.75 (33): 367 -> 376                            50 240, C = 512, 0.75 (59): 619 -> 570
-//   18 880, C = 1024, 0.35 (232): 870 -> 430                          15 680, C = 1024, 0.91 (27): 817 -> 657
-// Up to sixteen tiles the kernels without a plan share a tile's K steps over a cluster, and the longest tile, which needs
-// nearly every tap, is all that matters: 1 770, C = 1024, 0.35 (22): 118 -> 128.
+// input gradient) takes 10 us up to 7 000 rows, 16 at 18 880, 30 at 60 000, 48 at 113 000, and a few more for the kernel that
+// starts cold behind it; the pair lists (weight gradient; 3 x 3) 4 to 15, next to the input gradient.  A tile of ordered rows
+// needs about 1.2 times the taps that its rows have on average, so what the order saves goes by work * (1 - 1.2 density), and
+// on what it costs the line rises with the rows.  Measured, us of a training pass (forward + backward, graph replays) without
+// a plan and with one made for it, by that figure:
+//   4 720 rows, C = 512, density 0.35 (13 GFLOP): 79 -> 84             12 800, C = 320, 0.27 (16): 105 -> 86
+//   18 880, C = 256, 0.35 (13): 72 -> 93                              11 800, C = 384, 0.35 (18): 113 -> 88
+//   75 520, C = 128, 0.35 (13): 97 -> 119                             4 720, C = 768, 0.35 (29): 152 -> 129
+//   37 760, C = 192, 0.35 (15): 85 -> 88                              18 880, C = 384, 0.35 (29): 148 -> 108
+//   75 520, C = 256, 0.59 (26): 222 -> 233                            37 760, C = 384, 0.59 (29): 260 -> 225
+//   75 520, C = 192, 0.35 (29): 151 -> 151                            18 880, C = 1024, 0.35 (207): 768 -> 391
+// With few tiles the longest one, which needs nearly every tap, is all that matters, and up to sixteen the kernels without a
+// plan share a tile's K steps over a cluster: 1 770, C = 1024, 0.35 (19): 117 -> 140; 3 920, C = 1024, 0.51 (29): 183 -> 197.
 // Stencils beyond 3 x 3: the order is by the eight nearest neighbors, and a tile needs nearly all of the others (19.9 of 25
 // taps at density 0.28, 22.4 at 0.61): 2 360 rows, C = 512: forward 38 -> 78 us; 18 880, C = 256: 44 -> 43.  So these take the
-// lists alone, which take 8 to 19 us (backward with the lists' making): 4 720 rows, C = 384, 0.28 (25 GFLOP): 97 -> 76; 9 440,
-// C = 256, 0.28 (22): 69 -> 75; 18 880, C = 256, 0.28 (45): 109 -> 97; 9 440, C = 384, 0.52 (33): 156 -> 122.
+// lists alone (8 to 30 us), which save work * (1 - density): 4 720 rows, C = 384, 0.28 (25 GFLOP): 138 -> 113; 9 440, C = 256, 0.28
+// (22): 105 -> 111; 2 360, C = 512, 0.27 (22): 115 -> 131; 18 880, C = 256, 0.28 (45): 158 -> 148; 7 840, C = 512, 0.44 (58): 263 -> 226.
 // density = pairs per row and tap; negative: not known, the sparse case (0.35) is assumed.
+static double left_out(int64_t n, int cin, int cout, int kk, double there, double factor) {
+    return 2e-9 * (double)n * kk * cin * cout * (1 - factor * there);
+}
+static double known_density(double density) { return density < 0 ? 0.35 : density < 1 ? density : 1; }
+
 extern "C" int svtad_plan_wanted(int64_t n, int cin, int cout, int kk, int dtype, double density) {
     if (svtad_plan_bytes(n, kk) == 0 || kk < 2) return 0;
-    const double there = density < 0 ? 0.35 : density < 1 ? density : 1;
-    const double saved = 2e-9 * (double)n * kk * cin * cout * (1 - there);
+    const double there = known_density(density);
     const bool near = kk <= 9;
-    if (saved < (near ? 15.0 : 23.0) + (double)n / 2500 || !use_tc(SVTAD_OP_FWD, n, cin, cout, kk, dtype)) return 0;
-    return (near && n > 2048 ? SVTAD_PLAN_ROWS : 0) | ((!near || n > 2048) && pairs_wgrad_wanted(cin, kk) ? SVTAD_PLAN_PAIRS : 0);
+    const bool pays = near ? n > 2048 && (n > 4096 || there < 0.4) && left_out(n, cin, cout, kk, there, 1.2) >= 13.2 + (double)n / 5000
+                           : left_out(n, cin, cout, kk, there, 1.0) >= 23 + (double)n / 2500;
+    if (!pays || !use_tc(SVTAD_OP_FWD, n, cin, cout, kk, dtype)) return 0;
+    return (near ? SVTAD_PLAN_ROWS : 0) | (pairs_wgrad_wanted(cin, kk) ? SVTAD_PLAN_PAIRS : 0);
+}
+
+// The same for a forward alone, which has to earn its row order by itself: 18 880 rows, C = 512, density 0.35 (52 GFLOP): 64 -> 55 us;
+// 7 840, C = 768, 0.51 (33): 77 -> 67; 37 760, C = 384, 0.35 (58): 78 -> 65; 18 880, C = 384, 0.35 (29): 44 -> 44; 4 720, C = 1024,
+// 0.35 (52): 61 -> 64; 75 520, C = 384, 0.59 (59): 154 -> 157; 75 520, C = 256, 0.35 (52): 66 -> 77; 50 240, C = 768, 0.75 (55): 370 -> 381.
+extern "C" int svtad_plan_wanted_fwd(int64_t n, int cin, int cout, int kk, int dtype, double density) {
+    const int rows = svtad_plan_wanted(n, cin, cout, kk, dtype, density) & SVTAD_PLAN_ROWS;
+    return rows && n > 6144 && left_out(n, cin, cout, kk, known_density(density), 1.2) >= 24 + (double)n / 1600 ? rows : 0;
 }
 
 extern "C" int svtad_conv_fwd(const void* x, const int32_t* nbr, const void* w, const void* bias,
@@ -281,21 +295,25 @@ extern "C" int svtad_conv_bwd_planned(const void* gy, const void* x, const int32
                                       size_t workspace_bytes, void* stream) {
     SV_CHECK_ARG(grad_dtype == dtype || grad_dtype == SVTAD_F32,
                  "svtad_conv_bwd: weight gradients come in the features' type or in float32, not in type %d", grad_dtype);
-    SV_CHECK_ARG((plan_make & ~SVTAD_PLAN_PAIRS) == 0, "svtad_conv_bwd: only the pair lists are made here, not parts %d", plan_make);
     const void* rows_plan = plan_use & SVTAD_PLAN_ROWS ? plan : nullptr;
     const void* pairs_plan = plan_use & SVTAD_PLAN_PAIRS ? plan : nullptr;
-    // where the lists are to be made, in front of the weight gradient on its stream
-    auto make_lists = [&](cudaStream_t on) {
-        if (plan_make == 0 || pairs_plan == nullptr || gw == nullptr || n == 0) return SVTAD_OK;
-        return svtad_plan_build_parts(nbr, n, kk, tokens_per_batch, SVTAD_PLAN_PAIRS, plan, on);
+    // Parts that are to be made first.  The lists alone go in front of the weight gradient on its stream.  With the row order
+    // both come in one launch in front of the two kernels: made side by side, the lists are there first, the weight gradient
+    // fills the GPU and the input gradient has to wait for it (4 720 rows, C = 768: a training pass 185 instead of 166 us).
+    const int to_make = plan_make & ((gx != nullptr && rows_plan != nullptr ? SVTAD_PLAN_ROWS : 0) |
+                                     (gw != nullptr && pairs_plan != nullptr ? SVTAD_PLAN_PAIRS : 0));
+    auto make = [&](cudaStream_t on) {
+        return to_make == 0 || n == 0 ? (int)SVTAD_OK : svtad_plan_build_parts(nbr, n, kk, tokens_per_batch, to_make, plan, on);
     };
     SV_CHECK_ARG(gx != nullptr || gw != nullptr, "svtad_conv_bwd: neither gx nor gw requested");
     SV_CHECK_ARG(gb == nullptr || gw != nullptr, "svtad_conv_bwd: gb needs gw");
-    if (gw == nullptr)
+    if (gw == nullptr) {
+        if (int rc = make((cudaStream_t)stream)) return rc;
         return conv_dgrad_planned(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, rows_plan, table_status,
                                   workspace, workspace_bytes, stream);
+    }
     if (gx == nullptr) {
-        if (int rc = make_lists((cudaStream_t)stream)) return rc;
+        if (int rc = make((cudaStream_t)stream)) return rc;
         return conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, pairs_plan,
                                 workspace, workspace_bytes, stream);
     }
@@ -310,7 +328,7 @@ extern "C" int svtad_conv_bwd_planned(const void* gy, const void* x, const int32
     int dev = 0;
     SV_CUDA(cudaGetDevice(&dev));
     if (!overlap_backward() || n == 0 || dev >= MAX_DEVICES) {
-        int rc = make_lists(s);
+        int rc = make(s);
         if (rc) return rc;
         rc = conv_wgrad_typed(gy, x, nbr, gw, gb, n, cin, cout, kk, tokens_per_batch, dtype, grad_dtype, pairs_plan,
                                   workspace, w_part, s);
@@ -332,6 +350,10 @@ extern "C" int svtad_conv_bwd_planned(const void* gy, const void* x, const int32
         explicit FloorGuard(int floor) : old(tc_set_share_floor(floor)) {}
         ~FloorGuard() { tc_set_share_floor(old); }
     } floor_guard(whole_gpu ? 1 : 2);
+    if (to_make & SVTAD_PLAN_ROWS) {
+        rc = make(s);
+        if (rc) return rc;
+    }
     // fork: the side stream starts where the caller's stream stands
     SV_CUDA(cudaEventRecord(lane.fork, s));
     SV_CUDA(cudaStreamWaitEvent(lane.stream, lane.fork, 0));
@@ -341,7 +363,7 @@ extern "C" int svtad_conv_bwd_planned(const void* gy, const void* x, const int32
                                 w_part, lane.stream);
     };
     if (pairs_plan == nullptr) wgrad();
-    else rc_w = make_lists(lane.stream);
+    else if (to_make == SVTAD_PLAN_PAIRS) rc_w = make(lane.stream);
     rc_d = conv_dgrad_planned(gy, nbr, w, gx, n, cin, cout, kk, tokens_per_batch, dtype, rows_plan, table_status, ws_d, d_part, s);
     if (pairs_plan != nullptr && rc_w == SVTAD_OK) wgrad();
     // join, also after an error: whatever was launched on the side stream is ordered before the caller's next work

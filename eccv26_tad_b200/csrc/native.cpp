@@ -335,12 +335,19 @@ Tensor int32_table(const Tensor& table, void* stream) {
     return form;
 }
 
-// Which parts of a work plan a layer should use: only where the table's density is known, which for a caller's table means
-// that this call, as one that reads the indices' kind from the values (see tokens_per_batch), may ask the device; once per
-// table, and only for layers that a sparse table would bring a plan.  So the kernels that run, and with them the order of
-// their sums, do not hang on when an answer arrives.
-int plan_parts(const Tensor& table, int64_t n, int cin, int cout, int kk, int code, bool may_ask, void* stream) {
-    if (!svtad_plan_wanted(n, cin, cout, kk, code, 0.0)) return 0;
+// Which parts of a work plan a layer's backward should use, of those that it has kernels for (`kernels`: 0 without a
+// backward), and whether its forward should use one: only where the table's density is known, which for a caller's table
+// means that this call, as one that reads the indices' kind from the values (see tokens_per_batch), may ask the device; once
+// per table, and only for layers that a sparse table would bring a plan.  So the kernels that run, and with them the order of
+// their sums, do not hang on when an answer arrives.  Nor does the forward's output hang on whether there is a backward: up to
+// 74 tiles, where the forward without a plan may split a tile's K steps and give other bits, it goes by what a forward gains
+// alone; beyond, where a row's sum is the same either way, it also uses a plan that the input gradient needs anyway.
+struct Parts {
+    int backward = 0;
+    bool forward = false;
+};
+Parts plan_parts(const Tensor& table, int64_t n, int cin, int cout, int kk, int code, int kernels, bool may_ask, void* stream) {
+    if (!svtad_plan_wanted(n, cin, cout, kk, code, 0.0)) return {};
     double density = density_of(table);
     if (density < 0 && may_ask && !capturing(stream)) {
         if (auto f = store().find(table, true)) {
@@ -349,7 +356,11 @@ int plan_parts(const Tensor& table, int64_t n, int cin, int cout, int kk, int co
             f->density = density;
         }
     }
-    return density < 0 ? 0 : svtad_plan_wanted(n, cin, cout, kk, code, density);
+    if (density < 0) return {};
+    Parts p;
+    p.backward = svtad_plan_wanted(n, cin, cout, kk, code, density) & kernels;
+    p.forward = (p.backward & SVTAD_PLAN_ROWS && n > 74 * 128) || svtad_plan_wanted_fwd(n, cin, cout, kk, code, density);
+    return p;
 }
 
 // tokens_per_batch of a call on [B, N, C] features: N when the table's indices are local to each batch row, else 0.
@@ -397,7 +408,7 @@ struct SparseConvBackward : public torch::autograd::Node {
     at::ScalarType w_dtype, b_dtype;                     // of the parameters
     Tensor status;
     Tensor plan;                                         // the forward's, with its row order; undefined without one
-    bool lists = false;                                  // the weight gradient goes by pair lists, made by the backward
+    int parts = 0;                                       // of a plan that the backward uses; it makes what the forward has not
     bool released = false;
 
     std::string name() const override { return "SparseConv2dBackward"; }
@@ -440,7 +451,8 @@ struct SparseConvBackward : public torch::autograd::Node {
         }
         if (need_w) gw = empty_on({d.kk, d.cin, d.cout}, gdt, dev);
         if (need_b) gb = empty_on({d.cout}, gdt, dev);
-        const int make = lists && need_w ? SVTAD_PLAN_PAIRS : 0, use = (plan.defined() ? SVTAD_PLAN_ROWS : 0) | make;
+        const int use = parts & ((need_x ? SVTAD_PLAN_ROWS : 0) | (need_w ? SVTAD_PLAN_PAIRS : 0));
+        const int make = use & ~(plan.defined() ? SVTAD_PLAN_ROWS : 0);
         Tensor pl = plan;
         const size_t bytes = need_w ? svtad_bwd_workspace_bytes(d.n, d.cin, d.cout, d.kk, code, use, st.defined())
                                     : (st.defined() ? svtad_workspace_bytes(SVTAD_OP_DGRAD, d.n, d.cin, d.cout, d.kk, code) : 0);
@@ -489,7 +501,7 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
     const bool grad = at::GradMode::is_enabled() &&
                       (x.requires_grad() || weight.requires_grad() || (bias.defined() && bias.requires_grad()));
     Tensor y, nbr, status, plan;
-    int parts = 0;
+    Parts parts;
     {
         at::NoGradGuard no_grad;
         d.tpb = batched ? tokens_per_batch(table, x.size(0), x.size(1), d.kk, local) : 0;
@@ -502,8 +514,10 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
             y = empty_on({d.n, d.cout}, dt, dev);
         }
         if (grad && x.requires_grad()) status = status_for(table, nbr, d.n, d.kk, d.tpb, stream);
-        parts = plan_parts(table, d.n, d.cin, d.cout, d.kk, code, batched && local < 0, stream);
-        if (parts & SVTAD_PLAN_ROWS) {
+        const int kernels = !grad ? 0 : (x.requires_grad() ? SVTAD_PLAN_ROWS : 0) |
+                            (weight.requires_grad() || (bias.defined() && bias.requires_grad()) ? SVTAD_PLAN_PAIRS : 0);
+        parts = plan_parts(table, d.n, d.cin, d.cout, d.kk, code, kernels, batched && local < 0, stream);
+        if (parts.forward) {
             plan = empty_on({static_cast<int64_t>(svtad_plan_bytes(d.n, d.kk))}, at::kByte, dev);
             check(svtad_plan_build_parts(iptr(nbr), d.n, d.kk, static_cast<int>(d.tpb), SVTAD_PLAN_ROWS, mptr(plan), stream));
         }
@@ -518,7 +532,7 @@ Tensor conv(Tensor x, const Tensor& table, const Tensor& weight, const Tensor& b
         node->b_dtype = bias.defined() ? bias.scalar_type() : dt;
         node->status = status;
         node->plan = plan;
-        node->lists = (parts & SVTAD_PLAN_PAIRS) != 0;
+        node->parts = parts.backward;
         node->x = torch::autograd::SavedVariable(x, false);
         node->table = torch::autograd::SavedVariable(table, false);
         node->weight = torch::autograd::SavedVariable(weight_c, false);

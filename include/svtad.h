@@ -173,12 +173,14 @@ int svtad_conv_bwd(const void* gy, const void* x, const int32_t* nbr, const void
  * route, makes the plan anew.  Any number of layers may share it until then.
  *   svtad_plan_wanted  which parts of a plan gain one layer of this size, in one pass, more than making them costs:
  *                      SVTAD_PLAN_ROWS the row order (forward, input gradient), SVTAD_PLAN_PAIRS the pair lists (weight
- *                      gradient); density = pairs per row and tap of the table, negative where it is not known
+ *                      gradient); density = pairs per row and tap of the table, negative where it is not known;
+ *                      _fwd: in a forward pass without a backward
  *   svtad_plan_bytes   size of a plan (0: no plan for such a table: more than 131072 rows)
  *   svtad_plan_build   makes it in `plan` (device memory, 256-byte aligned); _parts: only the parts named
  *   svtad_plan_counts  where in a plan the kk lists' lengths are (int32, device memory)
  */
 int svtad_plan_wanted(int64_t n, int cin, int cout, int kk, int dtype, double density);
+int svtad_plan_wanted_fwd(int64_t n, int cin, int cout, int kk, int dtype, double density);
 #define SVTAD_PLAN_ROWS 1
 #define SVTAD_PLAN_PAIRS 2
 size_t svtad_plan_bytes(int64_t n, int kk);
@@ -198,8 +200,8 @@ int svtad_conv_fwd_planned(const void* x, const int32_t* nbr, const void* w, con
  * svtad_conv_bwd with a plan (NULL: none), the parts of it to use (bits as svtad_plan_wanted's) and with the type of gw
  * and gb chosen by the caller: grad_dtype is dtype, or SVTAD_F32 for fp32 master parameters of a 16-bit layer (mixed
  * precision).  The values are the same - one rounding to dtype - and are written as fp32, which saves the separate
- * conversion of the gradient.  svtad_conv_bwd_planned with plan_make = SVTAD_PLAN_PAIRS first makes the pair lists in
- * `plan`, next to the input gradient.
+ * conversion of the gradient.  svtad_conv_bwd_planned first makes the parts plan_make of the plan in `plan`, in front of the
+ * kernels that use them.
  */
 int svtad_conv_bwd_typed(const void* gy, const void* x, const int32_t* nbr, const void* w, void* gx, void* gw,
                          void* gb, int64_t n, int cin, int cout, int kk, int tokens_per_batch, int dtype,

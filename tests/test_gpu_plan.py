@@ -259,8 +259,8 @@ def test_one_table_serves_layers_of_different_stencils():
 
 
 @pytest.mark.parametrize("C,ks,T,keep,given", [(512, 3, 320, 0.3, True), (512, 3, 160, 0.5, True), (512, 3, 160, 0.6, True),
-                                               (512, 3, 80, 1.0, True), (512, 5, 25, 0.38, False), (768, 3, 80, 0.3, False),
-                                               (1024, 3, 30, 0.3, True)])
+                                               (512, 3, 80, 1.0, True), (512, 5, 25, 0.38, False), (768, 3, 80, 0.3, False), (768, 3, 160, 0.3, True),
+                                               (1024, 3, 30, 0.3, True), (256, 3, 1280, 0.3, False), (320, 3, 320, 0.2, False)])
 def test_passes_repeat_bit_for_bit(C, ks, T, keep, given):
     """Neither the first pass on a table nor one that follows a synchronisation takes other kernels than the rest."""
     import eccv26_tad_b200 as sv

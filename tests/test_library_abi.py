@@ -252,10 +252,16 @@ def test_a_plan_is_wanted_where_one_layer_pays_for_it():
     def wanted(n, c, kk, density, dtype=_lib.BF16):
         return lib.svtad_plan_wanted(n, c, c, kk, dtype, density)
     assert wanted(18880, 1024, 9, 0.35) == 3 and wanted(18880, 512, 9, 0.35) == 3 and wanted(18880, 384, 9, 0.35, _lib.F16) == 3
+    assert wanted(4720, 768, 9, 0.35) == 3 and wanted(3920, 1024, 9, 0.51) == 0 and wanted(75520, 256, 9, 0.59) == 0
     assert wanted(19600, 192, 9, 0.51) == 0 and wanted(43200, 128, 9, 0.55) == 0            # 17 to 25 us for 5 to 15
     assert wanted(18880, 256, 9, 0.35) == 0 and wanted(1770, 1024, 9, 0.35) == 0
     assert wanted(62720, 512, 9, 0.91) == 0 and wanted(50240, 384, 9, 0.75) == 0            # hardly a neighbor missing
     assert wanted(18880, 256, 25, 0.28) == 2 and wanted(2360, 512, 25, 0.52) == 0           # 5x5: the lists alone
+    assert wanted(12800, 320, 9, 0.27) == 3 and wanted(113280, 192, 9, 0.35) == 1           # lists of 256 channels for 192: rows alone
+    for n, c, density, alone in ((18880, 512, 0.35, 1), (113280, 384, 0.35, 1), (75520, 256, 0.35, 0), (50240, 512, 0.75, 0),
+                                 (4720, 768, 0.35, 0), (9440, 768, 0.35, 1), (7840, 768, 0.51, 1), (18880, 256, 0.35, 0)):
+        fwd = lib.svtad_plan_wanted_fwd(n, c, c, 9, _lib.BF16, density)
+        assert fwd == alone and fwd <= (wanted(n, c, 9, density) & 1)
     assert wanted(18880, 1024, 9, 0.35, _lib.F32) == 0 and wanted(140000, 1024, 9, 0.35) == 0 and wanted(18880, 1024, 1, 0.35) == 0
 
 
