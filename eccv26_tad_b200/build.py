@@ -16,7 +16,7 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "libsvtad.so")
 NATIVE = os.path.join(PKG, "_native.so")
-SOURCES = ["api.cu", "table.cu", "conv_simt.cu", "conv_f32.cu", "conv_tc.cu", "conv_tc_hybrid.cu", "conv_tc_pair.cu", "conv_tc_pairs.cu", "plan.cu", "allreduce.cu", "noalloc.cu"]
+SOURCES = ["api.cu", "table.cu", "conv_simt.cu", "conv_f32.cu", "conv_f32_tc.cu", "conv_tc.cu", "conv_tc_hybrid.cu", "conv_tc_pair.cu", "conv_tc_pairs.cu", "plan.cu", "allreduce.cu", "noalloc.cu"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 

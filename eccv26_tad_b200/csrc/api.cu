@@ -18,7 +18,7 @@ int set_error(int code, const char* fmt, ...) {
 }
 
 // 0 = automatic, 1 = force CUDA-core kernels, 2 = force tensor-core kernels
-static int forced_path() {
+int forced_path() {
     const char* e = getenv("SVTAD_FORCE_PATH");
     if (e == nullptr || *e == 0) return 0;
     if (strcmp(e, "simt") == 0 || strcmp(e, "fp32") == 0) return 1;

@@ -1,4 +1,5 @@
-// fp32 SparseConv2D on the CUDA cores: forward, input gradient (gather form) and weight gradient.
+// fp32 SparseConv2D on the CUDA cores: forward, input gradient (gather form) and weight gradient.  The tensor-core kernels
+// (conv_f32_tc.cu) take over where f32_tc_wanted() says so; SVTAD_FORCE_PATH=simt keeps everything here.
 //
 // fp32 tensors cannot go through the tensor cores as TF32 without losing the 1e-5 the reference's fp32 path holds
 // (opentad/models/bricks/2d_sparse_v3.cu:545-651, a 32 x 32 shared-memory tile kernel with two __syncthreads per
@@ -544,8 +545,14 @@ bool f32_supported(int cin, int cout, int kk, int dtype) {
     return dtype == SVTAD_F32 && cin % 4 == 0 && cout % 4 == 0 && kk <= F_MAX_KK;
 }
 
-int f32_fwd(const ConvArgs& p, cudaStream_t s) { return dispatch_conv_f32<false>(p, nullptr, s); }
-int f32_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) { return dispatch_conv_f32<true>(p, status, s); }
+static bool use_f32_tc(int cin, int cout) { return forced_path() != 1 && f32_tc_wanted(cin, cout); }
+
+int f32_fwd(const ConvArgs& p, cudaStream_t s) {
+    return use_f32_tc(p.cin, p.cout) ? f32_tc_fwd(p, s) : dispatch_conv_f32<false>(p, nullptr, s);
+}
+int f32_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
+    return use_f32_tc(p.cin, p.cout) ? f32_tc_dgrad(p, status, s) : dispatch_conv_f32<true>(p, status, s);
+}
 
 // Token ranges: about two full loads of the GPU (four CTAs an SM), so that the centre tap's CTAs, which have every token
 // for a pair, do not outlast the rest; each range at least 128 tokens, the partials of several ranges at most 31 MB, which
@@ -569,13 +576,13 @@ int f32_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void*
     const size_t need = f32_wgrad_ws_bytes(n, cin, cout, kk);
     if (ws_bytes < need)
         return set_error(SVTAD_ERR_WORKSPACE, "svtad_conv_wgrad: workspace %zu < %zu bytes", ws_bytes, need);
-    static std::atomic<uint64_t> ready{0};
-    int rc = f32_allow_smem(reinterpret_cast<const void*>(wgrad_f32_kernel), sizeof(WgradSmem), ready);
-    if (rc) return rc;
     const int splits = f32_wgrad_splits(n, cin, cout, kk);
     const long n_w = (long)kk * cin * cout, rows = (n + splits - 1) / splits;
     float* ws_w = static_cast<float*>(ws);
     float* ws_b = reinterpret_cast<float*>(static_cast<char*>(ws) + align_up((size_t)splits * n_w * sizeof(float), 256));
+    static std::atomic<uint64_t> ready{0};
+    int rc = f32_allow_smem(reinterpret_cast<const void*>(wgrad_f32_kernel), sizeof(WgradSmem), ready);
+    if (rc) return rc;
     const int tiles_m = (cin + 63) / 64, tiles_n = (cout + 63) / 64;
     dim3 grid((unsigned)(kk * tiles_m * tiles_n + (gb ? tiles_n : 0)), (unsigned)splits);
     wgrad_f32_kernel<<<grid, F_THREADS, sizeof(WgradSmem), s>>>((const float*)gy, (const float*)x, nbr, ws_w, ws_b, (long)n,

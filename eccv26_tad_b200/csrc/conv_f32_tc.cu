@@ -1,0 +1,494 @@
+// fp32 SparseConv2D on the tensor cores: forward and input gradient (gather form), every operand split into three
+// bf16 values.
+//
+// An fp32 value is the exact sum of three bf16 ones, x = x1 + x2 + x3 (8 + 8 + 8 bits, each the rounded rest of the ones
+// before), and a product needs six of the nine partial products: x1 w1, x1 w2, x2 w1, x1 w3, x2 w2, x3 w1; the three that
+// are left out are below 2^-26 of it.  What would spoil the result is the accumulator: tcgen05.mma cuts its sum off towards
+// zero at every instruction (measured, relative error of a sum of N(0,1) products against 64 bits: 2.4e-8 after one
+// instruction of 16 products, 6.5e-8 after 4, 1.2e-7 after 8, 4.7e-7 after 32, nearly all of it bias).  So a sum stays in
+// tensor memory for one step of 64 products only and is then added to the running sum in registers, rounded to nearest; the
+// small partial products have columns of their own.  Errors against 64 bits (2-norm) over 4 to 1024 channels, 9 to 49
+// taps, 59 to 7 080 rows: forward 5e-8 to 1.4e-7, input gradient 5e-8 to 1.2e-7; the CUDA-core kernels (conv_f32.cu)
+// 6e-8 to 4.7e-7 and 6e-8 to 3.0e-7, each call's larger than here.  The
+// planes of values below 2^-108 lose bits under bf16's range: tensors whose values are all below 4e-34 come out less exact.
+//
+// A value that is infinite, NaN or beyond bf16's range makes its planes NaN, also in sums that it has no part in (the rows
+// of a tile that lack a neighbor are rows of zeros).  Sums that are not finite are therefore made again from the fp32
+// values, pair by pair, before they are stored.
+//
+// Measured (graph replays, before: the CUDA-core kernels): 784 rows, C = 192, keep 50 %: forward 21.2 -> 12.2 us, input
+// gradient 22.2 -> 12.3; 4 720 rows, C = 192, keep 30 %: 54.5 -> 28.8, 57.1 -> 28.2; 5 880
+// rows, full grid, 320 -> 96: 144 -> 46, 134 -> 39.  What bounds the loops: eight warps that load, split and store
+// (835 issue slots per scheduler and step; 768 cycles of tensor work) and the trip of the operands from L2, which is one step
+// long.
+#include <cfloat>
+
+#include "tc_common.cuh"
+
+namespace svtad {
+
+constexpr int T3_A_WARPS = 8;
+constexpr int T3_E_WARPS = 4;
+constexpr int T3_THREADS = (T3_A_WARPS + 1 + T3_E_WARPS) * 32;      // the MMA warp (TMEM owner) sits between them
+constexpr int T3_BN = 64;
+constexpr int T3_B_PLANE = T3_BN * 128;
+constexpr int T3_RING = 2, T3_B_STAGE = 3 * T3_B_PLANE;
+constexpr int T3_A_COL = 256, T3_A_COLS = 96;               // behind two accumulators of 128 columns
+constexpr int T3_PARK = T3_BN + 4;                     // floats per row of the parked sums
+
+typedef unsigned long long t3_pair;                    // two fp32 values
+__device__ __forceinline__ t3_pair t3_pack(uint32_t lo, uint32_t hi) {
+    t3_pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ void t3_unpack(t3_pair v, uint32_t& lo, uint32_t& hi) { asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v)); }
+__device__ __forceinline__ t3_pair t3_add(t3_pair a, t3_pair b) {
+    t3_pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ t3_pair t3_neg_add(t3_pair a, t3_pair b) {      // b - a
+    t3_pair r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(b), "l"(a));
+    return r;
+}
+
+// Two values -> their three planes, packed, the second with its sign turned: plane minus value is one instruction on the
+// half of a packed register.  (Widening the plane by a shift and a mask first: 16.5 cycles per pair and scheduler instead of
+// 12.7 in a loop of its own - conversions, shifts, masks and selects go through a pipe of half the width.)
+__device__ __forceinline__ void t3_split2(float a, float b, uint32_t (&p)[3]) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        p[q] = pack2(a, b, false);
+        if (q < 2)
+            asm("{\n\t.reg .b16 lo, hi;\n\t"
+                "mov.b32 {lo, hi}, %2;\n\t"
+                "sub.rn.f32.bf16 %0, lo, %0;\n\t"
+                "sub.rn.f32.bf16 %1, hi, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(p[q]));
+    }
+}
+// eight values -> four packed words of each plane
+__device__ __forceinline__ void t3_split8(const float (&v)[8], uint32_t (&p)[3][4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        uint32_t w[3];
+        t3_split2(v[2 * e], v[2 * e + 1], w);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) p[q][e] = w[q];
+    }
+}
+
+// What is read for a row that is not there: an address like any other instead of a branch or a select at the load.  Rows
+// of more channels than this are refused by f32_tc_wanted().
+constexpr int T3_MOST = 4096;
+__device__ __align__(32) float t3_zeros[T3_MOST];
+
+// FULL: all channels are there and 32-byte aligned; else those four for which first / second say so
+template <bool FULL>
+__device__ __forceinline__ void t3_load8(float (&v)[8], const float* p, bool first, bool second) {
+    if constexpr (FULL) {
+        asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
+    } else {
+        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 a = first ? __ldg(reinterpret_cast<const float4*>(p)) : none, b = second ? __ldg(reinterpret_cast<const float4*>(p) + 1) : none;
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    }
+}
+__device__ __forceinline__ void t3_sts16(uint32_t dst, const uint32_t (&v)[4]) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void t3_sts8(uint32_t dst, uint32_t lo, uint32_t hi) {
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst), "r"(lo), "r"(hi) : "memory");
+}
+// 16 rows x 32 words of tensor memory: lane t holds words 8 j + 2 (t % 4), + 1 of row t / 4 (v[4 j], v[4 j + 1]) and of row
+// t / 4 + 8 (v[4 j + 2], v[4 j + 3])
+__device__ __forceinline__ void t3_tmem_st(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+                 ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+                   "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void t3_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D += A (tensor memory) . B
+__device__ __forceinline__ void t3_umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+// all lanes wait, and agree on the outcome
+__device__ __forceinline__ bool t3_wait(uint32_t bar, uint32_t parity, volatile int* s_abort, int* err, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, s_abort, err, code));
+}
+// what the warp wrote to a buffer is the tensor core's to read
+__device__ __forceinline__ void t3_filled(uint32_t bar, int lane) {
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
+
+// A step's instructions: A in tensor memory (three planes of 32 columns), the accumulator two blocks of 64 columns: x1 w1, and
+// all others with their sign turned (the second planes are stored negative).
+template <bool B_MN>
+__device__ __forceinline__ void t3_issue_ts(uint32_t d, uint32_t a_tmem, uint32_t b_tile) {
+    const uint32_t b1 = ((b_tile & 0x3FFFFu) >> 4) | (B_MN ? smem_desc_lbo_bits(8192) : 0u), b2 = b1 + (T3_B_PLANE >> 4), b3 = b2 + (T3_B_PLANE >> 4);
+    constexpr uint32_t hi = smem_desc_hi(1024), neg = 1u << 13;
+    constexpr uint32_t i2 = make_idesc(1, 0, B_MN, TILE_M, 2 * T3_BN), i1 = make_idesc(1, 0, B_MN, TILE_M, T3_BN);
+#pragma unroll
+    for (int ks = 0; ks < STAGE_K / 16; ++ks) {
+        const uint32_t a = a_tmem + ks * 8, o = ks * (B_MN ? 128 : 2);
+        t3_umma_ts(d, a, b1 + o, hi, i2, ks != 0 ? 1u : 0u);                      // x1 w1, -(x1 w2)
+        t3_umma_ts(d + T3_BN, a + 32, b1 + o, hi, i1, 1u);                        // -(x2 w1)
+        t3_umma_ts(d + T3_BN, a, b3 + o, hi, i1 | neg, 1u);                       // -(x1 w3)
+        t3_umma_ts(d + T3_BN, a + 32, b2 + o, hi, i1 | neg, 1u);                  // -(x2 w2)
+        t3_umma_ts(d + T3_BN, a + 64, b1 + o, hi, i1 | neg, 1u);                  // -(x3 w1)
+    }
+}
+// a step's accumulator, added to the lane's running sums
+__device__ __forceinline__ void t3_drain(t3_pair (&sum)[T3_BN / 2], uint32_t t_addr) {
+#pragma unroll
+    for (int c = 0; c < T3_BN; c += 16) {
+        uint32_t g0[16], g1[16];
+        tmem_ld16(t_addr + c, g0);
+        tmem_ld16(t_addr + T3_BN + c, g1);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const t3_pair step = t3_neg_add(t3_pack(g1[2 * e], g1[2 * e + 1]), t3_pack(g0[2 * e], g0[2 * e + 1]));
+            sum[c / 2 + e] = t3_add(sum[c / 2 + e], step);
+        }
+    }
+}
+
+__device__ __forceinline__ bool t3_finite(float v) { return fabsf(v) <= FLT_MAX; }
+
+// out[row][col] of the forward or input gradient without its bias, from the fp32 values
+template <bool DGRAD>
+__device__ __noinline__ float t3_row_sum(const float* a, const int32_t* nbr, const float* w, long row, int col, long n, int cred,
+                                         int cin, int cout, int kk, int tpb) {
+    float s = 0.f;
+    const long off = tpb > 0 ? (row / tpb) * (long)tpb : 0;
+    for (int k = 0; k < kk; ++k) {
+        const int raw = __ldg(nbr + row * kk + k);
+        const long j = (long)raw + off;
+        if (raw < 0 || j >= n) continue;
+        const float* ar = a + j * cred;
+        const float* wr = DGRAD ? w + ((long)(kk - 1 - k) * cin + col) * cout : w + (long)k * cin * cout + col;
+        const long step = DGRAD ? 1 : cout;
+        for (int c = 0; c < cred; ++c) {
+            s = fmaf(__ldg(ar + c), __ldg(wr + c * step), s);
+            if (s != s) return s;
+        }
+    }
+    return s;
+}
+
+// ---------------------------------------------------------------------------------------------
+// forward / input gradient: a CTA per 128 rows x 64 columns; K steps are (tap, 64 channels)
+// ---------------------------------------------------------------------------------------------
+// A goes from registers to tensor memory, B through shared memory: with both in shared memory its 128 bytes a cycle were the bound
+// (72 KB written, 96 KB read and the loads' way through L1 a step; 4 720 rows, C = 192: 34.2 us instead of 28.8).
+// SPLIT: a cluster of G CTAs shares the tile's K steps; the sums meet in shared memory, in the order of the CTAs.
+template <bool DGRAD, bool SPLIT, bool FULL>
+__global__ void __launch_bounds__(T3_THREADS, 1)
+conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr, const float* __restrict__ w,
+                   const float* __restrict__ bias, float* __restrict__ out, const int32_t* __restrict__ status, long n, int cred,
+                   int cn, int cin, int cout, int kk, int tpb, int n_blks, int G, int* __restrict__ err) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    TmaTail* tail = reinterpret_cast<TmaTail*>(smem + T3_RING * T3_B_STAGE);
+    const float** s_row = reinterpret_cast<const float**>(tail + 1);      // [kk][128] gathered rows, or the row of zeros
+    volatile int* s_abort = &tail->abort_flag;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t stage_base = smem_u32(smem);
+    const int share = SPLIT ? (int)blockIdx.x % G : 0, item = SPLIT ? (int)blockIdx.x / G : (int)blockIdx.x;
+    const long row0 = (long)(item / n_blks) * TILE_M;
+    const int n0 = item % n_blks * T3_BN;
+    const int chunks = (cred + STAGE_K - 1) / STAGE_K, total = kk * chunks;
+    const int k_lo = SPLIT ? total * share / G : 0, k_hi = SPLIT ? total * (share + 1) / G : total;
+
+    if (warp == T3_A_WARPS) {
+        tmem_alloc(smem_u32(&tail->tmem_slot), 512);
+        tmem_relinquish();
+    }
+    if (tid == T3_A_WARPS * 32) {
+        for (int s = 0; s < T3_RING; ++s) {
+            mbar_init(smem_u32(&tail->full[s]), T3_A_WARPS);
+            mbar_init(smem_u32(&tail->empty[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&tail->accum_full[b]), 1);
+            mbar_init(smem_u32(&tail->accum_empty[b]), T3_E_WARPS * 32);
+        }
+        tail->abort_flag = 0;
+        fence_mbar_init();
+    }
+    pdl_wait();
+    if (DGRAD && status != nullptr && (__ldg(status) & SVTAD_TABLE_ASYMMETRIC)) {      // uniform over the grid
+        __syncthreads();
+        if (warp == T3_A_WARPS) tmem_dealloc(tail->tmem_slot, 512);
+        return;
+    }
+    {
+        const int32_t* rows = nbr + row0 * kk;
+        const int valid = (int)(n - row0 < TILE_M ? n - row0 : TILE_M) * kk;
+        for (int e = tid; e < TILE_M * kk; e += T3_THREADS) {
+            const int r = e / kk, k = e - r * kk;
+            const int raw = e < valid ? __ldg(rows + e) : -1;
+            const long j = (long)raw + (tpb > 0 ? ((row0 + r) / tpb) * (long)tpb : 0);
+            s_row[k * TILE_M + r] = raw >= 0 && j < n ? a + j * cred : t3_zeros;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = tail->tmem_slot;
+    pdl_trigger();
+
+    t3_pair sum[T3_BN / 2];
+    const int q = warp & 3;
+    bool whole = true;
+    if (warp < T3_A_WARPS) {
+        // ------------------------------------------------------------------ producers: all of them fill every buffer
+        // A: 16 rows per warp, straight from registers to tensor memory.  A lane loads channels 8 c .. + 7 and 32 + 8 c .. + 7
+        // (c = lane % 4) of rows lane / 4 and lane / 4 + 8; its j-th four channels become products 16 j + 4 c .. + 3 of the
+        // step, an order that B's rows (forward) or 8-byte pieces of them (input gradient) follow.
+        const int c8 = (lane & 3) * 8, r16 = (warp & 3) * 32 + (warp >> 2) * 16 + (lane >> 2);
+        const uint32_t a_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32 + (warp >> 2) * 16) << 16) + T3_A_COL;
+        // B: rows warp * 8 + {0 .. 3}, + 4, eight lanes each.  Rows r and r + 2 share a half-warp, for the input gradient's stores.
+        const int sub = lane & 7, row4 = (lane >> 4) + (lane >> 3 & 1) * 2, b_row = warp * 8 + row4;
+        uint32_t b_place;
+        if (DGRAD) {
+            b_place = b_row * 128 + ((((sub >> 2) * 4 + (sub >> 1 & 1)) ^ (b_row & 7)) << 4) + (sub & 1) * 8;
+        } else {
+            const int r = (warp >> 2) * 32 + (warp & 3) * 4 + row4;
+            b_place = r * 128 + ((sub ^ (r & 7)) << 4);
+        }
+        const uint32_t b_next = DGRAD ? 4 * 128 : 16 * 128;       // rows of the second four
+        float va[2][2][8], vb[2][8];
+        int k = k_lo / chunks, c0 = (k_lo - k * chunks) * STAGE_K;
+        const float* const* my_row = s_row + r16;
+        // forward: a row of B is a channel, along the columns; input gradient: a column, along the channels
+        auto b_at = [&] { return w + ((long)(DGRAD ? kk - 1 - k : k) * cin + (DGRAD ? n0 : c0) + b_row) * cout + (DGRAD ? c0 : n0) + 8 * sub; };
+        const float* b_ptr = b_at();
+        auto load_a = [&] {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const float* row = my_row[k * TILE_M + 8 * r] + c0 + c8;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) t3_load8<FULL>(va[r][h], row + 32 * h, c0 + c8 + 32 * h < cred, c0 + c8 + 32 * h + 4 < cred);
+            }
+        };
+        auto load_b = [&] {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int along = (DGRAD ? c0 : n0) + 8 * sub;
+                const bool in = FULL || (DGRAD ? n0 : c0) + b_row + 4 * h < cin;
+                t3_load8<FULL>(vb[h], b_ptr + 4 * h * cout, in && along < cout, in && along + 4 < cout);
+            }
+        };
+        if (k_lo < k_hi) {
+            load_a();
+            load_b();
+        }
+        int s = 0;
+        uint32_t ph = 1;
+        for (int st = k_lo; st < k_hi; ++st) {
+            uint32_t pa[3][16];
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t p[3][4];
+                    t3_split8(va[r][h], p);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) pa[q][8 * h + 4 * (e >> 1) + 2 * r + (e & 1)] = p[q][e];
+                }
+            // the next step's loads are on their way while this one is multiplied; behind the last step this one's again
+            if (st + 1 < k_hi) {
+                c0 += STAGE_K;
+                b_ptr += DGRAD ? STAGE_K : STAGE_K * cout;
+                if (c0 >= cred) { c0 = 0; ++k; b_ptr = b_at(); }
+            }
+            load_a();
+            if (!t3_wait(smem_u32(&tail->empty[s]), ph, s_abort, err, 71)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int q = 0; q < 3; ++q) t3_tmem_st(a_addr + s * T3_A_COLS + q * 32, pa[q]);
+            const uint32_t b_tile = stage_base + s * T3_B_STAGE + b_place;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t p[3][4];
+                t3_split8(vb[h], p);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const uint32_t dst = b_tile + q * T3_B_PLANE + h * b_next;
+                    if (DGRAD) {
+                        t3_sts8(dst ^ (h ? 64u : 0u), p[q][0], p[q][1]);
+                        t3_sts8(dst ^ (h ? 96u : 32u), p[q][2], p[q][3]);
+                    } else {
+                        t3_sts16(dst, p[q]);
+                    }
+                }
+            }
+            load_b();
+            t3_tmem_st_wait();
+            tc_fence_before();
+            t3_filled(smem_u32(&tail->full[s]), lane);
+            if (++s == T3_RING) { s = 0; ph ^= 1u; }
+        }
+    } else if (warp == T3_A_WARPS) {
+        // ------------------------------------------------------------------ MMA issuer (whole warp waits, one lane issues)
+        int s = 0;
+        uint32_t ph = 0;
+        for (int st = 0; st < k_hi - k_lo; ++st) {
+            const int buf = st & 1;
+            if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((st >> 1) & 1) ^ 1, s_abort, err, 72)) break;
+            if (!mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 73)) break;
+            tc_fence_after();
+            if (elect_one_sync()) {
+                t3_issue_ts<!DGRAD>(tmem_base + buf * (2 * T3_BN), tmem_base + T3_A_COL + s * T3_A_COLS, stage_base + s * T3_B_STAGE);
+                umma_commit(smem_u32(&tail->empty[s]));
+                umma_commit(smem_u32(&tail->accum_full[buf]));
+            }
+            __syncwarp();
+            if (++s == T3_RING) { s = 0; ph ^= 1u; }
+        }
+    } else {
+        // ------------------------------------------------------------------ the last four warps keep the sums
+#pragma unroll
+        for (int c = 0; c < T3_BN / 2; ++c) sum[c] = 0;
+        const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+        for (int st = 0; st < k_hi - k_lo; ++st) {
+            const int buf = st & 1;
+            if (!t3_wait(smem_u32(&tail->accum_full[buf]), (st >> 1) & 1, s_abort, err, 74)) { whole = false; break; }
+            tc_fence_after();
+            t3_drain(sum, t_addr + buf * (2 * T3_BN));
+            tc_fence_before();
+            mbar_arrive(smem_u32(&tail->accum_empty[buf]));
+        }
+    }
+    // four columns of a row: + bias, and sums that are not finite from the fp32 values
+    auto finish = [&](long row, int col, float4 f) {
+        float* e = reinterpret_cast<float*>(&f);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (!t3_finite(e[c])) e[c] = t3_row_sum<DGRAD>(a, nbr, w, row, col + c, n, cred, cin, cout, kk, tpb);
+        if (!DGRAD && bias != nullptr) {
+            const float4 b = __ldg(reinterpret_cast<const float4*>(bias + col));
+            f.x += b.x; f.y += b.y; f.z += b.z; f.w += b.w;
+        }
+        *reinterpret_cast<float4*>(out + row * cn + col) = f;
+    };
+    if constexpr (!SPLIT) {
+        const long row = row0 + q * 32 + lane;
+        if (warp > T3_A_WARPS && whole && row < n) {
+#pragma unroll
+            for (int c = 0; c < T3_BN / 4; ++c) {
+                uint32_t u[4];
+                t3_unpack(sum[2 * c], u[0], u[1]);
+                t3_unpack(sum[2 * c + 1], u[2], u[3]);
+                if (n0 + 4 * c < cn)
+                    finish(row, n0 + 4 * c, make_float4(__uint_as_float(u[0]), __uint_as_float(u[1]), __uint_as_float(u[2]), __uint_as_float(u[3])));
+            }
+        }
+    } else {
+        // a CTA whose wait gave up stops the whole cluster: the others' sums are not finished with what it left behind
+        __syncthreads();
+        if (tid < G && *s_abort) store_to_cta(smem_u32(&tail->abort_flag), tid, 1);
+        cluster_barrier();          // every CTA's instructions are done: nothing is left in the rings, which take the sums now
+        const bool all = *s_abort == 0;
+        const int per = (TILE_M + G - 1) / G;               // rows that a CTA finishes: [share * per, ...)
+        const uint32_t park = stage_base;                   // [CTA the sums come from][row][T3_PARK]
+        if (all && warp > T3_A_WARPS) {
+            const int r = q * 32 + lane, owner = r / per;
+            const uint32_t dst = map_to_cta(park + ((share * per + r - owner * per) * T3_PARK) * 4, owner);
+#pragma unroll
+            for (int c = 0; c < T3_BN / 4; ++c) {
+                uint32_t u[4];
+                t3_unpack(sum[2 * c], u[0], u[1]);
+                t3_unpack(sum[2 * c + 1], u[2], u[3]);
+                asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + c * 16), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]) : "memory");
+            }
+        }
+        cluster_barrier();
+        const float* sums = reinterpret_cast<const float*>(smem);
+        const int rows = !all ? 0 : share * per + per <= TILE_M ? per : TILE_M - share * per;
+        for (int e = tid; e < rows * (T3_BN / 4); e += T3_THREADS) {
+            const int r = e / (T3_BN / 4), c = e % (T3_BN / 4) * 4;
+            const long row = row0 + share * per + r;
+            if (row >= n || n0 + c >= cn) continue;
+            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int p = 0; p < G; ++p) {
+                const float4 u = *reinterpret_cast<const float4*>(sums + (p * per + r) * T3_PARK + c);
+                f.x += u.x; f.y += u.y; f.z += u.z; f.w += u.w;
+            }
+            finish(row, n0 + c, f);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == T3_A_WARPS) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------
+// whole blocks of 64 channels, rows that 32-byte loads may read
+static bool t3_full(int cin, int cout, const void* a, const void* b) {
+    return cin % STAGE_K == 0 && cout % STAGE_K == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 31) == 0;
+}
+
+template <bool DGRAD, bool SPLIT, bool FULL>
+static int launch_f32_tc(const ConvArgs& p, const int32_t* status, int G, cudaStream_t s) {
+    const int cn = DGRAD ? p.cin : p.cout, cred = DGRAD ? p.cout : p.cin;
+    const size_t table = (size_t)p.kk * TILE_M * sizeof(float*);
+    const int n_blks = (cn + T3_BN - 1) / T3_BN;
+    const long tiles = (p.n + TILE_M - 1) / TILE_M * n_blks;
+    const size_t smem = 1024 + T3_RING * T3_B_STAGE + sizeof(TmaTail) + table;
+    auto kern = conv_f32_tc_kernel<DGRAD, SPLIT, FULL>;
+    int rc = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem);
+    if (rc) return rc;
+    SV_CUDA(launch_pdl(kern, dim3((unsigned)(tiles * G)), dim3(T3_THREADS), smem, s, SPLIT ? G : 1, (const float*)p.a, p.nbr,
+                       (const float*)p.w, (const float*)p.bias, (float*)p.out, status, (long)p.n, cred, cn, p.cin, p.cout, p.kk, p.tpb,
+                       n_blks, G, tc_error_ptr()));
+    return SVTAD_OK;
+}
+
+template <bool DGRAD>
+static int dispatch_f32_tc(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
+    const int cn = DGRAD ? p.cin : p.cout, cred = DGRAD ? p.cout : p.cin;
+    const long tiles = (p.n + TILE_M - 1) / TILE_M * ((cn + T3_BN - 1) / T3_BN), sms = tc_num_sms();
+    const int steps = p.kk * ((cred + STAGE_K - 1) / STAGE_K);
+    // a step takes 0.72 us and sharing a tile out 2.5; clusters of three and more do not pack a GPC's SMs completely
+    const int sizes[5] = {2, 3, 4, 5, 8}, limit[5] = {148, 120, 120, 112, 112};
+    double best = (double)((tiles + sms - 1) / sms) * steps * 0.72;
+    int G = 1;
+    for (int g = 0; g < 5; ++g) {
+        if (tiles * sizes[g] * 148 > limit[g] * sms) continue;
+        const double u = (steps + sizes[g] - 1) / sizes[g] * 0.72 + 2.5;
+        if (u < best) { best = u; G = sizes[g]; }
+    }
+    const bool full = t3_full(p.cin, p.cout, p.a, p.w);
+    if (G > 1) return full ? launch_f32_tc<DGRAD, true, true>(p, status, G, s) : launch_f32_tc<DGRAD, true, false>(p, status, G, s);
+    return full ? launch_f32_tc<DGRAD, false, true>(p, status, 1, s) : launch_f32_tc<DGRAD, false, false>(p, status, 1, s);
+}
+
+// They win at every size measured (59 rows, 16 -> 16 channels: 8.6 -> 8.3 us; 1024 -> 1024: 57 -> 32).
+bool f32_tc_wanted(int cin, int cout) { return cin <= T3_MOST && cout <= T3_MOST; }
+
+int f32_tc_fwd(const ConvArgs& p, cudaStream_t s) { return dispatch_f32_tc<false>(p, nullptr, s); }
+int f32_tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) { return dispatch_f32_tc<true>(p, status, s); }
+
+}  // namespace svtad
