@@ -1,5 +1,5 @@
-// fp32 SparseConv2D on the tensor cores: forward and input gradient (gather form), every operand split into three
-// bf16 values.
+// fp32 SparseConv2D on the tensor cores: forward, input gradient (gather form) and weight gradient, every operand split
+// into three bf16 values.
 //
 // An fp32 value is the exact sum of three bf16 ones, x = x1 + x2 + x3 (8 + 8 + 8 bits, each the rounded rest of the ones
 // before), and a product needs six of the nine partial products: x1 w1, x1 w2, x2 w1, x1 w3, x2 w2, x3 w1; the three that
@@ -8,8 +8,8 @@
 // instruction of 16 products, 6.5e-8 after 4, 1.2e-7 after 8, 4.7e-7 after 32, nearly all of it bias).  So a sum stays in
 // tensor memory for one step of 64 products only and is then added to the running sum in registers, rounded to nearest; the
 // small partial products have columns of their own.  Errors against 64 bits (2-norm) over 4 to 1024 channels, 9 to 49
-// taps, 59 to 7 080 rows: forward 5e-8 to 1.4e-7, input gradient 5e-8 to 1.2e-7; the CUDA-core kernels (conv_f32.cu)
-// 6e-8 to 4.7e-7 and 6e-8 to 3.0e-7, each call's larger than here.  The
+// taps, 59 to 7 080 rows: forward 5e-8 to 1.4e-7, input gradient 5e-8 to 1.2e-7, weight gradient 5e-8 to 1.4e-7; the
+// CUDA-core kernels (conv_f32.cu) 6e-8 to 4.7e-7, 6e-8 to 3.0e-7, 1.2e-7 to 3.6e-7, each call's larger than here.  The
 // planes of values below 2^-108 lose bits under bf16's range: tensors whose values are all below 4e-34 come out less exact.
 //
 // A value that is infinite, NaN or beyond bf16's range makes its planes NaN, also in sums that it has no part in (the rows
@@ -17,8 +17,8 @@
 // values, pair by pair, before they are stored.
 //
 // Measured (graph replays, before: the CUDA-core kernels): 784 rows, C = 192, keep 50 %: forward 21.2 -> 12.2 us, input
-// gradient 22.2 -> 12.3; 4 720 rows, C = 192, keep 30 %: 54.5 -> 28.8, 57.1 -> 28.2; 5 880
-// rows, full grid, 320 -> 96: 144 -> 46, 134 -> 39.  What bounds the loops: eight warps that load, split and store
+// gradient 22.2 -> 12.3; 4 720 rows, C = 192, keep 30 %: 54.5 -> 28.8, 57.1 -> 28.2, weight gradient 47.8 -> 23.2; 5 880
+// rows, full grid, 320 -> 96: 144 -> 46, 134 -> 39, 103 -> 62.  What bounds the loops: eight warps that load, split and store
 // (835 issue slots per scheduler and step; 768 cycles of tensor work) and the trip of the operands from L2, which is one step
 // long.
 #include <cfloat>
@@ -31,9 +31,11 @@ constexpr int T3_A_WARPS = 8;
 constexpr int T3_E_WARPS = 4;
 constexpr int T3_THREADS = (T3_A_WARPS + 1 + T3_E_WARPS) * 32;      // the MMA warp (TMEM owner) sits between them
 constexpr int T3_BN = 64;
-constexpr int T3_B_PLANE = T3_BN * 128;
-constexpr int T3_RING = 2, T3_B_STAGE = 3 * T3_B_PLANE;
+constexpr int T3_A_PLANE = A_TILE_BYTES, T3_B_PLANE = T3_BN * 128;
+constexpr int T3_STAGE = 3 * (T3_A_PLANE + T3_B_PLANE);      // weight gradient
+constexpr int T3_RING = 2, T3_B_STAGE = 3 * T3_B_PLANE;      // forward, input gradient: A in tensor memory
 constexpr int T3_A_COL = 256, T3_A_COLS = 96;               // behind two accumulators of 128 columns
+constexpr int T3_COLS = 3 * T3_BN;                     // accumulator columns of a step
 constexpr int T3_PARK = T3_BN + 4;                     // floats per row of the parked sums
 
 typedef unsigned long long t3_pair;                    // two fp32 values
@@ -132,7 +134,24 @@ __device__ __forceinline__ void t3_filled(uint32_t bar, int lane) {
     if (lane == 0) mbar_arrive(bar);
 }
 
-// A step's instructions: A in tensor memory (three planes of 32 columns), the accumulator two blocks of 64 columns: x1 w1, and
+// A step's instructions, A and B in shared memory and both MN-major: 16 products further are 16 rows of 128 bytes.  Columns
+// [0, 64) of the accumulator get x1 w1, [64, 128) x1 w2 + x2 w1, [128, 192) the rest.  The planes w1, w2, w3 lie one behind the
+// other, so three instructions do the six products: x1 . [w1 w2 w3] (N = 192), x2 . [w1 w2] (N = 128), x3 . w1 (N = 64), and
+// read A three times instead of six (with N = 64 throughout, shared memory would be the bound by a factor of 1.5).
+__device__ __forceinline__ void t3_issue(uint32_t d, uint32_t stage) {
+    const uint32_t a_lo = ((stage & 0x3FFFFu) >> 4) | smem_desc_lbo_bits(8192);
+    const uint32_t b_lo = a_lo + (3 * T3_A_PLANE >> 4);
+    constexpr uint32_t hi = smem_desc_hi(1024);
+    constexpr uint32_t i3 = make_idesc(1, 1, 1, TILE_M, 3 * T3_BN), i2 = make_idesc(1, 1, 1, TILE_M, 2 * T3_BN), i1 = make_idesc(1, 1, 1, TILE_M, T3_BN);
+#pragma unroll
+    for (int ks = 0; ks < STAGE_K / 16; ++ks) {
+        const uint32_t a = a_lo + ks * 128, b = b_lo + ks * 128;
+        umma_f16_lh(d, a, hi, b, hi, i3, ks != 0 ? 1u : 0u);
+        umma_f16_lh_acc(d + T3_BN, a + (T3_A_PLANE >> 4), hi, b, hi, i2);
+        umma_f16_lh_acc(d + 2 * T3_BN, a + 2 * (T3_A_PLANE >> 4), hi, b, hi, i1);
+    }
+}
+// The same with A in tensor memory (three planes of 32 columns), where the accumulator is left two blocks of 64 columns: x1 w1, and
 // all others with their sign turned (the second planes are stored negative).
 template <bool B_MN>
 __device__ __forceinline__ void t3_issue_ts(uint32_t d, uint32_t a_tmem, uint32_t b_tile) {
@@ -150,16 +169,21 @@ __device__ __forceinline__ void t3_issue_ts(uint32_t d, uint32_t a_tmem, uint32_
     }
 }
 // a step's accumulator, added to the lane's running sums
+template <int BLOCKS>
 __device__ __forceinline__ void t3_drain(t3_pair (&sum)[T3_BN / 2], uint32_t t_addr) {
 #pragma unroll
     for (int c = 0; c < T3_BN; c += 16) {
-        uint32_t g0[16], g1[16];
+        uint32_t g0[16], g1[16], g2[16];
         tmem_ld16(t_addr + c, g0);
         tmem_ld16(t_addr + T3_BN + c, g1);
+        if (BLOCKS == 3) tmem_ld16(t_addr + 2 * T3_BN + c, g2);
         tmem_ld_wait();
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const t3_pair step = t3_neg_add(t3_pack(g1[2 * e], g1[2 * e + 1]), t3_pack(g0[2 * e], g0[2 * e + 1]));
+            t3_pair step = t3_pack(g0[2 * e], g0[2 * e + 1]);
+            const t3_pair turned = t3_pack(g1[2 * e], g1[2 * e + 1]);
+            if (BLOCKS == 3) step = t3_add(step, t3_neg_add(turned, t3_pack(g2[2 * e], g2[2 * e + 1])));
+            else step = t3_neg_add(turned, step);
             sum[c / 2 + e] = t3_add(sum[c / 2 + e], step);
         }
     }
@@ -370,7 +394,7 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
             const int buf = st & 1;
             if (!t3_wait(smem_u32(&tail->accum_full[buf]), (st >> 1) & 1, s_abort, err, 74)) { whole = false; break; }
             tc_fence_after();
-            t3_drain(sum, t_addr + buf * (2 * T3_BN));
+            t3_drain<2>(sum, t_addr + buf * (2 * T3_BN));
             tc_fence_before();
             mbar_arrive(smem_u32(&tail->accum_empty[buf]));
         }
@@ -443,6 +467,318 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
 }
 
 // ---------------------------------------------------------------------------------------------
+// weight gradient: D[128 input channels of a tap][64 columns] over the (row, neighbor) pairs that exist, 64 a step
+// ---------------------------------------------------------------------------------------------
+// A CTA takes a range of tokens, lists the pairs that its tap has there (1.3 of 4 tokens at keep 30 %, against a step for every
+// 64 tokens) and works through the list.  The centre tap has every token for a pair, so its tokens are cut into more ranges than
+// the others' (a CTA whose list is empty costs little, one whose list is three times as long sets the time).  Both operands lie
+// as rows of tokens (MN-major).  Partials to ws_w[range][kk][cin][cout].  The bias gradient's CTAs, behind all others, add up
+// gy's columns to ws_b[range][cout].
+constexpr int T3_SEG = 4096;               // tokens listed at a time
+struct T3Units {
+    int m_blks, n_blks, centre;
+    int own, others, bias;                 // ranges of tokens for the centre tap, the other taps, the bias gradient (0: not wanted)
+};
+
+template <bool FULL>
+__global__ void __launch_bounds__(T3_THREADS, 1)
+wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, const int32_t* __restrict__ nbr,
+                    float* __restrict__ ws_w, float* __restrict__ ws_b, long n, int cin, int cout, int kk, int tpb, T3Units u,
+                    int* __restrict__ err) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    TmaTail* tail = reinterpret_cast<TmaTail*>(smem + T3_RING * T3_STAGE);
+    int2* s_pair = reinterpret_cast<int2*>(tail + 1);      // [T3_SEG] the pairs: row of gy, row of x
+    __shared__ int s_count[T3_A_WARPS], s_pairs, s_end;      // s_end: number of steps, once known
+    volatile int* s_abort = &tail->abort_flag;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t stage_base = smem_u32(smem);
+
+    // which (tap, blocks, range)
+    const int tiles = u.m_blks * u.n_blks, own_units = tiles * u.own, all_units = own_units + (kk - 1) * tiles * u.others;
+    int tap, tile, range, ranges;
+    if ((int)blockIdx.x < own_units) {
+        tap = u.centre; ranges = u.own;
+        tile = blockIdx.x / ranges; range = blockIdx.x - tile * ranges;
+    } else if ((int)blockIdx.x < all_units) {
+        const int b = blockIdx.x - own_units;
+        ranges = u.others;
+        tile = b / ranges; range = b - tile * ranges;
+        tap = tile / tiles; tile -= tap * tiles;
+        if (tap >= u.centre) ++tap;
+    } else {
+        const int b = blockIdx.x - all_units;
+        ranges = u.bias;
+        tile = b / ranges; range = b - tile * ranges;
+        tap = kk;
+    }
+    const int m0 = tap < kk ? tile / u.n_blks * TILE_M : 0, n0 = (tap < kk ? tile % u.n_blks : tile) * T3_BN;
+    const long each = (n + ranges - 1) / ranges, i_begin = min(n, range * each), i_end = min(n, i_begin + each);
+
+    if (tap == kk) {
+        // column sums of gy: four columns and every 16th row per thread in two chains, the 32 sums added in pairs
+        pdl_wait();
+        pdl_trigger();
+        const int by = tid >> 4, col = n0 + (tid & 15) * 4;
+        float4* part = reinterpret_cast<float4*>(smem);     // [16][16]
+        auto add = [](float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
+        if (by < 16) {
+            float4 sum[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+#pragma unroll 2
+            for (long i = i_begin + by; i < i_end; i += 32) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (col < cout && i + 16 * h < i_end) add(sum[h], __ldg(reinterpret_cast<const float4*>(gy + (i + 16 * h) * cout + col)));
+            }
+            add(sum[0], sum[1]);
+            part[tid] = sum[0];
+        }
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1) {
+            __syncthreads();
+            if (by < d) add(part[tid], part[tid + d * 16]);
+        }
+        if (by == 0 && col < cout) *reinterpret_cast<float4*>(ws_b + (long)range * cout + col) = part[tid];
+        return;
+    }
+
+    if (warp == T3_A_WARPS) {
+        tmem_alloc(smem_u32(&tail->tmem_slot), 512);
+        tmem_relinquish();
+    }
+    if (tid == T3_A_WARPS * 32) {
+        for (int s = 0; s < T3_RING; ++s) {
+            mbar_init(smem_u32(&tail->full[s]), T3_A_WARPS);
+            mbar_init(smem_u32(&tail->empty[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&tail->accum_full[b]), 1);
+            mbar_init(smem_u32(&tail->accum_empty[b]), T3_E_WARPS * 32);
+        }
+        tail->abort_flag = 0;
+        fence_mbar_init();
+    }
+    // producers: the first half of the warps fills the first 64 channels of A, the others the second; eight lanes per row,
+    // eight channels each
+    constexpr int A_ITS = TILE_M / T3_A_WARPS / 4, B_ITS = STAGE_K / T3_A_WARPS / 4;
+    const int sub8 = (lane & 7) * 8, rg = lane >> 3;
+    const int half = warp / (T3_A_WARPS / 2), a_tok = warp % (T3_A_WARPS / 2) * (A_ITS * 4), b_tok = warp * (B_ITS * 4);
+    const int ca = m0 + half * 64 + sub8, cb = n0 + sub8;
+    const bool real = m0 + half * 64 < cin;                // else zeros, written once
+    if (warp < T3_A_WARPS && !real) {
+        for (int s = 0; s < T3_RING; ++s)
+            for (int p = 0; p < 3; ++p)
+#pragma unroll
+                for (int c = 0; c < A_ITS; ++c)
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(stage_base + s * T3_STAGE + p * T3_A_PLANE + warp * (A_ITS * 512) + c * 512 + lane * 16), "r"(0) : "memory");
+        fence_proxy_async();
+    }
+    if (tid == 0) s_end = 0x7fffffff;
+    pdl_wait();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = tail->tmem_slot;
+    pdl_trigger();
+
+    if (warp < T3_A_WARPS) {
+        // ------------------------------------------------------------------ producers: all of them fill every buffer
+        constexpr int Q = T3_SEG / T3_A_WARPS / 32;
+        const uint32_t place[2] = {(uint32_t)(rg * 128 + (((lane & 7) ^ rg) << 4)), (uint32_t)((4 + rg) * 128 + (((lane & 7) ^ (4 + rg)) << 4))};
+        float v[A_ITS + B_ITS][8];
+        auto store = [&](uint32_t rows, uint32_t plane, int it, const float (&f)[8]) {
+            uint32_t p[3][4];
+            t3_split8(f, p);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) t3_sts16(rows + (it >> 1) * 1024 + place[it & 1] + q * plane, p[q]);
+        };
+        auto load = [&](int st, int it) {
+            if (it < A_ITS) {
+                const int j = s_pair[st * STAGE_K + a_tok + 4 * it + rg].y;
+                t3_load8<FULL>(v[it], j >= 0 ? x + (long)j * cin + ca : t3_zeros + sub8, ca < cin, ca + 4 < cin);
+            } else {
+                const int i = s_pair[st * STAGE_K + b_tok + 4 * (it - A_ITS) + rg].x;
+                t3_load8<FULL>(v[it], i >= 0 ? gy + (long)i * cout + cb : t3_zeros + sub8, cb < cout, cb + 4 < cout);
+            }
+        };
+        bool alive = true;
+        int s = 0, done = 0;
+        uint32_t ph = 1;
+        for (long seg = i_begin; alive && seg < i_end; seg += T3_SEG) {
+            // ---- the segment's pairs, ascending: a warp lists an eighth of it
+            const int len = (int)min((long)T3_SEG, i_end - seg), eighth = (len + 255) / 256 * 32;
+            {
+                int jj[Q], cnt = 0;
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const int at = warp * eighth + q * 32 + lane;
+                    jj[q] = q * 32 < eighth && at < len ? __ldg(nbr + (seg + at) * kk + tap) : -1;
+                }
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const long i = seg + warp * eighth + q * 32 + lane, j = (long)jj[q] + (tpb > 0 ? (i / tpb) * (long)tpb : 0);
+                    jj[q] = jj[q] >= 0 && j < n ? (int)j : -1;
+                    cnt += __popc(__ballot_sync(0xffffffffu, jj[q] >= 0));
+                }
+                if (lane == 0) s_count[warp] = cnt;
+                named_bar_sync(1, T3_A_WARPS * 32);         // also: nobody reads the last segment's list any more
+                int at = 0, pairs = 0;
+#pragma unroll
+                for (int q = 0; q < T3_A_WARPS; ++q) {
+                    at += q < warp ? s_count[q] : 0;
+                    pairs += s_count[q];
+                }
+                if (tid == 0) s_pairs = pairs;
+                if (tid < STAGE_K && pairs + tid < (pairs + STAGE_K - 1) / STAGE_K * STAGE_K) s_pair[pairs + tid] = make_int2(-1, -1);
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const unsigned m = __ballot_sync(0xffffffffu, jj[q] >= 0);
+                    if (jj[q] >= 0) s_pair[at + __popc(m & ((1u << lane) - 1u))] = make_int2((int)(seg + warp * eighth + q * 32 + lane), jj[q]);
+                    at += __popc(m);
+                }
+                named_bar_sync(1, T3_A_WARPS * 32);
+            }
+            const int steps = (s_pairs + STAGE_K - 1) / STAGE_K;
+            if (steps > 0) {
+#pragma unroll
+                for (int it = 0; it < A_ITS + B_ITS; ++it)
+                    if (it >= A_ITS || real) load(0, it);
+            }
+            for (int st = 0; st < steps; ++st) {
+                if (!t3_wait(smem_u32(&tail->empty[s]), ph, s_abort, err, 75)) { alive = false; break; }
+                const uint32_t a_rows = stage_base + s * T3_STAGE + warp * (A_ITS * 512), b_rows = stage_base + s * T3_STAGE + 3 * T3_A_PLANE + b_tok * 128;
+                const int next = st + 1 < steps ? st + 1 : st;
+                if (real) {
+#pragma unroll
+                    for (int it = 0; it < A_ITS; ++it) {
+                        store(a_rows, T3_A_PLANE, it, v[it]);
+                        load(next, it);
+                    }
+                }
+#pragma unroll
+                for (int it = A_ITS; it < A_ITS + B_ITS; ++it) {
+                    store(b_rows, T3_B_PLANE, it - A_ITS, v[it]);
+                    load(next, it);
+                }
+                t3_filled(smem_u32(&tail->full[s]), lane);
+                if (++s == T3_RING) { s = 0; ph ^= 1u; }
+            }
+            done += steps;
+        }
+        // one more round, which carries nothing: the end
+        if (alive && t3_wait(smem_u32(&tail->empty[s]), ph, s_abort, err, 75)) {
+            if (tid == 0) s_end = done;
+            t3_filled(smem_u32(&tail->full[s]), lane);
+        }
+    } else if (warp == T3_A_WARPS) {
+        // ------------------------------------------------------------------ MMA issuer (whole warp waits, one lane issues)
+        for (int g = 0;; ++g) {
+            const int s = g % T3_RING, buf = g & 1;
+            if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((g >> 1) & 1) ^ 1, s_abort, err, 76)) break;
+            if (!mbar_wait(smem_u32(&tail->full[s]), g / T3_RING & 1, s_abort, err, 77)) break;
+            const bool end = *reinterpret_cast<volatile int*>(&s_end) == g;
+            __syncwarp();
+            tc_fence_after();
+            if (elect_one_sync()) {
+                if (!end) {
+                    t3_issue(tmem_base + buf * T3_COLS, stage_base + s * T3_STAGE);
+                    umma_commit(smem_u32(&tail->empty[s]));
+                }
+                umma_commit(smem_u32(&tail->accum_full[buf]));
+            }
+            __syncwarp();
+            if (end) break;
+        }
+    } else {
+        // ------------------------------------------------------------------ the last four warps keep the sums
+        t3_pair sum[T3_BN / 2];
+#pragma unroll
+        for (int c = 0; c < T3_BN / 2; ++c) sum[c] = 0;
+        const uint32_t t_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        bool whole = true;
+        for (int g = 0;; ++g) {
+            const int buf = g & 1;
+            if (!t3_wait(smem_u32(&tail->accum_full[buf]), (g >> 1) & 1, s_abort, err, 78)) { whole = false; break; }
+            if (*reinterpret_cast<volatile int*>(&s_end) == g) break;
+            tc_fence_after();
+            t3_drain<3>(sum, t_addr + buf * T3_COLS);
+            tc_fence_before();
+            mbar_arrive(smem_u32(&tail->accum_empty[buf]));
+        }
+        const int ci = m0 + (warp & 3) * 32 + lane;
+        float* dst = ws_w + (((long)range * kk + tap) * cin + ci) * cout + n0;
+        if (whole && ci < cin) {
+#pragma unroll
+            for (int c = 0; c < T3_BN / 4; ++c) {
+                uint32_t f[4];
+                t3_unpack(sum[2 * c], f[0], f[1]);
+                t3_unpack(sum[2 * c + 1], f[2], f[3]);
+                if (n0 + 4 * c < cout) *reinterpret_cast<uint4*>(dst + 4 * c) = make_uint4(f[0], f[1], f[2], f[3]);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == T3_A_WARPS) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+}
+
+// gw[k][ci][co] (k < kk) or gb[co] (k == kk) from the fp32 values
+__device__ __noinline__ float t3_pair_sum(const float* gy, const float* x, const int32_t* nbr, int k, int ci, int co, long n, int cin,
+                                          int cout, int kk, int tpb) {
+    float s = 0.f;
+    for (long i = 0; i < n && s == s; ++i) {
+        if (k == kk) {
+            s += __ldg(gy + i * cout + co);
+            continue;
+        }
+        const int raw = __ldg(nbr + i * kk + k);
+        const long j = (long)raw + (tpb > 0 ? (i / tpb) * (long)tpb : 0);
+        if (raw >= 0 && j < n) s = fmaf(__ldg(x + j * cin + ci), __ldg(gy + i * cout + co), s);
+    }
+    return s;
+}
+
+// fixed-order sum of the ranges' partials, four elements per thread; the bias gradient behind the weights
+__global__ void __launch_bounds__(128)
+wgrad_f32_tc_sum_kernel(const float* __restrict__ ws_w, const float* __restrict__ ws_b, T3Units u, float* __restrict__ gw,
+                        float* __restrict__ gb, const float* __restrict__ gy, const float* __restrict__ x,
+                        const int32_t* __restrict__ nbr, long n, int cin, int cout, int kk, int tpb) {
+    pdl_wait();
+    pdl_trigger();
+    const long n_w = (long)kk * cin * cout;
+    long e = (blockIdx.x * 128l + threadIdx.x) * 4;
+    const float* src = ws_w;
+    float* dst = gw;
+    long stride = n_w;
+    int k = kk, ci = 0, ranges = u.bias;
+    if (e >= n_w) {
+        e -= n_w;
+        if (gb == nullptr || e >= cout) return;
+        src = ws_b; dst = gb; stride = cout;
+    } else {
+        const long row = e / cout;
+        k = (int)(row / cin);
+        ci = (int)(row - (long)k * cin);
+        ranges = k == u.centre ? u.own : u.others;
+    }
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int q = 0; q < ranges; ++q) {
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(src + q * stride + e));
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    float* f = reinterpret_cast<float*>(&s);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        if (!t3_finite(f[c])) f[c] = t3_pair_sum(gy, x, nbr, k, ci, (int)(e % cout) + c, n, cin, cout, kk, tpb);
+    *reinterpret_cast<float4*>(dst + e) = s;
+}
+
+// ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
 // whole blocks of 64 channels, rows that 32-byte loads may read
@@ -485,10 +821,42 @@ static int dispatch_f32_tc(const ConvArgs& p, const int32_t* status, cudaStream_
     return full ? launch_f32_tc<DGRAD, false, true>(p, status, 1, s) : launch_f32_tc<DGRAD, false, false>(p, status, 1, s);
 }
 
-// They win at every size measured (59 rows, 16 -> 16 channels: 8.6 -> 8.3 us; 1024 -> 1024: 57 -> 32).
-bool f32_tc_wanted(int cin, int cout) { return cin <= T3_MOST && cout <= T3_MOST; }
+// Forward and input gradient win at every size measured (59 rows, 16 -> 16 channels: 8.6 -> 8.3 us; 1024 -> 1024: 57 -> 32).  The
+// weight gradient has a fixed cost of 7 us per CTA: 118 rows, C = 192: 8.7 and 11.2 us; 472: 12.2 and 12.7, 64 -> 1024: 15.2 and 19.2;
+// 944: 17.4 and 13.6, 64 -> 1024: 24.6 and 22.6.
+bool f32_tc_wanted(int op, int64_t n, int cin, int cout) {
+    return (op == SVTAD_OP_WGRAD ? n >= 640 : n > 0) && cin <= T3_MOST && cout <= T3_MOST;
+}
 
 int f32_tc_fwd(const ConvArgs& p, cudaStream_t s) { return dispatch_f32_tc<false>(p, nullptr, s); }
 int f32_tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) { return dispatch_f32_tc<true>(p, status, s); }
+
+// at most `limit` ranges of tokens (what the workspace of the kernels without tensor cores holds the partials of)
+int f32_tc_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin, int cout, int kk, int tpb,
+                 float* ws_w, float* ws_b, int limit, cudaStream_t s) {
+    T3Units u{(cin + TILE_M - 1) / TILE_M, (cout + T3_BN - 1) / T3_BN, kk / 2, 1, 1, 0};
+    const long tiles = (long)u.m_blks * u.n_blks, sms = tc_num_sms();
+    // one in three tokens is assumed to have a pair; a step takes 0.9 us, a CTA 7 besides, the partials go through L2 twice
+    double best = 0;
+    for (int c = 1; c <= limit; ++c) {
+        const int own = 3 * c < limit ? 3 * c : limit;
+        const long ctas = tiles * ((kk - 1) * c + own);
+        const double steps = n * 0.33 / c > (double)n / own ? n * 0.33 / c : (double)n / own;
+        const double t = (double)((ctas + sms - 1) / sms) * (steps / STAGE_K * 0.9 + 7) + ((double)c * (kk - 1) + own) * cin * cout * 8 / 6e6;
+        if (c == 1 || t < best * 0.98) { best = t; u.others = c; u.own = own; }
+    }
+    if (gb != nullptr) u.bias = limit < 16 ? limit : 16;
+    const size_t smem = 1024 + T3_RING * T3_STAGE + sizeof(TmaTail) + T3_SEG * sizeof(int2);
+    auto kern = t3_full(cin, cout, x, gy) ? wgrad_f32_tc_kernel<true> : wgrad_f32_tc_kernel<false>;
+    int rc = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem);
+    if (rc) return rc;
+    const long ctas = tiles * ((kk - 1) * u.others + u.own) + (long)u.n_blks * u.bias;
+    SV_CUDA(launch_pdl(kern, dim3((unsigned)ctas), dim3(T3_THREADS), smem, s, 1, (const float*)gy, (const float*)x, nbr, ws_w, ws_b, (long)n,
+                       cin, cout, kk, tpb, u, tc_error_ptr()));
+    const long quads = ((long)kk * cin * cout + (gb ? cout : 0)) / 4;
+    SV_CUDA(launch_pdl(wgrad_f32_tc_sum_kernel, dim3((unsigned)((quads + 127) / 128)), dim3(128), 0, s, 1, ws_w, ws_b, u, (float*)gw,
+                       (float*)gb, (const float*)gy, (const float*)x, nbr, (long)n, cin, cout, kk, tpb));
+    return SVTAD_OK;
+}
 
 }  // namespace svtad
