@@ -89,6 +89,7 @@ int tc_read_error(int32_t* code_out);
 int tc_set_share(int n);
 int tc_get_share();
 int tc_num_sms();               // of the current device
+int tc_ensure_smem(const void* kern, size_t bytes);
 int tc_set_share_floor(int n);
 
 // the single-CTA tensor-core kernels behind tc_* (conv_tc_hybrid.cu)

@@ -6,6 +6,7 @@
 // order-preserving integer keys, compaction is a ballot/popc prefix scan, and the table is
 // emitted straight from the kept set without materialising the old-to-new map in HBM.
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -14,10 +15,10 @@ namespace svtad {
 // float -> uint32 key with the same order as "a > b" on floats; every NaN maps to the largest
 // key (torch.topk ranks NaN above all numbers); -0.0 and +0.0 map to the same key.
 __device__ __forceinline__ uint32_t score_key(float f) {
-    if (f != f) return 0xFFFFFFFFu;
-    if (f == 0.0f) f = 0.0f;
-    uint32_t b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+    // the sum makes -0.0 +0.0 and any NaN the one that arithmetic returns, 0x7fffffff; it goes through another pipe than
+    // compares and selects, which the builders' loops are short of
+    const int b = __float_as_int(__fadd_rn(f, 0.0f));
+    return (uint32_t)(b ^ (b >> 31 | (int)0x80000000));
 }
 
 // a score with that key (the canonical one of those that share it)
@@ -28,30 +29,40 @@ __device__ __forceinline__ float key_score(uint32_t key) {
 // ------------------------------------------------------------------------------------------
 // init
 // ------------------------------------------------------------------------------------------
+// Four entries per thread from 32-bit indices (UINT: fewer than 2^32 entries), one division for the row and one for its place
+// in the grid.
+template <typename UINT>
 __global__ void table_init_kernel(int32_t* __restrict__ table, long total, int hw, int h, int w,
                                   int ksize, int kk) {
     pdl_wait();
     pdl_trigger();
-    long f0 = (long)(blockIdx.x * (long)blockDim.x + threadIdx.x) * 4;
-    if (f0 >= total) return;
-    int r = ksize >> 1;
+    const UINT f0 = ((UINT)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (f0 >= (UINT)total) return;
+    const int r = ksize >> 1;
+    UINT row = f0 / (UINT)kk;
+    int tap = (int)(f0 - row * (UINT)kk), p = (int)(row % (UINT)hw), y = p / w, x = p - y * w;
+    int ty = tap / ksize, tx = tap - ty * ksize;
     int32_t v[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        long f = f0 + e;
-        long row = f / kk;
-        int tap = (int)(f - row * kk);
-        int p = (int)(row % hw);
-        int y = p / w, x = p - y * w;
-        int dy = tap / ksize - r, dx = tap % ksize - r;
-        int yy = y + dy, xx = x + dx;
-        v[e] = ((unsigned)yy < (unsigned)h && (unsigned)xx < (unsigned)w)
-                   ? (int32_t)(row + dy * w + dx) : -1;
+        const int dy = ty - r, dx = tx - r;
+        v[e] = ((unsigned)(y + dy) < (unsigned)h && (unsigned)(x + dx) < (unsigned)w) ? (int32_t)row + dy * w + dx : -1;
+        if (++tx == ksize) {
+            tx = 0;
+            if (++ty == ksize) {
+                ty = 0;
+                ++row;
+                if (++x == w) {
+                    x = 0;
+                    if (++y == h) y = 0;
+                }
+            }
+        }
     }
-    if (f0 + 3 < total && (reinterpret_cast<uintptr_t>(table) & 15) == 0) {
+    if (f0 + 3 < (UINT)total && (reinterpret_cast<uintptr_t>(table) & 15) == 0) {
         *reinterpret_cast<int4*>(table + f0) = make_int4(v[0], v[1], v[2], v[3]);
     } else {
-        for (int e = 0; e < 4 && f0 + e < total; ++e) table[f0 + e] = v[e];
+        for (int e = 0; e < 4 && f0 + e < (UINT)total; ++e) table[f0 + e] = v[e];
     }
 }
 
@@ -238,19 +249,22 @@ table_build_warp_kernel(const float* __restrict__ scores, int n_seg, int L, int 
 }
 
 // ------------------------------------------------------------------------------------------
-// build: a thread-block cluster per segment (seg_len > 256: a clip, or a long batch row)
+// build: several CTAs per segment (seg_len > 256: a clip, or a long batch row)
 // ------------------------------------------------------------------------------------------
-// What bounds it: latency.  A clip of 15 680 scores is 60 KB and its table 340 KB, but every step of the selection
-// (four radix passes, two prefix sums) waits for the one before.  One CTA per clip took 115 us for 15 680 -> 9 408
-// tokens, most of it in 83 dependent trips to memory per thread while the rows were written out by two SMs of 148.
-// So G CTAs (one per 2048 tokens, at most 8) share a segment:
-//   * scores are read once and stay in registers as order-preserving keys;
-//   * per radix pass the CTAs count their own keys and add the G histograms up through distributed shared memory, each
-//     for itself, so a pass costs one cluster barrier;
-//   * what is kept travels as one bit per token: every CTA gets the whole bit set (6.4 KB at the longest segment) and
-//     scans it, after which rank(token) is a word, a mask and a popcount in its own shared memory;
-//   * the rows of a word's kept tokens are contiguous in the output: a warp writes them with coalesced stores.
-constexpr int SEG_THREADS = 1024, SEG_MAX = 51200, SEG_WORDS = SEG_MAX / 32;
+// What bounds it: latency, and the issue slots of the few SMs that write the rows out.  A clip of 15 680 scores is 60 KB
+// and its table 340 KB, but every step of the selection (radix passes, prefix sums) waits for the one before.  So the CTAs
+// of a segment share nothing: each makes the whole selection from all scores, in its registers and its own shared memory,
+// and writes the rows of its part of the tokens; there are as many CTAs as half the GPU holds, and the next round's take
+// the other half.  Measured in cycles of a CTA, 15 680 -> 9 408 tokens, two clips: scores 2 900, radix passes 5 700, ranks 1 600,
+// rows 3 400.  Clusters of up to eight CTAs that shared the selection through distributed shared memory, one barrier per
+// radix pass, took 2 900, 10 900, 3 700 and 7 800; three rounds of two 160-frame clips 42 us where these kernels take 24.
+//   * scores are read once and stay in registers as order-preserving keys; radix passes of 12, 10 and 10 bits, the last two
+//     over the keys of the first one's bin, and only until every key of a bin is kept;
+//   * what is kept is one bit per token: after a scan over the words rank(token) is a word, a mask and a popcount;
+//   * the rows of a word's kept tokens are contiguous in the output: warps write them with coalesced stores, several per
+//     word where a CTA has few.
+// Segments beyond 16 384 tokens keep the clusters: their keys do not fit one CTA's registers.
+constexpr int SEG_THREADS = 1024, SEG_WARPS = SEG_THREADS / 32, SEG_MAX = 51200, SEG_ALONE = 16384;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint32_t in_cta(uint32_t saddr, int cta) {
@@ -258,91 +272,305 @@ __device__ __forceinline__ uint32_t in_cta(uint32_t saddr, int cta) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
     return r;
 }
-template <int G>
 __device__ __forceinline__ void cluster_sync() {
-    if constexpr (G == 1) {
-        __syncthreads();
-    } else {
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// exclusive prefix sum of v over the block in thread order
-__device__ __forceinline__ int block_excl_scan(int v, int* s_w) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int incl = v;
+__device__ __forceinline__ int warp_incl_scan(int v) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += t;
+        const int t = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += t;
     }
+    return v;
+}
+// exclusive prefix sum of v over the block in thread order (all threads call)
+__device__ __forceinline__ int block_excl_scan(int v, int* s_w) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int incl = warp_incl_scan(v);
     __syncthreads();               // s_w free for reuse
     if (lane == 31) s_w[wid] = incl;
     __syncthreads();
-    int w = s_w[lane];             // SEG_THREADS / 32 = 32 warps
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, w, d);
-        if (lane >= d) w += t;
-    }
-    const int before = __shfl_sync(0xffffffffu, w, (wid + 31) & 31);
-    return (wid > 0 ? before : 0) + incl - v;
+    return __reduce_add_sync(0xffffffffu, lane < wid ? s_w[lane] : 0) + incl - v;
 }
 
-// ITEMS = words of 32 tokens a warp holds; table_in: rows to renumber (a later pruning round), else the grid's own
-template <int G, int ITEMS>
+struct SegArgs {
+    const float* scores;
+    int L, k, h, w, ksize;
+    uint32_t magic_w, magic_hw, magic_ks;
+    int kk;
+    int32_t* kept_idx;
+    int32_t* table;
+    int64_t* idx64;
+    const int32_t* table_in;               // rows to renumber (a later pruning round); null: the grid's own
+    int staged;                            // this CTA's rows of table_in fit its shared memory
+    int words;                             // of 32 tokens per CTA
+    int ctas;                              // per segment
+};
+
+// The rows of a later round start their trip to shared memory; source and target stay equally aligned.
+__device__ __forceinline__ int seg_shift(const int32_t* rows_in) { return (int)((reinterpret_cast<uintptr_t>(rows_in) >> 2) & 3); }
+__device__ __forceinline__ void seg_stage_rows(const int32_t* rows_in, int n_rows, int kk, int32_t* s_rows) {
+    const int shift = seg_shift(rows_in), total = n_rows * kk, lead = min(total, (4 - shift) & 3), vec = (total - lead) >> 2, tid = threadIdx.x;
+    auto copy = [&](int f, int bytes) {
+        const uint32_t dst = smem_addr(s_rows + shift + f);
+        if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(rows_in + f) : "memory");
+        else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(rows_in + f) : "memory");
+    };
+    if (tid < lead) copy(tid, 4);
+    for (int v = tid; v < vec; v += SEG_THREADS) copy(lead + 4 * v, 16);
+    for (int f = lead + 4 * vec + tid; f < total; f += SEG_THREADS) copy(f, 4);
+}
+
+// s_rank: per word its kept bits and the output row of its first kept token.  A warp writes part `part` of `parts` of a word's
+// kept positions and table rows; `in`: the word's rows of the previous table.
+__device__ __forceinline__ void seg_write_word(const SegArgs& p, const uint2* s_rank, uint32_t* list, int seg, int word, int part,
+                                               int parts, const int32_t* in) {
+    const int lane = threadIdx.x & 31, hw = p.h * p.w, r0 = p.ksize >> 1, seg0 = seg * p.L;      // row numbers fit 31 bits
+    const uint2 rk = s_rank[word];
+    const int e = word * 32 + lane;
+    auto renumbered = [&](unsigned loc) -> int32_t {
+        const uint2 r = s_rank[loc >> 5];
+        const uint32_t below = r.x << (31 - (loc & 31));        // the token's own bit on top
+        return below >> 31 ? (int32_t)(r.y + __popc(below) - 1) : -1;
+    };
+    if ((rk.x >> lane) & 1u) {
+        const int r = __popc(rk.x & ((1u << lane) - 1u));
+        if (part == 0 && p.kept_idx != nullptr) p.kept_idx[rk.y + r] = e;
+        if (part == 0 && p.idx64 != nullptr) p.idx64[rk.y + r] = e;
+        const int q = hw == 1 ? 0 : e - div_magic(e, p.magic_hw) * hw;
+        const int y = p.w == 1 ? q : div_magic(q, p.magic_w), x = q - y * p.w;
+        list[r] = (uint32_t)lane | (uint32_t)(y & 0xFF) << 8 | (uint32_t)(x & 0xFF) << 16;
+    }
+    if (p.table == nullptr) return;
+    __syncwarp();
+    const int kk = p.kk, entries = __popc(rk.x) * kk, step = 32 * parts, d_row = step / kk, d_tap = step - d_row * kk;
+    int32_t* out = p.table + (long)rk.y * kk;
+    int r = (part * 32 + lane) / kk, tap = part * 32 + lane - r * kk;
+    auto advance = [&] {
+        r += d_row;
+        tap += d_tap;
+        if (tap >= kk) { tap -= kk; ++r; }
+    };
+    if (p.table_in != nullptr) {
+        // later round: the kept rows of the previous table, renumbered
+#pragma unroll 4
+        for (int f = part * 32 + lane; f < entries; f += step) {
+            const int32_t old = in[(int)(list[r] & 31u) * kk + tap];
+            const unsigned loc = (unsigned)(old - seg0);
+            out[f] = old >= 0 && loc < (unsigned)p.L ? renumbered(loc) : -1;
+            advance();
+        }
+    } else {
+        for (int f = part * 32 + lane; f < entries; f += step) {
+            const int ty = p.ksize == 1 ? tap : div_magic(tap, p.magic_ks);
+            const int dy = ty - r0, dx = tap - ty * p.ksize - r0;
+            const uint32_t it = list[r];
+            const int y = (int)(it >> 8 & 0xFFu) + dy, x = (int)(it >> 16) + dx;
+            out[f] = (unsigned)y < (unsigned)p.h && (unsigned)x < (unsigned)p.w ? renumbered(word * 32 + (int)(it & 31u) + dy * p.w + dx) : -1;
+            advance();
+        }
+    }
+    __syncwarp();
+}
+
+constexpr int SEG_FEW = 2048;              // keys of a bin that are gathered
+
+// ITEMS = words per warp: all of the segment's, word 32 j + warp for j < ITEMS
+template <int ITEMS>
 __global__ void __launch_bounds__(SEG_THREADS)
-table_build_segment_kernel(const float* __restrict__ scores, int L, int k, int h, int w, int ksize, uint32_t magic_w,
-                           uint32_t magic_hw, uint32_t magic_ks, int kk,
-                           int32_t* __restrict__ kept_idx, int32_t* __restrict__ table, int64_t* __restrict__ idx64,
-                           const int32_t* __restrict__ table_in, int staged) {
+table_select_kernel(const SegArgs p) {
+    extern __shared__ __align__(16) int32_t s_rows[];     // this CTA's rows of table_in, if they fit
+    constexpr int WORDS = ITEMS * SEG_WARPS;
+    __shared__ __align__(16) int s_hist[4096 + 2 * 1024];
+    __shared__ int s_found[3], s_w[SEG_WARPS];
+    __shared__ uint32_t s_from[WORDS], s_eq[WORDS];        // keys from the threshold on, and equal to it
+    __shared__ uint2 s_rank[WORDS];                        // see seg_write_word
+    __shared__ uint32_t s_few[SEG_FEW];
+    __shared__ int s_n;
+    __shared__ uint32_t s_list[SEG_WARPS][32];             // per warp: its word's kept tokens, lane | y << 8 | x << 16
+    const int seg = blockIdx.x / p.ctas, cta = blockIdx.x - seg * p.ctas;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, L = p.L;
+    const int n_words = (L + 31) >> 5, w_begin = cta * p.words, w_end = min(n_words, w_begin + p.words);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) s_hist[q * 1024 + tid] = 0;
+    if (tid == 0) s_n = 0;
+    pdl_wait();
+    pdl_trigger();
+    const float* sc = p.scores + (long)seg * L;
+    float score[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const int e = (j * SEG_WARPS + wid) * 32 + lane;
+        score[j] = __ldg(sc + (e < L ? e : 0));
+    }
+    const int32_t* rows_in = p.table_in != nullptr ? p.table_in + ((long)seg * L + w_begin * 32) * p.kk : nullptr;
+    if (p.staged) seg_stage_rows(rows_in, max(0, min(L, w_end * 32) - w_begin * 32), p.kk, s_rows);
+    uint32_t key[ITEMS];       // 0 behind the segment's end: below every real key (those begin at 0x007fffff)
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) key[j] = (j * SEG_WARPS + wid) * 32 + lane < L ? score_key(score[j]) : 0u;
+    __syncthreads();
+
+    // (1) radix select of the k-th largest key: the bin that holds the need-th of the keys that match so far, from the top
+    uint32_t T = 0;
+    int need = p.k, at_T = 0;
+    auto find = [&](const int* hist, auto quads) {         // 1024 * quads bins, by eight warps (all threads call)
+        __syncthreads();
+        if (tid < 256) {
+            constexpr int Q = decltype(quads)::value;
+            int4 c[Q];
+            int sum = 0;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                c[q] = reinterpret_cast<const int4*>(hist)[(255 - tid) * Q + q];
+                sum += c[q].x + c[q].y + c[q].z + c[q].w;
+            }
+            int above = warp_incl_scan(sum);
+            if (lane == 31) s_w[wid] = above;
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            above += __reduce_add_sync(0xffffffffu, lane < wid ? s_w[lane] : 0) - sum;      // keys in higher bins
+            if (above < need && above + sum >= need) {
+                int bin = ((255 - tid) * Q + Q) * 4 - 1, count = 0;
+#pragma unroll
+                for (int q = Q - 1; q >= 0; --q) {
+                    const int v[4] = {c[q].w, c[q].z, c[q].y, c[q].x};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if (count == 0 && above + v[e] >= need) count = v[e];
+                        if (count == 0) { above += v[e]; --bin; }
+                    }
+                }
+                s_found[0] = bin;
+                s_found[1] = need - above;
+                s_found[2] = count;
+            }
+        }
+        __syncthreads();
+        need = s_found[1];
+        at_T = s_found[2];
+        return (uint32_t)s_found[0];
+    };
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) atomicAdd(&s_hist[key[j] >> 20], 1);
+    T = find(s_hist, std::integral_constant<int, 4>());
+    // The bin's keys, a few hundred of 15 680 normal ones, are gathered for the two passes that are left; there is nothing to
+    // be found out once every key of a bin is kept.
+    int shift = 20;
+    if (at_T != need) {
+        const bool few = at_T <= SEG_FEW;
+        if (few) {
+            int mine = 0;
+#pragma unroll
+            for (int j = 0; j < ITEMS; ++j) mine += key[j] >> 20 == T;
+            const int incl = warp_incl_scan(mine);
+            int at = 0;
+            if (lane == 31) at = atomicAdd(&s_n, incl);
+            at = __shfl_sync(0xffffffffu, at, 31) + incl - mine;
+            if (mine > 0) {
+#pragma unroll
+                for (int j = 0; j < ITEMS; ++j)
+                    if (key[j] >> 20 == T) s_few[at++] = key[j];
+            }
+            __syncthreads();
+        }
+        const int n_few = few ? at_T : 0;
+#pragma unroll 1
+        for (int pass = 0; pass < 2 && at_T != need; ++pass) {
+            int* hist = s_hist + 4096 + 1024 * pass;
+            shift -= 10;
+            auto count = [&](uint32_t key) {
+                if (key >> shift >> 10 == T) atomicAdd(&hist[key >> shift & 1023], 1);
+            };
+            if (few) {
+                for (int e = tid; e < n_few; e += SEG_THREADS) count(s_few[e]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < ITEMS; ++j) count(key[j]);
+            }
+            T = T << 10 | find(hist, std::integral_constant<int, 1>());
+        }
+    }
+    T <<= shift;
+
+    // (2) kept bits: keys from T on; where not every key equal to T is kept, lower tokens first
+    const bool ties = at_T != need;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const uint32_t from = __ballot_sync(0xffffffffu, key[j] >= T);
+        if (lane == 0) s_from[j * SEG_WARPS + wid] = from;
+    }
+    if (ties) {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const uint32_t eq = __ballot_sync(0xffffffffu, key[j] == T);
+            if (lane == 0) s_eq[j * SEG_WARPS + wid] = eq;
+        }
+    }
+    __syncthreads();
+    {
+        uint32_t kept = tid < n_words ? s_from[tid] : 0u;
+        if (ties) {
+            uint32_t eq = tid < n_words ? s_eq[tid] : 0u;
+            kept &= ~eq;
+            const int room = max(0, need - block_excl_scan(__popc(eq), s_w));
+            while (__popc(eq) > room) eq &= ~(0x80000000u >> __clz(eq));         // drop the highest
+            kept |= eq;
+        }
+        const int before = block_excl_scan(__popc(kept), s_w);
+        if (tid < n_words) s_rank[tid] = make_uint2(kept, seg * p.k + before);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+
+    // (3) kept positions and table rows of this CTA's words, each by as many warps as there are to spare
+    const int parts = max(1, SEG_WARPS / p.words);
+    for (int u = wid; u < (w_end - w_begin) * parts; u += SEG_WARPS) {
+        const int at = u / parts, word = w_begin + at;
+        const int32_t* in = p.staged ? s_rows + seg_shift(rows_in) + at * 32 * p.kk : rows_in + at * 32 * (long)p.kk;
+        seg_write_word(p, s_rank, s_list[wid], seg, word, u - at * parts, parts, in);
+    }
+}
+
+// Segments beyond SEG_ALONE: eight CTAs of a cluster hold seven words per warp of it and add their histograms up through
+// distributed shared memory, each for itself; every CTA gets the whole bit set.
+constexpr int SEG_G = 8, SEG_ITEMS = 7, SEG_WORDS = SEG_MAX / 32;
+
+__global__ void __launch_bounds__(SEG_THREADS)
+table_select_cluster_kernel(const SegArgs p) {
     extern __shared__ __align__(16) int32_t s_rows[];     // this CTA's rows of table_in, if they fit
     __shared__ int s_hist[4][256];
     __shared__ int s_found[3];
     __shared__ uint32_t s_keep[SEG_WORDS], s_eq[SEG_WORDS];
-    __shared__ uint2 s_rank[SEG_WORDS];               // a word's kept bits and the output row of its first kept token
-    __shared__ uint32_t s_list[SEG_THREADS / 32][32]; // per warp: its word's kept tokens, lane | y << 8 | x << 16
-    __shared__ int s_w[SEG_THREADS / 32];
-    const int seg = blockIdx.x / G, cta = blockIdx.x % G;
+    __shared__ uint2 s_rank[SEG_WORDS];
+    __shared__ uint32_t s_list[SEG_WARPS][32];
+    __shared__ int s_w[SEG_WARPS];
+    const int seg = blockIdx.x / SEG_G, cta = blockIdx.x % SEG_G, L = p.L;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    const int n_words = (L + 31) >> 5, per_cta = (n_words + G - 1) / G;
-    const int w_begin = cta * per_cta, w_end = min(n_words, w_begin + per_cta);
-    const float* sc = scores + (long)seg * L;
+    const int n_words = (L + 31) >> 5, w_begin = cta * p.words, w_end = min(n_words, w_begin + p.words);
+    const float* sc = p.scores + (long)seg * L;
     pdl_wait();
     pdl_trigger();
 
-    uint32_t key[ITEMS];
+    uint32_t key[SEG_ITEMS];
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
+    for (int j = 0; j < SEG_ITEMS; ++j) {
         const int word = w_begin + wid + 32 * j, e = word * 32 + lane;
         key[j] = word < w_end && e < L ? score_key(__ldg(sc + e)) : 0u;     // 0 is below every real key
     }
     s_hist[tid >> 8][tid & 255] = 0;
-    // the rows this CTA may have to renumber start their trip now and are in shared memory when the selection is done
-    const int row_begin = w_begin * 32, n_rows = max(0, min(L, w_end * 32) - row_begin);
-    const int32_t* rows_in = table_in != nullptr ? table_in + ((long)seg * L + row_begin) * kk : nullptr;
-    const int shift = (int)((reinterpret_cast<uintptr_t>(rows_in) >> 2) & 3);     // keeps source and target equally aligned
-    if (staged) {
-        const int total = n_rows * kk, lead = min(total, (4 - shift) & 3), vec = (total - lead) >> 2;
-        auto copy = [&](int f, int bytes) {
-            const uint32_t dst = smem_addr(s_rows + shift + f);
-            if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(rows_in + f) : "memory");
-            else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(rows_in + f) : "memory");
-        };
-        if (tid < lead) copy(tid, 4);
-        for (int v = tid; v < vec; v += SEG_THREADS) copy(lead + 4 * v, 16);
-        for (int f = lead + 4 * vec + tid; f < total; f += SEG_THREADS) copy(f, 4);
-    }
+    const int32_t* rows_in = p.table_in != nullptr ? p.table_in + ((long)seg * L + w_begin * 32) * p.kk : nullptr;
+    if (p.staged) seg_stage_rows(rows_in, max(0, min(L, w_end * 32) - w_begin * 32), p.kk, s_rows);
     __syncthreads();
 
     // (1) radix select of the k-th largest key, one byte per pass, most significant first
     uint32_t T = 0, mask = 0;
-    int need = k, at_T = 0;
+    int need = p.k, at_T = 0;
 #pragma unroll 1
     for (int pass = 3; pass >= 0; --pass) {
 #pragma unroll
-        for (int j = 0; j < ITEMS; ++j) {
+        for (int j = 0; j < SEG_ITEMS; ++j) {
             const int word = w_begin + wid + 32 * j;
             const bool in = word < w_end && word * 32 + lane < L && (key[j] & mask) == T;
             const int bin = (key[j] >> (8 * pass)) & 255;
@@ -354,28 +582,19 @@ table_build_segment_kernel(const float* __restrict__ scores, int L, int k, int h
                 atomicAdd(&s_hist[pass][bin], 1);
             }
         }
-        cluster_sync<G>();
+        cluster_sync();
         // thread t adds up bin 255 - t; an inclusive scan over the bins in descending order names the one that holds
         // the need-th key (always found: matching keys >= need)
         int c = 0, incl = 0;
         if (tid < 256) {
-            if constexpr (G == 1) {
-                c = s_hist[pass][255 - tid];
-            } else {
-                const uint32_t mine = smem_addr(&s_hist[pass][255 - tid]);
+            const uint32_t mine = smem_addr(&s_hist[pass][255 - tid]);
 #pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    int v;
-                    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(in_cta(mine, g)) : "memory");
-                    c += v;
-                }
+            for (int g = 0; g < SEG_G; ++g) {
+                int v;
+                asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(in_cta(mine, g)) : "memory");
+                c += v;
             }
-            incl = c;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += t;
-            }
+            incl = warp_incl_scan(c);
             if (lane == 31) s_w[wid] = incl;
         }
         __syncthreads();
@@ -396,21 +615,17 @@ table_build_segment_kernel(const float* __restrict__ scores, int L, int k, int h
 
     // (2) kept bits: keys above T, and of those equal to T the first `need`
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
+    for (int j = 0; j < SEG_ITEMS; ++j) {
         const int word = w_begin + wid + 32 * j;
         const bool valid = word < w_end && word * 32 + lane < L;
         const uint32_t gt = __ballot_sync(0xffffffffu, valid && key[j] > T);
         const uint32_t eq = __ballot_sync(0xffffffffu, valid && key[j] == T);
-        if (word < w_end) {
-            if constexpr (G == 1) {
-                if (lane == 0) { s_keep[word] = gt; s_eq[word] = eq; }
-            } else if (lane < G) {
-                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_cta(smem_addr(&s_keep[word]), lane)), "r"(gt) : "memory");
-                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_cta(smem_addr(&s_eq[word]), lane)), "r"(eq) : "memory");
-            }
+        if (word < w_end && lane < SEG_G) {
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_cta(smem_addr(&s_keep[word]), lane)), "r"(gt) : "memory");
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_cta(smem_addr(&s_eq[word]), lane)), "r"(eq) : "memory");
         }
     }
-    cluster_sync<G>();                 // also the last access to another CTA's shared memory
+    cluster_sync();                    // also the last access to another CTA's shared memory
     constexpr int WPT = (SEG_WORDS + SEG_THREADS - 1) / SEG_THREADS;     // words per thread in the scans
     {
         int ties = 0;
@@ -440,99 +655,52 @@ table_build_segment_kernel(const float* __restrict__ scores, int L, int k, int h
 #pragma unroll
         for (int q = 0; q < WPT; ++q) {
             const int word = tid * WPT + q;
-            if (word < n_words) { s_rank[word] = make_uint2(kw[q], seg * k + before); before += __popc(kw[q]); }
+            if (word < n_words) { s_rank[word] = make_uint2(kw[q], seg * p.k + before); before += __popc(kw[q]); }
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 
     // (3) a word's kept positions and table rows
-    const int seg0 = seg * L;          // row numbers fit 31 bits
-    const int hw = h * w, r0 = ksize >> 1;
-    auto renumbered = [&](unsigned loc) -> int32_t {
-        const uint2 rk = s_rank[loc >> 5];
-        const uint32_t below = rk.x << (31 - (loc & 31));       // the token's own bit on top
-        return below >> 31 ? (int32_t)(rk.y + __popc(below) - 1) : -1;
-    };
-    const int d_row = 32 / kk, d_tap = 32 - d_row * kk;           // from one of a lane's entries to the next
-    const int row_of_lane = lane / kk, tap_of_lane = lane - row_of_lane * kk;
-    for (int word = w_begin + wid; word < w_end; word += SEG_THREADS / 32) {
-        const uint2 rk = s_rank[word];
-        const int e = word * 32 + lane;
-        if ((rk.x >> lane) & 1u) {
-            const int r = __popc(rk.x & lt);
-            if (kept_idx != nullptr) kept_idx[rk.y + r] = e;
-            if (idx64 != nullptr) idx64[rk.y + r] = e;
-            const int p = hw == 1 ? 0 : e - div_magic(e, magic_hw) * hw;
-            const int y = w == 1 ? p : div_magic(p, magic_w), x = p - y * w;
-            s_list[wid][r] = (uint32_t)lane | (uint32_t)(y & 0xFF) << 8 | (uint32_t)(x & 0xFF) << 16;
-        }
-        if (table == nullptr) continue;
-        __syncwarp();
-        const int entries = __popc(rk.x) * kk;
-        int32_t* out = table + (long)rk.y * kk;
-        int r = row_of_lane, tap = tap_of_lane;
-        auto advance = [&] {
-            r += d_row;
-            tap += d_tap;
-            if (tap >= kk) { tap -= kk; ++r; }
-        };
-        if (table_in != nullptr) {
-            // later round: the kept rows of the previous table, renumbered
-            const int32_t* in = staged ? s_rows + shift + (word - w_begin) * 32 * kk : rows_in + (word - w_begin) * 32 * (long)kk;
-#pragma unroll 4
-            for (int f = lane; f < entries; f += 32) {
-                const int32_t old = in[(int)(s_list[wid][r] & 31u) * kk + tap];
-                const unsigned loc = (unsigned)(old - seg0);
-                out[f] = old >= 0 && loc < (unsigned)L ? renumbered(loc) : -1;
-                advance();
-            }
-        } else {
-            for (int f = lane; f < entries; f += 32) {
-                const int ty = ksize == 1 ? tap : div_magic(tap, magic_ks);
-                const int dy = ty - r0, dx = tap - ty * ksize - r0;
-                const uint32_t it = s_list[wid][r];
-                const int y = (int)(it >> 8 & 0xFFu) + dy, x = (int)(it >> 16) + dx;
-                out[f] = (unsigned)y < (unsigned)h && (unsigned)x < (unsigned)w
-                             ? renumbered(word * 32 + (int)(it & 31u) + dy * w + dx) : -1;
-                advance();
-            }
-        }
-        __syncwarp();
+    for (int word = w_begin + wid; word < w_end; word += SEG_WARPS) {
+        const int at = word - w_begin;
+        const int32_t* in = p.staged ? s_rows + seg_shift(rows_in) + at * 32 * p.kk : rows_in + at * 32 * (long)p.kk;
+        seg_write_word(p, s_rank, s_list[wid], seg, word, 0, 1, in);
     }
 }
 
 // floor(e / d) = umulhi(e, magic) for e < 65536 (see div_magic)
 static uint32_t magic_of(int d) { return (uint32_t)((0x100000000ull + d - 1) / d); }
 
-template <int G, int ITEMS>
-static int segment_launch_as(const float* scores, int n_seg, int L, int k, int h, int w, int ksize, int kk, int32_t* kept_idx,
-                             int32_t* table, int64_t* idx64, const int32_t* table_in, cudaStream_t s) {
-    auto kern = table_build_segment_kernel<G, ITEMS>;
-    // rows of the previous table wait in shared memory while they leave room for it
-    const size_t rows = (size_t)(((L + 31) / 32 + G - 1) / G) * 32 * kk * sizeof(int32_t) + 16;
-    const int staged = table_in != nullptr && rows <= 180 * 1024;
-    if (staged) {
-        static std::atomic<uint64_t> ready{0};     // devices on which this kernel may use that much
-        int dev = 0;
-        SV_CUDA(cudaGetDevice(&dev));
-        const uint64_t bit = 1ull << (dev & 63);
-        if (!(ready.load() & bit)) {
-            SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 180 * 1024));
-            ready.fetch_or(bit);
-        }
-    }
-    SV_CUDA(launch_pdl(kern, dim3((unsigned)(n_seg * G)), dim3(SEG_THREADS), staged ? rows : 0, s, G, scores, L, k, h, w, ksize,
-                       magic_of(w), magic_of(h * w), magic_of(ksize), kk, kept_idx, table, idx64, table_in, staged));
-    return SVTAD_OK;
-}
-
 static int segment_launch(const float* scores, int n_seg, int L, int k, int h, int w, int ksize, int kk, int32_t* kept_idx,
                           int32_t* table, int64_t* idx64, const int32_t* table_in, cudaStream_t s) {
-    // two words (64 tokens) per warp: a CTA per 2048 tokens while a portable cluster covers the segment
-    auto as = L <= 2048 ? segment_launch_as<1, 2> : L <= 4096 ? segment_launch_as<2, 2> : L <= 8192 ? segment_launch_as<4, 2>
-              : L <= 16384 ? segment_launch_as<8, 2> : segment_launch_as<8, 7>;
-    return as(scores, n_seg, L, k, h, w, ksize, kk, kept_idx, table, idx64, table_in, s);
+    const int n_words = (L + 31) / 32;
+    int words, ctas;
+    if (L <= SEG_ALONE) {
+        // Half the GPU's SMs for all segments together where that leaves a warp no more than one word (three rounds of eight
+        // 80-frame clips: 27.7 us, on all SMs 30.2), else all of them (24 clips of 80 slices: 54 us, on half 73); at least
+        // four words, of up to eight warps each, per CTA.
+        const int half = tc_num_sms() / 2;
+        const int want = ((long)n_words * n_seg <= (long)half * SEG_WARPS ? half : 2 * half) / n_seg;
+        words = want > 1 ? (n_words + want - 1) / want : n_words;
+        if (words < 4) words = 4;
+        ctas = (n_words + words - 1) / words;
+    } else {
+        words = (n_words + SEG_G - 1) / SEG_G;
+        ctas = SEG_G;
+    }
+    auto kern = L <= 2048 ? table_select_kernel<2> : L <= 4096 ? table_select_kernel<4> : L <= 8192 ? table_select_kernel<8>
+                : L <= SEG_ALONE ? table_select_kernel<16> : table_select_cluster_kernel;
+    // rows of the previous table wait in shared memory while they leave room for it
+    const size_t rows = (size_t)words * 32 * kk * sizeof(int32_t) + 16;
+    const int staged = table_in != nullptr && rows <= 176 * 1024;
+    if (staged) {
+        int rc = tc_ensure_smem(reinterpret_cast<const void*>(kern), 176 * 1024);
+        if (rc) return rc;
+    }
+    const SegArgs p{scores, L, k, h, w, ksize, magic_of(w), magic_of(h * w), magic_of(ksize), kk, kept_idx, table, idx64, table_in, staged, words, ctas};
+    SV_CUDA(launch_pdl(kern, dim3((unsigned)(n_seg * ctas)), dim3(SEG_THREADS), staged ? rows : 0, s, L <= SEG_ALONE ? 1 : SEG_G, p));
+    return SVTAD_OK;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -608,7 +776,8 @@ extern "C" int svtad_table_init(int B, int T, int h, int w, int ksize, int32_t* 
     SV_CHECK_ARG(table != nullptr, "svtad_table_init: table is null");
     long total = rows * ksize * ksize;
     long threads = (total + 3) / 4;
-    SV_CUDA(launch_pdl(table_init_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, 1, table,
+    auto kern = total < (1l << 32) - 4096 ? table_init_kernel<uint32_t> : table_init_kernel<uint64_t>;
+    SV_CUDA(launch_pdl(kern, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, 1, table,
                        total, h * w, h, w, ksize, ksize * ksize));
     return SVTAD_OK;
 }

@@ -252,3 +252,30 @@ def test_wide_stencils_on_short_segments(ksize, h, w):
     ekept, etable = otab.build_table(scores.numpy(), k, h, w, ksize)
     kept, table = sv.build_neighbor_table(scores.cuda(), None, h, w, ksize, num_keep=k)
     assert np.array_equal(kept.cpu().numpy(), ekept) and np.array_equal(table.cpu().numpy(), etable)
+
+
+@pytest.mark.parametrize("dist", ["normal", "exp", "few_values", "one_value", "inf", "nan_some", "subnormal"])
+@pytest.mark.parametrize("n_seg,T,h,w", [(1, 2, 10, 13), (3, 20, 14, 14), (40, 5, 14, 14), (160, 11, 14, 14), (2, 64, 16, 16)])
+def test_several_ctas_per_long_segment(dist, n_seg, T, h, w):
+    """Shares of a segment from four words to all of it (with more segments than SMs; previous rows in shared memory or not),
+    the first radix bin gathered or not, ties, infinities and NaNs at the threshold."""
+    ops = _ops()
+    L = T * h * w
+    rng = np.random.default_rng(L)
+    s = rng.standard_normal((n_seg, L))
+    s = {"normal": s, "exp": np.exp(4 * s), "few_values": np.round(2 * s), "one_value": np.zeros_like(s), "subnormal": s * 1e-42,
+         "inf": np.where(s > 1, np.inf, np.where(s < -1, -np.inf, s)), "nan_some": np.where(s > 0.8, np.nan, s)}[dist].astype(np.float32)
+    if dist == "one_value":
+        s[:, ::2] = -0.0
+    sc = torch.from_numpy(s).cuda()
+    for k in (1, L // 3, L - 1):
+        kept, table = ops.table_build(sc, k, h, w, 3)
+        ekept, etable = otab.build_table(s, k, h, w, 3)
+        np.testing.assert_array_equal(kept.cpu().numpy(), ekept)
+        np.testing.assert_array_equal(table.cpu().numpy(), etable)
+    full = ops.table_init(n_seg, T, h, w, 3)
+    idx, out = ops.table_select_remap(sc, full, L // 3)
+    eidx = otab.select_topk(s, L // 3)
+    np.testing.assert_array_equal(idx.cpu().numpy(), eidx)
+    eout = otab.remap_table(otab.initial_table(h, w, T, n_seg, 3), eidx)
+    np.testing.assert_array_equal(out.cpu().numpy(), eout)
