@@ -1,7 +1,7 @@
 // Host side of the tcgen05 / TMEM SparseConv2D path: the device error word, tensor-map encoding, tile
 // and split planning, and the dispatch between the kernel families
 //   conv_tc_hybrid.cu   one CTA per tile: gathered rows by per-warp cp.async, weight / gy tiles by TMA
-//   conv_tc_pair.cu     forward / dgrad on CTA pairs (cta_group::2) once row tiles outnumber the SMs
+//   conv_tc_pair.cu     forward / dgrad on CTA pairs (cta_group::2) where they are faster, see use_pair()
 // They replace opentad/models/bricks/implicit_gemm_v2.cu:197-417 (gather kernel + cuBLAS batched GEMM +
 // reduce kernel) and the atomic backward kernels opentad/models/bricks/2d_sparse_v3.cu:656-745.
 #include <cstdlib>
@@ -387,24 +387,41 @@ bool tc_supported(int op, int64_t n, int cin, int cout, int kk, int dtype) {
     return true;
 }
 
-// Forward / dgrad on CTA pairs (tcgen05 cta_group::2) or on single CTAs.  Measured on B200 at C = 192: pairs win
-// once there are more row tiles than SMs (918-941 vs 820-850 TFLOP/s at 226 560 rows); below that one CTA
-// per (row tile, column block) starts sooner and uses narrower column blocks to fill the machine.
-// SVTAD_TC_IMPL=pair / hybrid overrides the choice.
-static bool use_pair(int64_t n) {
+// Forward / dgrad on CTA pairs (tcgen05 cta_group::2) or on single CTAs.  A pair stages half of the weight tile per CTA, so
+// its K steps are shorter; it starts later, and single CTAs may take narrower column blocks to fill the machine.  Times as
+// measured on a B200 (us; rows, layer: pair, single): 18 880, 256 -> 256, 5x5: 40.9, 43.2; 14 160, 384, 5x5: 94.5, 108;
+// 9 440, 384, 5x5: 50.4, 55.9; 18 880, 192, 3x3: 15.5, 14.5; 9 440, 768, 3x3: 79.1, 74.7; 37 760, 128, 3x3: 17.4, 16.8; 23 600,
+// 256, 5x5: 74.1, 81.7; 37 760, 64, 5x5: 18.7, 18.0.  The two estimates below choose within 0.2 % of the faster one on average
+// over 326 such calls; where they are close the kernel stays that was there first (pairs from as many row tiles as SMs on).
+// A tile whose K steps a cluster shares goes to single CTAs, and under a concurrency hint only the number of tiles counts.
+// A row's sum is the same either way.  SVTAD_TC_IMPL=pair / hybrid overrides the choice.
+static bool use_pair(int64_t n, int cred, int cn, int kk) {
     const char* e = getenv("SVTAD_TC_IMPL");
     if (e != nullptr && *e) return e[0] == 'p';
-    const long m_tiles = (n + TILE_M - 1) / TILE_M;
-    return m_tiles > (long)tc_num_sms();
+    const long m_tiles = (n + TILE_M - 1) / TILE_M, sms = tc_num_sms();
+    const bool many = m_tiles > sms;
+    if (tc_plan_sms() < sms) return many;
+    const int steps = kk * ((cred + STAGE_K - 1) / STAGE_K);
+    if (hybrid_splits(cn, m_tiles, steps)) return false;
+    auto at = [](int bn) { return bn == 256 ? 4 : bn == 192 ? 3 : bn == 128 ? 2 : bn == 96 ? 1 : 0; };
+    const double pair_step[5] = {0.20, 0.2375, 0.2375, 0.29, 0.316}, single_step[5] = {0.19, 0.245, 0.266, 0.352, 0.366};
+    auto time = [&](double start, long items, long slots, double step) {
+        const long waves = (items + slots - 1) / slots;
+        return start + (double)waves * steps * step + (double)(waves - 1) * 1.7;
+    };
+    const int wide = tc_widest_bn(cn), bn = tc_pick_bn(cn, m_tiles);
+    const double pair = time(7.0, (m_tiles + 1) / 2 * ((cn + wide - 1) / wide), sms / 2, pair_step[at(wide)]);
+    const double single = time(5.2, m_tiles * ((cn + bn - 1) / bn), sms, single_step[at(bn)]);
+    return many ? single >= 0.97 * pair : pair < 0.926 * single;
 }
 
 int tc_fwd(const ConvArgs& p, cudaStream_t s) {
-    if (p.plan == nullptr && use_pair(p.n)) return pair_fwd(p, s);
+    if (p.plan == nullptr && use_pair(p.n, p.cin, p.cout, p.kk)) return pair_fwd(p, s);
     return hybrid_fwd(p, s);
 }
 
 int tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
-    if (p.plan == nullptr && use_pair(p.n)) return pair_dgrad(p, status, s);
+    if (p.plan == nullptr && use_pair(p.n, p.cout, p.cin, p.kk)) return pair_dgrad(p, status, s);
     return hybrid_dgrad(p, status, s);
 }
 

@@ -23,8 +23,8 @@
 // consumer only on its own steps, and with more warps than buffers it could lap the consumer by two rounds,
 // which the barrier's phase parity cannot tell from "free".  No TMA load uses cluster multicast.  Every
 // mbarrier wait is bounded: when it runs out the CTA records a code in the device error word, stops, frees its
-// tensor memory and returns.  Inputs whose row tiles outnumber the SMs go to the CTA-pair kernels instead
-// (conv_tc_pair.cu).
+// tensor memory and returns.  Where CTA pairs are faster, mostly for many row tiles and long reductions, the kernels of
+// conv_tc_pair.cu run instead.
 #include <cstdlib>
 
 #include "plan.cuh"
@@ -785,6 +785,11 @@ static int pick_split(int cn, long m_tiles, int steps, int& G) {
         if (u < best) { best = u; bn = width[i]; }
     }
     return bn;
+}
+
+bool hybrid_splits(int cn, long m_tiles, int steps) {
+    int G = 1;
+    return pick_split(cn, m_tiles, steps, G) != 0;
 }
 
 // Column block of the forward by a plan (the input gradient, which shares the GPU with the weight gradient, takes the widest: with

@@ -631,3 +631,24 @@ def test_errors_are_python_exceptions():
     with pytest.raises(ValueError):
         ops.conv_fwd(torch.randn(4, 8).cuda().double(), torch.zeros(4, 9, dtype=torch.int32).cuda(),
                      torch.randn(9, 8, 8).cuda().double(), None)
+
+
+@pytest.mark.parametrize("n,cin,cout,ks,dtype", [
+    (148 * 128, 192, 192, 5, torch.bfloat16),       # as many tiles as SMs, a long reduction: pairs by default
+    (148 * 128 + 77, 128, 128, 3, torch.float16),   # more tiles than SMs, a short one: single CTAs
+    (111 * 128 - 5, 384, 320, 5, torch.bfloat16),   # three quarters as many tiles, two column blocks
+])
+def test_a_row_s_sum_does_not_hang_on_pairs_or_single_ctas(n, cin, cout, ks, dtype, monkeypatch):
+    """Where no cluster shares a tile's K steps (too many tiles here), the two kernels and the choice between them agree bit for bit."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(n)
+    table = torch.randint(-1, n, (n, ks * ks), generator=g, dtype=torch.int32).cuda()
+    x, w, b, gy = (t.cuda() for t in make_conv_inputs(n, cin, cout, ks, dtype, 3, bias="random"))
+    outs = []
+    for impl in ("", "pair", "hybrid"):
+        monkeypatch.setenv("SVTAD_TC_IMPL", impl)
+        outs.append((ops.conv_fwd(x, table, w, b), ops.conv_dgrad(gy, table, w, assume_symmetric=True)))
+    torch.cuda.synchronize()
+    assert ops.device_error() == 0
+    for y, gx in outs[1:]:
+        assert torch.equal(y, outs[0][0]) and torch.equal(gx, outs[0][1])
