@@ -117,8 +117,9 @@ int pairs_wgrad(const void* gy, const void* x, const void* plan, void* gw, void*
 // holds them until everything the predecessor wrote can be seen, so it comes before a kernel's first access to global
 // memory, reads and writes alike, and before any return.  pdl_trigger() lets the successor's CTAs come in turn.  Back
 // to back this hides a launch's 2 us or so (16-bit forward of 2868 rows, C=256: 14.3 -> 12.3 us a call; three pruning
-// rounds of two clips: 49 -> 42.5 us).  Not for kernels of many small CTAs: the successor's, resident early, cost the
-// per-slice table builder 1.5 of 10.2 us and the fp32 forward 2.5 of 23.5 us.  Nor where the caller says that kernels of
+// rounds of two clips: 49 -> 42.5 us).  Kernels of many small CTAs do without the trigger: the successor's, resident early,
+// cost the per-slice table builder 1 to 5 of 8 to 12 us; its launch alone, under the predecessor's tail, gains 1.3 us, since
+// kernels of a stream otherwise start 2 us apart at the least.  No early start where the caller says that kernels of
 // several streams share the GPU: a CTA that waits here holds an SM that another stream's kernel could work on (forward
 // and backward of three layers on their streams, hints 3 / 2 / 2: 91 us a step with early starts, 82 without).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
