@@ -16,11 +16,11 @@
 // of a tile that lack a neighbor are rows of zeros).  Sums that are not finite are therefore made again from the fp32
 // values, pair by pair, before they are stored.
 //
-// Measured (graph replays, before: the CUDA-core kernels): 784 rows, C = 192, keep 50 %: forward 21.2 -> 12.2 us, input
-// gradient 22.2 -> 12.3; 4 720 rows, C = 192, keep 30 %: 54.5 -> 28.8, 57.1 -> 28.2, weight gradient 47.8 -> 23.2; 5 880
-// rows, full grid, 320 -> 96: 144 -> 46, 134 -> 39, 103 -> 62.  What bounds the loops: eight warps that load, split and store
-// (835 issue slots per scheduler and step; 768 cycles of tensor work) and the trip of the operands from L2, which is one step
-// long.
+// Measured (graph replays, before: the CUDA-core kernels): 784 rows, C = 192, keep 50 %: forward 21.2 -> 11.1 us, input
+// gradient 22.2 -> 11.0; 4 720 rows, C = 192, keep 30 %: 54.5 -> 28.0, 57.1 -> 26.4, weight gradient 47.8 -> 23.2; 5 880
+// rows, full grid, 320 -> 96: 144 -> 43, 134 -> 39, 103 -> 62.  What bounds the loops: eight warps that load, split and store
+// (850 issue slots per scheduler and step of 1 480 cycles; 768 cycles of tensor work) and the gathered rows' trip from L2, which is
+// one step long.
 #include <cfloat>
 
 #include "tc_common.cuh"
@@ -30,10 +30,12 @@ namespace svtad {
 constexpr int T3_A_WARPS = 8;
 constexpr int T3_E_WARPS = 4;
 constexpr int T3_THREADS = (T3_A_WARPS + 1 + T3_E_WARPS) * 32;      // the MMA warp (TMEM owner) sits between them
+constexpr int T3_FW_THREADS = T3_THREADS + 32;         // forward, input gradient: a warp more, for the weights
 constexpr int T3_BN = 64;
 constexpr int T3_A_PLANE = A_TILE_BYTES, T3_B_PLANE = T3_BN * 128;
 constexpr int T3_STAGE = 3 * (T3_A_PLANE + T3_B_PLANE);      // weight gradient
 constexpr int T3_RING = 2, T3_B_STAGE = 3 * T3_B_PLANE;      // forward, input gradient: A in tensor memory
+constexpr int T3_RAWS = 4, T3_RAW = 64 * T3_BN * 4;          // ... and the weights' fp32 tiles
 constexpr int T3_A_COL = 256, T3_A_COLS = 96;               // behind two accumulators of 128 columns
 constexpr int T3_COLS = 3 * T3_BN;                     // accumulator columns of a step
 constexpr int T3_PARK = T3_BN + 4;                     // floats per row of the parked sums
@@ -217,19 +219,23 @@ __device__ __noinline__ float t3_row_sum(const float* a, const int32_t* nbr, con
 // ---------------------------------------------------------------------------------------------
 // A goes from registers to tensor memory, B through shared memory: with both in shared memory its 128 bytes a cycle were the bound
 // (72 KB written, 96 KB read and the loads' way through L1 a step; 4 720 rows, C = 192: 34.2 us instead of 28.8).
+// The weights' tiles come as fp32 through TMA, several steps ahead: every CTA reads each of them once, from L2, while most gathered
+// rows are found in L1 again by the taps that follow.  Loaded to registers one step ahead they were what the warps waited for:
+// 784 rows, C = 192: 12.2 -> 11.1 us, 4 720 rows: 28.8 -> 28.0, input gradient 28.2 -> 26.4, 80 rows, C = 1024: 31.3 -> 25.5.
 // SPLIT: a cluster of G CTAs shares the tile's K steps; the sums meet in shared memory, in the order of the CTAs.
 template <bool DGRAD, bool SPLIT, bool FULL>
-__global__ void __launch_bounds__(T3_THREADS, 1)
-conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr, const float* __restrict__ w,
+__global__ void __launch_bounds__(T3_FW_THREADS, 1)
+conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __restrict__ a, const int32_t* __restrict__ nbr, const float* __restrict__ w,
                    const float* __restrict__ bias, float* __restrict__ out, const int32_t* __restrict__ status, long n, int cred,
                    int cn, int cin, int cout, int kk, int tpb, int n_blks, int G, int* __restrict__ err) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    TmaTail* tail = reinterpret_cast<TmaTail*>(smem + T3_RING * T3_B_STAGE);
+    TmaTail* tail = reinterpret_cast<TmaTail*>(smem + T3_RING * T3_B_STAGE + T3_RAWS * T3_RAW);
     const float** s_row = reinterpret_cast<const float**>(tail + 1);      // [kk][128] gathered rows, or the row of zeros
     volatile int* s_abort = &tail->abort_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t stage_base = smem_u32(smem);
+    const uint32_t stage_base = smem_u32(smem), raw_base = stage_base + T3_RING * T3_B_STAGE;
+    __shared__ uint64_t s_raw_full[T3_RAWS], s_raw_empty[T3_RAWS];
     const int share = SPLIT ? (int)blockIdx.x % G : 0, item = SPLIT ? (int)blockIdx.x / G : (int)blockIdx.x;
     const long row0 = (long)(item / n_blks) * TILE_M;
     const int n0 = item % n_blks * T3_BN;
@@ -249,8 +255,13 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
             mbar_init(smem_u32(&tail->accum_full[b]), 1);
             mbar_init(smem_u32(&tail->accum_empty[b]), T3_E_WARPS * 32);
         }
+        for (int r = 0; r < T3_RAWS; ++r) {
+            mbar_init(smem_u32(&s_raw_full[r]), 1);
+            mbar_init(smem_u32(&s_raw_empty[r]), T3_A_WARPS);
+        }
         tail->abort_flag = 0;
         fence_mbar_init();
+        tma_prefetch_map(&map_w);
     }
     pdl_wait();
     if (DGRAD && status != nullptr && (__ldg(status) & SVTAD_TABLE_ASYMMETRIC)) {      // uniform over the grid
@@ -261,7 +272,7 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
     {
         const int32_t* rows = nbr + row0 * kk;
         const int valid = (int)(n - row0 < TILE_M ? n - row0 : TILE_M) * kk;
-        for (int e = tid; e < TILE_M * kk; e += T3_THREADS) {
+        for (int e = tid; e < TILE_M * kk; e += T3_FW_THREADS) {
             const int r = e / kk, k = e - r * kk;
             const int raw = e < valid ? __ldg(rows + e) : -1;
             const long j = (long)raw + (tpb > 0 ? ((row0 + r) / tpb) * (long)tpb : 0);
@@ -284,8 +295,10 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
         // step, an order that B's rows (forward) or 8-byte pieces of them (input gradient) follow.
         const int c8 = (lane & 3) * 8, r16 = (warp & 3) * 32 + (warp >> 2) * 16 + (lane >> 2);
         const uint32_t a_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32 + (warp >> 2) * 16) << 16) + T3_A_COL;
-        // B: rows warp * 8 + {0 .. 3}, + 4, eight lanes each.  Rows r and r + 2 share a half-warp, for the input gradient's stores.
-        const int sub = lane & 7, row4 = (lane >> 4) + (lane >> 3 & 1) * 2, b_row = warp * 8 + row4;
+        // B: rows warp * 8 + {0 .. 3}, + 4, eight columns per lane; the fp32 tile is two boxes of 32 columns.  Eight lanes are half of
+        // a row and the other half of its neighbor, a half-warp has four rows: neither the loads nor the stores meet a bank twice.
+        const int sub = lane & 7, row4 = ((lane >> 4) + (lane >> 3 & 1) * 2) ^ (sub >> 2), b_row = warp * 8 + row4;
+        const uint32_t b_raw = raw_base + (sub >> 2) * (T3_RAW / 2) + b_row * 128 + (((sub & 3) * 2 ^ (b_row & 7)) << 4);
         uint32_t b_place;
         if (DGRAD) {
             b_place = b_row * 128 + ((((sub >> 2) * 4 + (sub >> 1 & 1)) ^ (b_row & 7)) << 4) + (sub & 1) * 8;
@@ -294,12 +307,9 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
             b_place = r * 128 + ((sub ^ (r & 7)) << 4);
         }
         const uint32_t b_next = DGRAD ? 4 * 128 : 16 * 128;       // rows of the second four
-        float va[2][2][8], vb[2][8];
+        float va[2][2][8];
         int k = k_lo / chunks, c0 = (k_lo - k * chunks) * STAGE_K;
         const float* const* my_row = s_row + r16;
-        // forward: a row of B is a channel, along the columns; input gradient: a column, along the channels
-        auto b_at = [&] { return w + ((long)(DGRAD ? kk - 1 - k : k) * cin + (DGRAD ? n0 : c0) + b_row) * cout + (DGRAD ? c0 : n0) + 8 * sub; };
-        const float* b_ptr = b_at();
         auto load_a = [&] {
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
@@ -308,20 +318,9 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
                 for (int h = 0; h < 2; ++h) t3_load8<FULL>(va[r][h], row + 32 * h, c0 + c8 + 32 * h < cred, c0 + c8 + 32 * h + 4 < cred);
             }
         };
-        auto load_b = [&] {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int along = (DGRAD ? c0 : n0) + 8 * sub;
-                const bool in = FULL || (DGRAD ? n0 : c0) + b_row + 4 * h < cin;
-                t3_load8<FULL>(vb[h], b_ptr + 4 * h * cout, in && along < cout, in && along + 4 < cout);
-            }
-        };
-        if (k_lo < k_hi) {
-            load_a();
-            load_b();
-        }
-        int s = 0;
-        uint32_t ph = 1;
+        if (k_lo < k_hi) load_a();
+        int s = 0, rs = 0;
+        uint32_t ph = 1, rph = 0;
         for (int st = k_lo; st < k_hi; ++st) {
             uint32_t pa[3][16];
 #pragma unroll
@@ -338,8 +337,7 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
             // the next step's loads are on their way while this one is multiplied; behind the last step this one's again
             if (st + 1 < k_hi) {
                 c0 += STAGE_K;
-                b_ptr += DGRAD ? STAGE_K : STAGE_K * cout;
-                if (c0 >= cred) { c0 = 0; ++k; b_ptr = b_at(); }
+                if (c0 >= cred) { c0 = 0; ++k; }
             }
             load_a();
             if (!t3_wait(smem_u32(&tail->empty[s]), ph, s_abort, err, 71)) break;
@@ -347,10 +345,17 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
 #pragma unroll
             for (int q = 0; q < 3; ++q) t3_tmem_st(a_addr + s * T3_A_COLS + q * 32, pa[q]);
             const uint32_t b_tile = stage_base + s * T3_B_STAGE + b_place;
+            if (!t3_wait(smem_u32(&s_raw_full[rs]), rph, s_abort, err, 79)) break;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
+                // rows b_row and b_row + 4: the second one's chunks lie across the swizzle
+                float vb[8];
+                const uint32_t src = (b_raw + rs * T3_RAW + h * 512) ^ (h ? 64u : 0u);
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(vb[4 * q]), "=f"(vb[4 * q + 1]), "=f"(vb[4 * q + 2]), "=f"(vb[4 * q + 3]) : "r"(src ^ (q ? 16u : 0u)) : "memory");
                 uint32_t p[3][4];
-                t3_split8(vb[h], p);
+                t3_split8(vb, p);
 #pragma unroll
                 for (int q = 0; q < 3; ++q) {
                     const uint32_t dst = b_tile + q * T3_B_PLANE + h * b_next;
@@ -362,7 +367,9 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
                     }
                 }
             }
-            load_b();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&s_raw_empty[rs]));
+            if (++rs == T3_RAWS) { rs = 0; rph ^= 1u; }
             t3_tmem_st_wait();
             tc_fence_before();
             t3_filled(smem_u32(&tail->full[s]), lane);
@@ -385,8 +392,26 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
             __syncwarp();
             if (++s == T3_RING) { s = 0; ph ^= 1u; }
         }
+    } else if (warp == T3_A_WARPS + 1 + T3_E_WARPS) {
+        // ------------------------------------------------------------------ weights: fp32 tiles, T3_RAWS steps ahead
+        if (lane == 0) {
+            int k = k_lo / chunks, c0 = (k_lo - k * chunks) * STAGE_K, rs = 0;
+            uint32_t ph = 1;
+            for (int st = k_lo; st < k_hi; ++st) {
+                if (!mbar_wait(smem_u32(&s_raw_empty[rs]), ph, s_abort, err, 80)) break;
+                const uint32_t bar = smem_u32(&s_raw_full[rs]), dst = raw_base + rs * T3_RAW;
+                mbar_expect_tx(bar, T3_RAW);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    tma_load_3d(dst + h * (T3_RAW / 2), &map_w, (DGRAD ? c0 : n0) + 32 * h, DGRAD ? n0 : c0, DGRAD ? kk - 1 - k : k, bar);
+                c0 += STAGE_K;
+                if (c0 >= cred) { c0 = 0; ++k; }
+                if (++rs == T3_RAWS) { rs = 0; ph ^= 1u; }
+            }
+        }
+        __syncwarp();
     } else {
-        // ------------------------------------------------------------------ the last four warps keep the sums
+        // ------------------------------------------------------------------ four warps keep the sums
 #pragma unroll
         for (int c = 0; c < T3_BN / 2; ++c) sum[c] = 0;
         const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
@@ -413,7 +438,7 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
     };
     if constexpr (!SPLIT) {
         const long row = row0 + q * 32 + lane;
-        if (warp > T3_A_WARPS && whole && row < n) {
+        if (warp > T3_A_WARPS && warp <= T3_A_WARPS + T3_E_WARPS && whole && row < n) {
 #pragma unroll
             for (int c = 0; c < T3_BN / 4; ++c) {
                 uint32_t u[4];
@@ -431,7 +456,7 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
         const bool all = *s_abort == 0;
         const int per = (TILE_M + G - 1) / G;               // rows that a CTA finishes: [share * per, ...)
         const uint32_t park = stage_base;                   // [CTA the sums come from][row][T3_PARK]
-        if (all && warp > T3_A_WARPS) {
+        if (all && warp > T3_A_WARPS && warp <= T3_A_WARPS + T3_E_WARPS) {
             const int r = q * 32 + lane, owner = r / per;
             const uint32_t dst = map_to_cta(park + ((share * per + r - owner * per) * T3_PARK) * 4, owner);
 #pragma unroll
@@ -445,7 +470,7 @@ conv_f32_tc_kernel(const float* __restrict__ a, const int32_t* __restrict__ nbr,
         cluster_barrier();
         const float* sums = reinterpret_cast<const float*>(smem);
         const int rows = !all ? 0 : share * per + per <= TILE_M ? per : TILE_M - share * per;
-        for (int e = tid; e < rows * (T3_BN / 4); e += T3_THREADS) {
+        for (int e = tid; e < rows * (T3_BN / 4); e += T3_FW_THREADS) {
             const int r = e / (T3_BN / 4), c = e % (T3_BN / 4) * 4;
             const long row = row0 + share * per + r;
             if (row >= n || n0 + c >= cn) continue;
@@ -792,11 +817,16 @@ static int launch_f32_tc(const ConvArgs& p, const int32_t* status, int G, cudaSt
     const size_t table = (size_t)p.kk * TILE_M * sizeof(float*);
     const int n_blks = (cn + T3_BN - 1) / T3_BN;
     const long tiles = (p.n + TILE_M - 1) / TILE_M * n_blks;
-    const size_t smem = 1024 + T3_RING * T3_B_STAGE + sizeof(TmaTail) + table;
+    const size_t smem = 1024 + T3_RING * T3_B_STAGE + T3_RAWS * T3_RAW + sizeof(TmaTail) + table;
     auto kern = conv_f32_tc_kernel<DGRAD, SPLIT, FULL>;
     int rc = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem);
     if (rc) return rc;
-    SV_CUDA(launch_pdl(kern, dim3((unsigned)(tiles * G)), dim3(T3_THREADS), smem, s, SPLIT ? G : 1, (const float*)p.a, p.nbr,
+    CUtensorMap map_w;
+    const uint64_t dims[3] = {(uint64_t)p.cout, (uint64_t)p.cin, (uint64_t)p.kk};
+    const uint32_t box[3] = {32, 64, 1};
+    rc = tc_make_map_sw(&map_w, 3, p.w, dims, box, TC_MAP_F32, 128);
+    if (rc) return rc;
+    SV_CUDA(launch_pdl(kern, dim3((unsigned)(tiles * G)), dim3(T3_FW_THREADS), smem, s, SPLIT ? G : 1, map_w, (const float*)p.a, p.nbr,
                        (const float*)p.w, (const float*)p.bias, (float*)p.out, status, (long)p.n, cred, cn, p.cin, p.cout, p.kk, p.tpb,
                        n_blks, G, tc_error_ptr()));
     return SVTAD_OK;
@@ -808,10 +838,10 @@ static int dispatch_f32_tc(const ConvArgs& p, const int32_t* status, cudaStream_
     const long tiles = (p.n + TILE_M - 1) / TILE_M * ((cn + T3_BN - 1) / T3_BN), sms = tc_num_sms();
     const int steps = p.kk * ((cred + STAGE_K - 1) / STAGE_K);
     // a step takes 0.72 us and sharing a tile out 2.5; clusters of three and more do not pack a GPC's SMs completely
-    const int sizes[5] = {2, 3, 4, 5, 8}, limit[5] = {148, 120, 120, 112, 112};
+    const int sizes[6] = {2, 3, 4, 5, 6, 8}, limit[6] = {148, 132, 128, 125, 126, 112};
     double best = (double)((tiles + sms - 1) / sms) * steps * 0.72;
     int G = 1;
-    for (int g = 0; g < 5; ++g) {
+    for (int g = 0; g < 6; ++g) {
         if (tiles * sizes[g] * 148 > limit[g] * sms) continue;
         const double u = (steps + sizes[g] - 1) / sizes[g] * 0.72 + 2.5;
         if (u < best) { best = u; G = sizes[g]; }

@@ -125,18 +125,18 @@ int tc_make_map(CUtensorMap* map, int rank, const void* base, const uint64_t* di
     return tc_make_map_sw(map, rank, base, dims, box, fp16, 128);
 }
 
-int tc_make_map_sw(CUtensorMap* map, int rank, const void* base, const uint64_t* dims, const uint32_t* box, int fp16,
+int tc_make_map_sw(CUtensorMap* map, int rank, const void* base, const uint64_t* dims, const uint32_t* box, int type,
                    int swizzle_bytes) {
     // A descriptor depends only on (base, dims, box, element type, swizzle): a training step encodes the same few
     // again and again, so the last ones are kept per thread.
-    struct Key { const void* base; uint64_t dims[3]; uint32_t box[3]; int rank, fp16, swz, dev; };
+    struct Key { const void* base; uint64_t dims[3]; uint32_t box[3]; int rank, type, swz, dev; };
     struct Slot { Key key; CUtensorMap map; bool used; };
     constexpr int SLOTS = 32;
     static thread_local Slot cache[SLOTS];
     static thread_local unsigned next_slot = 0;
     Key key;
     memset(&key, 0, sizeof(key));
-    key.base = base; key.rank = rank; key.fp16 = fp16; key.swz = swizzle_bytes;
+    key.base = base; key.rank = rank; key.type = type; key.swz = swizzle_bytes;
     for (int i = 0; i < rank; ++i) { key.dims[i] = dims[i]; key.box[i] = box[i]; }
     if (cudaGetDevice(&key.dev) != cudaSuccess) key.dev = -1;
     for (int i = 0; i < SLOTS; ++i)
@@ -153,14 +153,14 @@ int tc_make_map_sw(CUtensorMap* map, int rank, const void* base, const uint64_t*
     }
     cuuint64_t gdim[3], gstride[2];
     cuuint32_t bx[3], es[3] = {1, 1, 1};
-    uint64_t stride = 2;
+    uint64_t stride = type == TC_MAP_F32 ? 4 : 2;
     for (int i = 0; i < rank; ++i) {
         gdim[i] = dims[i];
         bx[i] = box[i];
         stride *= dims[i];
         if (i < rank - 1) gstride[i] = stride;
     }
-    CUresult r = fn(map, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank,
+    CUresult r = fn(map, type == TC_MAP_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : type == 1 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank,
                     const_cast<void*>(base), gdim, gstride, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

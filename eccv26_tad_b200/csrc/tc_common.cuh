@@ -305,8 +305,9 @@ int tc_set_share_floor(int n);   // per calling thread; returns the previous flo
 int tc_ensure_smem(const void* kern, size_t bytes);
 // 16-bit tensor map with 128-byte swizzle and zero fill outside the tensor; dims[0] is the contiguous one
 int tc_make_map(CUtensorMap* map, int rank, const void* base, const uint64_t* dims, const uint32_t* box, int fp16);
-// same with a 64- or 128-byte swizzle
-int tc_make_map_sw(CUtensorMap* map, int rank, const void* base, const uint64_t* dims, const uint32_t* box, int fp16,
+// same with a 64- or 128-byte swizzle, and for fp32 tensors (type: 0 = bf16, 1 = f16, or TC_MAP_F32)
+constexpr int TC_MAP_F32 = 2;
+int tc_make_map_sw(CUtensorMap* map, int rank, const void* base, const uint64_t* dims, const uint32_t* box, int type,
                    int swizzle_bytes);
 // column-block width of a forward / dgrad CTA for an output of `cn` columns and `m_tiles` row tiles
 int tc_pick_bn(int cn, long m_tiles);
