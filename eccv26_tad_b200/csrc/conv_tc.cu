@@ -1,7 +1,7 @@
 // Host side of the tcgen05 / TMEM SparseConv2D path: the device error word, tensor-map encoding, tile
 // and split planning, and the dispatch between the kernel families
 //   conv_tc_hybrid.cu   one CTA per tile: gathered rows by per-warp cp.async, weight / gy tiles by TMA
-//   conv_tc_pair.cu     forward / dgrad on CTA pairs (cta_group::2) where they are faster, see use_pair()
+//   conv_tc_pair.cu     forward / dgrad on CTA pairs (cta_group::2) where they are faster, see tc_choose()
 // They replace opentad/models/bricks/implicit_gemm_v2.cu:197-417 (gather kernel + cuBLAS batched GEMM +
 // reduce kernel) and the atomic backward kernels opentad/models/bricks/2d_sparse_v3.cu:656-745.
 #include <cstdlib>
@@ -96,12 +96,19 @@ int tc_ensure_smem(const void* kern, size_t bytes) {
     static std::map<std::pair<const void*, int>, size_t> done;
     int dev = 0;
     SV_CUDA(cudaGetDevice(&dev));
+    // what this thread has asked for lately needs no lock
+    struct Seen { const void* kern; int dev; size_t bytes; };
+    static thread_local Seen seen[64];
+    Seen& hit = seen[(reinterpret_cast<uintptr_t>(kern) >> 4) % 64];
+    if (hit.kern == kern && hit.dev == dev && hit.bytes >= bytes) return SVTAD_OK;
     std::lock_guard<std::mutex> hold(mu);
     auto key = std::make_pair(kern, dev);
     auto it = done.find(key);
-    if (it != done.end() && it->second >= bytes) return SVTAD_OK;
-    SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    done[key] = bytes;
+    if (it == done.end() || it->second < bytes) {
+        SV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        it = done.insert_or_assign(key, bytes).first;
+    }
+    hit = Seen{kern, dev, it->second};
     return SVTAD_OK;
 }
 
@@ -128,19 +135,23 @@ int tc_make_map(CUtensorMap* map, int rank, const void* base, const uint64_t* di
 int tc_make_map_sw(CUtensorMap* map, int rank, const void* base, const uint64_t* dims, const uint32_t* box, int type,
                    int swizzle_bytes) {
     // A descriptor depends only on (base, dims, box, element type, swizzle): a training step encodes the same few
-    // again and again, so the last ones are kept per thread.
+    // again and again, so the last ones are kept per thread, found by a hash of these.
     struct Key { const void* base; uint64_t dims[3]; uint32_t box[3]; int rank, type, swz, dev; };
     struct Slot { Key key; CUtensorMap map; bool used; };
-    constexpr int SLOTS = 32;
+    constexpr unsigned SLOTS = 128;
     static thread_local Slot cache[SLOTS];
-    static thread_local unsigned next_slot = 0;
     Key key;
     memset(&key, 0, sizeof(key));
     key.base = base; key.rank = rank; key.type = type; key.swz = swizzle_bytes;
-    for (int i = 0; i < rank; ++i) { key.dims[i] = dims[i]; key.box[i] = box[i]; }
+    uint64_t h = reinterpret_cast<uintptr_t>(base) >> 4;
+    for (int i = 0; i < rank; ++i) {
+        key.dims[i] = dims[i];
+        key.box[i] = box[i];
+        h = h * 0x9E3779B97F4A7C15ull + dims[i] * 8 + box[i];
+    }
     if (cudaGetDevice(&key.dev) != cudaSuccess) key.dev = -1;
-    for (int i = 0; i < SLOTS; ++i)
-        if (cache[i].used && memcmp(&cache[i].key, &key, sizeof(Key)) == 0) { *map = cache[i].map; return SVTAD_OK; }
+    Slot& slot = cache[(h ^ (h >> 29) ^ (h >> 47)) % SLOTS];
+    if (slot.used && memcmp(&slot.key, &key, sizeof(Key)) == 0) { *map = slot.map; return SVTAD_OK; }
     EncodeTiledFn fn = encode_fn();
     if (fn == nullptr) return set_error(SVTAD_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     // the driver call needs this thread to hold the device's context (autograd worker threads may not yet)
@@ -166,7 +177,6 @@ int tc_make_map_sw(CUtensorMap* map, int rank, const void* base, const uint64_t*
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(SVTAD_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
-    Slot& slot = cache[next_slot++ % SLOTS];
     slot.key = key; slot.map = *map; slot.used = true;
     return SVTAD_OK;
 }
@@ -395,33 +405,56 @@ bool tc_supported(int op, int64_t n, int cin, int cout, int kk, int dtype) {
 // over 326 such calls; where they are close the kernel stays that was there first (pairs from as many row tiles as SMs on).
 // A tile whose K steps a cluster shares goes to single CTAs, and under a concurrency hint only the number of tiles counts.
 // A row's sum is the same either way.  SVTAD_TC_IMPL=pair / hybrid overrides the choice.
-static bool use_pair(int64_t n, int cred, int cn, int kk) {
-    const char* e = getenv("SVTAD_TC_IMPL");
-    if (e != nullptr && *e) return e[0] == 'p';
+static TcChoice choose(int64_t n, int cred, int cn, int kk) {
     const long m_tiles = (n + TILE_M - 1) / TILE_M, sms = tc_num_sms();
-    const bool many = m_tiles > sms;
-    if (tc_plan_sms() < sms) return many;
     const int steps = kk * ((cred + STAGE_K - 1) / STAGE_K);
-    if (hybrid_splits(cn, m_tiles, steps)) return false;
-    auto at = [](int bn) { return bn == 256 ? 4 : bn == 192 ? 3 : bn == 128 ? 2 : bn == 96 ? 1 : 0; };
-    const double pair_step[5] = {0.20, 0.2375, 0.2375, 0.29, 0.316}, single_step[5] = {0.19, 0.245, 0.266, 0.352, 0.366};
-    auto time = [&](double start, long items, long slots, double step) {
-        const long waves = (items + slots - 1) / slots;
-        return start + (double)waves * steps * step + (double)(waves - 1) * 1.7;
+    TcChoice c{m_tiles > sms, 0, 1};
+    c.bn = hybrid_split(cn, m_tiles, steps, c.split);
+    if (c.bn != 0) c.pair = false;
+    else c.bn = tc_pick_bn(cn, m_tiles);
+    const char* e = getenv("SVTAD_TC_IMPL");
+    if (e != nullptr && *e) {
+        c.pair = e[0] == 'p';
+    } else if (c.split == 1 && tc_plan_sms() == sms) {
+        auto at = [](int bn) { return bn == 256 ? 4 : bn == 192 ? 3 : bn == 128 ? 2 : bn == 96 ? 1 : 0; };
+        const double pair_step[5] = {0.20, 0.2375, 0.2375, 0.29, 0.316}, single_step[5] = {0.19, 0.245, 0.266, 0.352, 0.366};
+        auto time = [&](double start, long items, long slots, double step) {
+            const long waves = (items + slots - 1) / slots;
+            return start + (double)waves * steps * step + (double)(waves - 1) * 1.7;
+        };
+        const int wide = tc_widest_bn(cn);
+        const double pair = time(7.0, (m_tiles + 1) / 2 * ((cn + wide - 1) / wide), sms / 2, pair_step[at(wide)]);
+        const double single = time(5.2, m_tiles * ((cn + c.bn - 1) / c.bn), sms, single_step[at(c.bn)]);
+        c.pair = c.pair ? single >= 0.97 * pair : pair < 0.926 * single;
+    }
+    return c;
+}
+
+// The estimates cost the host 0.4 us; the last few answers are kept per thread, as those of tc_wgrad_plan().
+TcChoice tc_choose(int64_t n, int cred, int cn, int kk) {
+    if (getenv("SVTAD_TC_IMPL") != nullptr || getenv("SVTAD_TC_BN") != nullptr) return choose(n, cred, cn, kk);
+    struct Memo {
+        int64_t n = -1;
+        int cred, cn, kk, sms, all;
+        TcChoice choice;
     };
-    const int wide = tc_widest_bn(cn), bn = tc_pick_bn(cn, m_tiles);
-    const double pair = time(7.0, (m_tiles + 1) / 2 * ((cn + wide - 1) / wide), sms / 2, pair_step[at(wide)]);
-    const double single = time(5.2, m_tiles * ((cn + bn - 1) / bn), sms, single_step[at(bn)]);
-    return many ? single >= 0.97 * pair : pair < 0.926 * single;
+    constexpr unsigned SLOTS = 64;
+    static thread_local Memo memo[SLOTS];
+    const int sms = tc_plan_sms(), all = tc_num_sms();
+    const uint64_t h = ((uint64_t)n * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)cred << 40) ^ ((uint64_t)cn << 20) ^ (uint64_t)(kk * 1024 + sms);
+    Memo& m = memo[(h ^ (h >> 29) ^ (h >> 47)) % SLOTS];
+    if (m.n != n || m.cred != cred || m.cn != cn || m.kk != kk || m.sms != sms || m.all != all)
+        m = Memo{n, cred, cn, kk, sms, all, choose(n, cred, cn, kk)};
+    return m.choice;
 }
 
 int tc_fwd(const ConvArgs& p, cudaStream_t s) {
-    if (p.plan == nullptr && use_pair(p.n, p.cin, p.cout, p.kk)) return pair_fwd(p, s);
+    if (p.plan == nullptr && tc_choose(p.n, p.cin, p.cout, p.kk).pair) return pair_fwd(p, s);
     return hybrid_fwd(p, s);
 }
 
 int tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
-    if (p.plan == nullptr && use_pair(p.n, p.cout, p.cin, p.kk)) return pair_dgrad(p, status, s);
+    if (p.plan == nullptr && tc_choose(p.n, p.cout, p.cin, p.kk).pair) return pair_dgrad(p, status, s);
     return hybrid_dgrad(p, status, s);
 }
 

@@ -754,7 +754,7 @@ static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, int G, c
 // The order of the sums depends on the cluster size alone, so that is chosen for the whole GPU whatever the concurrency
 // hint says.  The column block is then chosen for the SMs the kernel may count on: next to a weight gradient, narrow blocks
 // over the whole GPU would make one kernel wait for the other (1 834 rows, C = 320: 27.9 against 20 us).
-static int pick_split(int cn, long m_tiles, int steps, int& G) {
+int hybrid_split(int cn, long m_tiles, int steps, int& G) {
     if (getenv("SVTAD_TC_BN") != nullptr) return 0;
     const int width[4] = {64, 128, 192, 256};
     const double step_us[4] = {0.19, 0.23, 0.28, 0.344}, sharing_us[4] = {1.9, 3.5, 4.0, 6.0};
@@ -785,11 +785,6 @@ static int pick_split(int cn, long m_tiles, int steps, int& G) {
         if (u < best) { best = u; bn = width[i]; }
     }
     return bn;
-}
-
-bool hybrid_splits(int cn, long m_tiles, int steps) {
-    int G = 1;
-    return pick_split(cn, m_tiles, steps, G) != 0;
 }
 
 // Column block of the forward by a plan (the input gradient, which shares the GPU with the weight gradient, takes the widest: with
@@ -825,16 +820,16 @@ static int dispatch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaSt
             default: return launch_conv_hybrid<256, DGRAD, true, false>(p, status, 1, s);
         }
     }
-    int G = 1;
-    const int split_bn = pick_split(cn, (p.n + TILE_M - 1) / TILE_M, p.kk * (((DGRAD ? p.cout : p.cin) + STAGE_K - 1) / STAGE_K), G);
-    switch (split_bn) {
-        case 64: return launch_conv_hybrid<64, DGRAD, false, true>(p, status, G, s);
-        case 128: return launch_conv_hybrid<128, DGRAD, false, true>(p, status, G, s);
-        case 192: return launch_conv_hybrid<192, DGRAD, false, true>(p, status, G, s);
-        case 256: return launch_conv_hybrid<256, DGRAD, false, true>(p, status, G, s);
+    const TcChoice c = tc_choose(p.n, DGRAD ? p.cout : p.cin, cn, p.kk);
+    if (c.split > 1) {
+        switch (c.bn) {
+            case 64: return launch_conv_hybrid<64, DGRAD, false, true>(p, status, c.split, s);
+            case 128: return launch_conv_hybrid<128, DGRAD, false, true>(p, status, c.split, s);
+            case 192: return launch_conv_hybrid<192, DGRAD, false, true>(p, status, c.split, s);
+            case 256: return launch_conv_hybrid<256, DGRAD, false, true>(p, status, c.split, s);
+        }
     }
-    int bn = tc_pick_bn(cn, (p.n + TILE_M - 1) / TILE_M);
-    switch (bn) {
+    switch (c.bn) {
         case 64: return launch_conv_hybrid<64, DGRAD, false, false>(p, status, 1, s);
         case 96: return launch_conv_hybrid<96, DGRAD, false, false>(p, status, 1, s);
         case 128: return launch_conv_hybrid<128, DGRAD, false, false>(p, status, 1, s);
