@@ -16,9 +16,9 @@
 // of a tile that lack a neighbor are rows of zeros).  Sums that are not finite are therefore made again from the fp32
 // values, pair by pair, before they are stored.
 //
-// Measured (graph replays, before: the CUDA-core kernels): 784 rows, C = 192, keep 50 %: forward 21.2 -> 11.1 us, input
-// gradient 22.2 -> 11.0; 4 720 rows, C = 192, keep 30 %: 54.5 -> 28.0, 57.1 -> 26.4, weight gradient 47.8 -> 23.2; 5 880
-// rows, full grid, 320 -> 96: 144 -> 43, 134 -> 39, 103 -> 62.  What bounds the loops: eight warps that load, split and store
+// Measured (graph replays, before: the CUDA-core kernels): 784 rows, C = 192, keep 50 %: forward 21.2 -> 10.4 us, input
+// gradient 22.2 -> 10.4; 4 720 rows, C = 192, keep 30 %: 54.5 -> 25.7, 57.1 -> 25.5, weight gradient 47.8 -> 22.1; 5 880
+// rows, full grid, 320 -> 96: 144 -> 42, 134 -> 38, 103 -> 61.  What bounds the loops: eight warps that load, split and store
 // (850 issue slots per scheduler and step of 1 480 cycles; 768 cycles of tensor work) and the gathered rows' trip from L2, which is
 // one step long.
 #include <cfloat>
@@ -38,7 +38,6 @@ constexpr int T3_RING = 2, T3_B_STAGE = 3 * T3_B_PLANE;      // forward, input g
 constexpr int T3_RAWS = 4, T3_RAW = 64 * T3_BN * 4;          // ... and the weights' fp32 tiles
 constexpr int T3_A_COL = 256, T3_A_COLS = 96;               // behind two accumulators of 128 columns
 constexpr int T3_COLS = 3 * T3_BN;                     // accumulator columns of a step
-constexpr int T3_PARK = T3_BN + 4;                     // floats per row of the parked sums
 
 typedef unsigned long long t3_pair;                    // two fp32 values
 __device__ __forceinline__ t3_pair t3_pack(uint32_t lo, uint32_t hi) {
@@ -287,7 +286,6 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
 
     t3_pair sum[T3_BN / 2];
     const int q = warp & 3;
-    bool whole = true;
     if (warp < T3_A_WARPS) {
         // ------------------------------------------------------------------ producers: all of them fill every buffer
         // A: 16 rows per warp, straight from registers to tensor memory.  A lane loads channels 8 c .. + 7 and 32 + 8 c .. + 7
@@ -417,7 +415,7 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
         const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
         for (int st = 0; st < k_hi - k_lo; ++st) {
             const int buf = st & 1;
-            if (!t3_wait(smem_u32(&tail->accum_full[buf]), (st >> 1) & 1, s_abort, err, 74)) { whole = false; break; }
+            if (!t3_wait(smem_u32(&tail->accum_full[buf]), (st >> 1) & 1, s_abort, err, 74)) break;
             tc_fence_after();
             t3_drain<2>(sum, t_addr + buf * (2 * T3_BN));
             tc_fence_before();
@@ -436,51 +434,44 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
         }
         *reinterpret_cast<float4*>(out + row * cn + col) = f;
     };
-    if constexpr (!SPLIT) {
-        const long row = row0 + q * 32 + lane;
-        if (warp > T3_A_WARPS && warp <= T3_A_WARPS + T3_E_WARPS && whole && row < n) {
-#pragma unroll
-            for (int c = 0; c < T3_BN / 4; ++c) {
-                uint32_t u[4];
-                t3_unpack(sum[2 * c], u[0], u[1]);
-                t3_unpack(sum[2 * c + 1], u[2], u[3]);
-                if (n0 + 4 * c < cn)
-                    finish(row, n0 + 4 * c, make_float4(__uint_as_float(u[0]), __uint_as_float(u[1]), __uint_as_float(u[2]), __uint_as_float(u[3])));
-            }
-        }
-    } else {
-        // a CTA whose wait gave up stops the whole cluster: the others' sums are not finished with what it left behind
-        __syncthreads();
+    // The sums go through shared memory, those of a shared tile to the CTA that finishes their rows, so that all threads store whole
+    // lines (a lane that stores its own row takes 16 bytes of 32 lines at a time: 4 720 rows, C = 192: 28.0 us, now 25.7; with the
+    // shared sums by rows as well, 784 rows took 11.1, now 10.4).  A CTA whose wait gave up stops the whole
+    // cluster: the others' sums are not finished with what it left behind.
+    __syncthreads();
+    if constexpr (SPLIT) {
         if (tid < G && *s_abort) store_to_cta(smem_u32(&tail->abort_flag), tid, 1);
         cluster_barrier();          // every CTA's instructions are done: nothing is left in the rings, which take the sums now
-        const bool all = *s_abort == 0;
-        const int per = (TILE_M + G - 1) / G;               // rows that a CTA finishes: [share * per, ...)
-        const uint32_t park = stage_base;                   // [CTA the sums come from][row][T3_PARK]
-        if (all && warp > T3_A_WARPS && warp <= T3_A_WARPS + T3_E_WARPS) {
-            const int r = q * 32 + lane, owner = r / per;
-            const uint32_t dst = map_to_cta(park + ((share * per + r - owner * per) * T3_PARK) * 4, owner);
+    }
+    const bool all = *s_abort == 0;
+    const int per = SPLIT ? (TILE_M + G - 1) / G : TILE_M;  // rows that a CTA finishes: [share * per, ...)
+    const int pitch = per | 1;                              // [CTA the sums come from][column / 4][row], an odd number of rows apart
+    if (all && warp > T3_A_WARPS && warp <= T3_A_WARPS + T3_E_WARPS) {
+        const int r = q * 32 + lane, owner = SPLIT ? r / per : 0;
+        const uint32_t here = stage_base + (share * (T3_BN / 4) * pitch + r - owner * per) * 16;
+        const uint32_t dst = SPLIT ? map_to_cta(here, owner) : here;
 #pragma unroll
-            for (int c = 0; c < T3_BN / 4; ++c) {
-                uint32_t u[4];
-                t3_unpack(sum[2 * c], u[0], u[1]);
-                t3_unpack(sum[2 * c + 1], u[2], u[3]);
-                asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + c * 16), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]) : "memory");
-            }
+        for (int c = 0; c < T3_BN / 4; ++c) {
+            uint32_t u[4];
+            t3_unpack(sum[2 * c], u[0], u[1]);
+            t3_unpack(sum[2 * c + 1], u[2], u[3]);
+            if (SPLIT) asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + c * pitch * 16), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]) : "memory");
+            else t3_sts16(dst + c * pitch * 16, u);
         }
-        cluster_barrier();
-        const float* sums = reinterpret_cast<const float*>(smem);
-        const int rows = !all ? 0 : share * per + per <= TILE_M ? per : TILE_M - share * per;
-        for (int e = tid; e < rows * (T3_BN / 4); e += T3_FW_THREADS) {
-            const int r = e / (T3_BN / 4), c = e % (T3_BN / 4) * 4;
-            const long row = row0 + share * per + r;
-            if (row >= n || n0 + c >= cn) continue;
-            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int p = 0; p < G; ++p) {
-                const float4 u = *reinterpret_cast<const float4*>(sums + (p * per + r) * T3_PARK + c);
-                f.x += u.x; f.y += u.y; f.z += u.z; f.w += u.w;
-            }
-            finish(row, n0 + c, f);
+    }
+    if constexpr (SPLIT) cluster_barrier(); else __syncthreads();
+    const float4* sums = reinterpret_cast<const float4*>(smem);
+    const int rows = !all ? 0 : share * per + per <= TILE_M ? per : TILE_M - share * per;
+    for (int e = tid; e < rows * (T3_BN / 4); e += T3_FW_THREADS) {
+        const int r = e / (T3_BN / 4), c = e % (T3_BN / 4);
+        const long row = row0 + share * per + r;
+        if (row >= n || n0 + 4 * c >= cn) continue;
+        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int p = 0; p < (SPLIT ? G : 1); ++p) {
+            const float4 u = sums[(p * (T3_BN / 4) + c) * pitch + r];
+            f.x += u.x; f.y += u.y; f.z += u.z; f.w += u.w;
         }
+        finish(row, n0 + 4 * c, f);
     }
     tc_fence_before();
     __syncthreads();
@@ -720,26 +711,32 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
 #pragma unroll
         for (int c = 0; c < T3_BN / 2; ++c) sum[c] = 0;
         const uint32_t t_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-        bool whole = true;
         for (int g = 0;; ++g) {
             const int buf = g & 1;
-            if (!t3_wait(smem_u32(&tail->accum_full[buf]), (g >> 1) & 1, s_abort, err, 78)) { whole = false; break; }
+            if (!t3_wait(smem_u32(&tail->accum_full[buf]), (g >> 1) & 1, s_abort, err, 78)) break;
             if (*reinterpret_cast<volatile int*>(&s_end) == g) break;
             tc_fence_after();
             t3_drain<3>(sum, t_addr + buf * T3_COLS);
             tc_fence_before();
             mbar_arrive(smem_u32(&tail->accum_empty[buf]));
         }
-        const int ci = m0 + (warp & 3) * 32 + lane;
-        float* dst = ws_w + (((long)range * kk + tap) * cin + ci) * cout + n0;
-        if (whole && ci < cin) {
+        // the sums leave through the ring, which nothing is in any more, as the forward's do
+        const uint32_t dst = stage_base + ((warp & 3) * 32 + lane) * 16;
 #pragma unroll
-            for (int c = 0; c < T3_BN / 4; ++c) {
-                uint32_t f[4];
-                t3_unpack(sum[2 * c], f[0], f[1]);
-                t3_unpack(sum[2 * c + 1], f[2], f[3]);
-                if (n0 + 4 * c < cout) *reinterpret_cast<uint4*>(dst + 4 * c) = make_uint4(f[0], f[1], f[2], f[3]);
-            }
+        for (int c = 0; c < T3_BN / 4; ++c) {
+            uint32_t f[4];
+            t3_unpack(sum[2 * c], f[0], f[1]);
+            t3_unpack(sum[2 * c + 1], f[2], f[3]);
+            t3_sts16(dst + c * (TILE_M + 1) * 16, f);
+        }
+    }
+    __syncthreads();
+    if (*s_abort == 0) {
+        const float4* sums = reinterpret_cast<const float4*>(smem);
+        float* to = ws_w + (((long)range * kk + tap) * cin + m0) * cout + n0;
+        for (int e = tid; e < TILE_M * (T3_BN / 4); e += T3_THREADS) {
+            const int r = e / (T3_BN / 4), c = e % (T3_BN / 4);
+            if (m0 + r < cin && n0 + 4 * c < cout) *reinterpret_cast<float4*>(to + (long)r * cout + 4 * c) = sums[c * (TILE_M + 1) + r];
         }
     }
     tc_fence_before();
@@ -851,9 +848,9 @@ static int dispatch_f32_tc(const ConvArgs& p, const int32_t* status, cudaStream_
     return full ? launch_f32_tc<DGRAD, false, true>(p, status, 1, s) : launch_f32_tc<DGRAD, false, false>(p, status, 1, s);
 }
 
-// Forward and input gradient win at every size measured (59 rows, 16 -> 16 channels: 8.6 -> 8.3 us; 1024 -> 1024: 57 -> 32).  The
-// weight gradient has a fixed cost of 7 us per CTA: 118 rows, C = 192: 8.7 and 11.2 us; 472: 12.2 and 12.7, 64 -> 1024: 15.2 and 19.2;
-// 944: 17.4 and 13.6, 64 -> 1024: 24.6 and 22.6.
+// Forward and input gradient win at every size measured (59 rows, 16 -> 16 channels: 8.6 -> 8.3 us; 1024 -> 1024: 57 -> 26).  The
+// weight gradient has a fixed cost of 6 us per CTA: 118 rows, C = 192: 8.7 and 10.0 us; 472: 12.2 and 11.5, 128 -> 128 9.6 and 10.0,
+// 64 -> 1024 15.2 and 19.1; 708: 13.9 and 11.4, 13.0 and 10.3, 21.3 and 20.9.
 bool f32_tc_wanted(int op, int64_t n, int cin, int cout) {
     return (op == SVTAD_OP_WGRAD ? n >= 640 : n > 0) && cin <= T3_MOST && cout <= T3_MOST;
 }
