@@ -77,7 +77,6 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
     constexpr int B_TX_BYTES = DGRAD ? BN * 128 : B_TILE_BYTES;
     constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
     constexpr int TM_COLS = tmem_cols2_for(BN);
-    constexpr int PARK = BN + 4;             // floats per row of the parked sums (SPLIT)
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -383,10 +382,12 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
         int tile, blk;
         item(0, tile, blk);
         const int per = (TILE_M + G - 1) / G;                   // rows that a CTA finishes: [share * per, ...)
-        const uint32_t park = smem_u32(smem);                   // [CTA the sums come from][row][PARK]
+        // [CTA the sums come from][column / 4][row], an odd number of rows apart: a warp's store goes to its owner in one run (row
+        // by row, 16 bytes of each at a time: 392 rows, C = 192: 8.2 us, now 7.3; 980 rows, C = 1024: 26.5, now 25.6)
+        const int pitch = per | 1;
         if (whole && warp > FW_A_WARPS) {
             const int r = (warp & 3) * 32 + lane, owner = r / per;
-            const uint32_t dst = map_to_cta(park + ((share * per + r - owner * per) * PARK) * 4, owner);
+            const uint32_t dst = map_to_cta(stage_base + (share * (BN / 4) * pitch + r - owner * per) * 16, owner);
             const uint32_t t_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
             uint32_t va[32], vb[32];
             tc_fence_after();
@@ -399,12 +400,12 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
 #pragma unroll
                 for (int g = 0; g < 8; ++g)
                     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
-                                 ::"r"(dst + (c * 32 + g * 4) * 4), "r"(v[4 * g]), "r"(v[4 * g + 1]), "r"(v[4 * g + 2]), "r"(v[4 * g + 3]) : "memory");
+                                 ::"r"(dst + (c * 8 + g) * pitch * 16), "r"(v[4 * g]), "r"(v[4 * g + 1]), "r"(v[4 * g + 2]), "r"(v[4 * g + 3]) : "memory");
             }
         }
         cluster_barrier();
         // eight columns of a row per thread, the CTAs' sums in their order
-        const float* sums = reinterpret_cast<const float*>(smem);
+        const float4* sums = reinterpret_cast<const float4*>(smem);
         const long row0 = (long)tile * TILE_M + share * per;
         const int rows = !whole ? 0 : share * per + per <= TILE_M ? per : TILE_M - share * per;
         for (int e = tid; e < rows * (BN / 8); e += FW_THREADS) {
@@ -412,8 +413,8 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             if (row0 + r >= n || col >= cn) continue;
             float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int p = 0; p < G; ++p) {
-                const float4* src = reinterpret_cast<const float4*>(sums + (p * per + r) * PARK + c);
-                const float4 u = src[0], v = src[1];
+                const float4* src = sums + (p * (BN / 4) + c / 4) * pitch + r;
+                const float4 u = src[0], v = src[pitch];
                 sum[0] += u.x; sum[1] += u.y; sum[2] += u.z; sum[3] += u.w;
                 sum[4] += v.x; sum[5] += v.y; sum[6] += v.z; sum[7] += v.w;
             }
@@ -747,18 +748,20 @@ static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, int G, c
 }
 
 // Few row tiles and a long reduction leave most SMs idle: cluster size and column block for the K split, or 0 where it does
-// not pay.  A K step takes what a CTA was measured to need at that width; sharing an item out costs 2 to 6 us more than
+// not pay.  A K step takes what a CTA was measured to need at that width; sharing an item out costs 2 to 5 us more than
 // finishing it alone (cluster launch, two cluster barriers, the sums' trip between SMs).  Clusters of three and more do not
-// pack a GPC's SMs completely, hence the limits on the grid.  1 180 rows, C = 1024: 41.6 -> 31.1 us; 2 360 rows, C = 512,
-// 5x5: 56 -> 38 us; 2 208 rows, C = 256: 11.9 -> 10.3 us.
+// pack a GPC's SMs completely: 45, 33, 26, 22 and 15 of 3, 4, 5, 6 and 8 CTAs run at a time (asked of the occupancy query on
+// a B200), hence the limits on the grid, a cluster short of these.  Before the split / with it: 1 180 rows, C = 1024: 41.6 /
+// 30.4 us; 2 360 rows, C = 512, 5x5: 56 / 37; 2 548 rows, C = 256: 11.8 / 10.9; 1 372 rows, C = 512: 18.7 with at most
+// 112 to 120 CTAs, 14.1 with these limits.
 // The order of the sums depends on the cluster size alone, so that is chosen for the whole GPU whatever the concurrency
 // hint says.  The column block is then chosen for the SMs the kernel may count on: next to a weight gradient, narrow blocks
 // over the whole GPU would make one kernel wait for the other (1 834 rows, C = 320: 27.9 against 20 us).
 int hybrid_split(int cn, long m_tiles, int steps, int& G) {
     if (getenv("SVTAD_TC_BN") != nullptr) return 0;
     const int width[4] = {64, 128, 192, 256};
-    const double step_us[4] = {0.19, 0.23, 0.28, 0.344}, sharing_us[4] = {1.9, 3.5, 4.0, 6.0};
-    const int sizes[5] = {2, 3, 4, 5, 8}, limit[5] = {148, 120, 120, 112, 112};
+    const double step_us[4] = {0.19, 0.23, 0.28, 0.344}, sharing_us[4] = {1.6, 3.0, 3.5, 5.2};
+    const int sizes[6] = {2, 3, 4, 5, 6, 8}, limit[6] = {148, 132, 128, 125, 126, 112};
     const long sms = tc_num_sms(), mine = tc_plan_sms();
     auto tiles_of = [&](int i) { return m_tiles * ((cn + width[i] - 1) / width[i]); };
     double alone = 1e30, best = 1e30;
@@ -768,7 +771,7 @@ int hybrid_split(int cn, long m_tiles, int steps, int& G) {
         const long tiles = tiles_of(i);
         const double t = (double)((tiles + sms - 1) / sms) * steps * step_us[i];
         if (t < alone) alone = t;
-        for (int g = 0; g < 5; ++g) {
+        for (int g = 0; g < 6; ++g) {
             if (tiles * sizes[g] * 148 > limit[g] * sms) continue;
             const double u = (steps + sizes[g] - 1) / sizes[g] * step_us[i] + sharing_us[i];
             if (u < best) { best = u; pick = g; }
