@@ -100,7 +100,7 @@ int tc_set_share_floor(int n);
                        int cin, int cout, int kk, int tpb, int dtype, int grad_dtype, void* ws,             \
                        size_t ws_bytes, bool fit, cudaStream_t s);
 SV_DECLARE_TC_FAMILY(hybrid)
-int hybrid_split(int cn, long m_tiles, int steps, int& G);    // column block and size of clusters that share a tile's K steps, or 0
+int hybrid_split(int cn, long m_tiles, int steps, bool dgrad, int& G);    // column block and size of clusters that share a tile's K steps, or 0
 // forward / dgrad on CTA pairs (conv_tc_pair.cu)
 int pair_fwd(const ConvArgs& p, cudaStream_t s);
 int pair_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s);

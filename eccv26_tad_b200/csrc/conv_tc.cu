@@ -204,8 +204,9 @@ int tc_pick_bn(int cn, long m_tiles) {
     return best;
 }
 
-// The column block with the least padding over the output width, the widest of equals (for kernels whose tiles fill the
-// GPU whatever the width).
+// The column block that covers the output width in the least time, blocks times what a K step takes at that width, for kernels whose
+// tiles fill the GPU whatever the width.  By least padding a width of 320 went in five blocks of 64, which gather a row tile five
+// times: 37 760 rows, C = 320: forward 108 us, in two blocks of 192 68, a training pass 200 and 154; 34 560 rows, C = 448: 184 and 98.
 int tc_widest_bn(int cn) {
     const int cand[4] = {256, 192, 128, 64};
     const char* e = getenv("SVTAD_TC_BN");
@@ -214,10 +215,12 @@ int tc_widest_bn(int cn) {
         for (int c : cand)
             if (v == c && cn % v == 0) return v;
     }
-    int best = 0, padded = 0;
-    for (int c : cand) {
-        const int p = (cn + c - 1) / c * c;
-        if (best == 0 || p < padded) { best = c; padded = p; }
+    const double step_us[4] = {0.344, 0.28, 0.23, 0.19};
+    int best = 0;
+    double least = 0;
+    for (int i = 0; i < 4; ++i) {
+        const double t = (cn + cand[i] - 1) / cand[i] * step_us[i];
+        if (best == 0 || t < least) { best = cand[i]; least = t; }
     }
     return best;
 }
@@ -405,11 +408,11 @@ bool tc_supported(int op, int64_t n, int cin, int cout, int kk, int dtype) {
 // over 326 such calls; where they are close the kernel stays that was there first (pairs from as many row tiles as SMs on).
 // A tile whose K steps a cluster shares goes to single CTAs, and under a concurrency hint only the number of tiles counts.
 // A row's sum is the same either way.  SVTAD_TC_IMPL=pair / hybrid overrides the choice.
-static TcChoice choose(int64_t n, int cred, int cn, int kk) {
+static TcChoice choose(int64_t n, int cred, int cn, int kk, bool dgrad) {
     const long m_tiles = (n + TILE_M - 1) / TILE_M, sms = tc_num_sms();
     const int steps = kk * ((cred + STAGE_K - 1) / STAGE_K);
     TcChoice c{m_tiles > sms, 0, 1};
-    c.bn = hybrid_split(cn, m_tiles, steps, c.split);
+    c.bn = hybrid_split(cn, m_tiles, steps, dgrad, c.split);
     if (c.bn != 0) c.pair = false;
     else c.bn = tc_pick_bn(cn, m_tiles);
     const char* e = getenv("SVTAD_TC_IMPL");
@@ -431,30 +434,30 @@ static TcChoice choose(int64_t n, int cred, int cn, int kk) {
 }
 
 // The estimates cost the host 0.4 us; the last few answers are kept per thread, as those of tc_wgrad_plan().
-TcChoice tc_choose(int64_t n, int cred, int cn, int kk) {
-    if (getenv("SVTAD_TC_IMPL") != nullptr || getenv("SVTAD_TC_BN") != nullptr) return choose(n, cred, cn, kk);
+TcChoice tc_choose(int64_t n, int cred, int cn, int kk, bool dgrad) {
+    if (getenv("SVTAD_TC_IMPL") != nullptr || getenv("SVTAD_TC_BN") != nullptr) return choose(n, cred, cn, kk, dgrad);
     struct Memo {
         int64_t n = -1;
-        int cred, cn, kk, sms, all;
+        int cred, cn, kk, sms, all, dgrad;
         TcChoice choice;
     };
     constexpr unsigned SLOTS = 64;
     static thread_local Memo memo[SLOTS];
     const int sms = tc_plan_sms(), all = tc_num_sms();
-    const uint64_t h = ((uint64_t)n * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)cred << 40) ^ ((uint64_t)cn << 20) ^ (uint64_t)(kk * 1024 + sms);
+    const uint64_t h = ((uint64_t)n * 0x9E3779B97F4A7C15ull) ^ ((uint64_t)cred << 40) ^ ((uint64_t)cn << 20) ^ (uint64_t)(kk * 2048 + sms * 2 + dgrad);
     Memo& m = memo[(h ^ (h >> 29) ^ (h >> 47)) % SLOTS];
-    if (m.n != n || m.cred != cred || m.cn != cn || m.kk != kk || m.sms != sms || m.all != all)
-        m = Memo{n, cred, cn, kk, sms, all, choose(n, cred, cn, kk)};
+    if (m.n != n || m.cred != cred || m.cn != cn || m.kk != kk || m.sms != sms || m.all != all || m.dgrad != dgrad)
+        m = Memo{n, cred, cn, kk, sms, all, dgrad, choose(n, cred, cn, kk, dgrad)};
     return m.choice;
 }
 
 int tc_fwd(const ConvArgs& p, cudaStream_t s) {
-    if (p.plan == nullptr && tc_choose(p.n, p.cin, p.cout, p.kk).pair) return pair_fwd(p, s);
+    if (p.plan == nullptr && tc_choose(p.n, p.cin, p.cout, p.kk, false).pair) return pair_fwd(p, s);
     return hybrid_fwd(p, s);
 }
 
 int tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
-    if (p.plan == nullptr && tc_choose(p.n, p.cout, p.cin, p.kk).pair) return pair_dgrad(p, status, s);
+    if (p.plan == nullptr && tc_choose(p.n, p.cout, p.cin, p.kk, true).pair) return pair_dgrad(p, status, s);
     return hybrid_dgrad(p, status, s);
 }
 

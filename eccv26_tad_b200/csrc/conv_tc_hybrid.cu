@@ -753,15 +753,18 @@ static int launch_conv_hybrid(const ConvArgs& p, const int32_t* status, int G, c
 // pack a GPC's SMs completely: 45, 33, 26, 22 and 15 of 3, 4, 5, 6 and 8 CTAs run at a time (asked of the occupancy query on
 // a B200), hence the limits on the grid, a cluster short of these.  Before the split / with it: 1 180 rows, C = 1024: 41.6 /
 // 30.4 us; 2 360 rows, C = 512, 5x5: 56 / 37; 2 548 rows, C = 256: 11.8 / 10.9; 1 372 rows, C = 512: 18.7 with at most
-// 112 to 120 CTAs, 14.1 with these limits.
+// 112 to 120 CTAs, 14.1 with these limits.  The input gradient, which mostly runs beside a weight gradient, keeps to those: in
+// clusters that fill the GPU it comes in two waves there (1 770 rows, C = 448: a training pass of 40 us became 52).
 // The order of the sums depends on the cluster size alone, so that is chosen for the whole GPU whatever the concurrency
 // hint says.  The column block is then chosen for the SMs the kernel may count on: next to a weight gradient, narrow blocks
 // over the whole GPU would make one kernel wait for the other (1 834 rows, C = 320: 27.9 against 20 us).
-int hybrid_split(int cn, long m_tiles, int steps, int& G) {
+int hybrid_split(int cn, long m_tiles, int steps, bool dgrad, int& G) {
     if (getenv("SVTAD_TC_BN") != nullptr) return 0;
     const int width[4] = {64, 128, 192, 256};
-    const double step_us[4] = {0.19, 0.23, 0.28, 0.344}, sharing_us[4] = {1.6, 3.0, 3.5, 5.2};
-    const int sizes[6] = {2, 3, 4, 5, 6, 8}, limit[6] = {148, 132, 128, 125, 126, 112};
+    const double step_us[4] = {0.19, 0.23, 0.28, 0.344}, fwd_us[4] = {1.6, 3.0, 3.5, 5.2}, dgrad_us[4] = {1.9, 3.5, 4.0, 6.0};
+    const int sizes[6] = {2, 3, 4, 5, 6, 8}, fwd_limit[6] = {148, 132, 128, 125, 126, 112}, dgrad_limit[6] = {148, 120, 120, 112, 0, 112};
+    const double* sharing_us = dgrad ? dgrad_us : fwd_us;
+    const int* limit = dgrad ? dgrad_limit : fwd_limit;
     const long sms = tc_num_sms(), mine = tc_plan_sms();
     auto tiles_of = [&](int i) { return m_tiles * ((cn + width[i] - 1) / width[i]); };
     double alone = 1e30, best = 1e30;
@@ -823,7 +826,7 @@ static int dispatch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaSt
             default: return launch_conv_hybrid<256, DGRAD, true, false>(p, status, 1, s);
         }
     }
-    const TcChoice c = tc_choose(p.n, DGRAD ? p.cout : p.cin, cn, p.kk);
+    const TcChoice c = tc_choose(p.n, DGRAD ? p.cout : p.cin, cn, p.kk, DGRAD);
     if (c.split > 1) {
         switch (c.bn) {
             case 64: return launch_conv_hybrid<64, DGRAD, false, true>(p, status, c.split, s);

@@ -317,7 +317,7 @@ struct TcChoice {
     bool pair;
     int bn, split;
 };
-TcChoice tc_choose(int64_t n, int cred, int cn, int kk);
+TcChoice tc_choose(int64_t n, int cred, int cn, int kk, bool dgrad);
 struct WgradPlan {
     int bn, n_nblk, n_pairs, splits, ones_block;
     long tokens_per_split;
