@@ -124,17 +124,17 @@ extern "C" size_t svtad_bwd_workspace_bytes(int64_t n, int cin, int cout, int kk
 }
 
 // Which parts of a plan gain a layer more than it costs to make them for this one layer and call: the row order (forward,
-// input gradient) takes 10 us up to 7 000 rows, 16 at 18 880, 30 at 60 000, 48 at 113 000, and a few more for the kernel that
+// input gradient) takes 7 us at 4 720 rows, 12 at 18 880, 15 at 37 760, 24 at 75 520, and a few more for the kernel that
 // starts cold behind it; the pair lists (weight gradient; 3 x 3) 4 to 15, next to the input gradient.  A tile of ordered rows
 // needs about 1.2 times the taps that its rows have on average, so what the order saves goes by work * (1 - 1.2 density), and
 // on what it costs the line rises with the rows.  Measured, us of a training pass (forward + backward, graph replays) without
 // a plan and with one made for it, by that figure:
-//   4 720 rows, C = 512, density 0.35 (13 GFLOP): 79 -> 84             12 800, C = 320, 0.27 (16): 105 -> 86
-//   18 880, C = 256, 0.35 (13): 72 -> 93                              11 800, C = 384, 0.35 (18): 113 -> 88
-//   75 520, C = 128, 0.35 (13): 97 -> 119                             4 720, C = 768, 0.35 (29): 152 -> 129
-//   37 760, C = 192, 0.35 (15): 85 -> 88                              18 880, C = 384, 0.35 (29): 148 -> 108
-//   75 520, C = 256, 0.59 (26): 222 -> 233                            37 760, C = 384, 0.59 (29): 260 -> 225
-//   75 520, C = 192, 0.35 (29): 151 -> 151                            18 880, C = 1024, 0.35 (207): 768 -> 391
+//   4 720 rows, C = 512, density 0.35 (13 GFLOP): 77 -> 80             11 800, C = 320, 0.35 (13): 90 -> 76
+//   18 880, C = 256, 0.35 (13): 70 -> 85                              11 800, C = 384, 0.35 (18): 112 -> 82
+//   75 520, C = 128, 0.35 (13): 95 -> 108                             4 720, C = 768, 0.35 (29): 152 -> 123
+//   37 760, C = 192, 0.35 (15): 83 -> 81                              18 880, C = 384, 0.35 (29): 145 -> 106
+//   21 600, C = 512, 0.55 (35): 258 -> 197                            37 760, C = 320, 0.35 (40): 218 -> 150
+//   75 520, C = 192, 0.35 (29): 150 -> 139                            18 880, C = 1024, 0.35 (207): 768 -> 391
 // With few tiles the longest one, which needs nearly every tap, is all that matters, and up to sixteen the kernels without a
 // plan share a tile's K steps over a cluster: 1 770, C = 1024, 0.35 (19): 117 -> 140; 3 920, C = 1024, 0.51 (29): 183 -> 197.
 // Stencils beyond 3 x 3: the order is by the eight nearest neighbors, and a tile needs nearly all of the others (19.9 of 25
@@ -157,12 +157,16 @@ extern "C" int svtad_plan_wanted(int64_t n, int cin, int cout, int kk, int dtype
     return (near ? SVTAD_PLAN_ROWS : 0) | (pairs_wgrad_wanted(cin, kk) ? SVTAD_PLAN_PAIRS : 0);
 }
 
-// The same for a forward alone, which has to earn its row order by itself: 18 880 rows, C = 512, density 0.35 (52 GFLOP): 64 -> 55 us;
-// 7 840, C = 768, 0.51 (33): 77 -> 67; 37 760, C = 384, 0.35 (58): 78 -> 65; 18 880, C = 384, 0.35 (29): 44 -> 44; 4 720, C = 1024,
-// 0.35 (52): 61 -> 64; 75 520, C = 384, 0.59 (59): 154 -> 157; 75 520, C = 256, 0.35 (52): 66 -> 77; 50 240, C = 768, 0.75 (55): 370 -> 381.
+// The same for a forward alone, which has to earn its row order by itself.  us without and with an order made for the call, by
+// the work (GFLOP) that it leaves out:
+//   12 960 rows, C = 512, density 0.55 (21): 56.5 -> 50.7        37 760, C = 320, 0.35 (40): 65.9 -> 53.1
+//   11 800, C = 384, 0.35 (18): 34.8 -> 33.1                     18 880, C = 320, 0.35 (20): 36.0 -> 36.3
+//   18 880, C = 384, 0.35 (29): 41.4 -> 39.7                     75 520, C = 256, 0.35 (52): 64.7 -> 67.0
+// A sweep of 104 shapes (1 920 to 75 520 rows, C = 128 to 1024) is on average 1.4 % from the better of the two, and on a line of
+// 24 + rows / 1600 2.9 %.  Below 48 tiles the longest one decides: 4 720, C = 768, 0.55 (17): 43.4 -> 56.2.
 extern "C" int svtad_plan_wanted_fwd(int64_t n, int cin, int cout, int kk, int dtype, double density) {
     const int rows = svtad_plan_wanted(n, cin, cout, kk, dtype, density) & SVTAD_PLAN_ROWS;
-    return rows && n > 6144 && left_out(n, cin, cout, kk, known_density(density), 1.2) >= 24 + (double)n / 1600 ? rows : 0;
+    return rows && n > 6144 && left_out(n, cin, cout, kk, known_density(density), 1.2) >= 12 + (double)n / 1800 ? rows : 0;
 }
 
 extern "C" int svtad_conv_fwd(const void* x, const int32_t* nbr, const void* w, const void* bias,
