@@ -3,7 +3,7 @@
 #include <cstring>
 #include <mutex>
 
-#include "common.cuh"
+#include "tc_common.cuh"
 
 namespace svtad {
 
@@ -157,16 +157,19 @@ extern "C" int svtad_plan_wanted(int64_t n, int cin, int cout, int kk, int dtype
     return (near ? SVTAD_PLAN_ROWS : 0) | (pairs_wgrad_wanted(cin, kk) ? SVTAD_PLAN_PAIRS : 0);
 }
 
-// The same for a forward alone, which has to earn its row order by itself.  us without and with an order made for the call, by
-// the work (GFLOP) that it leaves out:
-//   12 960 rows, C = 512, density 0.55 (21): 56.5 -> 50.7        37 760, C = 320, 0.35 (40): 65.9 -> 53.1
-//   11 800, C = 384, 0.35 (18): 34.8 -> 33.1                     18 880, C = 320, 0.35 (20): 36.0 -> 36.3
-//   18 880, C = 384, 0.35 (29): 41.4 -> 39.7                     75 520, C = 256, 0.35 (52): 64.7 -> 67.0
-// A sweep of 104 shapes (1 920 to 75 520 rows, C = 128 to 1024) is on average 1.4 % from the better of the two, and on a line of
-// 24 + rows / 1600 2.9 %.  Below 48 tiles the longest one decides: 4 720, C = 768, 0.55 (17): 43.4 -> 56.2.
+// The same for a forward alone, which has to earn its row order by itself.  What the order saves is the share of the time that
+// the kernel without one takes, which goes by its waves (8 736 rows, C = 384, are one wave of 70 tile pairs, 9 600 rows two).  us
+// without and with an order made for the call, and in brackets what it is expected to save, before it is made:
+//   12 960 rows, C = 512, density 0.55 (21): 56.5 -> 50.7        8 736, C = 384, 0.2 (18): 23.9 -> 28.7
+//   11 800, C = 384, 0.35 (22): 34.8 -> 33.1                     18 880, C = 320, 0.35 (21): 36.0 -> 36.3
+//   37 760, C = 320, 0.35 (40): 65.9 -> 53.1                     75 520, C = 256, 0.35 (36): 64.7 -> 67.0
+// A sweep of 104 shapes (1 920 to 75 520 rows, C = 128 to 1024) is on average 1.0 % from the better of the two; on a line by the
+// work left out (24 GFLOP + rows / 1600) 2.9 %.  Below 40 tiles the longest one decides: 4 720, C = 768, 0.55: 43.4 -> 56.2.
 extern "C" int svtad_plan_wanted_fwd(int64_t n, int cin, int cout, int kk, int dtype, double density) {
     const int rows = svtad_plan_wanted(n, cin, cout, kk, dtype, density) & SVTAD_PLAN_ROWS;
-    return rows && n > 6144 && left_out(n, cin, cout, kk, known_density(density), 1.2) >= 12 + (double)n / 1800 ? rows : 0;
+    if (!rows || n <= 5120) return 0;
+    const double saved = tc_choose(n, cin, cout, kk, false).us * (1 - 1.1 * known_density(density));
+    return saved >= 16 + (double)n / 3600 ? rows : 0;
 }
 
 extern "C" int svtad_conv_fwd(const void* x, const int32_t* nbr, const void* w, const void* bias,

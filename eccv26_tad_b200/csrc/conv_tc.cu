@@ -411,14 +411,14 @@ bool tc_supported(int op, int64_t n, int cin, int cout, int kk, int dtype) {
 static TcChoice choose(int64_t n, int cred, int cn, int kk, bool dgrad) {
     const long m_tiles = (n + TILE_M - 1) / TILE_M, sms = tc_num_sms();
     const int steps = kk * ((cred + STAGE_K - 1) / STAGE_K);
-    TcChoice c{m_tiles > sms, 0, 1};
+    TcChoice c{m_tiles > sms, 0, 1, 0.0};
     c.bn = hybrid_split(cn, m_tiles, steps, dgrad, c.split);
     if (c.bn != 0) c.pair = false;
     else c.bn = tc_pick_bn(cn, m_tiles);
     const char* e = getenv("SVTAD_TC_IMPL");
-    if (e != nullptr && *e) {
-        c.pair = e[0] == 'p';
-    } else if (c.split == 1 && tc_plan_sms() == sms) {
+    const bool forced = e != nullptr && *e;
+    if (forced) c.pair = e[0] == 'p';
+    if (c.split == 1) {
         auto at = [](int bn) { return bn == 256 ? 4 : bn == 192 ? 3 : bn == 128 ? 2 : bn == 96 ? 1 : 0; };
         const double pair_step[5] = {0.20, 0.2375, 0.2375, 0.29, 0.316}, single_step[5] = {0.19, 0.245, 0.266, 0.352, 0.366};
         auto time = [&](double start, long items, long slots, double step) {
@@ -428,7 +428,8 @@ static TcChoice choose(int64_t n, int cred, int cn, int kk, bool dgrad) {
         const int wide = tc_widest_bn(cn);
         const double pair = time(7.0, (m_tiles + 1) / 2 * ((cn + wide - 1) / wide), sms / 2, pair_step[at(wide)]);
         const double single = time(5.2, m_tiles * ((cn + c.bn - 1) / c.bn), sms, single_step[at(c.bn)]);
-        c.pair = c.pair ? single >= 0.97 * pair : pair < 0.926 * single;
+        if (!forced && tc_plan_sms() == sms) c.pair = c.pair ? single >= 0.97 * pair : pair < 0.926 * single;
+        c.us = pair < single ? pair : single;
     }
     return c;
 }

@@ -312,10 +312,12 @@ int tc_make_map_sw(CUtensorMap* map, int rank, const void* base, const uint64_t*
 // column-block width of a forward / dgrad CTA for an output of `cn` columns and `m_tiles` row tiles
 int tc_pick_bn(int cn, long m_tiles);
 int tc_widest_bn(int cn);
-// kernel of a forward / dgrad without a plan: CTA pairs, or single CTAs with a column block and `split` CTAs per tile
+// kernel of a forward / dgrad without a plan: CTA pairs, or single CTAs with a column block and `split` CTAs per tile; and what
+// it takes about, alone on the GPU (0: a cluster shares a tile's K steps)
 struct TcChoice {
     bool pair;
     int bn, split;
+    double us;
 };
 TcChoice tc_choose(int64_t n, int cred, int cn, int kk, bool dgrad);
 struct WgradPlan {
