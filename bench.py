@@ -1049,7 +1049,8 @@ def _graph_time(fn, reps=24):
 
 
 def ffma_peak_tflops():
-    """FFMA rate of this GPU (what the fp32 CUDA-core kernels are measured against): svtad_ffma_probe timed here."""
+    """FFMA rate of this GPU (what fp32 has without the tensor cores; the fp32 forward, sums of bf16 products, is given
+    as a share of it): svtad_ffma_probe timed here."""
     import torch
     from eccv26_tad_b200 import _lib
     lib = _lib.load()

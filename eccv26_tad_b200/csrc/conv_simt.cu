@@ -1,5 +1,5 @@
-// Generic CUDA-core (FFMA) SparseConv2D kernels: widths that neither the tensor-core path nor the fp32 kernels over
-// compacted pairs (conv_f32.cu) take, and the asymmetric-table dgrad.  Strict fp32 FMA accumulation in
+// Generic CUDA-core (FFMA) SparseConv2D kernels: widths that neither the tensor-core paths (16-bit, and conv_f32_tc.cu) nor the
+// fp32 kernels over compacted pairs (conv_f32.cu) take, and the asymmetric-table dgrad.  Strict fp32 FMA accumulation in
 // (tap, channel) ascending order - the order of the reference's tiled forward
 // (opentad/models/bricks/2d_sparse_v3.cu:574-629) - so fp32 results stay within 1e-5 relative.
 //
