@@ -265,6 +265,17 @@ def test_a_plan_is_wanted_where_one_layer_pays_for_it():
     assert wanted(18880, 1024, 9, 0.35, _lib.F32) == 0 and wanted(140000, 1024, 9, 0.35) == 0 and wanted(18880, 1024, 1, 0.35) == 0
 
 
+@pytest.mark.parametrize("n,cin,cout,density,wanted", [
+    (8736, 384, 384, 0.20, 0), (9700, 384, 384, 0.20, 1),        # one wave of tile pairs, two
+    (37760, 320, 320, 0.35, 1), (34496, 768, 192, 0.45, 1), (75520, 256, 256, 0.35, 0),
+    (5120, 1024, 1024, 0.20, 0), (5121, 1024, 1024, 0.20, 1),
+])
+def test_a_forward_s_row_order_is_wanted_by_the_waves_it_saves(n, cin, cout, density, wanted):
+    lib = _lib.load()
+    assert lib.svtad_plan_wanted_fwd(n, cin, cout, 9, _lib.BF16, density) == wanted
+    assert lib.svtad_plan_wanted_fwd(n, cin, cout, 9, _lib.F32, density) == 0
+
+
 def test_workspace_sizes_count_the_pair_lists_only_where_a_plan_is_used():
     """The weight gradient by pair lists parks pieces of its sums (74 MB at C = 256); a call without a plan does not."""
     lib = _lib.load()
