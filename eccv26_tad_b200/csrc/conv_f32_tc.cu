@@ -620,7 +620,8 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
         bool alive = true;
         int s = 0, done = 0;
         uint32_t ph = 1;
-        for (long seg = i_begin; alive && seg < i_end; seg += T3_SEG) {
+        // A warp whose wait gave up goes on taking part in every segment's two barriers, as the others may not know of it yet.
+        for (long seg = i_begin; seg < i_end; seg += T3_SEG) {
             // ---- the segment's pairs, ascending: a warp lists an eighth of it
             const int len = (int)min((long)T3_SEG, i_end - seg), eighth = (len + 255) / 256 * 32;
             {
@@ -654,6 +655,7 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
                 }
                 named_bar_sync(1, T3_A_WARPS * 32);
             }
+            if (!alive) continue;
             const int steps = (s_pairs + STAGE_K - 1) / STAGE_K;
             if (steps > 0) {
 #pragma unroll

@@ -67,3 +67,21 @@ def test_ctas_that_share_a_tile_store_nothing_once_a_wait_gave_up():
     known, parks = finish.index("const bool whole = *s_abort == 0;"), finish.index("if (whole && warp > FW_A_WARPS)")
     stores = finish.index("const int rows = !whole ? 0 :")
     assert finish.index("__syncthreads();") < told < barrier < known < parks < stores
+
+
+def _source(name):
+    import os
+    return open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "eccv26_tad_b200", "csrc", name)).read()
+
+
+def test_warps_that_list_pairs_meet_at_every_segment_whoever_gave_up():
+    """The fp32 weight gradient's producers (conv_f32_tc.cu) list each segment's pairs between two barriers of all eight warps,
+    which have no limit: a warp whose wait gave up may not miss one.  Reads the order of the steps."""
+    text = _source("conv_f32_tc.cu")
+    loop = text[text.index("for (long seg = i_begin;"):text.index("// one more round, which carries nothing: the end")]
+    assert "alive" not in loop[:loop.index("{")]
+    first = loop.index("named_bar_sync(1, T3_A_WARPS * 32);")
+    second = loop.index("named_bar_sync(1, T3_A_WARPS * 32);", first + 1)
+    for leaves in ("break", "continue", "return", "alive"):
+        assert leaves not in loop[loop.index("{"):second], leaves
+    assert second < loop.index("if (!alive) continue;") < loop.index("t3_wait(")
