@@ -124,10 +124,6 @@ __device__ __forceinline__ void t3_umma_ts(uint32_t d_tmem, uint32_t a_tmem, uin
         ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// all lanes wait, and agree on the outcome
-__device__ __forceinline__ bool t3_wait(uint32_t bar, uint32_t parity, volatile int* s_abort, int* err, int code) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, s_abort, err, code));
-}
 // what the warp wrote to a buffer is the tensor core's to read
 __device__ __forceinline__ void t3_filled(uint32_t bar, int lane) {
     fence_proxy_async();
@@ -338,12 +334,12 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
                 if (c0 >= cred) { c0 = 0; ++k; }
             }
             load_a();
-            if (!t3_wait(smem_u32(&tail->empty[s]), ph, s_abort, err, 71)) break;
+            if (!mbar_wait_warp(smem_u32(&tail->empty[s]), ph, s_abort, err, 71)) break;
             tc_fence_after();
 #pragma unroll
             for (int q = 0; q < 3; ++q) t3_tmem_st(a_addr + s * T3_A_COLS + q * 32, pa[q]);
             const uint32_t b_tile = stage_base + s * T3_B_STAGE + b_place;
-            if (!t3_wait(smem_u32(&s_raw_full[rs]), rph, s_abort, err, 79)) break;
+            if (!mbar_wait_warp(smem_u32(&s_raw_full[rs]), rph, s_abort, err, 79)) break;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 // rows b_row and b_row + 4: the second one's chunks lie across the swizzle
@@ -379,15 +375,15 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
         uint32_t ph = 0;
         for (int st = 0; st < k_hi - k_lo; ++st) {
             const int buf = st & 1;
-            if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((st >> 1) & 1) ^ 1, s_abort, err, 72)) break;
-            if (!mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 73)) break;
+            const bool ok = mbar_wait(smem_u32(&tail->accum_empty[buf]), ((st >> 1) & 1) ^ 1, s_abort, err, 72) &&
+                            mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 73);
             tc_fence_after();
             if (elect_one_sync()) {
                 t3_issue_ts<!DGRAD>(tmem_base + buf * (2 * T3_BN), tmem_base + T3_A_COL + s * T3_A_COLS, stage_base + s * T3_B_STAGE);
                 umma_commit(smem_u32(&tail->empty[s]));
                 umma_commit(smem_u32(&tail->accum_full[buf]));
             }
-            __syncwarp();
+            if (!__all_sync(0xffffffffu, ok)) break;
             if (++s == T3_RING) { s = 0; ph ^= 1u; }
         }
     } else if (warp == T3_A_WARPS + 1 + T3_E_WARPS) {
@@ -415,7 +411,7 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
         const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
         for (int st = 0; st < k_hi - k_lo; ++st) {
             const int buf = st & 1;
-            if (!t3_wait(smem_u32(&tail->accum_full[buf]), (st >> 1) & 1, s_abort, err, 74)) break;
+            if (!mbar_wait_warp(smem_u32(&tail->accum_full[buf]), (st >> 1) & 1, s_abort, err, 74)) break;
             tc_fence_after();
             t3_drain<2>(sum, t_addr + buf * (2 * T3_BN));
             tc_fence_before();
@@ -663,7 +659,7 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
                     if (it >= A_ITS || real) load(0, it);
             }
             for (int st = 0; st < steps; ++st) {
-                if (!t3_wait(smem_u32(&tail->empty[s]), ph, s_abort, err, 75)) { alive = false; break; }
+                if (!mbar_wait_warp(smem_u32(&tail->empty[s]), ph, s_abort, err, 75)) { alive = false; break; }
                 const uint32_t a_rows = stage_base + s * T3_STAGE + warp * (A_ITS * 512), b_rows = stage_base + s * T3_STAGE + 3 * T3_A_PLANE + b_tok * 128;
                 const int next = st + 1 < steps ? st + 1 : st;
                 if (real) {
@@ -684,7 +680,7 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
             done += steps;
         }
         // one more round, which carries nothing: the end
-        if (alive && t3_wait(smem_u32(&tail->empty[s]), ph, s_abort, err, 75)) {
+        if (alive && mbar_wait_warp(smem_u32(&tail->empty[s]), ph, s_abort, err, 75)) {
             if (tid == 0) s_end = done;
             t3_filled(smem_u32(&tail->full[s]), lane);
         }
@@ -692,8 +688,8 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
         // ------------------------------------------------------------------ MMA issuer (whole warp waits, one lane issues)
         for (int g = 0;; ++g) {
             const int s = g % T3_RING, buf = g & 1;
-            if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((g >> 1) & 1) ^ 1, s_abort, err, 76)) break;
-            if (!mbar_wait(smem_u32(&tail->full[s]), g / T3_RING & 1, s_abort, err, 77)) break;
+            const bool ok = mbar_wait(smem_u32(&tail->accum_empty[buf]), ((g >> 1) & 1) ^ 1, s_abort, err, 76) &&
+                            mbar_wait(smem_u32(&tail->full[s]), g / T3_RING & 1, s_abort, err, 77);
             const bool end = *reinterpret_cast<volatile int*>(&s_end) == g;
             __syncwarp();
             tc_fence_after();
@@ -704,8 +700,7 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
                 }
                 umma_commit(smem_u32(&tail->accum_full[buf]));
             }
-            __syncwarp();
-            if (end) break;
+            if (!__all_sync(0xffffffffu, ok && !end)) break;
         }
     } else {
         // ------------------------------------------------------------------ the last four warps keep the sums
@@ -715,7 +710,7 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
         const uint32_t t_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
         for (int g = 0;; ++g) {
             const int buf = g & 1;
-            if (!t3_wait(smem_u32(&tail->accum_full[buf]), (g >> 1) & 1, s_abort, err, 78)) break;
+            if (!mbar_wait_warp(smem_u32(&tail->accum_full[buf]), (g >> 1) & 1, s_abort, err, 78)) break;
             if (*reinterpret_cast<volatile int*>(&s_end) == g) break;
             tc_fence_after();
             t3_drain<3>(sum, t_addr + buf * T3_COLS);

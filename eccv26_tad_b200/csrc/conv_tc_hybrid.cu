@@ -297,14 +297,14 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
             const int last_ks = (cred - (kchunks - 1) * STAGE_K + 15) / 16;     // 16-channel MMA steps of the last chunk
             const bool whole = last_ks == STAGE_K / 16;
             int tile, blk;
-            for (; alive && item(local, tile, blk); ++local) {
+            for (; item(local, tile, blk); ++local) {
                 const int steps = PLAN ? __popcll(taps_of(tile)) * kchunks : k_hi - k_lo, sp_pad = padded(steps);
                 const int buf = local & 1;
-                if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((local >> 1) & 1) ^ 1, s_abort, err, 42)) { alive = false; break; }
+                if (!mbar_wait_warp(smem_u32(&tail->accum_empty[buf]), ((local >> 1) & 1) ^ 1, s_abort, err, 42)) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
                 for (int st = 0; st < sp_pad; st += RB) {
-                    if (!mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 43)) { alive = false; break; }
+                    const bool ok = mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 43);
                     fence_proxy_async();   // cp.async (generic proxy) writes -> tcgen05.mma (async proxy) reads
                     tc_fence_after();
                     const uint32_t a_tile = stage_base + (uint32_t)(RB * s) * STAGE_BYTES;
@@ -328,7 +328,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
                         }
                         umma_commit(smem_u32(&tail->empty[s]));
                     }
-                    __syncwarp();
+                    if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
                     if (!whole) { kc += halves; if (kc >= kchunks) kc -= kchunks; }
                     if (++s == nbig) { s = 0; ph ^= 1u; }
                 }
@@ -625,7 +625,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
         int s = 0;
         uint32_t ph = 0;
         for (int it = 0; it < total_stages; ++it) {
-            if (!mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 52)) { alive = false; break; }
+            const bool ok = mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 52);
             fence_proxy_async();
             tc_fence_after();
             const uint32_t a_tile = stage_base + (uint32_t)s * STAGE_BYTES;
@@ -639,7 +639,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
                     umma_f16_lh_acc(tmem_base, a_lo + ks * 128, smem_desc_hi(1024), b_lo + ks * 128, smem_desc_hi(1024), idesc);
                 umma_commit(smem_u32(&tail->empty[s]));
             }
-            __syncwarp();
+            if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
             if (++s == nstage) { s = 0; ph ^= 1u; }
         }
         if (alive && total_stages > 0 && elect_one_sync()) umma_commit(smem_u32(&tail->accum_full[0]));
@@ -648,7 +648,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
         // epilogue: fp32 partial tile -> ws_w[split][(tap, ci)][co]; the all-ones block -> ws_b[split][co].  direct: there
         // is one split, and the rounded values go to the gradients themselves (ws_w, ws_b are gw, gb)
         bool have = true;
-        if (total_stages > 0) have = mbar_wait(smem_u32(&tail->accum_full[0]), 0, s_abort, err, 53);
+        if (total_stages > 0) have = mbar_wait_warp(smem_u32(&tail->accum_full[0]), 0, s_abort, err, 53);
         tc_fence_after();
         if (have) {
             const int q = warp & 3;

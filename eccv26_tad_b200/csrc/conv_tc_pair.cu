@@ -275,13 +275,13 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
             const bool whole = last_ks == STAGE_K / 16;
             // distance from one of this CTA's shared-memory addresses to the same location in the odd CTA
             const uint32_t to_peer = map_to_cta(stage_base, 1) - stage_base;
-            for (int item = cid; item < items_total && alive; item += n_clusters, ++local) {
+            for (int item = cid; item < items_total; item += n_clusters, ++local) {
                 const int buf = local & 1;
-                if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((local >> 1) & 1) ^ 1, s_abort, err, 52)) { alive = false; break; }
+                if (!mbar_wait_warp(smem_u32(&tail->accum_empty[buf]), ((local >> 1) & 1) ^ 1, s_abort, err, 52)) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
                 for (int st = 0; st < sp_pad; st += 2) {
-                    if (!mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 53)) { alive = false; break; }
+                    const bool ok = mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 53);
                     fence_proxy_async();
                     tc_fence_after();
                     const uint32_t a_tile = stage_base + (uint32_t)(2 * s) * STAGE_BYTES;
@@ -311,7 +311,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
                         umma_pair_commit(e_local);
                         umma_pair_commit(e_local + to_peer);
                     }
-                    __syncwarp();
+                    if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
                     if (!whole) { kc += halves; if (kc >= kchunks) kc -= kchunks; }
                     if (++s == nbig) { s = 0; ph ^= 1u; }
                 }

@@ -238,13 +238,13 @@ wgrad_pairs_kernel(const uint16_t* __restrict__ gy, const uint16_t* __restrict__
         bool alive = true;
         int s = 0;
         uint32_t ph = 0;
-        for (int local = 0; alive && next_piece(); ++local) {
+        for (int local = 0; next_piece(); ++local) {
             const int buf = local % NBUF, steps = s1 - s0;
-            if (!mbar_wait(smem_u32(&tail->accum_empty[buf]), ((local / NBUF) & 1) ^ 1, s_abort, err, 62)) break;
+            if (!mbar_wait_warp(smem_u32(&tail->accum_empty[buf]), ((local / NBUF) & 1) ^ 1, s_abort, err, 62)) break;
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + buf * BN;
             for (int st = 0; st < steps; ++st) {
-                if (!mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 63)) { alive = false; break; }
+                const bool ok = mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 63);
                 fence_proxy_async();       // cp.async (generic proxy) writes -> tcgen05.mma (async proxy) reads
                 tc_fence_after();
                 const uint32_t a_tile = stage_base + (uint32_t)s * STAGE_BYTES;
@@ -262,7 +262,7 @@ wgrad_pairs_kernel(const uint16_t* __restrict__ gy, const uint16_t* __restrict__
                     }
                     umma_commit(smem_u32(&tail->empty[s]));
                 }
-                __syncwarp();
+                if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
                 if (++s == nstage) { s = 0; ph ^= 1u; }
             }
             if (!alive) break;

@@ -84,4 +84,25 @@ def test_warps_that_list_pairs_meet_at_every_segment_whoever_gave_up():
     second = loop.index("named_bar_sync(1, T3_A_WARPS * 32);", first + 1)
     for leaves in ("break", "continue", "return", "alive"):
         assert leaves not in loop[loop.index("{"):second], leaves
-    assert second < loop.index("if (!alive) continue;") < loop.index("t3_wait(")
+    assert second < loop.index("if (!alive) continue;") < loop.index("mbar_wait_warp(")
+
+
+def test_no_warp_wide_step_behind_a_wait_of_single_lanes():
+    """A warp in which one lane's wait gave up and another's came through never meets again.  So every wait of the tensor-core
+    kernels is one lane's (its outcome shuffled, or the lane on its own from there), the whole warp's, or one whose outcome
+    ``ok`` all lanes carry to the vote behind the step."""
+    import re
+    for name in ("conv_f32_tc.cu", "conv_tc_hybrid.cu", "conv_tc_pair.cu", "conv_tc_pairs.cu"):
+        lines = _source(name).split("\n")
+        for at, line in enumerate(lines):
+            where = f"{name}:{at + 1}: {line.strip()}"
+            if not re.search(r"\bmbar_wait\(", line) or "lane == 0" in line:
+                continue
+            if "bool ok = " in lines[at - 1] + line:
+                rest = "\n".join(lines[at + 1:at + 50])
+                to_vote = rest[:rest.index("__all_sync(0xffffffffu, ok")]
+                assert "break" not in to_vote and "return" not in to_vote, where
+                continue
+            depth = len(line) - len(line.lstrip())
+            guard = [b for b in lines[:at] if b.rstrip().endswith("{") and len(b) - len(b.lstrip()) < depth and "lane == 0" in b]
+            assert guard and "elect" not in "".join(lines[at:at + 12]), where
