@@ -471,6 +471,7 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
     }
     tc_fence_before();
     __syncthreads();
+    settle_after_abort(s_abort);
     if (warp == T3_A_WARPS) {
         __syncwarp();
         tc_fence_after();
@@ -738,6 +739,7 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
     }
     tc_fence_before();
     __syncthreads();
+    settle_after_abort(s_abort);
     if (warp == T3_A_WARPS) {
         __syncwarp();
         tc_fence_after();

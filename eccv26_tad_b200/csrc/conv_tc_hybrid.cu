@@ -436,6 +436,7 @@ conv_hybrid_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __
     }
     tc_fence_before();
     __syncthreads();
+    settle_after_abort(s_abort);
     if (warp == FW_A_WARPS) {
         __syncwarp();
         tc_fence_after();
@@ -703,6 +704,7 @@ wgrad_hybrid_kernel(const __grid_constant__ CUtensorMap map_gy, const uint16_t* 
     }
     tc_fence_before();
     __syncthreads();
+    settle_after_abort(s_abort);
     if (warp == 4) {
         __syncwarp();
         tc_fence_after();

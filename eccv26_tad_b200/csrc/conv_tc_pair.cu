@@ -373,6 +373,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_w, const uint16_t* __re
     }
     tc_fence_before();
     __syncthreads();
+    settle_after_abort(s_abort);
     cluster_barrier();          // nobody frees tensor memory or leaves while the other CTA's work may still touch it
     if (warp == PR_A_WARPS) {
         __syncwarp();

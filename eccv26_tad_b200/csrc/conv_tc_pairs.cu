@@ -349,6 +349,7 @@ wgrad_pairs_kernel(const uint16_t* __restrict__ gy, const uint16_t* __restrict__
     }
     tc_fence_before();
     __syncthreads();
+    settle_after_abort(s_abort);
     if (warp == WP_A_WARPS) {
         __syncwarp();
         tc_fence_after();

@@ -70,6 +70,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* s_abort, int* err, int code) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, s_abort, err, code));
 }
+// Behind the last wait of a CTA in which one gave up: what copies and MMAs are still in flight have a millisecond to finish, before
+// tensor memory is freed and the CTA's shared memory is another's.
+__device__ __forceinline__ void settle_after_abort(volatile int* s_abort) {
+    if (*s_abort == 0) return;
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000ll) {}
+}
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t src_bytes) {

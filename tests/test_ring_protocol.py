@@ -106,3 +106,11 @@ def test_no_warp_wide_step_behind_a_wait_of_single_lanes():
             depth = len(line) - len(line.lstrip())
             guard = [b for b in lines[:at] if b.rstrip().endswith("{") and len(b) - len(b.lstrip()) < depth and "lane == 0" in b]
             assert guard and "elect" not in "".join(lines[at:at + 12]), where
+
+
+def test_nothing_is_in_flight_when_a_cta_that_gave_up_leaves():
+    """Every tensor-core kernel gives what is in flight time to finish behind a wait that gave up, before it frees tensor memory."""
+    for name, kernels in (("conv_f32_tc.cu", 2), ("conv_tc_hybrid.cu", 2), ("conv_tc_pair.cu", 1), ("conv_tc_pairs.cu", 1)):
+        ends = _source(name).split("tmem_dealloc")
+        ends = [e for e in ends[:-1] if "tcgen05.dealloc" not in e[-200:] and "SVTAD_TABLE_ASYMMETRIC" not in e[-300:] and "void " not in e[-10:]]
+        assert len(ends) == kernels and all("settle_after_abort(s_abort);" in e[-300:] for e in ends), name
