@@ -9,12 +9,14 @@
 // tensor memory for one step of 64 products only and is then added to the running sum in registers, rounded to nearest; the
 // small partial products have columns of their own.  Errors against 64 bits (2-norm) over 4 to 1024 channels, 9 to 49
 // taps, 59 to 7 080 rows: forward 5e-8 to 1.4e-7, input gradient 5e-8 to 1.2e-7, weight gradient 5e-8 to 1.4e-7; the
-// CUDA-core kernels (conv_f32.cu) 6e-8 to 4.7e-7, 6e-8 to 3.0e-7, 1.2e-7 to 3.6e-7, each call's larger than here.  The
-// planes of values below 2^-108 lose bits under bf16's range: tensors whose values are all below 4e-34 come out less exact.
+// CUDA-core kernels (conv_f32.cu) 6e-8 to 4.7e-7, 6e-8 to 3.0e-7, 1.2e-7 to 3.6e-7, each call's larger than here.  Values
+// are split as 2^16 times what they are, and the sums brought back by 2^-32: the last bit that fp32 has, 2^-149, is then the
+// last that bf16 has, and planes lose nothing however small the value is (without it: all of a tensor below 4e-34 made errors
+// of 3e-6 at 1e-35, 3e-4 at 1e-37).
 //
-// A value that is infinite, NaN or beyond bf16's range makes its planes NaN, also in sums that it has no part in (the rows
-// of a tile that lack a neighbor are rows of zeros).  Sums that are not finite are therefore made again from the fp32
-// values, pair by pair, before they are stored.
+// A value that is infinite, NaN or above 2^112 makes its planes NaN, also in sums that it has no part in (the rows of a tile
+// that lack a neighbor are rows of zeros), and a sum above 2^96 is infinite.  Sums that are not finite are therefore made again from
+// the fp32 values, pair by pair, before they are stored.
 //
 // Measured (graph replays, before: the CUDA-core kernels): 784 rows, C = 192, keep 50 %: forward 21.2 -> 10.4 us, input
 // gradient 22.2 -> 10.4; 4 720 rows, C = 192, keep 30 %: 54.5 -> 25.7, 57.1 -> 25.5, weight gradient 47.8 -> 22.1; 5 880
@@ -51,16 +53,26 @@ __device__ __forceinline__ t3_pair t3_add(t3_pair a, t3_pair b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ t3_pair t3_mul(t3_pair a, t3_pair b) {
+    t3_pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+constexpr t3_pair T3_UP = 0x4780000047800000ull, T3_DOWN = 0x2F8000002F800000ull;      // 2^16 and 2^-32, twice
 __device__ __forceinline__ t3_pair t3_neg_add(t3_pair a, t3_pair b) {      // b - a
     t3_pair r;
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(b), "l"(a));
     return r;
 }
 
-// Two values -> their three planes, packed, the second with its sign turned: plane minus value is one instruction on the
+// Two values -> the three planes of 2^16 times them, packed, the second with its sign turned: plane minus value is one instruction on the
 // half of a packed register.  (Widening the plane by a shift and a mask first: 16.5 cycles per pair and scheduler instead of
 // 12.7 in a loop of its own - conversions, shifts, masks and selects go through a pipe of half the width.)
 __device__ __forceinline__ void t3_split2(float a, float b, uint32_t (&p)[3]) {
+    uint32_t lo, hi;
+    t3_unpack(t3_mul(t3_pack(__float_as_uint(a), __float_as_uint(b)), T3_UP), lo, hi);
+    a = __uint_as_float(lo);
+    b = __uint_as_float(hi);
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         p[q] = pack2(a, b, false);
@@ -449,8 +461,8 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
 #pragma unroll
         for (int c = 0; c < T3_BN / 4; ++c) {
             uint32_t u[4];
-            t3_unpack(sum[2 * c], u[0], u[1]);
-            t3_unpack(sum[2 * c + 1], u[2], u[3]);
+            t3_unpack(t3_mul(sum[2 * c], T3_DOWN), u[0], u[1]);
+            t3_unpack(t3_mul(sum[2 * c + 1], T3_DOWN), u[2], u[3]);
             if (SPLIT) asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + c * pitch * 16), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]) : "memory");
             else t3_sts16(dst + c * pitch * 16, u);
         }
@@ -723,8 +735,8 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
 #pragma unroll
         for (int c = 0; c < T3_BN / 4; ++c) {
             uint32_t f[4];
-            t3_unpack(sum[2 * c], f[0], f[1]);
-            t3_unpack(sum[2 * c + 1], f[2], f[3]);
+            t3_unpack(t3_mul(sum[2 * c], T3_DOWN), f[0], f[1]);
+            t3_unpack(t3_mul(sum[2 * c + 1], T3_DOWN), f[2], f[3]);
             t3_sts16(dst + c * (TILE_M + 1) * 16, f);
         }
     }

@@ -104,6 +104,18 @@ def test_precision_does_not_hang_on_the_scale(sx, sw):
     _close(_run(table, x, w, b, gy), _truth(table, x, w, b, gy))
 
 
+@pytest.mark.parametrize("small", ["x", "w", "gy"])
+@pytest.mark.parametrize("scale", [2.0 ** -112, 2.0 ** -120, 2.0 ** -127])
+def test_the_planes_hold_values_down_to_the_last_bit_of_fp32(small, scale):
+    """Down to subnormal values, the other operands large enough for results in the normal range."""
+    _, _, table = make_table(1, 8, 14, 14, 0.5, 3, 6)
+    x, w, b, gy = make_conv_inputs(table.shape[0], 64, 64, 3, torch.float32, 6)
+    t = {"x": x, "w": w, "gy": gy}
+    t = {name: v * (scale if name == small else 2.0 ** 36) for name, v in t.items()}
+    got, truth = _run(table, t["x"], t["w"], b, t["gy"]), _truth(table, t["x"], t["w"], b, t["gy"])
+    _close(got[:3], truth[:3])
+
+
 @pytest.mark.parametrize("where", ["x", "w", "gy"])
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38])
 @pytest.mark.parametrize("n", [700, 200])
