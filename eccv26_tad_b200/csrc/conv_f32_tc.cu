@@ -16,7 +16,9 @@
 //
 // A value that is infinite, NaN or above 2^112 makes its planes NaN, also in sums that it has no part in (the rows of a tile
 // that lack a neighbor are rows of zeros), and a sum above 2^96 is infinite.  Sums that are not finite are therefore made again from
-// the fp32 values, pair by pair, before they are stored.
+// the fp32 values, by all warps of the CTA, before they are stored.  us a call of 4 720 rows, C = 192, ordinary values / one
+// infinity in each operand / all infinite (a thread per sum: 1 150 and 7 430 with one): forward 27 / 164 / 200, input gradient 27 /
+// 152 / 195, weight gradient 25 / 114 / 114; the CUDA-core kernels, whatever the values, 59, 62 and 51.
 //
 // Measured (graph replays, before: the CUDA-core kernels): 784 rows, C = 192, keep 50 %: forward 21.2 -> 10.4 us, input
 // gradient 22.2 -> 10.4; 4 720 rows, C = 192, keep 30 %: 54.5 -> 25.7, 57.1 -> 25.5, weight gradient 47.8 -> 22.1; 5 880
@@ -199,26 +201,83 @@ __device__ __forceinline__ void t3_drain(t3_pair (&sum)[T3_BN / 2], uint32_t t_a
 }
 
 __device__ __forceinline__ bool t3_finite(float v) { return fabsf(v) <= FLT_MAX; }
+__device__ __forceinline__ bool t3_finite(const float4& v) { return t3_finite(v.x) && t3_finite(v.y) && t3_finite(v.z) && t3_finite(v.w); }
 
-// out[row][col] of the forward or input gradient without its bias, from the fp32 values
+// The values of `rows` rows of the tile from row `lo` on, of 64 columns, that came out infinite or NaN, from the fp32 values: a warp
+// per four rows and sixteen columns; lanes l % 4 have four columns each and lanes l / 4 four of 32 channels, whose sums are added up
+// at the end.  All threads of the CTA call; out and s_row as they left them.  A function of its own, so that the kernel keeps its
+// registers.
 template <bool DGRAD>
-__device__ __noinline__ float t3_row_sum(const float* a, const int32_t* nbr, const float* w, long row, int col, long n, int cred,
-                                         int cin, int cout, int kk, int tpb) {
-    float s = 0.f;
-    const long off = tpb > 0 ? (row / tpb) * (long)tpb : 0;
-    for (int k = 0; k < kk; ++k) {
-        const int raw = __ldg(nbr + row * kk + k);
-        const long j = (long)raw + off;
-        if (raw < 0 || j >= n) continue;
-        const float* ar = a + j * cred;
-        const float* wr = DGRAD ? w + ((long)(kk - 1 - k) * cin + col) * cout : w + (long)k * cin * cout + col;
-        const long step = DGRAD ? 1 : cout;
-        for (int c = 0; c < cred; ++c) {
-            s = fmaf(__ldg(ar + c), __ldg(wr + c * step), s);
-            if (s != s) return s;
+__device__ __noinline__ void t3_redo(float* out, const float* const* s_row, const float* w, const float* bias, long row0, int lo, int rows,
+                                     int n0, long n, int cred, int cn, int cin, int cout, int kk) {
+    const int lane = threadIdx.x & 31, items = (rows + 3) / 4 * 4;
+    for (int item = threadIdx.x >> 5; item < items; item += T3_FW_THREADS / 32) {
+        const int r0 = lo + item / 4 * 4, col = n0 + item % 4 * 16 + (lane & 3) * 4;
+        int at[4];
+        bool bad = false;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            at[r] = r0 + r < lo + rows && row0 + r0 + r < n ? r0 + r : r0;
+            if (r == lane >> 3 && row0 + r0 < n && col < cn) bad = !t3_finite(*reinterpret_cast<const float4*>(out + (row0 + at[r]) * cn + col));
+        }
+        if (!__any_sync(0xffffffffu, bad)) continue;
+        float sum[4][4] = {};
+        for (int k = 0; k < kk; ++k) {
+            const float* a[4];
+            bool there[4], any = false;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                a[r] = s_row[k * TILE_M + at[r]];
+                there[r] = a[r] != t3_zeros;
+                any = any || there[r];
+            }
+            if (!any) continue;
+            if (col < cn) {
+                const float* wk = DGRAD ? w + ((long)(kk - 1 - k) * cin + col) * cout : w + (long)k * cin * cout + col;
+#pragma unroll 2
+                for (int c = (lane >> 2) * 4; c < cred; c += 32) {
+                    float4 av[4], wv[4];
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) av[r] = __ldg(reinterpret_cast<const float4*>(a[r] + c));
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) wv[q] = __ldg(reinterpret_cast<const float4*>(DGRAD ? wk + (long)q * cout + c : wk + (long)(c + q) * cout));
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        if (!there[r]) continue;           // zeros would make NaN of an infinite weight
+                        const float x[4] = {av[r].x, av[r].y, av[r].z, av[r].w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                const float4 v = DGRAD ? wv[q] : wv[i];
+                                const int c4 = DGRAD ? i : q;
+                                sum[r][q] = fmaf(x[i], c4 == 0 ? v.x : c4 == 1 ? v.y : c4 == 2 ? v.z : v.w, sum[r][q]);
+                            }
+                    }
+                }
+            }
+            // a lane's NaN is one of the whole sum; once all are NaN that is what they stay
+            unsigned nans = 0;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) nans |= (sum[e >> 2][e & 3] != sum[e >> 2][e & 3] ? 1u : 0u) << e;
+#pragma unroll
+            for (int d = 4; d < 32; d <<= 1) nans |= __shfl_xor_sync(0xffffffffu, nans, d);
+            if (__all_sync(0xffffffffu, nans == 0xffffu || col >= cn)) break;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int d = 4; d < 32; d <<= 1) sum[r][q] += __shfl_xor_sync(0xffffffffu, sum[r][q], d);
+            if (r != lane >> 2 || row0 + r0 >= n || col >= cn) continue;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float* to = out + (row0 + at[r]) * cn + col + q;
+                if (!t3_finite(*to)) *to = sum[r][q] + (!DGRAD && bias != nullptr ? __ldg(bias + col + q) : 0.f);
+            }
         }
     }
-    return s;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -430,18 +489,6 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
             mbar_arrive(smem_u32(&tail->accum_empty[buf]));
         }
     }
-    // four columns of a row: + bias, and sums that are not finite from the fp32 values
-    auto finish = [&](long row, int col, float4 f) {
-        float* e = reinterpret_cast<float*>(&f);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            if (!t3_finite(e[c])) e[c] = t3_row_sum<DGRAD>(a, nbr, w, row, col + c, n, cred, cin, cout, kk, tpb);
-        if (!DGRAD && bias != nullptr) {
-            const float4 b = __ldg(reinterpret_cast<const float4*>(bias + col));
-            f.x += b.x; f.y += b.y; f.z += b.z; f.w += b.w;
-        }
-        *reinterpret_cast<float4*>(out + row * cn + col) = f;
-    };
     // The sums go through shared memory, those of a shared tile to the CTA that finishes their rows, so that all threads store whole
     // lines (a lane that stores its own row takes 16 bytes of 32 lines at a time: 4 720 rows, C = 192: 28.0 us, now 25.7; with the
     // shared sums by rows as well, 784 rows took 11.1, now 10.4).  A CTA whose wait gave up stops the whole
@@ -470,19 +517,25 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
     if constexpr (SPLIT) cluster_barrier(); else __syncthreads();
     const float4* sums = reinterpret_cast<const float4*>(smem);
     const int rows = !all ? 0 : share * per + per <= TILE_M ? per : TILE_M - share * per;
+    bool again = false;
     for (int e = tid; e < rows * (T3_BN / 4); e += T3_FW_THREADS) {
-        const int r = e / (T3_BN / 4), c = e % (T3_BN / 4);
+        const int r = e / (T3_BN / 4), c = e % (T3_BN / 4), col = n0 + 4 * c;
         const long row = row0 + share * per + r;
-        if (row >= n || n0 + 4 * c >= cn) continue;
+        if (row >= n || col >= cn) continue;
         float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int p = 0; p < (SPLIT ? G : 1); ++p) {
             const float4 u = sums[(p * (T3_BN / 4) + c) * pitch + r];
             f.x += u.x; f.y += u.y; f.z += u.z; f.w += u.w;
         }
-        finish(row, n0 + 4 * c, f);
+        if (!DGRAD && bias != nullptr) {
+            const float4 b = __ldg(reinterpret_cast<const float4*>(bias + col));
+            f.x += b.x; f.y += b.y; f.z += b.z; f.w += b.w;
+        }
+        again = again || !t3_finite(f);
+        *reinterpret_cast<float4*>(out + row * cn + col) = f;
     }
     tc_fence_before();
-    __syncthreads();
+    if (__syncthreads_or(again)) t3_redo<DGRAD>(out, s_row, w, bias, row0, share * per, rows, n0, n, cred, cn, cin, cout, kk);
     settle_after_abort(s_abort);
     if (warp == T3_A_WARPS) {
         __syncwarp();
@@ -504,6 +557,80 @@ struct T3Units {
     int m_blks, n_blks, centre;
     int own, others, bias;                 // ranges of tokens for the centre tap, the other taps, the bias gradient (0: not wanted)
 };
+
+// Segments of T3_SEG tokens: their pairs (row of gy, row of x), ascending, and behind them (-1, -1) up to a whole step.  Each of the
+// first eight warps, all of which call, lists an eighth of it between two barriers of theirs.
+__device__ __forceinline__ void t3_list_pairs(int2* s_pair, int* s_count, int* s_pairs, const int32_t* nbr, long seg, long i_end,
+                                              long n, int kk, int tap, int tpb) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int Q = T3_SEG / T3_A_WARPS / 32;
+    const int len = (int)min((long)T3_SEG, i_end - seg), eighth = (len + 255) / 256 * 32;
+    int jj[Q], cnt = 0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int at = warp * eighth + q * 32 + lane;
+        jj[q] = q * 32 < eighth && at < len ? __ldg(nbr + (seg + at) * kk + tap) : -1;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const long i = seg + warp * eighth + q * 32 + lane, j = (long)jj[q] + (tpb > 0 ? (i / tpb) * (long)tpb : 0);
+        jj[q] = jj[q] >= 0 && j < n ? (int)j : -1;
+        cnt += __popc(__ballot_sync(0xffffffffu, jj[q] >= 0));
+    }
+    if (lane == 0) s_count[warp] = cnt;
+    named_bar_sync(1, T3_A_WARPS * 32);         // also: nobody reads the last segment's list any more
+    int at = 0, pairs = 0;
+#pragma unroll
+    for (int q = 0; q < T3_A_WARPS; ++q) {
+        at += q < warp ? s_count[q] : 0;
+        pairs += s_count[q];
+    }
+    if (tid == 0) *s_pairs = pairs;
+    if (tid < STAGE_K && pairs + tid < (pairs + STAGE_K - 1) / STAGE_K * STAGE_K) s_pair[pairs + tid] = make_int2(-1, -1);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const unsigned m = __ballot_sync(0xffffffffu, jj[q] >= 0);
+        if (jj[q] >= 0) s_pair[at + __popc(m & ((1u << lane) - 1u))] = make_int2((int)(seg + warp * eighth + q * 32 + lane), jj[q]);
+        at += __popc(m);
+    }
+    named_bar_sync(1, T3_A_WARPS * 32);
+}
+
+// The tile's sums [column / 4][row] that came out infinite or NaN, from the fp32 values of the pairs, ascending, eight rows by four
+// columns per thread of the first eight warps, all of which call.  A function of its own, so that the kernel keeps its registers.
+__device__ __noinline__ void t3_redo_wgrad(float* sums, int2* s_pair, int* s_count, int* s_pairs, const float* gy, const float* x,
+                                           const int32_t* nbr, long i_begin, long i_end, long n, int m0, int n0, int cin, int cout,
+                                           int kk, int tap, int tpb) {
+    const int r0 = (threadIdx.x >> 4) * 8, c = threadIdx.x & 15, ci = m0 + r0, co = n0 + 4 * c;
+    const bool g_there = co < cout, lo_there = ci < cin, hi_there = ci + 4 < cin;
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    float acc[8][4] = {};
+    for (long seg = i_begin; seg < i_end; seg += T3_SEG) {
+        t3_list_pairs(s_pair, s_count, s_pairs, nbr, seg, i_end, n, kk, tap, tpb);
+        const int pairs = *s_pairs;
+#pragma unroll 4
+        for (int p = 0; p < pairs; ++p) {
+            const int2 ij = s_pair[p];
+            const float4* xr = reinterpret_cast<const float4*>(x + (long)ij.y * cin + ci);
+            const float4 g = g_there ? __ldg(reinterpret_cast<const float4*>(gy + (long)ij.x * cout + co)) : none;
+            const float4 lo = lo_there ? __ldg(xr) : none, hi = hi_there ? __ldg(xr + 1) : none;
+            const float xv[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                acc[r][0] = fmaf(xv[r], g.x, acc[r][0]);
+                acc[r][1] = fmaf(xv[r], g.y, acc[r][1]);
+                acc[r][2] = fmaf(xv[r], g.z, acc[r][2]);
+                acc[r][3] = fmaf(xv[r], g.w, acc[r][3]);
+            }
+        }
+    }
+    sums += (c * (TILE_M + 1) + r0) * 4;
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (!t3_finite(sums[r * 4 + q])) sums[r * 4 + q] = acc[r][q];
+}
 
 template <bool FULL>
 __global__ void __launch_bounds__(T3_THREADS, 1)
@@ -606,9 +733,9 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
     const uint32_t tmem_base = tail->tmem_slot;
     pdl_trigger();
 
+    bool again = false;
     if (warp < T3_A_WARPS) {
         // ------------------------------------------------------------------ producers: all of them fill every buffer
-        constexpr int Q = T3_SEG / T3_A_WARPS / 32;
         const uint32_t place[2] = {(uint32_t)(rg * 128 + (((lane & 7) ^ rg) << 4)), (uint32_t)((4 + rg) * 128 + (((lane & 7) ^ (4 + rg)) << 4))};
         float v[A_ITS + B_ITS][8];
         auto store = [&](uint32_t rows, uint32_t plane, int it, const float (&f)[8]) {
@@ -631,39 +758,7 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
         uint32_t ph = 1;
         // A warp whose wait gave up goes on taking part in every segment's two barriers, as the others may not know of it yet.
         for (long seg = i_begin; seg < i_end; seg += T3_SEG) {
-            // ---- the segment's pairs, ascending: a warp lists an eighth of it
-            const int len = (int)min((long)T3_SEG, i_end - seg), eighth = (len + 255) / 256 * 32;
-            {
-                int jj[Q], cnt = 0;
-#pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    const int at = warp * eighth + q * 32 + lane;
-                    jj[q] = q * 32 < eighth && at < len ? __ldg(nbr + (seg + at) * kk + tap) : -1;
-                }
-#pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    const long i = seg + warp * eighth + q * 32 + lane, j = (long)jj[q] + (tpb > 0 ? (i / tpb) * (long)tpb : 0);
-                    jj[q] = jj[q] >= 0 && j < n ? (int)j : -1;
-                    cnt += __popc(__ballot_sync(0xffffffffu, jj[q] >= 0));
-                }
-                if (lane == 0) s_count[warp] = cnt;
-                named_bar_sync(1, T3_A_WARPS * 32);         // also: nobody reads the last segment's list any more
-                int at = 0, pairs = 0;
-#pragma unroll
-                for (int q = 0; q < T3_A_WARPS; ++q) {
-                    at += q < warp ? s_count[q] : 0;
-                    pairs += s_count[q];
-                }
-                if (tid == 0) s_pairs = pairs;
-                if (tid < STAGE_K && pairs + tid < (pairs + STAGE_K - 1) / STAGE_K * STAGE_K) s_pair[pairs + tid] = make_int2(-1, -1);
-#pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    const unsigned m = __ballot_sync(0xffffffffu, jj[q] >= 0);
-                    if (jj[q] >= 0) s_pair[at + __popc(m & ((1u << lane) - 1u))] = make_int2((int)(seg + warp * eighth + q * 32 + lane), jj[q]);
-                    at += __popc(m);
-                }
-                named_bar_sync(1, T3_A_WARPS * 32);
-            }
+            t3_list_pairs(s_pair, s_count, &s_pairs, nbr, seg, i_end, n, kk, tap, tpb);
             if (!alive) continue;
             const int steps = (s_pairs + STAGE_K - 1) / STAGE_K;
             if (steps > 0) {
@@ -737,10 +832,16 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
             uint32_t f[4];
             t3_unpack(t3_mul(sum[2 * c], T3_DOWN), f[0], f[1]);
             t3_unpack(t3_mul(sum[2 * c + 1], T3_DOWN), f[2], f[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) again = again || !t3_finite(__uint_as_float(f[e]));
             t3_sts16(dst + c * (TILE_M + 1) * 16, f);
         }
     }
-    __syncthreads();
+    if (__syncthreads_or(again) && *s_abort == 0) {
+        if (warp < T3_A_WARPS)
+            t3_redo_wgrad(reinterpret_cast<float*>(smem), s_pair, s_count, &s_pairs, gy, x, nbr, i_begin, i_end, n, m0, n0, cin, cout, kk, tap, tpb);
+        __syncthreads();
+    }
     if (*s_abort == 0) {
         const float4* sums = reinterpret_cast<const float4*>(smem);
         float* to = ws_w + (((long)range * kk + tap) * cin + m0) * cout + n0;
@@ -759,27 +860,10 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
     }
 }
 
-// gw[k][ci][co] (k < kk) or gb[co] (k == kk) from the fp32 values
-__device__ __noinline__ float t3_pair_sum(const float* gy, const float* x, const int32_t* nbr, int k, int ci, int co, long n, int cin,
-                                          int cout, int kk, int tpb) {
-    float s = 0.f;
-    for (long i = 0; i < n && s == s; ++i) {
-        if (k == kk) {
-            s += __ldg(gy + i * cout + co);
-            continue;
-        }
-        const int raw = __ldg(nbr + i * kk + k);
-        const long j = (long)raw + (tpb > 0 ? (i / tpb) * (long)tpb : 0);
-        if (raw >= 0 && j < n) s = fmaf(__ldg(x + j * cin + ci), __ldg(gy + i * cout + co), s);
-    }
-    return s;
-}
-
 // fixed-order sum of the ranges' partials, four elements per thread; the bias gradient behind the weights
 __global__ void __launch_bounds__(128)
 wgrad_f32_tc_sum_kernel(const float* __restrict__ ws_w, const float* __restrict__ ws_b, T3Units u, float* __restrict__ gw,
-                        float* __restrict__ gb, const float* __restrict__ gy, const float* __restrict__ x,
-                        const int32_t* __restrict__ nbr, long n, int cin, int cout, int kk, int tpb) {
+                        float* __restrict__ gb, int cin, int cout, int kk) {
     pdl_wait();
     pdl_trigger();
     const long n_w = (long)kk * cin * cout;
@@ -787,16 +871,13 @@ wgrad_f32_tc_sum_kernel(const float* __restrict__ ws_w, const float* __restrict_
     const float* src = ws_w;
     float* dst = gw;
     long stride = n_w;
-    int k = kk, ci = 0, ranges = u.bias;
+    int ranges = u.bias;
     if (e >= n_w) {
         e -= n_w;
         if (gb == nullptr || e >= cout) return;
         src = ws_b; dst = gb; stride = cout;
     } else {
-        const long row = e / cout;
-        k = (int)(row / cin);
-        ci = (int)(row - (long)k * cin);
-        ranges = k == u.centre ? u.own : u.others;
+        ranges = e / ((long)cin * cout) == u.centre ? u.own : u.others;
     }
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
@@ -804,10 +885,6 @@ wgrad_f32_tc_sum_kernel(const float* __restrict__ ws_w, const float* __restrict_
         const float4 v = __ldcg(reinterpret_cast<const float4*>(src + q * stride + e));
         s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
-    float* f = reinterpret_cast<float*>(&s);
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-        if (!t3_finite(f[c])) f[c] = t3_pair_sum(gy, x, nbr, k, ci, (int)(e % cout) + c, n, cin, cout, kk, tpb);
     *reinterpret_cast<float4*>(dst + e) = s;
 }
 
@@ -893,7 +970,7 @@ int f32_tc_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, vo
                        cin, cout, kk, tpb, u, tc_error_ptr()));
     const long quads = ((long)kk * cin * cout + (gb ? cout : 0)) / 4;
     SV_CUDA(launch_pdl(wgrad_f32_tc_sum_kernel, dim3((unsigned)((quads + 127) / 128)), dim3(128), 0, s, 1, ws_w, ws_b, u, (float*)gw,
-                       (float*)gb, (const float*)gy, (const float*)x, nbr, (long)n, cin, cout, kk, tpb));
+                       (float*)gb, cin, cout, kk));
     return SVTAD_OK;
 }
 

@@ -139,3 +139,48 @@ def test_values_beyond_the_planes(where, value, n):
         # finite sums: as above, but for the size of the largest product of their own that a fp32 sum is rounded at
         err = (a[ok].double() - e[ok].double()).abs() / e[ok].double().abs().clamp_min(1.0)
         assert err.max() < 1e-4, (name, err.max())
+
+
+def test_sums_beyond_the_scaled_range_are_those_of_the_fp32_values():
+    """2^16 times each value: sums above 2^96 leave fp32's range before they are brought back, and are made again."""
+    n = 9000                                # several lists per range of tokens
+    table = _chain(n, 9, 0.3, 2)
+    x, w, b, gy = make_conv_inputs(n, 8, 12, 3, torch.float32, 2)
+    x, w, gy = x * 2.0 ** 62, w * 2.0 ** 45, gy * 2.0 ** 50
+    x[n // 2] *= 2.0 ** -62                 # rows of one tile on both sides of the line
+    got, truth = _run(table, x, w, b, gy), _truth(table, x, w, b, gy)
+    _close(got[:3], truth[:3])
+
+
+def test_infinities_cost_a_small_multiple_of_an_ordinary_call():
+    """One value, a row, all of them: 5 to 7 times an ordinary call's time were measured, 20 to 450 with a thread per element."""
+    ops = _ops()
+    n, c = 4720, 192
+    table = _chain(n, 9, 0.2, 1).cuda()
+    plain = [t.cuda() for t in make_conv_inputs(n, c, c, 3, torch.float32, 1)]
+
+    def times(x, w, gy):
+        out = []
+        for f in (lambda: ops.conv_fwd(x, table, w), lambda: ops.conv_dgrad(gy, table, w, assume_symmetric=True),
+                  lambda: ops.conv_wgrad(gy, x, table, 9)):
+            best = 1e9
+            for _ in range(5):
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record()
+                for _ in range(8):
+                    f()
+                b.record()
+                b.synchronize()
+                best = min(best, a.elapsed_time(b))
+            out.append(best)
+        return out
+
+    ordinary = times(plain[0], plain[1], plain[3])
+    for where in ("one", "row", "all"):
+        x, w, gy = plain[0].clone(), plain[1].clone(), plain[3].clone()
+        for t in (x, gy):
+            t.view(-1)[{"one": slice(5000, 5001), "row": slice(5 * c, 6 * c), "all": slice(None)}[where]] = float("inf")
+        if where == "one":
+            w.view(-1)[5000] = float("inf")
+        for ours, usual in zip(times(x, w, gy), ordinary):
+            assert ours < 14 * usual, (where, ours, usual)

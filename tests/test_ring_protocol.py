@@ -78,13 +78,14 @@ def test_warps_that_list_pairs_meet_at_every_segment_whoever_gave_up():
     """The fp32 weight gradient's producers (conv_f32_tc.cu) list each segment's pairs between two barriers of all eight warps,
     which have no limit: a warp whose wait gave up may not miss one.  Reads the order of the steps."""
     text = _source("conv_f32_tc.cu")
-    loop = text[text.index("for (long seg = i_begin;"):text.index("// one more round, which carries nothing: the end")]
-    assert "alive" not in loop[:loop.index("{")]
-    first = loop.index("named_bar_sync(1, T3_A_WARPS * 32);")
-    second = loop.index("named_bar_sync(1, T3_A_WARPS * 32);", first + 1)
-    for leaves in ("break", "continue", "return", "alive"):
-        assert leaves not in loop[loop.index("{"):second], leaves
-    assert second < loop.index("if (!alive) continue;") < loop.index("mbar_wait_warp(")
+    lists = text[text.index("__device__ __forceinline__ void t3_list_pairs("):]
+    lists = lists[:lists.index("\n}\n")]
+    assert lists.count("named_bar_sync(1, T3_A_WARPS * 32);") == 2
+    assert not any(leaves in lists for leaves in ("break", "continue", "return"))
+    loop = text[text.index("// one more round, which carries nothing: the end") - 3000:text.index("// one more round, which carries nothing: the end")]
+    loop = loop[loop.index("for (long seg = i_begin;"):]
+    assert "alive" not in loop[:loop.index("t3_list_pairs(")]
+    assert loop.index("t3_list_pairs(") < loop.index("if (!alive) continue;") < loop.index("mbar_wait_warp(")
 
 
 def test_no_warp_wide_step_behind_a_wait_of_single_lanes():
