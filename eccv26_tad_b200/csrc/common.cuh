@@ -65,7 +65,7 @@ size_t f32_wgrad_ws_bytes(int64_t n, int cin, int cout, int kk);
 int forced_path();              // SVTAD_FORCE_PATH: 0 = automatic, 1 = CUDA-core kernels, 2 = tensor-core kernels
 
 // fp32 kernels on the tensor cores (conv_f32_tc.cu)
-bool f32_tc_wanted(int op, int64_t n, int cin, int cout);
+bool f32_tc_wanted(int op, int64_t n, int cin, int cout, int kk);
 int f32_tc_fwd(const ConvArgs& p, cudaStream_t s);
 int f32_tc_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s);
 int f32_tc_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void* gb, int64_t n, int cin, int cout, int kk,

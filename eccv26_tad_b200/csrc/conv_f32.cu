@@ -545,13 +545,13 @@ bool f32_supported(int cin, int cout, int kk, int dtype) {
     return dtype == SVTAD_F32 && cin % 4 == 0 && cout % 4 == 0 && kk <= F_MAX_KK;
 }
 
-static bool use_f32_tc(int op, int64_t n, int cin, int cout) { return forced_path() != 1 && f32_tc_wanted(op, n, cin, cout); }
+static bool use_f32_tc(int op, int64_t n, int cin, int cout, int kk) { return forced_path() != 1 && f32_tc_wanted(op, n, cin, cout, kk); }
 
 int f32_fwd(const ConvArgs& p, cudaStream_t s) {
-    return use_f32_tc(SVTAD_OP_FWD, p.n, p.cin, p.cout) ? f32_tc_fwd(p, s) : dispatch_conv_f32<false>(p, nullptr, s);
+    return use_f32_tc(SVTAD_OP_FWD, p.n, p.cin, p.cout, p.kk) ? f32_tc_fwd(p, s) : dispatch_conv_f32<false>(p, nullptr, s);
 }
 int f32_dgrad(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
-    return use_f32_tc(SVTAD_OP_DGRAD, p.n, p.cin, p.cout) ? f32_tc_dgrad(p, status, s) : dispatch_conv_f32<true>(p, status, s);
+    return use_f32_tc(SVTAD_OP_DGRAD, p.n, p.cin, p.cout, p.kk) ? f32_tc_dgrad(p, status, s) : dispatch_conv_f32<true>(p, status, s);
 }
 
 // Token ranges: about two full loads of the GPU (four CTAs an SM), so that the centre tap's CTAs, which have every token
@@ -580,7 +580,7 @@ int f32_wgrad(const void* gy, const void* x, const int32_t* nbr, void* gw, void*
     const long n_w = (long)kk * cin * cout, rows = (n + splits - 1) / splits;
     float* ws_w = static_cast<float*>(ws);
     float* ws_b = reinterpret_cast<float*>(static_cast<char*>(ws) + align_up((size_t)splits * n_w * sizeof(float), 256));
-    if (use_f32_tc(SVTAD_OP_WGRAD, n, cin, cout)) return f32_tc_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tpb, ws_w, ws_b, splits, s);
+    if (use_f32_tc(SVTAD_OP_WGRAD, n, cin, cout, kk)) return f32_tc_wgrad(gy, x, nbr, gw, gb, n, cin, cout, kk, tpb, ws_w, ws_b, splits, s);
     static std::atomic<uint64_t> ready{0};
     int rc = f32_allow_smem(reinterpret_cast<const void*>(wgrad_f32_kernel), sizeof(WgradSmem), ready);
     if (rc) return rc;

@@ -280,6 +280,33 @@ __device__ __noinline__ void t3_redo(float* out, const float* const* s_row, cons
     }
 }
 
+// A walk over a tile's K steps, (tap, 64 channels), the taps ascending; SKIP: those of a mask alone
+template <bool SKIP>
+struct T3Steps {
+    uint64_t left;                         // SKIP: the current tap is the lowest bit
+    int k, c0;
+    __device__ __forceinline__ T3Steps(uint64_t taps, int st, int chunks) {
+        k = st / chunks;
+        c0 = (st - k * chunks) * STAGE_K;
+        if constexpr (SKIP) {
+            left = taps;
+            for (; k > 0; --k) left &= left - 1;
+            k = __ffsll((long long)left) - 1;
+        }
+    }
+    __device__ __forceinline__ void next(int cred) {
+        c0 += STAGE_K;
+        if (c0 < cred) return;
+        c0 = 0;
+        if constexpr (SKIP) {
+            left &= left - 1;
+            k = __ffsll((long long)left) - 1;
+        } else {
+            ++k;
+        }
+    }
+};
+
 // ---------------------------------------------------------------------------------------------
 // forward / input gradient: a CTA per 128 rows x 64 columns; K steps are (tap, 64 channels)
 // ---------------------------------------------------------------------------------------------
@@ -288,8 +315,10 @@ __device__ __noinline__ void t3_redo(float* out, const float* const* s_row, cons
 // The weights' tiles come as fp32 through TMA, several steps ahead: every CTA reads each of them once, from L2, while most gathered
 // rows are found in L1 again by the taps that follow.  Loaded to registers one step ahead they were what the warps waited for:
 // 784 rows, C = 192: 12.2 -> 11.1 us, 4 720 rows: 28.8 -> 28.0, input gradient 28.2 -> 26.4, 80 rows, C = 1024: 31.3 -> 25.5.
+// SKIP: taps that none of the tile's rows has a neighbor at are left out.  With few rows that may be most of them (8 rows, C = 192,
+// four tokens a slice, 7 x 7: 23.4 -> 12.3 us), with more hardly one, and finding out costs 0.25 us and the loop 1 to 2 %: up to 64 rows.
 // SPLIT: a cluster of G CTAs shares the tile's K steps; the sums meet in shared memory, in the order of the CTAs.
-template <bool DGRAD, bool SPLIT, bool FULL>
+template <bool DGRAD, bool SPLIT, bool FULL, bool SKIP>
 __global__ void __launch_bounds__(T3_FW_THREADS, 1)
 conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __restrict__ a, const int32_t* __restrict__ nbr, const float* __restrict__ w,
                    const float* __restrict__ bias, float* __restrict__ out, const int32_t* __restrict__ status, long n, int cred,
@@ -302,11 +331,12 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t stage_base = smem_u32(smem), raw_base = stage_base + T3_RING * T3_B_STAGE;
     __shared__ uint64_t s_raw_full[T3_RAWS], s_raw_empty[T3_RAWS];
+    __shared__ uint32_t s_taps[2][T3_FW_THREADS / 32];         // SKIP: per warp, the taps of the neighbors it has seen
     const int share = SPLIT ? (int)blockIdx.x % G : 0, item = SPLIT ? (int)blockIdx.x / G : (int)blockIdx.x;
     const long row0 = (long)(item / n_blks) * TILE_M;
     const int n0 = item % n_blks * T3_BN;
-    const int chunks = (cred + STAGE_K - 1) / STAGE_K, total = kk * chunks;
-    const int k_lo = SPLIT ? total * share / G : 0, k_hi = SPLIT ? total * (share + 1) / G : total;
+    const int chunks = (cred + STAGE_K - 1) / STAGE_K;
+    int total = kk * chunks, k_lo = SPLIT ? total * share / G : 0, k_hi = SPLIT ? total * (share + 1) / G : total;
 
     if (warp == T3_A_WARPS) {
         tmem_alloc(smem_u32(&tail->tmem_slot), 512);
@@ -338,11 +368,21 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
     {
         const int32_t* rows = nbr + row0 * kk;
         const int valid = (int)(n - row0 < TILE_M ? n - row0 : TILE_M) * kk;
+        uint64_t mine = 0;
         for (int e = tid; e < TILE_M * kk; e += T3_FW_THREADS) {
             const int r = e / kk, k = e - r * kk;
             const int raw = e < valid ? __ldg(rows + e) : -1;
             const long j = (long)raw + (tpb > 0 ? ((row0 + r) / tpb) * (long)tpb : 0);
-            s_row[k * TILE_M + r] = raw >= 0 && j < n ? a + j * cred : t3_zeros;
+            const bool there = raw >= 0 && j < n;
+            s_row[k * TILE_M + r] = there ? a + j * cred : t3_zeros;
+            if (SKIP && there) mine |= 1ull << k;
+        }
+        if constexpr (SKIP) {
+            const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)mine), hi = __reduce_or_sync(0xffffffffu, (uint32_t)(mine >> 32));
+            if (lane == 0) {
+                s_taps[0][warp] = lo;
+                s_taps[1][warp] = hi;
+            }
         }
     }
     tc_fence_before();
@@ -350,6 +390,14 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
     tc_fence_after();
     const uint32_t tmem_base = tail->tmem_slot;
     pdl_trigger();
+    uint64_t taps = 0;
+    if constexpr (SKIP) {
+        taps = (uint64_t)__reduce_or_sync(0xffffffffu, lane < T3_FW_THREADS / 32 ? s_taps[1][lane] : 0u) << 32 |
+               __reduce_or_sync(0xffffffffu, lane < T3_FW_THREADS / 32 ? s_taps[0][lane] : 0u);
+        total = __popcll(taps) * chunks;
+        k_lo = SPLIT ? total * share / G : 0;
+        k_hi = SPLIT ? total * (share + 1) / G : total;
+    }
 
     t3_pair sum[T3_BN / 2];
     const int q = warp & 3;
@@ -373,14 +421,14 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
         }
         const uint32_t b_next = DGRAD ? 4 * 128 : 16 * 128;       // rows of the second four
         float va[2][2][8];
-        int k = k_lo / chunks, c0 = (k_lo - k * chunks) * STAGE_K;
+        T3Steps<SKIP> at(taps, k_lo, chunks);
         const float* const* my_row = s_row + r16;
         auto load_a = [&] {
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-                const float* row = my_row[k * TILE_M + 8 * r] + c0 + c8;
+                const float* row = my_row[at.k * TILE_M + 8 * r] + at.c0 + c8;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) t3_load8<FULL>(va[r][h], row + 32 * h, c0 + c8 + 32 * h < cred, c0 + c8 + 32 * h + 4 < cred);
+                for (int h = 0; h < 2; ++h) t3_load8<FULL>(va[r][h], row + 32 * h, at.c0 + c8 + 32 * h < cred, at.c0 + c8 + 32 * h + 4 < cred);
             }
         };
         if (k_lo < k_hi) load_a();
@@ -400,10 +448,7 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
                         for (int e = 0; e < 4; ++e) pa[q][8 * h + 4 * (e >> 1) + 2 * r + (e & 1)] = p[q][e];
                 }
             // the next step's loads are on their way while this one is multiplied; behind the last step this one's again
-            if (st + 1 < k_hi) {
-                c0 += STAGE_K;
-                if (c0 >= cred) { c0 = 0; ++k; }
-            }
+            if (st + 1 < k_hi) at.next(cred);
             load_a();
             if (!mbar_wait_warp(smem_u32(&tail->empty[s]), ph, s_abort, err, 71)) break;
             tc_fence_after();
@@ -460,7 +505,8 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
     } else if (warp == T3_A_WARPS + 1 + T3_E_WARPS) {
         // ------------------------------------------------------------------ weights: fp32 tiles, T3_RAWS steps ahead
         if (lane == 0) {
-            int k = k_lo / chunks, c0 = (k_lo - k * chunks) * STAGE_K, rs = 0;
+            T3Steps<SKIP> at(taps, k_lo, chunks);
+            int rs = 0;
             uint32_t ph = 1;
             for (int st = k_lo; st < k_hi; ++st) {
                 if (!mbar_wait(smem_u32(&s_raw_empty[rs]), ph, s_abort, err, 80)) break;
@@ -468,9 +514,8 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
                 mbar_expect_tx(bar, T3_RAW);
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
-                    tma_load_3d(dst + h * (T3_RAW / 2), &map_w, (DGRAD ? c0 : n0) + 32 * h, DGRAD ? n0 : c0, DGRAD ? kk - 1 - k : k, bar);
-                c0 += STAGE_K;
-                if (c0 >= cred) { c0 = 0; ++k; }
+                    tma_load_3d(dst + h * (T3_RAW / 2), &map_w, (DGRAD ? at.c0 : n0) + 32 * h, DGRAD ? n0 : at.c0, DGRAD ? kk - 1 - at.k : at.k, bar);
+                at.next(cred);
                 if (++rs == T3_RAWS) { rs = 0; ph ^= 1u; }
             }
         }
@@ -896,14 +941,14 @@ static bool t3_full(int cin, int cout, const void* a, const void* b) {
     return cin % STAGE_K == 0 && cout % STAGE_K == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 31) == 0;
 }
 
-template <bool DGRAD, bool SPLIT, bool FULL>
+template <bool DGRAD, bool SPLIT, bool FULL, bool SKIP>
 static int launch_f32_tc(const ConvArgs& p, const int32_t* status, int G, cudaStream_t s) {
     const int cn = DGRAD ? p.cin : p.cout, cred = DGRAD ? p.cout : p.cin;
     const size_t table = (size_t)p.kk * TILE_M * sizeof(float*);
     const int n_blks = (cn + T3_BN - 1) / T3_BN;
     const long tiles = (p.n + TILE_M - 1) / TILE_M * n_blks;
     const size_t smem = 1024 + T3_RING * T3_B_STAGE + T3_RAWS * T3_RAW + sizeof(TmaTail) + table;
-    auto kern = conv_f32_tc_kernel<DGRAD, SPLIT, FULL>;
+    auto kern = conv_f32_tc_kernel<DGRAD, SPLIT, FULL, SKIP>;
     int rc = tc_ensure_smem(reinterpret_cast<const void*>(kern), smem);
     if (rc) return rc;
     CUtensorMap map_w;
@@ -932,15 +977,26 @@ static int dispatch_f32_tc(const ConvArgs& p, const int32_t* status, cudaStream_
         if (u < best) { best = u; G = sizes[g]; }
     }
     const bool full = t3_full(p.cin, p.cout, p.a, p.w);
-    if (G > 1) return full ? launch_f32_tc<DGRAD, true, true>(p, status, G, s) : launch_f32_tc<DGRAD, true, false>(p, status, G, s);
-    return full ? launch_f32_tc<DGRAD, false, true>(p, status, 1, s) : launch_f32_tc<DGRAD, false, false>(p, status, 1, s);
+    if (G == 1) return full ? launch_f32_tc<DGRAD, false, true, false>(p, status, 1, s) : launch_f32_tc<DGRAD, false, false, false>(p, status, 1, s);
+    if (p.n <= 64) return full ? launch_f32_tc<DGRAD, true, true, true>(p, status, G, s) : launch_f32_tc<DGRAD, true, false, true>(p, status, G, s);
+    return full ? launch_f32_tc<DGRAD, true, true, false>(p, status, G, s) : launch_f32_tc<DGRAD, true, false, false>(p, status, G, s);
 }
 
-// Forward and input gradient win at every size measured (59 rows, 16 -> 16 channels: 8.6 -> 8.3 us; 1024 -> 1024: 57 -> 26).  The
-// weight gradient has a fixed cost of 6 us per CTA: 118 rows, C = 192: 8.7 and 10.0 us; 472: 12.2 and 11.5, 128 -> 128 9.6 and 10.0,
-// 64 -> 1024 15.2 and 19.1; 708: 13.9 and 11.4, 13.0 and 10.3, 21.3 and 20.9.
-bool f32_tc_wanted(int op, int64_t n, int cin, int cout) {
-    return (op == SVTAD_OP_WGRAD ? n >= 640 : n > 0) && cin <= T3_MOST && cout <= T3_MOST;
+// Where these kernels take over from those on the CUDA cores, us there and here.  Forward and input gradient from four rows on: 1
+// row, C = 192, 3 x 3: 6.2 and 6.9; 8 rows, one neighbor in nine / five / all: 6.4 and 7.1 / 10.1 and 8.9 / 10.7 and 9.7; 96 rows, C = 512:
+// 32.2 and 13.6 at one in four, 39.5 and 14.1 at all.  (Above 64 rows a table in which hardly a row has any neighbor is the exception: 96
+// rows, C = 512, none: 10.1 and 13.8.)
+// The weight gradient has 7 us per CTA whatever it holds, one CTA an SM, and cuts its tokens for one pair in three tokens.  So it
+// loses where there is little to do, mostly on full tables (64 -> 64, 3 x 3, density 0.15 / 0.95: 1 100 rows 9.8 and 9.5 / 9.8 and
+// 12.9, 2 400 rows 12.4 and 11.3 / 15.1 and 14.8), and where many CTAs have few pairs each, as with wide
+// stencils (density 0.15: 800 rows, C = 512, 5 x 5: 64 and 66, 7 x 7: 105 and 125; 1 100 rows: 85 and 70, 140 and 133; at density 0.3 it
+// wins at 640; C = 1024, 3 x 3, 640 rows, density 0.2 / 0.4: 91 and 96 / 131 and 109).
+bool f32_tc_wanted(int op, int64_t n, int cin, int cout, int kk) {
+    if (cin > T3_MOST || cout > T3_MOST) return false;
+    if (op != SVTAD_OP_WGRAD) return n >= 4 || (n > 0 && kk == 1);
+    const double work = (double)n * kk * ((cin + 63) / 64 * 64) * ((cout + 63) / 64 * 64);
+    const long ctas = (long)kk * ((cin + TILE_M - 1) / TILE_M) * ((cout + T3_BN - 1) / T3_BN);
+    return n >= (kk > 9 && ctas > 600 ? 900 : 640) && (n >= 2600 || work >= 7e7);
 }
 
 int f32_tc_fwd(const ConvArgs& p, cudaStream_t s) { return dispatch_f32_tc<false>(p, nullptr, s); }

@@ -81,6 +81,25 @@ def test_edges_of_tiles_chunks_and_lists(n, cin, cout, kk):
     _close(_run(table, x, w, b, gy), _truth(table, x, w, b, gy))
 
 
+@pytest.mark.parametrize("n,kk,density", [(n, kk, d) for n in (3, 4, 8, 64, 65) for kk, d in ((9, 0.0), (49, 0.03), (49, 1.0))])
+def test_taps_without_a_neighbor_are_left_out_of_few_rows(n, kk, density):
+    table = _chain(n, kk, density, n)
+    x, w, b, gy = make_conv_inputs(n, 192, 68, int(kk ** 0.5), torch.float32, n, bias="random")
+    _close(_run(table, x, w, b, gy), _truth(table, x, w, b, gy))
+    if n == 64:                 # nothing at all: the bias, and zeros
+        table[:] = -1
+        y, gx, gw, gb = _run(table, x, w, b, gy)
+        assert torch.equal(y, b.expand(n, -1)) and not gx.any() and not gw.any()
+
+
+@pytest.mark.parametrize("n,cin,cout,kk", [(1898, 64, 64, 9), (1899, 64, 64, 9), (2599, 16, 20, 9), (2600, 16, 20, 9),
+                                           (899, 64, 1024, 49), (900, 64, 1024, 49)])
+def test_both_sides_of_the_weight_gradient_s_rule(n, cin, cout, kk):
+    table = _chain(n, kk, 0.2, n)
+    x, w, b, gy = make_conv_inputs(n, cin, cout, int(kk ** 0.5), torch.float32, n, bias="random")
+    _close(_run(table, x, w, b, gy), _truth(table, x, w, b, gy))
+
+
 def test_rows_that_are_16_but_not_32_byte_aligned_and_batch_local_indices():
     n, c = 900, 64
     table = _chain(n // 3, 9, 0.5, 3).repeat(3, 1)
@@ -184,3 +203,34 @@ def test_infinities_cost_a_small_multiple_of_an_ordinary_call():
             w.view(-1)[5000] = float("inf")
         for ours, usual in zip(times(x, w, gy), ordinary):
             assert ours < 14 * usual, (where, ours, usual)
+
+
+@pytest.mark.parametrize("what,n,cin,cout,kk,density", [("fwd", 8, 512, 512, 49, 0.0), ("dgrad", 32, 512, 512, 49, 0.0),
+                                                        ("wgrad", 800, 64, 1024, 49, 0.05), ("wgrad", 1100, 64, 64, 9, 1.0)])
+def test_the_tensor_cores_do_not_take_what_the_cuda_cores_do_faster(what, n, cin, cout, kk, density, monkeypatch):
+    """Few rows without neighbors (2.3 to 2.9 times the time with every tap worked through), weight gradients of many CTAs with
+    few pairs each (1.5 times) or of little work on a full table (1.3 times)."""
+    ops = _ops()
+    table = _chain(n, kk, density, n).cuda()
+    x, w, _, gy = (t.cuda() for t in make_conv_inputs(n, cin, cout, int(kk ** 0.5), torch.float32, n))
+    f = {"fwd": lambda: ops.conv_fwd(x, table, w), "dgrad": lambda: ops.conv_dgrad(gy, table, w, assume_symmetric=True),
+         "wgrad": lambda: ops.conv_wgrad(gy, x, table, kk)}[what]
+
+    def time(path):
+        monkeypatch.setenv("SVTAD_FORCE_PATH", path)
+        f()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                f()
+        best = 1e9
+        for _ in range(10):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            graph.replay()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    assert time("") < 1.2 * time("simt")
