@@ -450,12 +450,12 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
             // the next step's loads are on their way while this one is multiplied; behind the last step this one's again
             if (st + 1 < k_hi) at.next(cred);
             load_a();
-            if (!mbar_wait_warp(smem_u32(&tail->empty[s]), ph, s_abort, err, 71)) break;
+            if (!mbar_wait_warp(smem_u32(&tail->empty[s]), ph, s_abort, err, 81)) break;
             tc_fence_after();
 #pragma unroll
             for (int q = 0; q < 3; ++q) t3_tmem_st(a_addr + s * T3_A_COLS + q * 32, pa[q]);
             const uint32_t b_tile = stage_base + s * T3_B_STAGE + b_place;
-            if (!mbar_wait_warp(smem_u32(&s_raw_full[rs]), rph, s_abort, err, 79)) break;
+            if (!mbar_wait_warp(smem_u32(&s_raw_full[rs]), rph, s_abort, err, 89)) break;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 // rows b_row and b_row + 4: the second one's chunks lie across the swizzle
@@ -491,8 +491,8 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
         uint32_t ph = 0;
         for (int st = 0; st < k_hi - k_lo; ++st) {
             const int buf = st & 1;
-            const bool ok = mbar_wait(smem_u32(&tail->accum_empty[buf]), ((st >> 1) & 1) ^ 1, s_abort, err, 72) &&
-                            mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 73);
+            const bool ok = mbar_wait(smem_u32(&tail->accum_empty[buf]), ((st >> 1) & 1) ^ 1, s_abort, err, 82) &&
+                            mbar_wait(smem_u32(&tail->full[s]), ph, s_abort, err, 83);
             tc_fence_after();
             if (elect_one_sync()) {
                 t3_issue_ts<!DGRAD>(tmem_base + buf * (2 * T3_BN), tmem_base + T3_A_COL + s * T3_A_COLS, stage_base + s * T3_B_STAGE);
@@ -509,7 +509,7 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
             int rs = 0;
             uint32_t ph = 1;
             for (int st = k_lo; st < k_hi; ++st) {
-                if (!mbar_wait(smem_u32(&s_raw_empty[rs]), ph, s_abort, err, 80)) break;
+                if (!mbar_wait(smem_u32(&s_raw_empty[rs]), ph, s_abort, err, 90)) break;
                 const uint32_t bar = smem_u32(&s_raw_full[rs]), dst = raw_base + rs * T3_RAW;
                 mbar_expect_tx(bar, T3_RAW);
 #pragma unroll
@@ -527,7 +527,7 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
         const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
         for (int st = 0; st < k_hi - k_lo; ++st) {
             const int buf = st & 1;
-            if (!mbar_wait_warp(smem_u32(&tail->accum_full[buf]), (st >> 1) & 1, s_abort, err, 74)) break;
+            if (!mbar_wait_warp(smem_u32(&tail->accum_full[buf]), (st >> 1) & 1, s_abort, err, 84)) break;
             tc_fence_after();
             t3_drain<2>(sum, t_addr + buf * (2 * T3_BN));
             tc_fence_before();
@@ -812,7 +812,7 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
                     if (it >= A_ITS || real) load(0, it);
             }
             for (int st = 0; st < steps; ++st) {
-                if (!mbar_wait_warp(smem_u32(&tail->empty[s]), ph, s_abort, err, 75)) { alive = false; break; }
+                if (!mbar_wait_warp(smem_u32(&tail->empty[s]), ph, s_abort, err, 85)) { alive = false; break; }
                 const uint32_t a_rows = stage_base + s * T3_STAGE + warp * (A_ITS * 512), b_rows = stage_base + s * T3_STAGE + 3 * T3_A_PLANE + b_tok * 128;
                 const int next = st + 1 < steps ? st + 1 : st;
                 if (real) {
@@ -833,7 +833,7 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
             done += steps;
         }
         // one more round, which carries nothing: the end
-        if (alive && mbar_wait_warp(smem_u32(&tail->empty[s]), ph, s_abort, err, 75)) {
+        if (alive && mbar_wait_warp(smem_u32(&tail->empty[s]), ph, s_abort, err, 85)) {
             if (tid == 0) s_end = done;
             t3_filled(smem_u32(&tail->full[s]), lane);
         }
@@ -841,8 +841,8 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
         // ------------------------------------------------------------------ MMA issuer (whole warp waits, one lane issues)
         for (int g = 0;; ++g) {
             const int s = g % T3_RING, buf = g & 1;
-            const bool ok = mbar_wait(smem_u32(&tail->accum_empty[buf]), ((g >> 1) & 1) ^ 1, s_abort, err, 76) &&
-                            mbar_wait(smem_u32(&tail->full[s]), g / T3_RING & 1, s_abort, err, 77);
+            const bool ok = mbar_wait(smem_u32(&tail->accum_empty[buf]), ((g >> 1) & 1) ^ 1, s_abort, err, 86) &&
+                            mbar_wait(smem_u32(&tail->full[s]), g / T3_RING & 1, s_abort, err, 87);
             const bool end = *reinterpret_cast<volatile int*>(&s_end) == g;
             __syncwarp();
             tc_fence_after();
@@ -863,7 +863,7 @@ wgrad_f32_tc_kernel(const float* __restrict__ gy, const float* __restrict__ x, c
         const uint32_t t_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
         for (int g = 0;; ++g) {
             const int buf = g & 1;
-            if (!mbar_wait_warp(smem_u32(&tail->accum_full[buf]), (g >> 1) & 1, s_abort, err, 78)) break;
+            if (!mbar_wait_warp(smem_u32(&tail->accum_full[buf]), (g >> 1) & 1, s_abort, err, 88)) break;
             if (*reinterpret_cast<volatile int*>(&s_end) == g) break;
             tc_fence_after();
             t3_drain<3>(sum, t_addr + buf * T3_COLS);

@@ -303,6 +303,7 @@ def device_error():
 
 
 def path_for(op, n, cin, cout, kk, dtype):
+    """"tc": a 16-bit tensor-core kernel.  "simt": any other, the fp32 ones among them, most of which use the tensor cores too."""
     return "tc" if _lib.load().svtad_path_for(op, n, cin, cout, kk, _DTYPES[dtype]) else "simt"
 
 

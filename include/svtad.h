@@ -281,7 +281,7 @@ int svtad_allreduce_sum_emulated(void* const* bufs, int world, int64_t n_elems, 
  * Concurrency hint (no counterpart in the reference): how many of this library's kernels the caller expects to
  * share the GPU at a time - independent layers on streams of their own, forward next to backward.  The default, 1,
  * plans every kernel for the whole GPU, which gives a kernel that runs alone its shortest latency.  With a hint of
- * k the tensor-core kernels are planned for (SMs / k) multiprocessors each: wide column blocks, persistent CTAs
+ * k the 16-bit tensor-core kernels are planned for (SMs / k) multiprocessors each: wide column blocks, persistent CTAs
  * that take several row tiles in turn, fewer token splits in the weight gradient.  Every CTA pays a few
  * microseconds of set-up, first-operand latency and epilogue whatever its share of the work, so fewer and longer
  * CTAs cost a lone kernel latency but save SM time when the SMs are contended anyway (three layers' passes in one
@@ -298,8 +298,9 @@ int svtad_get_concurrency(void);
 
 /*
  * Reads (and clears) the device-side error word of the current device: non-zero means a bounded
- * wait inside a kernel gave up and that launch's output is invalid.  Synchronises
- * the device.  No reference counterpart.
+ * wait inside a kernel gave up and that launch's output is invalid.  41 to 64: a 16-bit tensor-core
+ * kernel, 81 to 90: an fp32 one, 71 and 72: the exchange (above).  Synchronises the device.  No
+ * reference counterpart.
  */
 int svtad_device_error(int32_t* code_out);
 
@@ -312,8 +313,10 @@ int svtad_device_error(int32_t* code_out);
 int svtad_ffma_probe(int ctas, int iters, float* scratch, void* stream);
 
 /*
- * Which implementation the given problem dispatches to: 0 = CUDA-core (SIMT) kernels,
- * 1 = tcgen05 tensor-core kernels.  Honours the SVTAD_FORCE_PATH=simt|tc environment override.
+ * Which implementation the given problem dispatches to: 1 = the 16-bit tensor-core kernels, 0 = all
+ * others.  Those of fp32 are among the others although most fp32 calls run on the tensor cores too (operands as
+ * bf16 planes; the error word counts for them as well).  Honours the SVTAD_FORCE_PATH=simt|tc environment
+ * override: simt keeps every call on the CUDA cores, tc refuses what has no 16-bit tensor-core kernel.
  */
 int svtad_path_for(int op, int64_t n, int cin, int cout, int kk, int dtype);
 

@@ -115,3 +115,12 @@ def test_nothing_is_in_flight_when_a_cta_that_gave_up_leaves():
         ends = _source(name).split("tmem_dealloc")
         ends = [e for e in ends[:-1] if "tcgen05.dealloc" not in e[-200:] and "SVTAD_TABLE_ASYMMETRIC" not in e[-300:] and "void " not in e[-10:]]
         assert len(ends) == kernels and all("settle_after_abort(s_abort);" in e[-300:] for e in ends), name
+
+
+def test_the_exchange_s_error_codes_are_its_own():
+    """71 and 72 are documented as the exchange's; 81 to 90 as the fp32 kernels', 41 to 64 as the 16-bit ones'."""
+    import re
+    for name, low, high in (("conv_f32_tc.cu", 81, 90), ("conv_tc_hybrid.cu", 41, 64), ("conv_tc_pair.cu", 41, 64),
+                            ("conv_tc_pairs.cu", 41, 64), ("allreduce.cu", 71, 72)):
+        codes = {int(c) for c in re.findall(r"\berr, (\d+)\b", _source(name))}
+        assert codes and low <= min(codes) and max(codes) <= high, (name, codes)
