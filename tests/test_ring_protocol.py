@@ -122,5 +122,5 @@ def test_the_exchange_s_error_codes_are_its_own():
     import re
     for name, low, high in (("conv_f32_tc.cu", 81, 90), ("conv_tc_hybrid.cu", 41, 64), ("conv_tc_pair.cu", 41, 64),
                             ("conv_tc_pairs.cu", 41, 64), ("allreduce.cu", 71, 72)):
-        codes = {int(c) for c in re.findall(r"\berr, (\d+)\b", _source(name))}
+        codes = {int(c) for c in re.findall(r", err, (\d+)\b", _source(name))}
         assert codes and low <= min(codes) and max(codes) <= high, (name, codes)
