@@ -2,7 +2,8 @@
 // into three bf16 values.
 //
 // An fp32 value is the exact sum of three bf16 ones, x = x1 + x2 + x3 (8 + 8 + 8 bits, each the rounded rest of the ones
-// before), and a product needs six of the nine partial products: x1 w1, x1 w2, x2 w1, x1 w3, x2 w2, x3 w1; the three that
+// before; the method of G. Henry, P. T. P. Tang and A. Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For
+// Higher-Precision Computations", ARITH 2019), and a product needs six of the nine partial products: x1 w1, x1 w2, x2 w1, x1 w3, x2 w2, x3 w1; the three that
 // are left out are below 2^-26 of it.  What would spoil the result is the accumulator: tcgen05.mma cuts its sum off towards
 // zero at every instruction (measured, relative error of a sum of N(0,1) products against 64 bits: 2.4e-8 after one
 // instruction of 16 products, 6.5e-8 after 4, 1.2e-7 after 8, 4.7e-7 after 32, nearly all of it bias).  So a sum stays in
@@ -20,10 +21,10 @@
 // infinity in each operand / all infinite (a thread per sum: 1 150 and 7 430 with one): forward 27 / 164 / 200, input gradient 27 /
 // 152 / 195, weight gradient 25 / 114 / 114; the CUDA-core kernels, whatever the values, 59, 62 and 51.
 //
-// Measured (graph replays, before: the CUDA-core kernels): 784 rows, C = 192, keep 50 %: forward 21.2 -> 10.4 us, input
-// gradient 22.2 -> 10.4; 4 720 rows, C = 192, keep 30 %: 54.5 -> 25.7, 57.1 -> 25.5, weight gradient 47.8 -> 22.1; 5 880
-// rows, full grid, 320 -> 96: 144 -> 42, 134 -> 38, 103 -> 61.  What bounds the loops: eight warps that load, split and store
-// (850 issue slots per scheduler and step of 1 480 cycles; 768 cycles of tensor work) and the gathered rows' trip from L2, which is
+// Measured (graph replays, before: the CUDA-core kernels): 784 rows, C = 192, keep 50 %: forward 21.7 -> 11.0 us, input
+// gradient 22.9 -> 11.0; 4 720 rows, C = 192, keep 30 %: 55.0 -> 26.8, 58.0 -> 27.1, weight gradient 49.8 -> 22.0; 5 880
+// rows, full grid, 320 -> 96: 144 -> 44, 134 -> 40, 103 -> 57.  What bounds the loops: eight warps that load, split and store
+// (900 issue slots per scheduler and step of 1 500 cycles; 768 cycles of tensor work) and the gathered rows' trip from L2, which is
 // one step long.
 #include <cfloat>
 
@@ -535,8 +536,8 @@ conv_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const float* __res
         }
     }
     // The sums go through shared memory, those of a shared tile to the CTA that finishes their rows, so that all threads store whole
-    // lines (a lane that stores its own row takes 16 bytes of 32 lines at a time: 4 720 rows, C = 192: 28.0 us, now 25.7; with the
-    // shared sums by rows as well, 784 rows took 11.1, now 10.4).  A CTA whose wait gave up stops the whole
+    // lines (a lane that stores its own row takes 16 bytes of 32 lines at a time: 4 720 rows, C = 192: 28.0 us instead of 25.7; with
+    // the shared sums by rows as well, 784 rows took 11.1 instead of 10.4).  A CTA whose wait gave up stops the whole
     // cluster: the others' sums are not finished with what it left behind.
     __syncthreads();
     if constexpr (SPLIT) {
