@@ -404,9 +404,10 @@ bool tc_supported(int op, int64_t n, int cin, int cout, int kk, int dtype) {
 // its K steps are shorter; it starts later, and single CTAs may take narrower column blocks to fill the machine.  Times as
 // measured on a B200 (us; rows, layer: pair, single): 18 880, 256 -> 256, 5x5: 40.9, 43.2; 14 160, 384, 5x5: 94.5, 108;
 // 9 440, 384, 5x5: 50.4, 55.9; 18 880, 192, 3x3: 15.5, 14.5; 9 440, 768, 3x3: 79.1, 74.7; 37 760, 128, 3x3: 17.4, 16.8; 23 600,
-// 256, 5x5: 74.1, 81.7; 37 760, 64, 5x5: 18.7, 18.0.  The two estimates below choose within 0.2 % of the faster one on average
-// over 326 such calls; where they are close the kernel stays that was there first (pairs from as many row tiles as SMs on).
-// A tile whose K steps a cluster shares goes to single CTAs, and under a concurrency hint only the number of tiles counts.
+// 256, 5x5: 74.1, 81.7; 37 760, 64, 5x5: 18.7, 18.0; 20 480, 1024 -> 32, 5x5: 163, 174; 9 984, 512, 7x7: 358, 266.  The two
+// estimates below choose within 0.2 % of the faster one on average over 326 such calls (3x3 and 5x5); where they are close the
+// kernel stays that was there first (pairs from as many row tiles as SMs on).  A tile whose K steps a cluster shares goes to
+// single CTAs, and under a concurrency hint only the number of tiles counts.
 // A row's sum is the same either way.  SVTAD_TC_IMPL=pair / hybrid overrides the choice.
 static TcChoice choose(int64_t n, int cred, int cn, int kk, bool dgrad) {
     const long m_tiles = (n + TILE_M - 1) / TILE_M, sms = tc_num_sms();
@@ -420,13 +421,16 @@ static TcChoice choose(int64_t n, int cred, int cn, int kk, bool dgrad) {
     if (forced) c.pair = e[0] == 'p';
     if (c.split == 1) {
         auto at = [](int bn) { return bn == 256 ? 4 : bn == 192 ? 3 : bn == 128 ? 2 : bn == 96 ? 1 : 0; };
-        const double pair_step[5] = {0.20, 0.2375, 0.2375, 0.29, 0.316}, single_step[5] = {0.19, 0.245, 0.266, 0.352, 0.366};
+        const double pair_step[5] = {0.20, 0.2375, 0.2375, 0.29, 0.316}, single_step[5] = {0.21, 0.245, 0.266, 0.352, 0.366};
         auto time = [&](double start, long items, long slots, double step) {
             const long waves = (items + slots - 1) / slots;
             return start + (double)waves * steps * step + (double)(waves - 1) * 1.7;
         };
         const int wide = tc_widest_bn(cn);
-        const double pair = time(7.0, (m_tiles + 1) / 2 * ((cn + wide - 1) / wide), sms / 2, pair_step[at(wide)]);
+        // the tables of stencils beyond 5x5 leave pairs with 256 columns room for two rounds of buffers instead of three: 0.455 us a step
+        const size_t table = 2 * (size_t)TILE_M * kk * sizeof(int) + 2048 + 512, stage = A_TILE_BYTES + (size_t)wide / 2 * 128;
+        const double ring = (TC_SMEM_LIMIT - 1024 - table) / stage < 6 ? 1.44 : 1.0;
+        const double pair = time(7.0, (m_tiles + 1) / 2 * ((cn + wide - 1) / wide), sms / 2, pair_step[at(wide)] * ring);
         const double single = time(5.2, m_tiles * ((cn + c.bn - 1) / c.bn), sms, single_step[at(c.bn)]);
         if (!forced && tc_plan_sms() == sms) c.pair = c.pair ? single >= 0.97 * pair : pair < 0.926 * single;
         c.us = pair < single ? pair : single;

@@ -652,3 +652,30 @@ def test_a_row_s_sum_does_not_hang_on_pairs_or_single_ctas(n, cin, cout, ks, dty
     assert ops.device_error() == 0
     for y, gx in outs[1:]:
         assert torch.equal(y, outs[0][0]) and torch.equal(gx, outs[0][1])
+
+
+@pytest.mark.parametrize("n,cin,cout,ks", [(9984, 512, 512, 7), (20480, 1024, 32, 5)])
+def test_pairs_or_single_ctas_by_the_faster(n, cin, cout, ks, monkeypatch):
+    """Few buffers beside a large table (single CTAs: 1.34 times the rate of pairs), a narrow output with a long reduction (pairs:
+    1.06 times)."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    table = torch.randint(-n, n, (n, ks * ks), generator=g, dtype=torch.int32, device="cuda").clamp_(min=-1)
+    x = torch.randn(n, cin, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(ks * ks, cin, cout, generator=g, device="cuda") * 0.02).bfloat16()
+
+    def time(impl):
+        monkeypatch.setenv("SVTAD_TC_IMPL", impl)
+        best = 1e9
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(4):
+                ops.conv_fwd(x, table, w)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    time("")
+    assert time("") < 1.035 * min(time("pair"), time("hybrid"))
