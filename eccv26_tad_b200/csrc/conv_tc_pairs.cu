@@ -15,6 +15,8 @@
 // Both operands are gathered rows in the MN-major 128-byte-swizzled layout (64 tokens x 64 channels = 8 KB blocks), so a
 // step of 128 x 256 copies 48 KB; what bounds the loop is the SM's path to L2 (48 KB in ~ 700 cycles against 512 cycles
 // of tensor work).
+#include <cstdlib>
+
 #include "plan.cuh"
 #include "tc_common.cuh"
 
@@ -416,9 +418,27 @@ wgrad_pairs_sum_kernel(const float* __restrict__ pieces, const int4* __restrict_
 // with the pieces' layout; C = 256, 5 x 5: 53 -> 41 us)
 static int pairs_halves(int cin) { return (cin + 255) / 256 * 256 * 8 <= cin * 9 ? 2 : 1; }
 
+// Column block of the weight gradient by pairs: blocks times what a step takes at that width, which goes nearly by the width with
+// 128 input channels a block (a step's time as a share of 256 columns': 0.38, 0.49, 0.74 at 64, 128, 192 columns) and less so with 256
+// (0.5, 0.675, 0.77); a narrower block from 3 % on.  With the other kernels' step times, 0.55, 0.67, 0.81, a width of 640 went in three
+// blocks of 256 instead of five of 128, and 960 in four of 256 instead of five of 192.  us with its sum kernel, C = 640: 14 160 rows,
+// density 0.35: 109 and 77; 26 550: 159 and 123; C = 896, 14 160 rows: 163 and 125; C = 960 (256 input channels a block): 148 and 128.
+static int pairs_bn(int cin, int cout) {
+    if (getenv("SVTAD_TC_BN") != nullptr) return tc_widest_bn(cout);
+    const int width[4] = {256, 192, 128, 64};
+    const double share[2][4] = {{1.0, 0.74, 0.49, 0.38}, {1.0, 0.77, 0.675, 0.5}};
+    int bn = 0;
+    double least = 1e30;
+    for (int i = 0; i < 4; ++i) {
+        const double t = (cout + width[i] - 1) / width[i] * share[pairs_halves(cin) - 1][i];
+        if (t < 0.97 * least) { least = t; bn = width[i]; }
+    }
+    return bn;
+}
+
 // per run two pieces and the boundary behind it
 size_t pairs_wgrad_ws_bytes(int cin, int cout) {
-    const size_t run = 2 * TILE_M * pairs_halves(cin) * tc_widest_bn(cout) * sizeof(float) + sizeof(int4);
+    const size_t run = 2 * TILE_M * pairs_halves(cin) * pairs_bn(cin, cout) * sizeof(float) + sizeof(int4);
     return (tc_num_sms() * run + 255) / 256 * 256;
 }
 
@@ -456,7 +476,7 @@ int pairs_wgrad(const void* gy, const void* x, const void* plan, void* gw, void*
     auto go = [&](auto one, auto two) {
         return (pairs_halves(cin) == 2 ? two : one)(gy, x, view, gw, gb, pieces, n, cin, cout, kk, fp16, out32, s);
     };
-    switch (tc_widest_bn(cout)) {
+    switch (pairs_bn(cin, cout)) {
         case 64: return go(launch_pairs<64, 1>, launch_pairs<64, 2>);
         case 128: return go(launch_pairs<128, 1>, launch_pairs<128, 2>);
         case 192: return go(launch_pairs<192, 1>, launch_pairs<192, 2>);

@@ -120,6 +120,18 @@ def test_planned_kernels_give_the_unplanned_results(B, T, keep, ks, cin, cout, d
     assert ops.device_error() == 0
 
 
+@pytest.mark.parametrize("cin,cout", [(640, 640), (384, 800), (512, 928), (256, 960)])
+def test_weight_gradient_in_narrower_column_blocks(cin, cout):
+    """Five and seven (the last partial) blocks of 128 columns, five of 192 (the last partial or not) instead of 256."""
+    from eccv26_tad_b200 import ops
+    table = make_table(1, 24, 14, 14, 0.3, 3, 9)[2].cuda()
+    x, w, b, gy = (t.cuda() for t in make_conv_inputs(table.shape[0], cin, cout, 3, torch.bfloat16, 9, bias="random"))
+    gw, gb = _planned(table, x, w, b, gy)[2:]
+    egw, egb = ops.conv_wgrad(gy, x, table, 9)
+    assert oconv.rel_err(f32np(gw), f32np(egw)) < 8e-3 and oconv.rel_err(f32np(gb), f32np(egb)) < 8e-3
+    assert ops.device_error() == 0
+
+
 @pytest.mark.parametrize("keep,table_kind", [(0.3, "built"), (0.5, "given"), (1.0, "given"), (1.0, "built")])
 def test_module_with_a_layer_that_wants_a_plan(keep, table_kind):
     """C = 512 at 18 880 / 31 360 / 62 720 rows: with the module's plan (a table built here that is sparse enough) and without

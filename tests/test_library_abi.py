@@ -276,6 +276,16 @@ def test_a_forward_s_row_order_is_wanted_by_the_waves_it_saves(n, cin, cout, den
     assert lib.svtad_plan_wanted_fwd(n, cin, cout, 9, _lib.F32, density) == 0
 
 
+@pytest.mark.parametrize("cin,cout,halves,bn", [(640, 640, 1, 128), (896, 896, 1, 128), (512, 960, 2, 192), (640, 1024, 1, 256),
+                                                (512, 640, 2, 256), (320, 320, 1, 192), (1024, 1024, 2, 256)])
+def test_column_block_of_a_weight_gradient_by_pairs(cin, cout, halves, bn):
+    """By what its own steps take, which shows in the pieces its workspace holds: two of 128 * halves rows and a block's columns, and
+    a record, for each of 148 CTAs."""
+    lib = _lib.load()
+    each = 2 * 128 * halves * bn * 4 + 16
+    assert lib.svtad_bwd_workspace_bytes(18880, cin, cout, 9, _lib.BF16, 2, 0) == (148 * each + 255) // 256 * 256
+
+
 def test_workspace_sizes_count_the_pair_lists_only_where_a_plan_is_used():
     """The weight gradient by pair lists parks pieces of its sums (74 MB at C = 256); a call without a plan does not."""
     lib = _lib.load()
