@@ -163,13 +163,18 @@ extern "C" int svtad_plan_wanted(int64_t n, int cin, int cout, int kk, int dtype
 //   12 960 rows, C = 512, density 0.55 (21): 56.5 -> 50.7        8 736, C = 384, 0.2 (18): 23.9 -> 28.7
 //   11 800, C = 384, 0.35 (22): 34.8 -> 33.1                     18 880, C = 320, 0.35 (21): 36.0 -> 36.3
 //   37 760, C = 320, 0.35 (40): 65.9 -> 53.1                     75 520, C = 256, 0.35 (36): 64.7 -> 67.0
-// A sweep of 104 shapes (1 920 to 75 520 rows, C = 128 to 1024) is on average 1.0 % from the better of the two; on a line by the
-// work left out (24 GFLOP + rows / 1600) 2.9 %.  Below 40 tiles the longest one decides: 4 720, C = 768, 0.55: 43.4 -> 56.2.
+// Where a CTA's share of the tiles is shorter than the longest tile, which needs every tap, that one decides: 18 940 rows, 512 ->
+// 192, density 0.19: 30.9 -> 42.1; 8 960 rows, 640 -> 256, 0.19: 30.5 -> 37.7; 4 720, C = 768, 0.55: 43.4 -> 56.2.  There the
+// order, 9 us and one per 3 200 rows, and that tile together have to be shorter than the kernel without.
+// Of 1 129 forwards of 41 to 180 tiles, 256 to 1 024 -> 128 to 1 024 channels, that the first line takes, 123 lost 3 to 27 % (1.3 %
+// from the better of the two on average), with the second 32 lose up to 17 % (0.4 %); of 926 up to 600 tiles 8 (0.07 %).
 extern "C" int svtad_plan_wanted_fwd(int64_t n, int cin, int cout, int kk, int dtype, double density) {
     const int rows = svtad_plan_wanted(n, cin, cout, kk, dtype, density) & SVTAD_PLAN_ROWS;
     if (!rows || n <= 5120) return 0;
-    const double saved = tc_choose(n, cin, cout, kk, false).us * (1 - 1.1 * known_density(density));
-    return saved >= 16 + (double)n / 3600 ? rows : 0;
+    const double there = known_density(density), without = tc_choose(n, cin, cout, kk, false).us;
+    if (without * (1 - 1.1 * there) < 16 + (double)n / 3600) return 0;
+    const double longest = hybrid_longest_us(n, cin, cout, kk, there);
+    return longest == 0 || 9 + (double)n / 3200 + longest < 1.06 * without ? rows : 0;
 }
 
 extern "C" int svtad_conv_fwd(const void* x, const int32_t* nbr, const void* w, const void* bias,

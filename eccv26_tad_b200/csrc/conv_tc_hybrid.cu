@@ -823,6 +823,16 @@ static int pick_planned(int cn, long m_tiles, int kk, int chunks) {
     return bn;
 }
 
+// About how long a forward by a plan takes its longest tile, which needs every tap, where that outlasts each CTA's share of all
+// tiles; 0 where it does not.
+double hybrid_longest_us(int64_t n, int cred, int cn, int kk, double density) {
+    const long m_tiles = (n + TILE_M - 1) / TILE_M;
+    const int chunks = (cred + STAGE_K - 1) / STAGE_K, bn = pick_planned(cn, m_tiles, kk, chunks);
+    const double step = bn == 256 ? 0.366 : bn == 192 ? 0.352 : bn == 128 ? 0.266 : 0.21, longest = kk * chunks * step;
+    const double taps = 1.2 * density * kk, items = (double)m_tiles * ((cn + bn - 1) / bn);
+    return items / tc_num_sms() * ((taps < 1 ? 1 : taps > kk ? kk : taps) * chunks * step + 2.4) < longest ? 1.05 * longest : 0;
+}
+
 template <bool DGRAD>
 static int dispatch_conv_hybrid(const ConvArgs& p, const int32_t* status, cudaStream_t s) {
     const int cn = DGRAD ? p.cin : p.cout;

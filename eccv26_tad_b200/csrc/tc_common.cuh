@@ -335,6 +335,7 @@ struct TcChoice {
     double us;
 };
 TcChoice tc_choose(int64_t n, int cred, int cn, int kk, bool dgrad);
+double hybrid_longest_us(int64_t n, int cred, int cn, int kk, double density);      // see conv_tc_hybrid.cu
 struct WgradPlan {
     int bn, n_nblk, n_pairs, splits, ones_block;
     long tokens_per_split;

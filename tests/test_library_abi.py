@@ -276,6 +276,14 @@ def test_a_forward_s_row_order_is_wanted_by_the_waves_it_saves(n, cin, cout, den
     assert lib.svtad_plan_wanted_fwd(n, cin, cout, 9, _lib.F32, density) == 0
 
 
+@pytest.mark.parametrize("n,cin,cout,density,wanted", [
+    (18940, 512, 192, 0.188, 0), (8960, 640, 256, 0.188, 0), (7644, 512, 384, 0.266, 0),      # the longest tile takes what the order saves
+    (8960, 640, 768, 0.188, 1), (10192, 1024, 1024, 0.509, 1), (56252, 384, 384, 0.508, 1),
+])
+def test_no_row_order_for_a_forward_whose_longest_tile_decides(n, cin, cout, density, wanted):
+    assert _lib.load().svtad_plan_wanted_fwd(n, cin, cout, 9, _lib.BF16, density) == wanted
+
+
 @pytest.mark.parametrize("cin,cout,halves,bn", [(640, 640, 1, 128), (896, 896, 1, 128), (512, 960, 2, 192), (640, 1024, 1, 256),
                                                 (512, 640, 2, 256), (320, 320, 1, 192), (1024, 1024, 2, 256)])
 def test_column_block_of_a_weight_gradient_by_pairs(cin, cout, halves, bn):
