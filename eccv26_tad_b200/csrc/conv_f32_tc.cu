@@ -986,7 +986,8 @@ static int dispatch_f32_tc(const ConvArgs& p, const int32_t* status, cudaStream_
 // Where these kernels take over from those on the CUDA cores, us there and here.  Forward and input gradient from four rows on: 1
 // row, C = 192, 3 x 3: 6.2 and 6.9; 8 rows, one neighbor in nine / five / all: 6.4 and 7.1 / 10.1 and 8.9 / 10.7 and 9.7; 96 rows, C = 512:
 // 32.2 and 13.6 at one in four, 39.5 and 14.1 at all.  (Above 64 rows a table in which hardly a row has any neighbor is the exception: 96
-// rows, C = 512, none: 10.1 and 13.8.)
+// rows, C = 512, none: 10.1 and 13.8; so are sparse tables over at most 32 channels, half of a step: 16 000 rows, 32 -> 192, density
+// 0.14: 27.5 and 34.9, 0.42: 38.9 and 35.7, 0.96: 70.5 and 36.0.)
 // The weight gradient has 7 us per CTA whatever it holds, one CTA an SM, and cuts its tokens for one pair in three tokens.  So it
 // loses where there is little to do, mostly on full tables (64 -> 64, 3 x 3, density 0.15 / 0.95: 1 100 rows 9.8 and 9.5 / 9.8 and
 // 12.9, 2 400 rows 12.4 and 11.3 / 15.1 and 14.8), and where many CTAs have few pairs each, as with wide
